@@ -9,6 +9,7 @@ ADKV_HIDDEN int adkv_tu_status_split(int *out);
 ADKV_HIDDEN int adkv_tu_status_wide(int *out);
 ADKV_HIDDEN int adkv_tu_status_half(int *out);
 ADKV_HIDDEN int adkv_tu_status_narrow(int *out);
+ADKV_HIDDEN int adkv_tu_status_segments(int *out);
 
 namespace adkv {
 
@@ -60,7 +61,7 @@ int adkv_device_status(int *status, void *stream)
     if (!status) return ADKV_E_NULL;
     const cudaError_t e = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return int(e);
-    int a = 0, b = 0, c = 0, d = 0, w = 0, t = 0, hf = 0, nr = 0;
+    int a = 0, b = 0, c = 0, d = 0, w = 0, t = 0, hf = 0, nr = 0, sg = 0;
     if (int rc = adkv_tu_status_fused(&a)) return rc;
     if (int rc = adkv_tu_status_unfused(&b)) return rc;
     if (int rc = adkv_tu_status_encode(&c)) return rc;
@@ -69,6 +70,8 @@ int adkv_device_status(int *status, void *stream)
     if (int rc = adkv_tu_status_capi(&t)) return rc;
     if (int rc = adkv_tu_status_half(&hf)) return rc;
     if (int rc = adkv_tu_status_narrow(&nr)) return rc;
+    if (int rc = adkv_tu_status_segments(&sg)) return rc;
+    if (sg) nr = sg;
     *status = a ? a : (b ? b : (c ? c : (d ? d : (w ? w : (hf ? hf : (nr ? nr : t))))));
     return 0;
 }

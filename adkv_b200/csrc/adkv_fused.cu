@@ -78,10 +78,21 @@ ADKV_HIDDEN int adkv_half_decode_attn(const KArgs &ka, const VArgs &va, const fl
                                       float scaling, int B, int bits, const int *seq_lens, cudaStream_t s);
 ADKV_HIDDEN int adkv_narrow_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b,
                                         float scaling, int B, int bits, bool exact, cudaStream_t s);
+ADKV_HIDDEN int adkv_segments_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b,
+                                          float scaling, int B, int bits, const int *seq_lens, cudaStream_t s);
 ADKV_HIDDEN int adkv_wide_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b,
                                       float scaling, int B, int bits, int mode, cudaStream_t s);
 
 ADKV_DEFINE_TU_STATUS(adkv_tu_status_fused)
+
+// Token segments of a stream side by side (adkv_segments.cu): up to this many streams per launch.
+constexpr long long kSegmentsMaxStreams = 444;
+
+static bool use_segments(const KArgs &ka, int B, bool exact, unsigned flags)
+{
+    return ka.tail && !exact && !(flags & (ADKV_FLAG_SPLIT_CHANNELS | ADKV_FLAG_NO_SPLIT_CHANNELS)) &&
+           ka.Hq / ka.Hkv <= 4 && (long long)B * ka.Hkv <= kSegmentsMaxStreams;
+}
 
 extern "C" {
 
@@ -112,6 +123,8 @@ int adkv_decode_attn(const void *q, void *k_cache, void *v_cache, const void *k_
                                      half ? 2 : int(exact), s);
     if (half)
         return adkv_half_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, nullptr, s);
+    if (use_segments(ka, B, exact, flags))
+        return adkv_segments_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, nullptr, s);
     // Very few streams: split every head over two warp pairs (adkv_narrow.cu).
     const bool split = (flags & ADKV_FLAG_SPLIT_CHANNELS) ||
                        (!(flags & ADKV_FLAG_NO_SPLIT_CHANNELS) && (long long)B * Hkv <= kSplitChannelsMaxStreams);
@@ -147,6 +160,8 @@ int adkv_decode_attn_varlen(const void *q, void *k_cache, void *v_cache, const v
     if (flags & ADKV_FLAG_HALF_STATE)
         return adkv_half_decode_attn(ka, va, nullptr, 0, scaling, B, bits, static_cast<const int *>(seq_lens), s);
     const bool exact = !(flags & ADKV_FLAG_FAST_REPLAY);
+    if (use_segments(ka, B, exact, flags))
+        return adkv_segments_decode_attn(ka, va, nullptr, 0, scaling, B, bits, static_cast<const int *>(seq_lens), s);
     ADKV_DISPATCH(bits, exact, Hq / Hkv,
                   (decode_attn_kernel<BITS, G, ARITH><<<B * Hkv, 64, 0, s>>>(ka, va, nullptr, 0, scaling,
                                                                             static_cast<const int *>(seq_lens))))

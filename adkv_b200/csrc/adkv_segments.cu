@@ -1,0 +1,434 @@
+// Part of libadkv_b200.so (sm_100a).  See include/adkv_b200.h for the contract of every entry point.
+//
+// Fused decode step for launches with few (batch, kv head) streams, next to tail states: the token axis of every stream
+// is cut into kSegPairs segments that run side by side in ONE CTA, a K and a V warp each.  Reached through
+// adkv_decode_attn and adkv_decode_attn_varlen.
+//
+// What bounds a step with few streams is one warp's dependent instruction stream: a K/V pair walks its stream at about
+// 100 cycles a token whatever the rest of the SM does, and splitting the channels of a head over more warps repeats the
+// per-token overhead in each.  The token axis looks serial, but the scale recurrence s' = clamp(s * (tc + beta*|q|)) is a
+// running product of factors that depend on the codes alone, and the zero point a running sum, so:
+//
+//  1. every warp forms the product F of the factors of its segment and the extremes of its running product (half the
+//     arithmetic of a scan, no clamps);
+//  2. the states at the segment starts follow from the products of the segments before.  A segment whose product,
+//     from the state it really starts with, cannot have met a clamp (nearly always: the extremes, widened by the
+//     worst case of four tokens, stay inside the bounds) contributes F; any other is replayed with clamps, the warps of
+//     the CTA taking turns, so a cache that clamps everywhere costs at most one scale-only scan more;
+//  3. the scans run with zero points relative to the segment start.  For K that shifts every logit of a segment by one
+//     number, sum_c q_c * zp_c(start), for V it leaves out (sum of weights) * zp(start): both are put back
+//  4. when the partial softmax results of the segments are merged in shared memory.
+//
+// Only the appended token needs the encoder's exact state, and that comes from the tail.
+// @MEASURED@
+#include "adkv_host.h"
+
+#include "adkv_softmax.cuh"
+
+namespace adkv {
+
+constexpr int kSegPairs = 8;      // segments per stream; 16 warps keep the four schedulers of an SM busy
+constexpr int kSegStages = 2;     // bulk-copy ring depth per warp
+constexpr int kPartFloats = 4 + kD;   // per (segment, head): maximum (log2 units), denominator, 2 pad, kD sums
+
+template <int BITS, int G>
+struct SegShared {
+    alignas(128) uint8_t buf[2][kSegPairs][kSegStages * Tile<BITS>::BYTES];
+    alignas(16) float red[kSegPairs][G * 8 * 36];
+    alignas(16) float2 wts[kSegPairs][G * kTileTok];
+    union {
+        alignas(16) float comp[2][kSegPairs][3][kD];     // steps 1 and 2: product, smallest and largest running product
+        alignas(16) float part[kSegPairs][G][kPartFloats];   // steps 3 and 4
+    };
+    alignas(16) float init[2][kSegPairs][2][kD];         // zero point (relative) and scale at the segment starts
+    alignas(16) float zp_end[kSegPairs][kD];             // V: zero points after the segment, relative to its start
+    alignas(16) float self_x[kD];                        // V: dequantised appended token
+    float z_end[kSegPairs][G];                           // K: sum_c q_c * zp_c after the segment, relative
+    float self_logit[G];
+    FusedShared<G> fs[kSegPairs];
+    uint64_t bar[2][kSegPairs][kSegStages];
+};
+
+template <int G>
+struct SegSink : RingSink<G> {
+    float *z_end;
+    bool done;
+    __device__ __forceinline__ void end_state(const Chan (&ch)[4], const float (&qv)[G][4], int lane)
+    {
+        done = true;
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            float z = 0.f;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) z = fmaf(qv[g][c], ch[c].zp, z);
+            z = warp_sum(z);
+            if (lane == 0) z_end[g] = z;
+        }
+    }
+};
+
+template <int G>
+struct SegSrc : SoftmaxSrc<G> {
+    float *part;       // [G][kPartFloats] of this segment
+    float *zp_end;
+    bool done;
+    __device__ __forceinline__ void end_state(const Chan (&ch)[4], int c0)
+    {
+        done = true;
+        *reinterpret_cast<float4 *>(zp_end + c0) = make_float4(ch[0].zp, ch[1].zp, ch[2].zp, ch[3].zp);
+    }
+    __device__ __forceinline__ void put(int c0, int g, float m, float l, float4 acc) const
+    {
+        if (c0 == 0) {
+            part[g * kPartFloats] = m;
+            part[g * kPartFloats + 1] = l;
+        }
+        *reinterpret_cast<float4 *>(part + g * kPartFloats + 4 + c0) = acc;
+    }
+    __device__ __forceinline__ void store(const VArgs &, int, int, int c0, const float (&acc)[G][4]) const
+    {
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+            put(c0, g, this->m[g], this->l[g], make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]));
+    }
+    // a bounded wait gave up: the merged output of these heads becomes NaN
+    __device__ __forceinline__ void give_up(int c0) const
+    {
+#pragma unroll
+        for (int g = 0; g < G; ++g) put(c0, g, -INFINITY, __int_as_float(0x7fc00000), make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+};
+
+// Scales of four channels and what advances them (contracted constants: ch[].tc = 1 - beta * target).
+struct ScaleConst {
+    f32x2 beta[2], tc[2];
+};
+
+// Step 1: product of the factors of `n_words` words of a stream and the extremes of the running product at every
+// fourth token (1 at the start included).  src: this lane's vector of the first word.
+template <int BITS>
+__device__ __forceinline__ void scale_product(const uint4 *src, int n_words, const ScaleConst &sc, float (&F)[4],
+                                              float (&mn)[4], float (&mx)[4])
+{
+    constexpr int kAhead = 4;
+    FieldConsts<BITS> fc;
+    fc.init();
+    f32x2 f2[2] = {pk2(1.f, 1.f), pk2(1.f, 1.f)};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) mn[c] = mx[c] = 1.f;
+    uint4 w[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) w[i] = src[min(i, n_words - 1) * (kD / 4)];
+#pragma unroll 1
+    for (int wd = 0; wd < n_words; wd += kAhead) {
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+            uint32_t grp[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+            w[i] = src[min(wd + kAhead + i, n_words - 1) * (kD / 4)];
+            if (wd + i < n_words) {
+#pragma unroll 1
+                for (int blk = 0; blk < Codec<BITS>::TPW / 4; ++blk) {
+                    static_for<4>([&](auto kc) {
+                        constexpr int k = decltype(kc)::value;
+#pragma unroll
+                        for (int p = 0; p < 2; ++p) {
+                            const f32x2 q2 = fc.template code2<k>(grp[2 * p], grp[2 * p + 1]);
+                            f2[p] = mul2(f2[p], fma2(sc.beta[p], abs2(q2), sc.tc[p]));
+                        }
+                    });
+                    upk2(f2[0], F[0], F[1]);
+                    upk2(f2[1], F[2], F[3]);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        mn[c] = fminf(mn[c], F[c]);
+                        mx[c] = fmaxf(mx[c], F[c]);
+                        grp[c] >>= 4 * BITS;
+                    }
+                }
+            }
+        }
+    }
+    upk2(f2[0], F[0], F[1]);
+    upk2(f2[1], F[2], F[3]);
+}
+
+// Step 2, the segments that may have met a clamp: the scales alone, with clamps where they can act.
+template <int BITS>
+__device__ __noinline__ float4 scale_replay(const uint4 *src, int n_words, float4 s4, ScaleConst sc, SafeRange safe, float smin,
+                                            float smax)
+{
+    FieldConsts<BITS> fc;
+    fc.init();
+    Chan ch[4];
+    ch[0].s = s4.x; ch[1].s = s4.y; ch[2].s = s4.z; ch[3].s = s4.w;
+    float be[4], tc[4];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        upk2(sc.beta[p], be[2 * p], be[2 * p + 1]);
+        upk2(sc.tc[p], tc[2 * p], tc[2 * p + 1]);
+    }
+#pragma unroll 1
+    for (int wd = 0; wd < n_words; ++wd) {
+        const uint4 w = src[wd * (kD / 4)];
+        uint32_t grp[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll 1
+        for (int c8 = 0; c8 < Codec<BITS>::TPW / 8; ++c8) {
+            const bool free = safe.holds(ch);
+#pragma unroll 1
+            for (int half = 0; half < 2; ++half) {
+                static_for<4>([&](auto kc) {
+                    constexpr int k = decltype(kc)::value;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float s = ch[c].s * fmaf(be[c], fabsf(fc.template code<k>(grp[c])), tc[c]);
+                        ch[c].s = free ? s : fminf(fmaxf(s, smin), smax);
+                    }
+                });
+#pragma unroll
+                for (int c = 0; c < 4; ++c) grp[c] >>= 4 * BITS;
+            }
+        }
+    }
+    return make_float4(ch[0].s, ch[1].s, ch[2].s, ch[3].s);
+}
+
+template <int BITS, int G>
+__global__ void __launch_bounds__(64 * kSegPairs, 1)
+    decode_attn_segments_kernel(KArgs ka, VArgs va, const float *__restrict__ mask, long long mask_stride_b, float scaling,
+                                const int *__restrict__ seq_lens)
+{
+    extern __shared__ uint8_t smem_raw[];
+    SegShared<BITS, G> &sh = *reinterpret_cast<SegShared<BITS, G> *>(smem_raw);
+    using C = Codec<BITS>;
+    const int bh = blockIdx.x, b = bh / ka.Hkv, h = bh % ka.Hkv;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // Warps go to the four schedulers round robin: a pair of warps is the K and the V warp of one segment, and the order
+    // flips with every other pair so that each scheduler holds as many K as V warps.
+    const int seg = warp >> 1, role = (warp ^ (warp >> 2)) & 1;
+    if (seq_lens) {   // as in decode_attn_kernel
+        const int T = seq_lens[b];
+        if (T < 0 || T / C::TPW >= ka.n_super_cap) {
+            if (threadIdx.x == 0) atomicExch(&g_status, kStatCapacity);
+            return;
+        }
+        ka.T = T;
+        va.T = T;
+    }
+    if (threadIdx.x < kSegPairs) {
+        for (int r = 0; r < 2; ++r)
+            for (int i = 0; i < kSegStages; ++i) mbar_init(&sh.bar[r][threadIdx.x][i], 1);
+        sh.fs[threadIdx.x].init_barriers(1);
+        for (int g = 0; g < G; ++g) sh.z_end[threadIdx.x][g] = 0.f;
+        mbar_init_fence();
+    }
+    const int T = ka.T, n_tiles = (T + kTileTok - 1) / kTileTok;
+    const int per_seg = (n_tiles + kSegPairs - 1) / kSegPairs * kTileTok;
+    const int t_begin = min(seg * per_seg, T), t_end = min(t_begin + per_seg, T);
+    const ParamPtrs &p = role ? va.p : ka.p;
+    const int c0 = 4 * lane;
+    const size_t poff = size_t(h) * kD + c0;
+    const uint4 *words = reinterpret_cast<const uint4 *>((role ? va.cache : ka.cache) +
+                                                         (size_t(bh) * ka.n_super_cap + t_begin / C::TPW) * kD * 4) + lane;
+
+    // 1. products of all segments that another one follows (those are whole tiles)
+    ScaleConst sc;
+    SafeRange safe8, safe4;
+    float s[4];
+    const bool followed = t_end < T;
+    {
+        Chan ch[4];
+        load_chan4<BITS, true>(ch, safe8, p, poff, ka.smin, ka.smax);
+        float be[4], tg[4], tc[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            be[c] = ch[c].beta;
+            tg[c] = ch[c].tc;
+            tc[c] = fmaf(-be[c], tg[c], 1.0f);
+            s[c] = ch[c].s;
+        }
+        safe4.template init<BITS, 4, 4>(be, tg, ka.smin, ka.smax);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            sc.beta[q] = pk2(be[2 * q], be[2 * q + 1]);
+            sc.tc[q] = pk2(tc[2 * q], tc[2 * q + 1]);
+        }
+    }
+    if (followed) {
+        float F[4], mn[4], mx[4];
+        scale_product<BITS>(words, per_seg / C::TPW, sc, F, mn, mx);
+        *reinterpret_cast<float4 *>(&sh.comp[role][seg][0][c0]) = make_float4(F[0], F[1], F[2], F[3]);
+        *reinterpret_cast<float4 *>(&sh.comp[role][seg][1][c0]) = make_float4(mn[0], mn[1], mn[2], mn[3]);
+        *reinterpret_cast<float4 *>(&sh.comp[role][seg][2][c0]) = make_float4(mx[0], mx[1], mx[2], mx[3]);
+    }
+    __syncthreads();
+
+    // 2. scale at the start of this warp's segment
+    // Advances x over segment i if that provably meets no clamp in any channel of the warp.
+    const auto advance = [&](int i, float (&x)[4]) {
+        const float4 F = *reinterpret_cast<const float4 *>(&sh.comp[role][i][0][c0]);
+        const float4 mn = *reinterpret_cast<const float4 *>(&sh.comp[role][i][1][c0]);
+        const float4 mx = *reinterpret_cast<const float4 *>(&sh.comp[role][i][2][c0]);
+        const float Fv[4] = {F.x, F.y, F.z, F.w}, mnv[4] = {mn.x, mn.y, mn.z, mn.w}, mxv[4] = {mx.x, mx.y, mx.z, mx.w};
+        bool ok = true;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) ok = ok && x[c] * mnv[c] >= safe4.lo && x[c] * mxv[c] <= safe4.hi;
+        ok = __all_sync(kFull, ok);
+        if (ok) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) x[c] *= Fv[c];
+        }
+        return ok;
+    };
+    bool proven = true;
+    const bool empty = seg > 0 && t_begin >= T;
+    if (!empty)
+        for (int i = 0; i < seg && proven; ++i) proven = advance(i, s);
+    if (__syncthreads_or(!proven)) {
+        // Some segment may clamp: the segments of a tensor advance the state one after another.
+        const bool first = seg == 0;
+        if (first) {
+            Chan ch[4];
+            SafeRange unused;
+            load_chan4<BITS, true>(ch, unused, p, poff, ka.smin, ka.smax);
+            *reinterpret_cast<float4 *>(&sh.init[role][0][1][c0]) = make_float4(ch[0].s, ch[1].s, ch[2].s, ch[3].s);
+        }
+        for (int i = 0; i + 1 < kSegPairs; ++i) {
+            if (seg == i && followed) {
+                const float4 x4 = *reinterpret_cast<const float4 *>(&sh.init[role][i][1][c0]);
+                float x[4] = {x4.x, x4.y, x4.z, x4.w};
+                float4 y;
+                if (advance(i, x)) y = make_float4(x[0], x[1], x[2], x[3]);
+                else y = scale_replay<BITS>(words, per_seg / C::TPW, x4, sc, safe8, ka.smin, ka.smax);
+                *reinterpret_cast<float4 *>(&sh.init[role][i + 1][1][c0]) = y;
+            }
+            __syncthreads();
+        }
+        if (!empty) {
+            const float4 x4 = *reinterpret_cast<const float4 *>(&sh.init[role][seg][1][c0]);
+            s[0] = x4.x; s[1] = x4.y; s[2] = x4.z; s[3] = x4.w;
+        }
+        __syncthreads();
+    }
+
+    // 3. the scans; a lane reads back only the state that it wrote itself
+    *reinterpret_cast<float4 *>(&sh.init[role][seg][0][c0]) = make_float4(0.f, 0.f, 0.f, 0.f);
+    *reinterpret_cast<float4 *>(&sh.init[role][seg][1][c0]) = make_float4(s[0], s[1], s[2], s[3]);
+    const Seg sg{t_begin, t_end, false, seg ? &sh.init[role][seg][0][0] : nullptr, nullptr, 0};
+    const float *mask_row = mask ? mask + size_t(b) * mask_stride_b : nullptr;
+    const float scale2 = scaling * 1.4426950408889634f;
+    const auto append = [&](const ParamPtrs &pp, float *tail, bool keep, const __half *x_new, uint8_t *cache, float (&xh)[4]) {
+        Chan ch[4];
+        SafeRange unused;
+        load_chan4<BITS, true>(ch, unused, pp, poff, ka.smin, ka.smax);
+        append_new_token<BITS, kArithCanon>(
+            ch, pp, poff, tail + size_t(bh) * 2 * kD, keep, x_new + size_t(bh) * kD + c0,
+            reinterpret_cast<uint4 *>(cache + (size_t(bh) * ka.n_super_cap + T / C::TPW) * kD * 4) + lane, T, ka.smin, ka.smax,
+            nullptr, c0, kD, xh);
+    };
+    // The appended token goes into the word behind the last cached one: only the warps that read that word may write it.
+    const bool last = t_end == T && (seg == 0 || t_begin < T);
+    if (role == 0) {
+        SegSink<G> sink;
+        sink.sh = &sh.fs[seg];
+        sink.slot = 0;
+        sink.sl = 0;
+        sink.z_end = sh.z_end[seg];
+        sink.done = false;
+        k_warp<BITS, G, kArithFma, SegSink<G>, kSegStages>(ka, sg, b, h, lane, sh.buf[0][seg], sh.bar[0][seg], sh.red[seg], sink);
+        if (last && sink.done) {
+            float xh[4];
+            append(ka.p, ka.tail, ka.tail_keep, ka.x_new, ka.cache, xh);
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                float qv[4], x = 0.f;
+                load_half4(qv, ka.q + (size_t(b) * ka.Hq + size_t(h) * G + g) * kD + c0);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) x = fmaf(qv[c], xh[c], x);
+                x = warp_sum(x);
+                if (lane == 0) sh.self_logit[g] = x;
+            }
+        }
+    } else {
+        SegSrc<G> src;
+        src.sh = &sh.fs[seg];
+        src.wts = sh.wts[seg];
+        src.mask = mask_row;
+        src.scale2 = scale2;
+        src.n_tiles = (t_end - t_begin + kTileTok - 1) / kTileTok;
+        src.t_begin = t_begin;
+        src.part = &sh.part[seg][0][0];
+        src.zp_end = sh.zp_end[seg];
+        src.done = false;
+        src.init();
+        v_warp<BITS, G, kArithFma, SegSrc<G>, kSegStages>(va, sg, b, h, lane, sh.buf[1][seg], sh.bar[1][seg], sh.wts[seg], src);
+        if (last && src.done) {
+            float xh[4];
+            append(va.p, va.tail, va.tail_keep, va.x_new, va.cache, xh);
+            *reinterpret_cast<float4 *>(&sh.self_x[c0]) = make_float4(xh[0], xh[1], xh[2], xh[3]);
+        }
+    }
+    __syncthreads();
+
+    // 4. merge: segment maxima shifted by the zero points K left out, sums completed with those V left out
+    const float mk = mask_row ? mask_row[T] * 1.4426950408889634f : 0.f;
+    for (int i = threadIdx.x; i < G * kD; i += 64 * kSegPairs) {
+        const int g = i / kD, c = i % kD;
+        float m[kSegPairs], z = 0.f;
+        const float v = fmaf(sh.self_logit[g], scale2, mk);
+        float M = v;
+#pragma unroll
+        for (int j = 0; j < kSegPairs; ++j) {
+            m[j] = sh.part[j][g][0];
+            if (m[j] != -INFINITY) m[j] = fmaf(z, scale2, m[j]);
+            z += sh.z_end[j][g];
+            M = fmaxf(M, m[j]);
+        }
+        const bool dead = M == -INFINITY;
+        const float w_self = dead ? 0.f : exp2f(v - M);
+        float L = w_self, A = w_self * sh.self_x[c], zp = 0.f;
+#pragma unroll
+        for (int j = 0; j < kSegPairs; ++j) {
+            const float w = m[j] == -INFINITY ? 0.f : exp2f(m[j] - M);
+            const float l = sh.part[j][g][1];
+            L = fmaf(l, w, L);
+            A = fmaf(fmaf(l, zp, sh.part[j][g][4 + c]), w, A);
+            zp += sh.zp_end[j][c];
+        }
+        va.out[(size_t(b) * ka.Hq + size_t(h) * G + g) * kD + c] = __float2half_rn(A / L);
+    }
+}
+
+}  // namespace adkv
+
+using namespace adkv;
+
+ADKV_DEFINE_TU_STATUS(adkv_tu_status_segments)
+
+template <int BITS, int G>
+static int launch_segments(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b, float scaling, int B,
+                           const int *seq_lens, cudaStream_t s)
+{
+    constexpr int bytes = int(sizeof(SegShared<BITS, G>));
+    static_assert(bytes <= 227 * 1024, "shared memory of one CTA");
+    // per device and process: cheap enough (a host-side call) to be made before every launch
+    const cudaError_t e = cudaFuncSetAttribute(decode_attn_segments_kernel<BITS, G>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return int(e);
+    decode_attn_segments_kernel<BITS, G><<<B * ka.Hkv, 64 * kSegPairs, bytes, s>>>(ka, va, mask, mask_stride_b, scaling, seq_lens);
+    return launch_status();
+}
+
+// Arguments checked by the caller (head dim 128, fp32 arithmetic, contracted, tail states present, Hq / Hkv at most 4).
+ADKV_HIDDEN int adkv_segments_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b,
+                                          float scaling, int B, int bits, const int *seq_lens, cudaStream_t s)
+{
+    switch (bits * 16 + ka.Hq / ka.Hkv) {
+    case 4 * 16 + 1: return launch_segments<4, 1>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
+    case 4 * 16 + 2: return launch_segments<4, 2>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
+    case 4 * 16 + 4: return launch_segments<4, 4>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
+    case 2 * 16 + 1: return launch_segments<2, 1>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
+    case 2 * 16 + 2: return launch_segments<2, 2>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
+    case 2 * 16 + 4: return launch_segments<2, 4>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
+    default: return ADKV_E_SHAPE;
+    }
+}
