@@ -411,6 +411,16 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
     return ok;
 }
 
+// The same with the polling out of line: a scan that waits twice per tile keeps a test and a vote in its loop.
+static __device__ __noinline__ bool mbar_wait_slow(uint64_t *bar, uint32_t parity, int code)
+{
+    return mbar_wait_bounded(bar, parity, code);
+}
+__device__ __forceinline__ bool mbar_wait_short(uint64_t *bar, uint32_t parity, int code)
+{
+    return __all_sync(kFull, mbar_try_wait(bar, parity)) || mbar_wait_slow(bar, parity, code);
+}
+
 // Global -> shared bulk copy completing on an mbarrier.  dst, src 16-byte aligned, bytes % 16 == 0.
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
 {

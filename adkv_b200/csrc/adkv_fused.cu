@@ -2,7 +2,7 @@
 // and the reference interface each one replaces.
 #include "adkv_host.h"
 
-#include "adkv_softmax.cuh"
+#include "adkv_tailscan.cuh"
 
 namespace adkv {
 
@@ -64,6 +64,56 @@ __global__ void __launch_bounds__(64) decode_attn_kernel(KArgs ka, VArgs va, con
     }
 }
 
+// The same step next to tail states in the contracted arithmetic (adkv_tailscan.cuh).
+template <int BITS, int G>
+__global__ void __launch_bounds__(64, 1) decode_attn_tail_kernel(KArgs ka, VArgs va, const float *__restrict__ mask,
+                                                                 long long mask_stride_b, float scaling,
+                                                                 const int *__restrict__ seq_lens)
+{
+    using Softmax = TailSoftmax<G, G == 1>;
+    __shared__ alignas(128) uint8_t kbuf[kTailStages * Tile<BITS>::BYTES];
+    __shared__ alignas(128) uint8_t vbuf[kTailStages * Tile<BITS>::BYTES];
+    __shared__ alignas(16) float red[kRedFloats];
+    __shared__ alignas(16) float4 wts[Softmax::kFloat4];
+    __shared__ alignas(16) float4 slow[2][2 * 32];
+    __shared__ FusedShared<G> fs;
+    __shared__ uint64_t kbar[kTailStages], vbar[kTailStages];
+
+    const int bh = blockIdx.x, b = bh / ka.Hkv, h = bh % ka.Hkv;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (seq_lens) {   // as in decode_attn_kernel
+        const int T = seq_lens[b];
+        if (T < 0 || T / Codec<BITS>::TPW >= ka.n_super_cap) {
+            if (threadIdx.x == 0) atomicExch(&g_status, kStatCapacity);
+            return;
+        }
+        ka.T = T;
+        va.T = T;
+    }
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kTailStages; ++i) { mbar_init(&kbar[i], 1); mbar_init(&vbar[i], 1); }
+        fs.init_barriers(1);
+        mbar_init_fence();
+    }
+    __syncthreads();
+    Seg seg{0, ka.T, true, nullptr, nullptr, 0};
+    if (warp == 0) {
+        RingSink<G> sink{&fs, 0, 0};
+        k_tail_warp<BITS, G, kTailStages>(ka, seg, b, h, lane, kbuf, kbar, red, slow[0], sink);
+    } else {
+        Softmax src;
+        src.sh = &fs;
+        src.wts = wts;
+        src.mask = mask ? mask + size_t(b) * mask_stride_b : nullptr;
+        src.scale2 = scaling * 1.4426950408889634f;
+        src.t_begin = 0;
+        src.init();
+        seg.zp_end = va.tail + size_t(bh) * 2 * kD;
+        v_tail_warp<BITS, G, G == 1, kTailStages>(va, seg, b, h, lane, vbuf, vbar, slow[1], src,
+                                                  TailStore<G>{va.out + size_t(bh) * G * kD});
+    }
+}
+
 }  // namespace adkv
 
 using namespace adkv;
@@ -92,6 +142,30 @@ static bool use_segments(const KArgs &ka, int B, bool exact, unsigned flags)
 {
     return ka.tail && !exact && !(flags & (ADKV_FLAG_SPLIT_CHANNELS | ADKV_FLAG_NO_SPLIT_CHANNELS)) &&
            ka.Hq / ka.Hkv <= 4 && (long long)B * ka.Hkv <= kSegmentsMaxStreams;
+}
+
+// One CTA per stream.  With tail states and the contracted arithmetic the scans of adkv_tailscan.cuh run, for one, two
+// and four query heads per KV head; with eight their constants and partial sums would not stay in registers.
+static int launch_decode(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b, float scaling, int B,
+                         int bits, bool exact, const int *seq_lens, cudaStream_t s)
+{
+    const int group = ka.Hq / ka.Hkv;
+    if (ka.tail && !exact && group <= 4) {
+        switch (bits * 16 + group) {
+#define ADKV_TAIL_CASE(BITS_, G_)                                                                                     \
+    case BITS_ * 16 + G_:                                                                                             \
+        decode_attn_tail_kernel<BITS_, G_><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling, seq_lens); \
+        return launch_status();
+            ADKV_TAIL_CASE(4, 1) ADKV_TAIL_CASE(4, 2) ADKV_TAIL_CASE(4, 4)
+            ADKV_TAIL_CASE(2, 1) ADKV_TAIL_CASE(2, 2) ADKV_TAIL_CASE(2, 4)
+#undef ADKV_TAIL_CASE
+        default: return ADKV_E_SHAPE;
+        }
+    }
+    ADKV_DISPATCH(bits, exact, group,
+                  (decode_attn_kernel<BITS, G, ARITH><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling,
+                                                                               seq_lens)))
+    return launch_status();
 }
 
 extern "C" {
@@ -130,10 +204,7 @@ int adkv_decode_attn(const void *q, void *k_cache, void *v_cache, const void *k_
                        (!(flags & ADKV_FLAG_NO_SPLIT_CHANNELS) && (long long)B * Hkv <= kSplitChannelsMaxStreams);
     if (split)
         return adkv_narrow_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, exact, s);
-    ADKV_DISPATCH(bits, exact, Hq / Hkv,
-                  (decode_attn_kernel<BITS, G, ARITH><<<B * Hkv, 64, 0, s>>>(
-                      ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, nullptr)))
-    return launch_status();
+    return launch_decode(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, exact, nullptr, s);
 }
 
 int adkv_decode_attn_varlen(const void *q, void *k_cache, void *v_cache, const void *k_new, const void *v_new,
@@ -162,10 +233,7 @@ int adkv_decode_attn_varlen(const void *q, void *k_cache, void *v_cache, const v
     const bool exact = !(flags & ADKV_FLAG_FAST_REPLAY);
     if (use_segments(ka, B, exact, flags))
         return adkv_segments_decode_attn(ka, va, nullptr, 0, scaling, B, bits, static_cast<const int *>(seq_lens), s);
-    ADKV_DISPATCH(bits, exact, Hq / Hkv,
-                  (decode_attn_kernel<BITS, G, ARITH><<<B * Hkv, 64, 0, s>>>(ka, va, nullptr, 0, scaling,
-                                                                            static_cast<const int *>(seq_lens))))
-    return launch_status();
+    return launch_decode(ka, va, nullptr, 0, scaling, B, bits, exact, static_cast<const int *>(seq_lens), s);
 }
 
 }  // extern "C"

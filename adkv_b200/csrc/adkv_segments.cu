@@ -23,7 +23,7 @@
 // @MEASURED@
 #include "adkv_host.h"
 
-#include "adkv_softmax.cuh"
+#include "adkv_tailscan.cuh"
 
 namespace adkv {
 
@@ -34,8 +34,9 @@ constexpr int kPartFloats = 4 + kD;   // per (segment, head): maximum (log2 unit
 template <int BITS, int G>
 struct SegShared {
     alignas(128) uint8_t buf[2][kSegPairs][kSegStages * Tile<BITS>::BYTES];
-    alignas(16) float red[kSegPairs][G * 8 * 36];
-    alignas(16) float2 wts[kSegPairs][G * kTileTok];
+    alignas(16) float red[kSegPairs][kRedFloats];
+    alignas(16) float4 wts[kSegPairs][TailSoftmax<G, false>::kFloat4];
+    alignas(16) float4 slow[2][kSegPairs][2 * 32];
     union {
         alignas(16) float comp[2][kSegPairs][3][kD];     // steps 1 and 2: product, smallest and largest running product
         alignas(16) float part[kSegPairs][G][kPartFloats];   // steps 3 and 4
@@ -53,29 +54,26 @@ template <int G>
 struct SegSink : RingSink<G> {
     float *z_end;
     bool done;
-    __device__ __forceinline__ void end_state(const Chan (&ch)[4], const float (&qv)[G][4], int lane)
+    __device__ __forceinline__ void end_shares(const float (&share)[G], int lane)
     {
         done = true;
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-            float z = 0.f;
-#pragma unroll
-            for (int c = 0; c < 4; ++c) z = fmaf(qv[g][c], ch[c].zp, z);
-            z = warp_sum(z);
+            const float z = warp_sum(share[g]);
             if (lane == 0) z_end[g] = z;
         }
     }
 };
 
 template <int G>
-struct SegSrc : SoftmaxSrc<G> {
+struct SegStore {
     float *part;       // [G][kPartFloats] of this segment
     float *zp_end;
     bool done;
-    __device__ __forceinline__ void end_state(const Chan (&ch)[4], int c0)
+    __device__ __forceinline__ void end_zp(const f32x2 (&zp)[2], int c0)
     {
         done = true;
-        *reinterpret_cast<float4 *>(zp_end + c0) = make_float4(ch[0].zp, ch[1].zp, ch[2].zp, ch[3].zp);
+        *reinterpret_cast<ulonglong2 *>(zp_end + c0) = make_ulonglong2(zp[0], zp[1]);
     }
     __device__ __forceinline__ void put(int c0, int g, float m, float l, float4 acc) const
     {
@@ -85,11 +83,11 @@ struct SegSrc : SoftmaxSrc<G> {
         }
         *reinterpret_cast<float4 *>(part + g * kPartFloats + 4 + c0) = acc;
     }
-    __device__ __forceinline__ void store(const VArgs &, int, int, int c0, const float (&acc)[G][4]) const
+    __device__ __forceinline__ void store(const float (&m)[G], const float (&l)[G], const float (&acc)[G][4], int c0) const
     {
 #pragma unroll
         for (int g = 0; g < G; ++g)
-            put(c0, g, this->m[g], this->l[g], make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]));
+            put(c0, g, m[g], l[g], make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]));
     }
     // a bounded wait gave up: the merged output of these heads becomes NaN
     __device__ __forceinline__ void give_up(int c0) const
@@ -317,13 +315,9 @@ __global__ void __launch_bounds__(64 * kSegPairs, 1)
     const float *mask_row = mask ? mask + size_t(b) * mask_stride_b : nullptr;
     const float scale2 = scaling * 1.4426950408889634f;
     const auto append = [&](const ParamPtrs &pp, float *tail, bool keep, const __half *x_new, uint8_t *cache, float (&xh)[4]) {
-        Chan ch[4];
-        SafeRange unused;
-        load_chan4<BITS, true>(ch, unused, pp, poff, ka.smin, ka.smax);
-        append_new_token<BITS, kArithCanon>(
-            ch, pp, poff, tail + size_t(bh) * 2 * kD, keep, x_new + size_t(bh) * kD + c0,
-            reinterpret_cast<uint4 *>(cache + (size_t(bh) * ka.n_super_cap + T / C::TPW) * kD * 4) + lane, T, ka.smin, ka.smax,
-            nullptr, c0, kD, xh);
+        append_from_tail<BITS>(pp, poff, tail + size_t(bh) * 2 * kD, keep, x_new + size_t(bh) * kD + c0,
+                               reinterpret_cast<uint4 *>(cache + (size_t(bh) * ka.n_super_cap + T / C::TPW) * kD * 4) + lane,
+                               T, ka.smin, ka.smax, nullptr, c0, xh);
     };
     // The appended token goes into the word behind the last cached one: only the warps that read that word may write it.
     const bool last = t_end == T && (seg == 0 || t_begin < T);
@@ -334,7 +328,7 @@ __global__ void __launch_bounds__(64 * kSegPairs, 1)
         sink.sl = 0;
         sink.z_end = sh.z_end[seg];
         sink.done = false;
-        k_warp<BITS, G, kArithFma, SegSink<G>, kSegStages>(ka, sg, b, h, lane, sh.buf[0][seg], sh.bar[0][seg], sh.red[seg], sink);
+        k_tail_warp<BITS, G, kSegStages>(ka, sg, b, h, lane, sh.buf[0][seg], sh.bar[0][seg], sh.red[seg], sh.slow[0][seg], sink);
         if (last && sink.done) {
             float xh[4];
             append(ka.p, ka.tail, ka.tail_keep, ka.x_new, ka.cache, xh);
@@ -349,19 +343,16 @@ __global__ void __launch_bounds__(64 * kSegPairs, 1)
             }
         }
     } else {
-        SegSrc<G> src;
+        TailSoftmax<G, false> src;
         src.sh = &sh.fs[seg];
         src.wts = sh.wts[seg];
         src.mask = mask_row;
         src.scale2 = scale2;
-        src.n_tiles = (t_end - t_begin + kTileTok - 1) / kTileTok;
         src.t_begin = t_begin;
-        src.part = &sh.part[seg][0][0];
-        src.zp_end = sh.zp_end[seg];
-        src.done = false;
         src.init();
-        v_warp<BITS, G, kArithFma, SegSrc<G>, kSegStages>(va, sg, b, h, lane, sh.buf[1][seg], sh.bar[1][seg], sh.wts[seg], src);
-        if (last && src.done) {
+        SegStore<G> store{&sh.part[seg][0][0], sh.zp_end[seg], false};
+        v_tail_warp<BITS, G, false, kSegStages>(va, sg, b, h, lane, sh.buf[1][seg], sh.bar[1][seg], sh.slow[1][seg], src, store);
+        if (last && store.done) {
             float xh[4];
             append(va.p, va.tail, va.tail_keep, va.x_new, va.cache, xh);
             *reinterpret_cast<float4 *>(&sh.self_x[c0]) = make_float4(xh[0], xh[1], xh[2], xh[3]);
