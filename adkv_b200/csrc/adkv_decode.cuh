@@ -208,7 +208,6 @@ struct Seg {
     const float *init;    // state before token t_begin of this stream, [2][head_dim] (zp, scale); nullptr = parameters
     float *ckpt_out;      // where to store the state after the appended token, [2][head_dim]; nullptr = nowhere
     int slice;            // which 128-channel slice of the head this warp owns (0 for head_dim 128)
-    const float *zp_end = nullptr;   // whole-stream V scan next to a tail: zero points after token t_end - 1, [head_dim]
 };
 
 __device__ __forceinline__ void load_init_state(Chan (&ch)[4], const float *init, int c0, int D)
@@ -308,6 +307,18 @@ __device__ __noinline__ Chan4 k_chunk_guarded(uint4 w, Chan4 st, QueryRegs<G> q,
     k_chunk<BITS, G, EXACT, true, true>(w, fc, st.c, q.v, red, lane, count, smin, smax);
     return st;
 }
+
+// A sink or source may want the state a scan without append ended in (end_state is optional): the segment kernel does.
+template <class S, int G>
+__device__ __forceinline__ auto sink_end_state(S &s, const Chan (&ch)[4], const float (&qv)[G][4], int lane, int)
+    -> decltype(s.end_state(ch, qv, lane), void()) { s.end_state(ch, qv, lane); }
+template <class S, int G>
+__device__ __forceinline__ void sink_end_state(S &, const Chan (&)[4], const float (&)[G][4], int, long) {}
+template <class S>
+__device__ __forceinline__ auto src_end_state(S &s, const Chan (&ch)[4], int c0, int)
+    -> decltype(s.end_state(ch, c0), void()) { s.end_state(ch, c0); }
+template <class S>
+__device__ __forceinline__ void src_end_state(S &, const Chan (&)[4], int, long) {}
 
 // Sink interface (duck-typed):
 //   bool begin_tile(int i)            wait for room; false = bounded wait gave up
@@ -420,7 +431,10 @@ __device__ __forceinline__ void k_warp(const KArgs &a, const Seg &seg, int b, in
         return;
     }
 
-    if (!seg.append) return;
+    if (!seg.append) {
+        sink_end_state(sink, ch, qv, lane, 0);
+        return;
+    }
     // Append k_new as token T with the state after token T-1, then its own logit from the
     // dequantised value.
     float xh[4];
@@ -677,6 +691,8 @@ __device__ __forceinline__ void v_warp(const VArgs &a, const Seg &seg, int b, in
         for (int g = 0; g < G; ++g)
 #pragma unroll
             for (int c = 0; c < 4; ++c) acc[g][c] = fmaf(w_self[g], xh[c], acc[g][c]);
+    } else {
+        src_end_state(src, ch, c0, 0);
     }
     src.store(a, b, h, c0, acc);
 }

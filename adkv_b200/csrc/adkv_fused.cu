@@ -64,19 +64,18 @@ __global__ void __launch_bounds__(64) decode_attn_kernel(KArgs ka, VArgs va, con
     }
 }
 
-// The same step next to tail states in the contracted arithmetic (adkv_tailscan.cuh).
-template <int BITS, int G>
+// The same step next to tail states in the contracted arithmetic, one query head per KV head (adkv_tailscan.cuh).
+template <int BITS>
 __global__ void __launch_bounds__(64, 1) decode_attn_tail_kernel(KArgs ka, VArgs va, const float *__restrict__ mask,
                                                                  long long mask_stride_b, float scaling,
                                                                  const int *__restrict__ seq_lens)
 {
-    using Softmax = TailSoftmax<G, G == 1>;
     __shared__ alignas(128) uint8_t kbuf[kTailStages * Tile<BITS>::BYTES];
     __shared__ alignas(128) uint8_t vbuf[kTailStages * Tile<BITS>::BYTES];
     __shared__ alignas(16) float red[kRedFloats];
-    __shared__ alignas(16) float4 wts[Softmax::kFloat4];
+    __shared__ alignas(16) float4 wts[kTileTok];
     __shared__ alignas(16) float4 slow[2][2 * 32];
-    __shared__ FusedShared<G> fs;
+    __shared__ FusedShared<1> fs;
     __shared__ uint64_t kbar[kTailStages], vbar[kTailStages];
 
     const int bh = blockIdx.x, b = bh / ka.Hkv, h = bh % ka.Hkv;
@@ -96,21 +95,13 @@ __global__ void __launch_bounds__(64, 1) decode_attn_tail_kernel(KArgs ka, VArgs
         mbar_init_fence();
     }
     __syncthreads();
-    Seg seg{0, ka.T, true, nullptr, nullptr, 0};
     if (warp == 0) {
-        RingSink<G> sink{&fs, 0, 0};
-        k_tail_warp<BITS, G, kTailStages>(ka, seg, b, h, lane, kbuf, kbar, red, slow[0], sink);
+        RingSink<1> sink{&fs, 0, 0};
+        const Seg seg{0, ka.T, true, nullptr, nullptr, 0};
+        k_tail_warp<BITS, kTailStages, true>(ka, seg, b, h, lane, kbuf, kbar, red, slow[0], sink);
     } else {
-        Softmax src;
-        src.sh = &fs;
-        src.wts = wts;
-        src.mask = mask ? mask + size_t(b) * mask_stride_b : nullptr;
-        src.scale2 = scaling * 1.4426950408889634f;
-        src.t_begin = 0;
-        src.init();
-        seg.zp_end = va.tail + size_t(bh) * 2 * kD;
-        v_tail_warp<BITS, G, G == 1, kTailStages>(va, seg, b, h, lane, vbuf, vbar, slow[1], src,
-                                                  TailStore<G>{va.out + size_t(bh) * G * kD});
+        TailSoftmax src{&fs, wts, mask ? mask + size_t(b) * mask_stride_b : nullptr, scaling * 1.4426950408889634f, -INFINITY, 0.f};
+        v_tail_warp<BITS, kTailStages>(va, b, h, lane, vbuf, vbar, slow[1], src);
     }
 }
 
@@ -136,7 +127,7 @@ ADKV_HIDDEN int adkv_wide_decode_attn(const KArgs &ka, const VArgs &va, const fl
 ADKV_DEFINE_TU_STATUS(adkv_tu_status_fused)
 
 // Token segments of a stream side by side (adkv_segments.cu): up to this many streams per launch.
-constexpr long long kSegmentsMaxStreams = 444;
+constexpr long long kSegmentsMaxStreams = 148;
 
 static bool use_segments(const KArgs &ka, int B, bool exact, unsigned flags)
 {
@@ -144,25 +135,18 @@ static bool use_segments(const KArgs &ka, int B, bool exact, unsigned flags)
            ka.Hq / ka.Hkv <= 4 && (long long)B * ka.Hkv <= kSegmentsMaxStreams;
 }
 
-// One CTA per stream.  With tail states and the contracted arithmetic the scans of adkv_tailscan.cuh run, for one, two
-// and four query heads per KV head; with eight their constants and partial sums would not stay in registers.
+// One CTA per stream.
 static int launch_decode(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b, float scaling, int B,
                          int bits, bool exact, const int *seq_lens, cudaStream_t s)
 {
-    const int group = ka.Hq / ka.Hkv;
-    if (ka.tail && !exact && group <= 4) {
-        switch (bits * 16 + group) {
-#define ADKV_TAIL_CASE(BITS_, G_)                                                                                     \
-    case BITS_ * 16 + G_:                                                                                             \
-        decode_attn_tail_kernel<BITS_, G_><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling, seq_lens); \
+    if (ka.tail && !exact && ka.Hq == ka.Hkv) {
+        if (bits == 4)
+            decode_attn_tail_kernel<4><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling, seq_lens);
+        else
+            decode_attn_tail_kernel<2><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling, seq_lens);
         return launch_status();
-            ADKV_TAIL_CASE(4, 1) ADKV_TAIL_CASE(4, 2) ADKV_TAIL_CASE(4, 4)
-            ADKV_TAIL_CASE(2, 1) ADKV_TAIL_CASE(2, 2) ADKV_TAIL_CASE(2, 4)
-#undef ADKV_TAIL_CASE
-        default: return ADKV_E_SHAPE;
-        }
     }
-    ADKV_DISPATCH(bits, exact, group,
+    ADKV_DISPATCH(bits, exact, ka.Hq / ka.Hkv,
                   (decode_attn_kernel<BITS, G, ARITH><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling,
                                                                                seq_lens)))
     return launch_status();

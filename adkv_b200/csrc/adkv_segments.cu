@@ -11,10 +11,9 @@
 //
 //  1. every warp forms the product F of the factors of its segment and the extremes of its running product (half the
 //     arithmetic of a scan, no clamps);
-//  2. the states at the segment starts follow from the products of the segments before.  A segment whose product,
-//     from the state it really starts with, cannot have met a clamp (nearly always: the extremes, widened by the
-//     worst case of four tokens, stay inside the bounds) contributes F; any other is replayed with clamps, the warps of
-//     the CTA taking turns, so a cache that clamps everywhere costs at most one scale-only scan more;
+//  2. the states at the segment starts follow from the products of the segments before.  If some segment, from the state
+//     it really starts with, may have met a clamp (rarely: the extremes, widened by the worst case of four tokens, reach
+//     a bound), all segments of the stream are gone through once more with clamps (scale_map), still side by side;
 //  3. the scans run with zero points relative to the segment start.  For K that shifts every logit of a segment by one
 //     number, sum_c q_c * zp_c(start), for V it leaves out (sum of weights) * zp(start): both are put back
 //  4. when the partial softmax results of the segments are merged in shared memory.
@@ -34,9 +33,9 @@ constexpr int kPartFloats = 4 + kD;   // per (segment, head): maximum (log2 unit
 template <int BITS, int G>
 struct SegShared {
     alignas(128) uint8_t buf[2][kSegPairs][kSegStages * Tile<BITS>::BYTES];
-    alignas(16) float red[kSegPairs][kRedFloats];
-    alignas(16) float4 wts[kSegPairs][TailSoftmax<G, false>::kFloat4];
-    alignas(16) float4 slow[2][kSegPairs][2 * 32];
+    alignas(16) float red[kSegPairs][G == 1 ? kRedFloats : G * 8 * 36];
+    alignas(16) float2 wts[kSegPairs][G * kTileTok];
+    alignas(16) float4 slow[kSegPairs][2 * 32];          // one head: constants of the K scans' guarded bodies
     union {
         alignas(16) float comp[2][kSegPairs][3][kD];     // steps 1 and 2: product, smallest and largest running product
         alignas(16) float part[kSegPairs][G][kPartFloats];   // steps 3 and 4
@@ -54,26 +53,29 @@ template <int G>
 struct SegSink : RingSink<G> {
     float *z_end;
     bool done;
-    __device__ __forceinline__ void end_shares(const float (&share)[G], int lane)
+    __device__ __forceinline__ void end_share(float share, int lane, int g = 0)
     {
         done = true;
+        const float z = warp_sum(share);
+        if (lane == 0) z_end[g] = z;
+    }
+    __device__ __forceinline__ void end_state(const Chan (&ch)[4], const float (&qv)[G][4], int lane)
+    {
 #pragma unroll
-        for (int g = 0; g < G; ++g) {
-            const float z = warp_sum(share[g]);
-            if (lane == 0) z_end[g] = z;
-        }
+        for (int g = 0; g < G; ++g)
+            end_share(fmaf(qv[g][3], ch[3].zp, fmaf(qv[g][2], ch[2].zp, fmaf(qv[g][1], ch[1].zp, qv[g][0] * ch[0].zp))), lane, g);
     }
 };
 
 template <int G>
-struct SegStore {
+struct SegSrc : SoftmaxSrc<G> {
     float *part;       // [G][kPartFloats] of this segment
     float *zp_end;
     bool done;
-    __device__ __forceinline__ void end_zp(const f32x2 (&zp)[2], int c0)
+    __device__ __forceinline__ void end_state(const Chan (&ch)[4], int c0)
     {
         done = true;
-        *reinterpret_cast<ulonglong2 *>(zp_end + c0) = make_ulonglong2(zp[0], zp[1]);
+        *reinterpret_cast<float4 *>(zp_end + c0) = make_float4(ch[0].zp, ch[1].zp, ch[2].zp, ch[3].zp);
     }
     __device__ __forceinline__ void put(int c0, int g, float m, float l, float4 acc) const
     {
@@ -83,11 +85,11 @@ struct SegStore {
         }
         *reinterpret_cast<float4 *>(part + g * kPartFloats + 4 + c0) = acc;
     }
-    __device__ __forceinline__ void store(const float (&m)[G], const float (&l)[G], const float (&acc)[G][4], int c0) const
+    __device__ __forceinline__ void store(const VArgs &, int, int, int c0, const float (&acc)[G][4]) const
     {
 #pragma unroll
         for (int g = 0; g < G; ++g)
-            put(c0, g, m[g], l[g], make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]));
+            put(c0, g, this->m[g], this->l[g], make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]));
     }
     // a bounded wait gave up: the merged output of these heads becomes NaN
     __device__ __forceinline__ void give_up(int c0) const
@@ -150,44 +152,49 @@ __device__ __forceinline__ void scale_product(const uint4 *src, int n_words, con
     upk2(f2[1], F[2], F[3]);
 }
 
-// Step 2, the segments that may have met a clamp: the scales alone, with clamps where they can act.
+// Step 2 where a clamp may have acted.  The composition of the clamped steps is again a clamped scaling: a state x inside
+// the bounds ends as clamp(F * x, lo, hi), where F is the product of the factors and lo and hi are what the two bounds
+// themselves end as.  (A factor below zero sends every state to the same bound: then lo == hi.)  lo, hi: in the states to
+// start from -- the bounds, or twice the state itself where it is known and may lie outside them.
 template <int BITS>
-__device__ __noinline__ float4 scale_replay(const uint4 *src, int n_words, float4 s4, ScaleConst sc, SafeRange safe, float smin,
-                                            float smax)
+__device__ __noinline__ void scale_map(const uint4 *src, int n_words, const ScaleConst &sc, float smin, float smax, float4 lo4,
+                                       float4 hi4, float4 *comp)
 {
     FieldConsts<BITS> fc;
     fc.init();
-    Chan ch[4];
-    ch[0].s = s4.x; ch[1].s = s4.y; ch[2].s = s4.z; ch[3].s = s4.w;
-    float be[4], tc[4];
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-        upk2(sc.beta[p], be[2 * p], be[2 * p + 1]);
-        upk2(sc.tc[p], tc[2 * p], tc[2 * p + 1]);
-    }
+    f32x2 F[2] = {pk2(1.f, 1.f), pk2(1.f, 1.f)};
+    f32x2 lo[2] = {pk2(lo4.x, lo4.y), pk2(lo4.z, lo4.w)}, hi[2] = {pk2(hi4.x, hi4.y), pk2(hi4.z, hi4.w)};
+    const auto clamped = [&](f32x2 v) {
+        float a, b;
+        upk2(v, a, b);
+        return pk2(fminf(fmaxf(a, smin), smax), fminf(fmaxf(b, smin), smax));
+    };
+    uint4 w = *src;
 #pragma unroll 1
     for (int wd = 0; wd < n_words; ++wd) {
-        const uint4 w = src[wd * (kD / 4)];
+        const uint4 next = src[min(wd + 1, n_words - 1) * (kD / 4)];
         uint32_t grp[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll 1
-        for (int c8 = 0; c8 < Codec<BITS>::TPW / 8; ++c8) {
-            const bool free = safe.holds(ch);
-#pragma unroll 1
-            for (int half = 0; half < 2; ++half) {
-                static_for<4>([&](auto kc) {
-                    constexpr int k = decltype(kc)::value;
+        for (int blk = 0; blk < Codec<BITS>::TPW / 4; ++blk) {
+            static_for<4>([&](auto kc) {
+                constexpr int k = decltype(kc)::value;
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const float s = ch[c].s * fmaf(be[c], fabsf(fc.template code<k>(grp[c])), tc[c]);
-                        ch[c].s = free ? s : fminf(fmaxf(s, smin), smax);
-                    }
-                });
+                for (int p = 0; p < 2; ++p) {
+                    const f32x2 f = fma2(sc.beta[p], abs2(fc.template code2<k>(grp[2 * p], grp[2 * p + 1])), sc.tc[p]);
+                    F[p] = mul2(F[p], f);
+                    lo[p] = clamped(mul2(lo[p], f));
+                    hi[p] = clamped(mul2(hi[p], f));
+                }
+            });
 #pragma unroll
-                for (int c = 0; c < 4; ++c) grp[c] >>= 4 * BITS;
-            }
+            for (int c = 0; c < 4; ++c) grp[c] >>= 4 * BITS;
         }
+        w = next;
     }
-    return make_float4(ch[0].s, ch[1].s, ch[2].s, ch[3].s);
+    const f32x2 *rows[3] = {F, lo, hi};
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+        *reinterpret_cast<ulonglong2 *>(comp + r * (kD / 4)) = make_ulonglong2(rows[r][0], rows[r][1]);
 }
 
 template <int BITS, int G>
@@ -230,7 +237,7 @@ __global__ void __launch_bounds__(64 * kSegPairs, 1)
 
     // 1. products of all segments that another one follows (those are whole tiles)
     ScaleConst sc;
-    SafeRange safe8, safe4;
+    SafeRange safe8, safe4;   // safe8: not used
     float s[4];
     const bool followed = t_end < T;
     {
@@ -261,49 +268,34 @@ __global__ void __launch_bounds__(64 * kSegPairs, 1)
     __syncthreads();
 
     // 2. scale at the start of this warp's segment
-    // Advances x over segment i if that provably meets no clamp in any channel of the warp.
-    const auto advance = [&](int i, float (&x)[4]) {
+    const float4 start = make_float4(s[0], s[1], s[2], s[3]);
+    const bool empty = seg > 0 && t_begin >= T;
+    bool proven = true;      // no segment up to this one can have met a clamp, in any channel of the warp
+    for (int i = 0; i < seg && proven && !empty; ++i) {
         const float4 F = *reinterpret_cast<const float4 *>(&sh.comp[role][i][0][c0]);
         const float4 mn = *reinterpret_cast<const float4 *>(&sh.comp[role][i][1][c0]);
         const float4 mx = *reinterpret_cast<const float4 *>(&sh.comp[role][i][2][c0]);
-        const float Fv[4] = {F.x, F.y, F.z, F.w}, mnv[4] = {mn.x, mn.y, mn.z, mn.w}, mxv[4] = {mx.x, mx.y, mx.z, mx.w};
-        bool ok = true;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) ok = ok && x[c] * mnv[c] >= safe4.lo && x[c] * mxv[c] <= safe4.hi;
-        ok = __all_sync(kFull, ok);
-        if (ok) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) x[c] *= Fv[c];
-        }
-        return ok;
-    };
-    bool proven = true;
-    const bool empty = seg > 0 && t_begin >= T;
-    if (!empty)
-        for (int i = 0; i < seg && proven; ++i) proven = advance(i, s);
+        const bool ok = s[0] * mn.x >= safe4.lo && s[1] * mn.y >= safe4.lo && s[2] * mn.z >= safe4.lo && s[3] * mn.w >= safe4.lo &&
+                        s[0] * mx.x <= safe4.hi && s[1] * mx.y <= safe4.hi && s[2] * mx.z <= safe4.hi && s[3] * mx.w <= safe4.hi;
+        proven = __all_sync(kFull, ok);
+        s[0] *= F.x; s[1] *= F.y; s[2] *= F.z; s[3] *= F.w;
+    }
     if (__syncthreads_or(!proven)) {
-        // Some segment may clamp: the segments of a tensor advance the state one after another.
-        const bool first = seg == 0;
-        if (first) {
-            Chan ch[4];
-            SafeRange unused;
-            load_chan4<BITS, true>(ch, unused, p, poff, ka.smin, ka.smax);
-            *reinterpret_cast<float4 *>(&sh.init[role][0][1][c0]) = make_float4(ch[0].s, ch[1].s, ch[2].s, ch[3].s);
-        }
-        for (int i = 0; i + 1 < kSegPairs; ++i) {
-            if (seg == i && followed) {
-                const float4 x4 = *reinterpret_cast<const float4 *>(&sh.init[role][i][1][c0]);
-                float x[4] = {x4.x, x4.y, x4.z, x4.w};
-                float4 y;
-                if (advance(i, x)) y = make_float4(x[0], x[1], x[2], x[3]);
-                else y = scale_replay<BITS>(words, per_seg / C::TPW, x4, sc, safe8, ka.smin, ka.smax);
-                *reinterpret_cast<float4 *>(&sh.init[role][i + 1][1][c0]) = y;
-            }
-            __syncthreads();
-        }
-        if (!empty) {
-            const float4 x4 = *reinterpret_cast<const float4 *>(&sh.init[role][seg][1][c0]);
-            s[0] = x4.x; s[1] = x4.y; s[2] = x4.z; s[3] = x4.w;
+        const float4 lo = seg ? make_float4(ka.smin, ka.smin, ka.smin, ka.smin) : start;
+        const float4 hi = seg ? make_float4(ka.smax, ka.smax, ka.smax, ka.smax) : start;
+        if (followed)
+            scale_map<BITS>(words, per_seg / C::TPW, sc, ka.smin, ka.smax, lo, hi,
+                            reinterpret_cast<float4 *>(&sh.comp[role][seg][0][c0]));
+        __syncthreads();
+        s[0] = start.x; s[1] = start.y; s[2] = start.z; s[3] = start.w;
+        for (int i = 0; i < seg && !empty; ++i) {
+            const float4 F = *reinterpret_cast<const float4 *>(&sh.comp[role][i][0][c0]);
+            const float4 l = *reinterpret_cast<const float4 *>(&sh.comp[role][i][1][c0]);
+            const float4 u = *reinterpret_cast<const float4 *>(&sh.comp[role][i][2][c0]);
+            s[0] = fminf(fmaxf(F.x * s[0], l.x), u.x);
+            s[1] = fminf(fmaxf(F.y * s[1], l.y), u.y);
+            s[2] = fminf(fmaxf(F.z * s[2], l.z), u.z);
+            s[3] = fminf(fmaxf(F.w * s[3], l.w), u.w);
         }
         __syncthreads();
     }
@@ -317,7 +309,7 @@ __global__ void __launch_bounds__(64 * kSegPairs, 1)
     const auto append = [&](const ParamPtrs &pp, float *tail, bool keep, const __half *x_new, uint8_t *cache, float (&xh)[4]) {
         append_from_tail<BITS>(pp, poff, tail + size_t(bh) * 2 * kD, keep, x_new + size_t(bh) * kD + c0,
                                reinterpret_cast<uint4 *>(cache + (size_t(bh) * ka.n_super_cap + T / C::TPW) * kD * 4) + lane,
-                               T, ka.smin, ka.smax, nullptr, c0, xh);
+                               T, ka.smin, ka.smax, c0, xh);
     };
     // The appended token goes into the word behind the last cached one: only the warps that read that word may write it.
     const bool last = t_end == T && (seg == 0 || t_begin < T);
@@ -328,7 +320,10 @@ __global__ void __launch_bounds__(64 * kSegPairs, 1)
         sink.sl = 0;
         sink.z_end = sh.z_end[seg];
         sink.done = false;
-        k_tail_warp<BITS, G, kSegStages>(ka, sg, b, h, lane, sh.buf[0][seg], sh.bar[0][seg], sh.red[seg], sh.slow[0][seg], sink);
+        if constexpr (G == 1)
+            k_tail_warp<BITS, kSegStages, false>(ka, sg, b, h, lane, sh.buf[0][seg], sh.bar[0][seg], sh.red[seg], sh.slow[seg], sink);
+        else
+            k_warp<BITS, G, kArithFma, SegSink<G>, kSegStages>(ka, sg, b, h, lane, sh.buf[0][seg], sh.bar[0][seg], sh.red[seg], sink);
         if (last && sink.done) {
             float xh[4];
             append(ka.p, ka.tail, ka.tail_keep, ka.x_new, ka.cache, xh);
@@ -343,16 +338,19 @@ __global__ void __launch_bounds__(64 * kSegPairs, 1)
             }
         }
     } else {
-        TailSoftmax<G, false> src;
+        SegSrc<G> src;
         src.sh = &sh.fs[seg];
         src.wts = sh.wts[seg];
         src.mask = mask_row;
         src.scale2 = scale2;
+        src.n_tiles = (t_end - t_begin + kTileTok - 1) / kTileTok;
         src.t_begin = t_begin;
+        src.part = &sh.part[seg][0][0];
+        src.zp_end = sh.zp_end[seg];
+        src.done = false;
         src.init();
-        SegStore<G> store{&sh.part[seg][0][0], sh.zp_end[seg], false};
-        v_tail_warp<BITS, G, false, kSegStages>(va, sg, b, h, lane, sh.buf[1][seg], sh.bar[1][seg], sh.slow[1][seg], src, store);
-        if (last && store.done) {
+        v_warp<BITS, G, kArithFma, SegSrc<G>, kSegStages>(va, sg, b, h, lane, sh.buf[1][seg], sh.bar[1][seg], sh.wts[seg], src);
+        if (last && src.done) {
             float xh[4];
             append(va.p, va.tail, va.tail_keep, va.x_new, va.cache, xh);
             *reinterpret_cast<float4 *>(&sh.self_x[c0]) = make_float4(xh[0], xh[1], xh[2], xh[3]);

@@ -1,22 +1,29 @@
-// Scans of the decode step next to a persisted tail state (contracted arithmetic, head dim 128).
+// Scans of the decode step next to a persisted tail state (contracted arithmetic, head dim 128, one query head per KV
+// head).
 //
 // The tail supplies the state the appended token is quantised with, so a replay only has to feed the two attention
 // sums.  What bounds it is instruction issue: a packed fp32 instruction holds the issue port for two cycles, and the
-// contracted recurrence as written (adkv_decode.cuh) needs 6 + G of them per channel pair and token with G query heads.
+// contracted recurrence as written (adkv_decode.cuh) needs seven of them per channel pair and token.  Three identities
+// leave 5.25:
 //
 //  * Scale.  s' = s * (tc + beta*|q|) with tc = 1 - beta*target.  With s = tc^k * u inside a block of four tokens
 //    (k = 0..3), u' = u + (beta/tc) * |q*u|: one multiply-add on the product q*u that the value needs anyway.  The
-//    powers tc^k are folded into constants; once per block u is scaled back by tc^4.  5.25 + G instructions.
-//  * K, one head.  The logit needs the zero points only as z_t = sum_c q_c * zp_c(t), a running sum over tokens like zp
-//    itself: each lane carries its share of z in ONE register pair instead of a zero point per channel.  5.25.
-//  * V, one head, whole stream.  zp_t = zp_T - alpha * sum_{u >= t} q_u*s_u, and zp_T is known before the scan: it is the
-//    tail.  Hence sum_t w_t*zp_t = zp_T * W - alpha * sum_u P_u*q_u*s_u with the running sums P_u = w_0 + .. + w_u, which
-//    the online softmax forms anyway (its denominator): no zero point is replayed, and tc^k goes into one accumulator
-//    per position.  5.25.
+//    powers tc^k are folded into constants (K) or into one accumulator per position (V); once per block u is scaled
+//    back by tc^4.
+//  * K.  The logit needs the zero points only as z_t = sum_c q_c * zp_c(t), a running sum over tokens like zp itself:
+//    each lane carries its share of z in ONE register pair instead of a zero point per channel.
+//  * V.  zp_t = zp_T - alpha * sum_{u >= t} q_u*s_u, and zp_T is known before the scan: it is the tail.  Hence
+//    sum_t w_t*zp_t = zp_T * W - alpha * sum_u P_u*q_u*s_u with the running sums P_u = w_0 + .. + w_u, which the online
+//    softmax forms anyway (its denominator): no zero point is replayed.
 //
 // Clamp and eps guard are left out where eight worst-case updates cannot reach a bound, else where four cannot (on the
 // benchmark data the eight-token test fails for 7 % of the 4-bit chunks and 16 % of the 2-bit ones, the four-token test
 // for none); only what is left runs guarded.
+//
+// Measured on a B200, 4-bit, 32 heads, against decode_attn_kernel: batch 128 x 4096 tokens 1340 us (1473), batch 24 x
+// 1531 tokens with mask 131 us (152), ragged batch 48 of up to 3000 tokens 303 us (352).  With two and four query heads
+// the first identity alone remains and the longer constants cost what it gains (2480 us against 2436 us at batch 32 x 8
+// KV heads x 32768 tokens, 2-bit), so those keep decode_attn_kernel.
 #pragma once
 #include "adkv_softmax.cuh"
 
@@ -149,27 +156,13 @@ __device__ __forceinline__ float guarded_scale_step(float q, float &s, float be,
 template <int BITS>
 __device__ __forceinline__ void append_from_tail(const ParamPtrs &p, size_t poff, float *tail, bool tail_keep,
                                                  const __half *x_new, uint4 *slot, int T, float smin, float smax,
-                                                 float *ckpt_out, int c0, float (&xh)[4])
+                                                 int c0, float (&xh)[4])
 {
     Chan ch[4];
     SafeRange unused;
     load_chan4<BITS, true>(ch, unused, p, poff, smin, smax);
-    append_new_token<BITS, kArithCanon>(ch, p, poff, tail, tail_keep, x_new, slot, T, smin, smax, ckpt_out, c0, kD, xh);
+    append_new_token<BITS, kArithCanon>(ch, p, poff, tail, tail_keep, x_new, slot, T, smin, smax, nullptr, c0, kD, xh);
 }
-
-// Optional members of sinks and stores: what a scan without append ends in.
-template <class S, int G>
-__device__ __forceinline__ auto sink_end_shares(S &s, const float (&z)[G], int lane, int)
-    -> decltype(s.end_shares(z, lane), void()) { s.end_shares(z, lane); }
-template <class S, int G>
-__device__ __forceinline__ void sink_end_shares(S &, const float (&)[G], int, long) {}
-template <class S>
-__device__ __forceinline__ auto store_end_zp(S &s, const f32x2 (&zp)[2], int c0, int) -> decltype(s.end_zp(zp, c0), void())
-{
-    s.end_zp(zp, c0);
-}
-template <class S>
-__device__ __forceinline__ void store_end_zp(S &, const f32x2 (&)[2], int, long) {}
 
 // ------------------------------------------------------------------------------------------ walking a tile
 
@@ -244,7 +237,7 @@ __device__ __forceinline__ float reduce_units(const float *red, int lane)
     return r;
 }
 
-// ------------------------------------------------------------------------------------------ K side, one head
+// ------------------------------------------------------------------------------------------ K side
 
 struct KTailState {
     f32x2 s[2];
@@ -336,73 +329,18 @@ __device__ __noinline__ KTailState k_tail_slow(uint4 w, KTailState st, float4 q,
     return st;
 }
 
-// ------------------------------------------------------------------------------------------ value form (both sides)
-
-// Replays four tokens; value(k, xh) takes the dequantised values of position k as two pairs.  aE[k] = alpha * tc^k.
-template <int BITS, class Value>
-__device__ __forceinline__ void x_tail_block(const uint32_t (&grp)[4], const PairFields<BITS> &fc, f32x2 (&s)[2], f32x2 (&zp)[2],
-                                             const TailChan &t, const f32x2 (&aE)[4][2], Value &&value)
-{
-    static_for<4>([&](auto kc) {
-        constexpr int k = decltype(kc)::value;
-        f32x2 xh[2];
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            const f32x2 r = mul2(fc.template code2<k>(grp[2 * p], grp[2 * p + 1]), s[p]);
-            xh[p] = k == 0 ? add2(r, zp[p]) : fma2(t.e[k ? k - 1 : 0][p], r, zp[p]);
-            zp[p] = fma2(aE[k][p], r, zp[p]);
-            s[p] = fma2(t.bp[p], abs2(r), s[p]);
-        }
-        value(kc, xh);
-    });
-#pragma unroll
-    for (int p = 0; p < 2; ++p) s[p] = mul2(s[p], t.e[3][p]);
-}
-
-// The same with guards and clamp for one token (inline: with several heads the operands of a call would not fit the
-// registers of the calling convention).
-template <int BITS>
-__device__ __forceinline__ void x_tail_guarded(const uint32_t (&grp)[4], int j, f32x2 (&s2)[2], f32x2 (&zp2)[2],
-                                               const f32x2 (&alpha)[2], const float4 *slow, float smin, float smax, f32x2 (&xh)[2])
-{
-    float be[4], tc[4], s[4];
-    load_slow_consts(slow, be, tc);
-    upk2(s2[0], s[0], s[1]);
-    upk2(s2[1], s[2], s[3]);
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-        const float a = guarded_scale_step(code_f_rt<BITS>(grp[2 * p], j), s[2 * p], be[2 * p], tc[2 * p], smin, smax);
-        const float b = guarded_scale_step(code_f_rt<BITS>(grp[2 * p + 1], j), s[2 * p + 1], be[2 * p + 1], tc[2 * p + 1], smin, smax);
-        const f32x2 r = pk2(a, b);
-        xh[p] = add2(r, zp2[p]);
-        zp2[p] = fma2(alpha[p], r, zp2[p]);
-        s2[p] = pk2(s[2 * p], s[2 * p + 1]);
-    }
-}
-
-__device__ __forceinline__ void scaled_alpha(const TailChan &t, f32x2 (&aE)[4][2])
-{
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-        aE[0][p] = t.alpha[p];
-#pragma unroll
-        for (int k = 1; k < 4; ++k) aE[k][p] = mul2(t.alpha[p], t.e[k - 1][p]);
-    }
-}
-
 // ------------------------------------------------------------------------------------------ K warp
 
-// Sink: RingSink<G> (begin_tile, put, end_tile, put_self, finish) or one with end_state(share of sum_c q_c * zp_c per
-// lane and head, lane) for a scan without append.  red: kRedFloats floats, 16-byte aligned.
-template <int BITS, int G, int STAGES, class Sink>
+// Sink: RingSink<1> (begin_tile_short, put, end_tile, put_self, finish); without APPEND (a scan that does not reach the
+// end of its stream) also end_share(this lane's share of sum_c q_c * zp_c after the last token, lane).
+// red: kRedFloats floats, 16-byte aligned; slow: 64 float4.
+template <int BITS, int STAGES, bool APPEND, class Sink>
 __device__ __forceinline__ void k_tail_warp(const KArgs &a, const Seg &seg, int b, int h, int lane, uint8_t *ring_buf,
                                             uint64_t *ring_bar, float *red, float4 *slow, Sink &sink)
 {
     using C = Codec<BITS>;
-    constexpr int kBlocks = kRedUnits / G;            // blocks of 4 tokens per reduction pass
     const int bh = b * a.Hkv + h, c0 = 4 * lane;
     const size_t poff = size_t(h) * kD + c0;
-    const __half *q = a.q + (size_t(b) * a.Hq + size_t(h) * G) * kD + c0;
     uint8_t *stream = a.cache + size_t(bh) * a.n_super_cap * kD * 4;
     const int n_tok = seg.t_end - seg.t_begin;
     StreamRing<BITS, STAGES> ring{ring_buf, ring_bar, stream + size_t(seg.t_begin / C::TPW) * (kD * 4),
@@ -412,152 +350,83 @@ __device__ __forceinline__ void k_tail_warp(const KArgs &a, const Seg &seg, int 
     fc.init();
     float4 *red4 = reinterpret_cast<float4 *>(red) + lane;
     slow += lane;
-    bool ok = true;
-    int i = 0;
-    float z_lane[G];
-
-    // Walks the tiles; tile_body(words, valid tokens) replays one.
-    const auto scan = [&](auto &&tile_body, f32x2 (&scale)[2], const uint32_t (&drift)[2]) {
-        for (; i < ring.n_tiles; ++i) {
-            if (!(ok = ring.wait_short(i))) break;
-            if (!(ok = sink.begin_tile_short(i))) break;
-            tile_body(ring.tile(i, lane), min(kTileTok, n_tok - i * kTileTok));
-            if ((i + 1) % kDriftTiles == 0) correct_drift(scale, drift);
-            if constexpr (G == 1) sink.put(0, lane, reduce_units(red, lane));
-            sink.end_tile(i, lane);
-            ring.release_and_refill(i, lane);
-        }
-    };
-
     TailChan t;
     load_tail_chan<BITS>(t, a.p, poff, seg.init, c0, a.smin, a.smax, slow);
-    if constexpr (G == 1) {
-        float qv[4], al[4];
-        load_half4(qv, q);
-        upk2(t.alpha[0], al[0], al[1]);
-        upk2(t.alpha[1], al[2], al[3]);
-        const float4 qf = make_float4(qv[0], qv[1], qv[2], qv[3]);
-        const float4 qaf = make_float4(qv[0] * al[0], qv[1] * al[1], qv[2] * al[2], qv[3] * al[3]);
-        f32x2 Q[4][2], A[4][2], e4[2];
+    float qv[4], al[4];
+    load_half4(qv, a.q + (size_t(b) * a.Hq + h) * kD + c0);
+    upk2(t.alpha[0], al[0], al[1]);
+    upk2(t.alpha[1], al[2], al[3]);
+    const float4 qf = make_float4(qv[0], qv[1], qv[2], qv[3]);
+    const float4 qaf = make_float4(qv[0] * al[0], qv[1] * al[1], qv[2] * al[2], qv[3] * al[3]);
+    f32x2 Q[4][2], A[4][2];
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            Q[0][p] = p ? pk2(qf.z, qf.w) : pk2(qf.x, qf.y);
-            A[0][p] = p ? pk2(qaf.z, qaf.w) : pk2(qaf.x, qaf.y);
-            e4[p] = t.e[3][p];
+    for (int p = 0; p < 2; ++p) {
+        Q[0][p] = p ? pk2(qf.z, qf.w) : pk2(qf.x, qf.y);
+        A[0][p] = p ? pk2(qaf.z, qaf.w) : pk2(qaf.x, qaf.y);
 #pragma unroll
-            for (int k = 1; k < 4; ++k) {
-                Q[k][p] = mul2(Q[0][p], t.e[k - 1][p]);
-                A[k][p] = mul2(A[0][p], t.e[k - 1][p]);
-            }
+        for (int k = 1; k < 4; ++k) {
+            Q[k][p] = mul2(Q[0][p], t.e[k - 1][p]);
+            A[k][p] = mul2(A[0][p], t.e[k - 1][p]);
         }
-        KTailState st;
-        st.s[0] = t.s[0];
-        st.s[1] = t.s[1];
-        st.z = fma2(Q[0][1], t.zp[1], mul2(Q[0][0], t.zp[0]));
-        const auto slow_chunk = [&](const uint4 &w, int tok, int count) {
-            st = k_tail_slow<BITS>(w, st, qf, qaf, slow, red4 + (tok >> 2) * 32, count, t.safe4, a.smin, a.smax);
-        };
-        const auto chunk = [&](const uint4 &w, int tok) {
-            if (tail_safe(t.safe, st.s)) {
-                float4 *dst = red4 + (tok >> 2) * 32;
-                uint32_t grp[4] = {w.x, w.y, w.z, w.w};
-                k_tail_block<BITS>(grp, fc, st, t.bp, e4, Q, A, dst);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) grp[c] >>= 4 * BITS;
-                k_tail_block<BITS>(grp, fc, st, t.bp, e4, Q, A, dst + 32);
-            } else {
-                slow_chunk(w, tok, 8);
-            }
-        };
-        scan(
-            [&](const uint4 *tile, int ntok) {
-                if (ntok == kTileTok) walk_full_tile<BITS>(tile, chunk);
-                else walk_tile<BITS>(tile, ntok, slow_chunk);
-            },
-            st.s, t.drift);
-        float lo, hi;
-        upk2(st.z, lo, hi);
-        z_lane[0] = lo + hi;
-    } else {
-        f32x2 aE[4][2], qv2[G][2];
-        scaled_alpha(t, aE);
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            float qv[4];
-            load_half4(qv, q + size_t(g) * kD);
-            qv2[g][0] = pk2(qv[0], qv[1]);
-            qv2[g][1] = pk2(qv[2], qv[3]);
-        }
-        const auto dot = [&](int g, const f32x2 (&x)[2]) {
-            float lo, hi;
-            upk2(fma2(qv2[g][1], x[1], mul2(qv2[g][0], x[0])), lo, hi);
-            return lo + hi;
-        };
-        const auto body = [&](const uint4 &w, int tok, int count) {
+    }
+    KTailState st;
+    st.s[0] = t.s[0];
+    st.s[1] = t.s[1];
+    st.z = fma2(Q[0][1], t.zp[1], mul2(Q[0][0], t.zp[0]));
+    const auto slow_chunk = [&](const uint4 &w, int tok, int count) {
+        st = k_tail_slow<BITS>(w, st, qf, qaf, slow, red4 + (tok >> 2) * 32, count, t.safe4, a.smin, a.smax);
+    };
+    const auto chunk = [&](const uint4 &w, int tok) {
+        if (tail_safe(t.safe, st.s)) {
+            float4 *dst = red4 + (tok >> 2) * 32;
             uint32_t grp[4] = {w.x, w.y, w.z, w.w};
-            const bool free8 = count >= 8 && tail_safe(t.safe, t.s);
-#pragma unroll 1
-            for (int half = 0; half < 2; ++half) {     // one body, two trips: the code has to stay in the instruction cache
-                float4 *dst = red4 + (((tok >> 2) + half) % kBlocks) * 32;
-                const int n = count - 4 * half;
-                if (free8 || (n >= 4 && tail_safe(t.safe4, t.s))) {
-                    float v[G][4];
-                    x_tail_block<BITS>(grp, fc, t.s, t.zp, t, aE, [&](auto kc, const f32x2 (&xh)[2]) {
+            k_tail_block<BITS>(grp, fc, st, t.bp, t.e[3], Q, A, dst);
 #pragma unroll
-                        for (int g = 0; g < G; ++g) v[g][decltype(kc)::value] = dot(g, xh);
-                    });
-#pragma unroll
-                    for (int g = 0; g < G; ++g) dst[g * kBlocks * 32] = make_float4(v[g][0], v[g][1], v[g][2], v[g][3]);
-                } else {
-#pragma unroll 1
-                    for (int j = 0; j < 4 && j < n; ++j) {
-                        f32x2 xh[2];
-                        x_tail_guarded<BITS>(grp, j, t.s, t.zp, t.alpha, slow, a.smin, a.smax, xh);
-#pragma unroll
-                        for (int g = 0; g < G; ++g) reinterpret_cast<float *>(dst + g * kBlocks * 32)[j] = dot(g, xh);
-                    }
-                }
-#pragma unroll
-                for (int c = 0; c < 4; ++c) grp[c] >>= 4 * BITS;
-            }
-            // a pass is complete after kBlocks blocks, or with the last tokens of the tile
-            if (((tok >> 2) + 2) % kBlocks == 0 || count <= 8) {
-                const float v = reduce_units(red, lane);
-                const int unit = lane >> 2;
-                sink.put(unit / kBlocks, ((tok >> 2) / kBlocks * kBlocks + unit % kBlocks) * 4 + (lane & 3), v);
-            }
-        };
-        scan([&](const uint4 *tile, int ntok) { walk_tile<BITS>(tile, ntok, body); }, t.s, t.drift);
-#pragma unroll
-        for (int g = 0; g < G; ++g) z_lane[g] = dot(g, t.zp);
+            for (int c = 0; c < 4; ++c) grp[c] >>= 4 * BITS;
+            k_tail_block<BITS>(grp, fc, st, t.bp, t.e[3], Q, A, dst + 32);
+        } else {
+            slow_chunk(w, tok, 8);
+        }
+    };
+    bool ok = true;
+    int i = 0;
+    for (; i < ring.n_tiles; ++i) {
+        if (!(ok = ring.wait_short(i))) break;
+        if (!(ok = sink.begin_tile_short(i))) break;
+        const uint4 *tile = ring.tile(i, lane);
+        const int ntok = min(kTileTok, n_tok - i * kTileTok);
+        if (ntok == kTileTok) walk_full_tile<BITS>(tile, chunk);
+        else walk_tile<BITS>(tile, ntok, slow_chunk);
+        if ((i + 1) % kDriftTiles == 0) correct_drift(st.s, t.drift);
+        sink.put(0, lane, reduce_units(red, lane));
+        sink.end_tile(i, lane);
+        ring.release_and_refill(i, lane);
     }
     if (!ok) {
         ring.drain(i);
         return;
     }
-    if (!seg.append) {
-        sink_end_shares(sink, z_lane, lane, 0);
-        return;
-    }
-    // Append k_new as token T from the tail, then its own logit from the dequantised value.
-    float xh[4];
-    append_from_tail<BITS>(a.p, poff, a.tail + size_t(bh) * 2 * kD, a.tail_keep, a.x_new + size_t(bh) * kD + c0,
-                           reinterpret_cast<uint4 *>(stream + size_t(a.T / C::TPW) * (kD * 4)) + lane, a.T, a.smin, a.smax,
-                           seg.ckpt_out, c0, xh);
-    if (!sink.begin_tile_short(ring.n_tiles)) return;
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-        float qv[4], s = 0.f;
-        load_half4(qv, q + size_t(g) * kD);
+    if constexpr (APPEND) {
+        // Append k_new as token T from the tail, then its own logit from the dequantised value.
+        float xh[4];
+        append_from_tail<BITS>(a.p, poff, a.tail + size_t(bh) * 2 * kD, a.tail_keep, a.x_new + size_t(bh) * kD + c0,
+                               reinterpret_cast<uint4 *>(stream + size_t(a.T / C::TPW) * (kD * 4)) + lane, a.T, a.smin,
+                               a.smax, c0, xh);
+        if (!sink.begin_tile_short(ring.n_tiles)) return;
+        float s = 0.f;
 #pragma unroll
         for (int c = 0; c < 4; ++c) s = fmaf(qv[c], xh[c], s);
         s = warp_sum(s);
-        if (lane == 0) sink.put_self(g, s);
+        if (lane == 0) sink.put_self(0, s);
+        sink.finish(lane);
+    } else {
+        float lo, hi;
+        upk2(st.z, lo, hi);
+        sink.end_share(lo + hi, lane);
     }
-    sink.finish(lane);
 }
 
-// ------------------------------------------------------------------------------------------ V side, one head
+// ------------------------------------------------------------------------------------------ V side
 
 struct VTailState {
     f32x2 s[2];
@@ -636,303 +505,165 @@ __device__ __forceinline__ void v_tail_block(const uint32_t (&grp)[4], const Pai
     for (int p = 0; p < 2; ++p) s[p] = mul2(s[p], e4[p]);
 }
 
-// ------------------------------------------------------------------------------------------ softmax of a V warp
+// ------------------------------------------------------------------------------------------ V warp
 
-// Online softmax.  Weights of a tile: PREFIX (one head): (w, w, P, P) per token with the running sum P of the weights;
-// otherwise [G][32] (w, w).
-template <int G, bool PREFIX>
+// Online softmax of a V warp.  Weights of a tile: (w, w, P, P) per token, P the running sum of the weights.
 struct TailSoftmax {
-    static constexpr int kFloat4 = PREFIX ? kTileTok : G * kTileTok / 2;
-    FusedShared<G> *sh;
-    float4 *wts;           // kFloat4 entries
+    FusedShared<1> *sh;
+    float4 *wts;           // [kTileTok]
     const float *mask;     // row of this batch or nullptr
     float scale2;          // scaling * log2(e)
-    int t_begin;           // first token of this segment (mask index of local token 0)
-    float m[G];            // running maximum (log2 units)
-    float l[G];            // PREFIX: sum of the weights so far; otherwise this lane's share of it
+    float m, l;            // running maximum (log2 units), sum of the weights so far
 
-    __device__ __forceinline__ void init()
-    {
-#pragma unroll
-        for (int g = 0; g < G; ++g) { m[g] = -INFINITY; l[g] = 0.f; }
-    }
     __device__ __forceinline__ static float redux_max(float v)
     {
         float r;
         asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
         return r;
     }
-    // Fills the weights of tile i; corr[g] is what the accumulators of head g have to be scaled with (warp-uniform).
-    __device__ __forceinline__ bool tile(int i, int ntok, int lane, float (&corr)[G])
+    // Fills the weights of tile i; corr is what the accumulators have to be scaled with (warp-uniform).
+    __device__ __forceinline__ bool tile(int i, int ntok, int lane, float &corr)
     {
         const int slot = unsigned(i) % kLogitSlots;
-        const float mk = (mask && lane < ntok) ? mask[t_begin + i * kTileTok + lane] * 1.4426950408889634f : 0.f;
+        const float mk = (mask && lane < ntok) ? mask[i * kTileTok + lane] * 1.4426950408889634f : 0.f;
         if (!mbar_wait_short(&sh->lfull[slot], (unsigned(i) / kLogitSlots) & 1, kStatLFullWait)) return false;
-        float x[G];
-#pragma unroll
-        for (int g = 0; g < G; ++g) x[g] = sh->lring[slot][0][g][lane];
+        const float x = sh->lring[slot][0][0][lane];
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh->lempty[slot]);
+        const float v = lane < ntok ? fmaf(x, scale2, mk) : -INFINITY;
+        const float m_new = fmaxf(m, redux_max(v));
+        const bool dead = m_new == -INFINITY;
+        corr = dead ? 1.f : exp2f(m - m_new);
+        const float w = dead ? 0.f : exp2f(v - m_new);
+        m = m_new;
+        float P = w;
 #pragma unroll
-        for (int g = 0; g < G; ++g) {
-            const float v = lane < ntok ? fmaf(x[g], scale2, mk) : -INFINITY;
-            const float m_new = fmaxf(m[g], redux_max(v));
-            const bool dead = m_new == -INFINITY;
-            corr[g] = dead ? 1.f : exp2f(m[g] - m_new);
-            const float w = dead ? 0.f : exp2f(v - m_new);
-            m[g] = m_new;
-            if constexpr (PREFIX) {
-                float P = w;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const float y = __shfl_up_sync(kFull, P, o);
-                    if (lane >= o) P += y;
-                }
-                P = fmaf(l[0], corr[0], P);
-                l[0] = __shfl_sync(kFull, P, 31);
-                wts[lane] = make_float4(w, w, P, P);
-            } else {
-                l[g] = fmaf(l[g], corr[g], w);
-                reinterpret_cast<float2 *>(wts)[g * kTileTok + lane] = make_float2(w, w);
-            }
+        for (int o = 1; o < 32; o <<= 1) {
+            const float y = __shfl_up_sync(kFull, P, o);
+            if (lane >= o) P += y;
         }
+        P = fmaf(l, corr, P);
+        l = __shfl_sync(kFull, P, 31);
+        wts[lane] = make_float4(w, w, P, P);
         __syncwarp();
         return true;
     }
-    // after the last tile: l = the sum of the weights, in every lane
-    __device__ __forceinline__ void close()
-    {
-        if constexpr (!PREFIX) {
-#pragma unroll
-            for (int g = 0; g < G; ++g) l[g] = warp_sum(l[g]);
-        }
-    }
-    // after close(): weight of the appended token, whose logit is the single entry of tile n_tiles
-    __device__ __forceinline__ bool self(int n_tiles, int T, float (&out)[G][4], float (&w_self)[G])
+    // weight of the appended token, whose logit is the single entry of tile n_tiles
+    __device__ __forceinline__ bool self(int n_tiles, int T, float (&out)[4], float &w_self)
     {
         const int slot = unsigned(n_tiles) % kLogitSlots;
         if (!mbar_wait_short(&sh->lfull[slot], (unsigned(n_tiles) / kLogitSlots) & 1, kStatLFullWait)) return false;
         const float mk = mask ? mask[T] * 1.4426950408889634f : 0.f;
+        const float v = fmaf(sh->lring[slot][0][0][0], scale2, mk);
+        const float m_new = fmaxf(m, v);
+        const bool dead = m_new == -INFINITY;
+        const float corr = dead ? 1.f : exp2f(m - m_new);
+        w_self = dead ? 0.f : exp2f(v - m_new);
+        l = fmaf(l, corr, w_self);
 #pragma unroll
-        for (int g = 0; g < G; ++g) {
-            const float v = fmaf(sh->lring[slot][0][g][0], scale2, mk);
-            const float m_new = fmaxf(m[g], v);
-            const bool dead = m_new == -INFINITY;
-            const float corr = dead ? 1.f : exp2f(m[g] - m_new);
-            w_self[g] = dead ? 0.f : exp2f(v - m_new);
-            l[g] = fmaf(l[g], corr, w_self[g]);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) out[g][c] *= corr;
-            m[g] = m_new;
-        }
+        for (int c = 0; c < 4; ++c) out[c] *= corr;
+        m = m_new;
         return true;
     }
 };
 
-// ------------------------------------------------------------------------------------------ V warp
-
-// store: store(m, l, sums, c0) with the un-normalised sums, give_up(c0) when a bounded wait ran out, and optionally
-// end_zp(zero points, c0) for a scan without append (value form).  PREFIX needs one head and the zero points after the
-// last token in seg.zp_end.
-template <int BITS, int G, bool PREFIX, int STAGES, class Store>
-__device__ __forceinline__ void v_tail_warp(const VArgs &a, const Seg &seg, int b, int h, int lane, uint8_t *ring_buf,
-                                            uint64_t *ring_bar, float4 *slow, TailSoftmax<G, PREFIX> &src, Store &&store)
+// The whole stream of (b, h); writes the normalised output.
+template <int BITS, int STAGES>
+__device__ __forceinline__ void v_tail_warp(const VArgs &a, int b, int h, int lane, uint8_t *ring_buf, uint64_t *ring_bar,
+                                            float4 *slow, TailSoftmax &src)
 {
     using C = Codec<BITS>;
-    static_assert(!PREFIX || G == 1, "running sums of the weights: one head");
     const int bh = b * a.Hkv + h, c0 = 4 * lane;
     const size_t poff = size_t(h) * kD + c0;
     uint8_t *stream = a.cache + size_t(bh) * a.n_super_cap * kD * 4;
-    const int n_tok = seg.t_end - seg.t_begin;
-    StreamRing<BITS, STAGES> ring{ring_buf, ring_bar, stream + size_t(seg.t_begin / C::TPW) * (kD * 4),
-                                  (n_tok + kTileTok - 1) / kTileTok, n_tok, kStatVWait, kD * 4};
+    StreamRing<BITS, STAGES> ring{ring_buf, ring_bar, stream, (a.T + kTileTok - 1) / kTileTok, a.T, kStatVWait, kD * 4};
     ring.prologue(lane);
     PairFields<BITS> fc;
     fc.init();
     slow += lane;
-    bool ok = true;
-    int i = 0;
-    const auto scan = [&](auto &&rescale, auto &&tile_body, f32x2 (&scale)[2], const uint32_t (&drift)[2]) {
-        for (; i < ring.n_tiles; ++i) {
-            const int ntok = min(kTileTok, n_tok - i * kTileTok);
-            float corr[G];
-            if (!(ok = src.tile(i, ntok, lane, corr))) break;
-            rescale(corr);
-            if (!(ok = ring.wait_short(i))) break;
-            tile_body(ring.tile(i, lane), ntok);
-            if ((i + 1) % kDriftTiles == 0) correct_drift(scale, drift);
-            ring.release_and_refill(i, lane);   // also orders this tile's reads of wts before the next fill
+    float *tail = a.tail + size_t(bh) * 2 * kD;
+    TailChan t;
+    load_tail_chan<BITS>(t, a.p, poff, nullptr, c0, a.smin, a.smax, slow);
+    f32x2 s[2] = {t.s[0], t.s[1]}, acc[4][2], accp[4][2];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int p = 0; p < 2; ++p) acc[k][p] = accp[k][p] = 0ull;
+    const auto slow_chunk = [&](const uint4 &w, int tok, int count) {
+        VTailState st;
+#pragma unroll
+        for (int p = 0; p < 2; ++p) { st.s[p] = s[p]; st.acc[p] = acc[0][p]; st.accp[p] = accp[0][p]; }
+        st = v_tail_slow<BITS>(w, st, slow, src.wts + tok, count, t.safe4, a.smin, a.smax);
+#pragma unroll
+        for (int p = 0; p < 2; ++p) { s[p] = st.s[p]; acc[0][p] = st.acc[p]; accp[0][p] = st.accp[p]; }
+    };
+    const auto chunk = [&](const uint4 &w, int tok) {
+        if (tail_safe(t.safe, s)) {
+            const float4 *wt = src.wts + tok;
+            uint32_t grp[4] = {w.x, w.y, w.z, w.w};
+            v_tail_block<BITS>(grp, fc, s, t.bp, t.e[3], wt, acc, accp);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) grp[c] >>= 4 * BITS;
+            v_tail_block<BITS>(grp, fc, s, t.bp, t.e[3], wt + 4, acc, accp);
+        } else {
+            slow_chunk(w, tok, 8);
         }
     };
-
-    float out[G][4];
-    TailChan t;
-    load_tail_chan<BITS>(t, a.p, poff, seg.init, c0, a.smin, a.smax, slow);
-    if constexpr (PREFIX) {
-        f32x2 s[2] = {t.s[0], t.s[1]}, e4[2] = {t.e[3][0], t.e[3][1]}, acc[4][2], accp[4][2];
+    bool ok = true;
+    int i = 0;
+    for (; i < ring.n_tiles; ++i) {
+        const int ntok = min(kTileTok, a.T - i * kTileTok);
+        float corr;
+        if (!(ok = src.tile(i, ntok, lane, corr))) break;
+        if (corr != 1.f) {       // warp-uniform; rare once the running maximum has settled
+            const f32x2 f = pk2(corr, corr);
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+            for (int k = 0; k < 4; ++k)
 #pragma unroll
-            for (int p = 0; p < 2; ++p) acc[k][p] = accp[k][p] = 0ull;
-        const auto slow_chunk = [&](const uint4 &w, int tok, int count) {
-            VTailState st;
-#pragma unroll
-            for (int p = 0; p < 2; ++p) { st.s[p] = s[p]; st.acc[p] = acc[0][p]; st.accp[p] = accp[0][p]; }
-            st = v_tail_slow<BITS>(w, st, slow, src.wts + tok, count, t.safe4, a.smin, a.smax);
-#pragma unroll
-            for (int p = 0; p < 2; ++p) { s[p] = st.s[p]; acc[0][p] = st.acc[p]; accp[0][p] = st.accp[p]; }
-        };
-        const auto chunk = [&](const uint4 &w, int tok) {
-            if (tail_safe(t.safe, s)) {
-                const float4 *wt = src.wts + tok;
-                uint32_t grp[4] = {w.x, w.y, w.z, w.w};
-                v_tail_block<BITS>(grp, fc, s, t.bp, e4, wt, acc, accp);
-#pragma unroll
-                for (int c = 0; c < 4; ++c) grp[c] >>= 4 * BITS;
-                v_tail_block<BITS>(grp, fc, s, t.bp, e4, wt + 4, acc, accp);
-            } else {
-                slow_chunk(w, tok, 8);
-            }
-        };
-        scan(
-            [&](const float (&corr)[G]) {
-                if (corr[0] != 1.f) {       // warp-uniform; rare once the running maximum has settled
-                    const f32x2 f = pk2(corr[0], corr[0]);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-#pragma unroll
-                        for (int p = 0; p < 2; ++p) {
-                            acc[k][p] = mul2(acc[k][p], f);
-                            accp[k][p] = mul2(accp[k][p], f);
-                        }
+                for (int p = 0; p < 2; ++p) {
+                    acc[k][p] = mul2(acc[k][p], f);
+                    accp[k][p] = mul2(accp[k][p], f);
                 }
-            },
-            [&](const uint4 *tile, int ntok) {
-                if (ntok == kTileTok) walk_full_tile<BITS>(tile, chunk);
-                else walk_tile<BITS>(tile, ntok, slow_chunk);
-            },
-            s, t.drift);
-        if (ok) {
-            // sum_k tc^k * (acc_k - alpha * accp_k) + W * zp_end; the constants are loaded again rather than kept
-            load_tail_chan<BITS>(t, a.p, poff, nullptr, c0, a.smin, a.smax, slow);
-            const f32x2 minus = pk2(-1.f, -1.f);
-#pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                const f32x2 nal = mul2(t.alpha[p], minus);
-                f32x2 sum = fma2(nal, accp[0][p], acc[0][p]);
-#pragma unroll
-                for (int k = 1; k < 4; ++k) sum = fma2(t.e[k - 1][p], fma2(nal, accp[k][p], acc[k][p]), sum);
-                upk2(sum, out[0][2 * p], out[0][2 * p + 1]);
-            }
-            if (n_tok > 0) {
-                const float4 ze = *reinterpret_cast<const float4 *>(seg.zp_end + c0);
-                out[0][0] = fmaf(src.l[0], ze.x, out[0][0]);
-                out[0][1] = fmaf(src.l[0], ze.y, out[0][1]);
-                out[0][2] = fmaf(src.l[0], ze.z, out[0][2]);
-                out[0][3] = fmaf(src.l[0], ze.w, out[0][3]);
-            }
         }
-    } else {
-        f32x2 aE[4][2], acc[G][2];
-        scaled_alpha(t, aE);
-#pragma unroll
-        for (int g = 0; g < G; ++g) acc[g][0] = acc[g][1] = 0ull;
-        const float2 *wts = reinterpret_cast<const float2 *>(src.wts);
-        const auto body = [&](const uint4 &w, int tok, int count) {
-            uint32_t grp[4] = {w.x, w.y, w.z, w.w};
-            const bool free8 = count >= 8 && tail_safe(t.safe, t.s);
-#pragma unroll 1
-            for (int half = 0; half < 2; ++half) {
-                const float2 *wt = wts + tok + 4 * half;
-                const int n = count - 4 * half;
-                if (free8 || (n >= 4 && tail_safe(t.safe4, t.s))) {
-                    f32x2 w4[G][4];
-#pragma unroll
-                    for (int g = 0; g < G; ++g) {
-                        const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(wt + g * kTileTok);
-                        const ulonglong2 y = *reinterpret_cast<const ulonglong2 *>(wt + g * kTileTok + 2);
-                        w4[g][0] = x.x; w4[g][1] = x.y; w4[g][2] = y.x; w4[g][3] = y.y;
-                    }
-                    x_tail_block<BITS>(grp, fc, t.s, t.zp, t, aE, [&](auto kc, const f32x2 (&xh)[2]) {
-#pragma unroll
-                        for (int g = 0; g < G; ++g)
-#pragma unroll
-                            for (int p = 0; p < 2; ++p) acc[g][p] = fma2(w4[g][decltype(kc)::value], xh[p], acc[g][p]);
-                    });
-                } else {
-#pragma unroll 1
-                    for (int j = 0; j < 4 && j < n; ++j) {
-                        f32x2 xh[2];
-                        x_tail_guarded<BITS>(grp, j, t.s, t.zp, t.alpha, slow, a.smin, a.smax, xh);
-#pragma unroll
-                        for (int g = 0; g < G; ++g) {
-                            const f32x2 w1 = *reinterpret_cast<const f32x2 *>(wt + g * kTileTok + j);
-                            acc[g][0] = fma2(w1, xh[0], acc[g][0]);
-                            acc[g][1] = fma2(w1, xh[1], acc[g][1]);
-                        }
-                    }
-                }
-#pragma unroll
-                for (int c = 0; c < 4; ++c) grp[c] >>= 4 * BITS;
-            }
-        };
-        scan(
-            [&](const float (&corr)[G]) {
-#pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    const f32x2 f = pk2(corr[g], corr[g]);
-                    acc[g][0] = mul2(acc[g][0], f);
-                    acc[g][1] = mul2(acc[g][1], f);
-                }
-            },
-            [&](const uint4 *tile, int ntok) { walk_tile<BITS>(tile, ntok, body); }, t.s, t.drift);
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            upk2(acc[g][0], out[g][0], out[g][1]);
-            upk2(acc[g][1], out[g][2], out[g][3]);
-        }
+        if (!(ok = ring.wait_short(i))) break;
+        const uint4 *tile = ring.tile(i, lane);
+        if (ntok == kTileTok) walk_full_tile<BITS>(tile, chunk);
+        else walk_tile<BITS>(tile, ntok, slow_chunk);
+        if ((i + 1) % kDriftTiles == 0) correct_drift(s, t.drift);
+        ring.release_and_refill(i, lane);   // also orders this tile's reads of wts before the next fill
     }
     if (!ok) {
         ring.drain(i);
-        store.give_up(c0);
         return;
     }
-    src.close();
-    if (seg.append) {
-        float w_self[G], xh[4];
-        if (!src.self(ring.n_tiles, a.T, out, w_self)) {
-            store.give_up(c0);
-            return;
-        }
-        append_from_tail<BITS>(a.p, poff, a.tail + size_t(bh) * 2 * kD, a.tail_keep, a.x_new + size_t(bh) * kD + c0,
-                               reinterpret_cast<uint4 *>(stream + size_t(a.T / C::TPW) * (kD * 4)) + lane, a.T, a.smin,
-                               a.smax, seg.ckpt_out, c0, xh);
+    // sum_k tc^k * (acc_k - alpha * accp_k) + W * zp_T; the constants are loaded again rather than kept
+    float out[4];
+    load_tail_chan<BITS>(t, a.p, poff, nullptr, c0, a.smin, a.smax, slow);
+    const f32x2 minus = pk2(-1.f, -1.f);
 #pragma unroll
-        for (int g = 0; g < G; ++g)
+    for (int p = 0; p < 2; ++p) {
+        const f32x2 nal = mul2(t.alpha[p], minus);
+        f32x2 sum = fma2(nal, accp[0][p], acc[0][p]);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) out[g][c] = fmaf(w_self[g], xh[c], out[g][c]);
-    } else {
-        if constexpr (!PREFIX) store_end_zp(store, t.zp, c0, 0);
+        for (int k = 1; k < 4; ++k) sum = fma2(t.e[k - 1][p], fma2(nal, accp[k][p], acc[k][p]), sum);
+        upk2(sum, out[2 * p], out[2 * p + 1]);
     }
-    store.store(src.m, src.l, out, c0);
+    if (a.T > 0) {
+        const float4 zp = *reinterpret_cast<const float4 *>(tail + c0);
+        out[0] = fmaf(src.l, zp.x, out[0]);
+        out[1] = fmaf(src.l, zp.y, out[1]);
+        out[2] = fmaf(src.l, zp.z, out[2]);
+        out[3] = fmaf(src.l, zp.w, out[3]);
+    }
+    float w_self, xh[4];
+    if (!src.self(ring.n_tiles, a.T, out, w_self)) return;
+    append_from_tail<BITS>(a.p, poff, tail, a.tail_keep, a.x_new + size_t(bh) * kD + c0,
+                           reinterpret_cast<uint4 *>(stream + size_t(a.T / C::TPW) * (kD * 4)) + lane, a.T, a.smin, a.smax,
+                           c0, xh);
+    const float inv = 1.0f / src.l;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) out[c] = fmaf(w_self, xh[c], out[c]) * inv;
+    store_half4(a.out + size_t(bh) * kD + c0, out);
 }
-
-// Normalised fp16 result of a whole stream.
-template <int G>
-struct TailStore {
-    __half *out;      // [G][kD] of this stream
-    __device__ __forceinline__ void store(const float (&)[G], const float (&l)[G], const float (&acc)[G][4], int c0) const
-    {
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            const float inv = 1.0f / l[g];
-            float o[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) o[c] = acc[g][c] * inv;
-            store_half4(out + size_t(g) * kD + c0, o);
-        }
-    }
-    __device__ __forceinline__ void give_up(int) const {}
-};
 
 }  // namespace adkv
