@@ -22,6 +22,7 @@ from __future__ import annotations
 import collections
 import ctypes
 
+import numpy as np
 import torch
 
 from . import _lib
@@ -291,11 +292,24 @@ class LayerSet:
             d.kp, d.vp = kp, vp
             d.k_tail, d.v_tail = _tail_ptr(kt, self.B, self.H, self.D), _tail_ptr(vt, self.B, self.H, self.D)
             self._keep.append((kc, vc, kt, vt, keep_k, keep_v))
+        self.has_tails = all(d.k_tail and d.v_tail for d in self.desc)
+        # the same memory as 64-bit words, one row per layer: the new tokens' pointers are written as two columns
+        words = np.frombuffer(self.desc, dtype=np.uint64).reshape(self.n, ctypes.sizeof(_lib.LayerKV) // 8)
+        self._k_col, self._v_col = words[:, _lib.LayerKV.k.offset // 8], words[:, _lib.LayerKV.v.offset // 8]
+        self._layer_index = np.arange(self.n, dtype=np.uint64)
 
     def _bind_new(self, k_new, v_new, tokens_dims):
         """Point the descriptors at the new tokens: two lists of per-layer tensors, or two stacked tensors
         ``[n_layers, B, H, ...]``."""
         _require(len(k_new) == self.n and len(v_new) == self.n, "one K and one V tensor per layer")
+        stacked = isinstance(k_new, torch.Tensor) and isinstance(v_new, torch.Tensor)
+        if stacked and k_new.is_contiguous() and v_new.is_contiguous():
+            # two buffers: their layers lie at a fixed distance, so nothing has to be asked of each layer's slice
+            for x, col in ((k_new, self._k_col), (v_new, self._v_col)):
+                _require(x.dtype == torch.float16 and x.is_cuda, "new tokens must be float16 CUDA tensors")
+                _require(x.numel() == self.n * tokens_dims, "new tokens have the wrong shape")
+                np.add(self._layer_index * np.uint64(2 * tokens_dims), np.uint64(x.data_ptr()), out=col)
+            return k_new, v_new
         keep = []
         for i in range(self.n):
             for x in (k_new[i], v_new[i]):
@@ -331,7 +345,7 @@ def append_kv_layers(layer_set: LayerSet, k_new, v_new, T: int, scale_min, scale
     tensor stacked along a leading layer axis, e.g. one ``[n_layers, B, nh, DIM]`` buffer the layers wrote into)."""
     ls = layer_set
     _require(T >= 0 and T // (32 // ls.bits) < ls.n_super_cap, f"cache has no free supergroup to append token {T}")
-    _require(all(ls.desc[i].k_tail and ls.desc[i].v_tail for i in range(ls.n)), "append needs the tail states")
+    _require(ls.has_tails, "append needs the tail states")
     keep = ls._bind_new(k_new, v_new, ls.B * ls.H * ls.D)
     with _on_device(ls.device):
         rc = _lib.load().adkv_append_kv_layers(ctypes.addressof(ls.desc), ls.n, ls.B, ls.H, T, ls.D, ls.n_super_cap,
