@@ -1,4 +1,5 @@
-"""Decode steps over token segments (launches with few streams, next to tail states) against the oracle.  Needs a B200.
+"""Decode steps next to tail states against the oracle, over token segments (launches with few streams) and with one
+warp pair per stream.  Needs a B200.
 
 Sizes are the edges of the split: no token, fewer tiles than segments, whole tiles, one token more or less; scales that
 never clamp, clamp at one bound, at both, and start outside the bounds.
@@ -32,12 +33,13 @@ def _clamping(case, kind):
         case[n] = (zp, sc, al, be, tg)
 
 
+@pytest.mark.parametrize("split", [None, False], ids=["segments", "whole_head"])
 @pytest.mark.parametrize("clamp", ["none", "pinned_low", "both", "start_outside", "odd_factor"])
 @pytest.mark.parametrize("B,Hq,Hkv,T,bits", [
     (1, 2, 2, 0, 4), (1, 2, 2, 1, 2), (2, 2, 2, 31, 4), (1, 4, 2, 32, 4), (1, 4, 1, 33, 2), (2, 2, 2, 255, 4), (1, 2, 1, 256, 2),
     (1, 2, 2, 257, 4), (1, 8, 2, 290, 2), (1, 2, 2, 777, 2), (2, 4, 2, 1031, 4),
 ])
-def test_segments_against_oracle(B, Hq, Hkv, T, bits, clamp):
+def test_against_oracle(B, Hq, Hkv, T, bits, clamp, split):
     case = make_case(500 + T, B, Hq, Hkv, T, bits)
     _clamping(case, clamp)
     dk, dv, tk, tv, ok_, ov_, sk, sv = _prefill(case, T + 1)
@@ -52,7 +54,7 @@ def test_segments_against_oracle(B, Hq, Hkv, T, bits, clamp):
                                scale_min=SMIN, scale_max=SMAX)
         got = gemv.decode_attn(dev(case["q"]), dk, dv, dev(kn[:, :, None]), dev(vn[:, :, None]), dev(case["kp"]), dev(case["vp"]),
                                T, 0.07, SMIN, SMAX, mask=None if m is None else dev(m), bits=bits, k_tail=tk, v_tail=tv,
-                               tail_keep=name == "mask")
+                               tail_keep=name == "mask", split_channels=split)
         _status_ok()
         np.testing.assert_allclose(got.float().cpu().numpy(), want, rtol=RTOL, atol=ATOL)
         assert np.array_equal(dk.cpu().numpy(), ok2) and np.array_equal(dv.cpu().numpy(), ov2)
@@ -84,3 +86,35 @@ def test_segments_varlen(bits):
                                   SMAX, bits=bits, k_tail=tk, v_tail=tv)
     _status_ok()
     np.testing.assert_allclose(got.float().cpu().numpy(), want.float().cpu().numpy(), rtol=RTOL, atol=ATOL)
+
+
+def test_layered_append_forms():
+    """33 layers (one more than a launch takes): stacked buffers, lists of tensors and pointers that are only aligned to
+    their type give the bytes and states of one append per layer."""
+    L, B, H, D, T, bits = 33, 1, 3, 128, 37, 4
+    g = torch.Generator(device="cuda").manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    shape = (L, B, H, orc.n_super_for(T + 1, bits), D // 4, 4, 4)
+    base = torch.randint(0, 256, shape, generator=g, device="cuda", dtype=torch.uint8)
+    tails = rnd(2, L, B, H, 2, D)
+    tails[:, :, :, :, 1] = tails[:, :, :, :, 1].abs() + 0.1
+    params = [[tuple(t.half().abs() * 0.3 for t in rnd(5, H, D)) for _ in range(2)] for _ in range(L)]
+    x = rnd(2, L, B, H, D).half()
+
+    def fresh():
+        return base.clone(), base.clone(), tails[0].clone(), tails[1].clone()
+
+    kc, vc, kt, vt = want = fresh()
+    for i in range(L):
+        gemv.append_kv_pair(kc[i], x[0, i][:, :, None], params[i][0], kt[i], vc[i], x[1, i][:, :, None], params[i][1], vt[i], T,
+                            SMIN, SMAX, bits=bits)
+    odd = torch.empty(x.numel() + 1, dtype=torch.float16, device="cuda")[1:].view_as(x)   # 2 bytes off
+    odd.copy_(x)
+    for k, v in ((x[0], x[1]), (list(x[0].unbind()), list(x[1].unbind())), (odd[0], odd[1])):
+        kc, vc, kt, vt = got = fresh()
+        ls = gemv.LayerSet([(kc[i], params[i][0], kt[i], vc[i], params[i][1], vt[i]) for i in range(L)], bits=bits)
+        gemv.append_kv_layers(ls, k, v, T, SMIN, SMAX)
+        for a, b in zip(got, want):
+            assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+    with pytest.raises(RuntimeError, match="wrong shape"):
+        gemv.append_kv_layers(ls, x[0, :, :, :2].contiguous(), x[1], T, SMIN, SMAX)
