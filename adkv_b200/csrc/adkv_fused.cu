@@ -126,8 +126,11 @@ ADKV_HIDDEN int adkv_wide_decode_attn(const KArgs &ka, const VArgs &va, const fl
 
 ADKV_DEFINE_TU_STATUS(adkv_tu_status_fused)
 
-// Token segments of a stream side by side (adkv_segments.cu): up to this many streams per launch.
-constexpr long long kSegmentsMaxStreams = 148;
+// Token segments of a stream side by side (adkv_segments.cu), next to tail states: up to two streams per SM.  Measured on
+// a B200 there (256 streams): 88 us against 92 us with one pair per stream for one query head per KV head, 258 us against
+// 307 us for four.  From three streams per SM on the schedulers are busy without segments (12 x 32 streams of 2000
+// tokens, two rounds of segments: 137 us against 131 us).
+constexpr long long kSegmentsMaxStreams = 296;
 
 static bool use_segments(const KArgs &ka, int B, bool exact, unsigned flags)
 {

@@ -1,7 +1,7 @@
 // Part of libadkv_b200.so (sm_100a).  See include/adkv_b200.h for the contract of every entry point.
 //
 // Fused decode step for launches with few (batch, kv head) streams, next to tail states: the token axis of every stream
-// is cut into kSegPairs segments that run side by side in ONE CTA, a K and a V warp each.  Reached through
+// is cut into NS segments that run side by side in ONE CTA, a K and a V warp each.  Reached through
 // adkv_decode_attn and adkv_decode_attn_varlen.
 //
 // What bounds a step with few streams is one warp's dependent instruction stream: a K/V pair walks its stream at about
@@ -13,40 +13,46 @@
 //     arithmetic of a scan, no clamps);
 //  2. the states at the segment starts follow from the products of the segments before.  If some segment, from the state
 //     it really starts with, may have met a clamp (rarely: the extremes, widened by the worst case of four tokens, reach
-//     a bound), all segments of the stream are gone through once more with clamps (scale_map), still side by side;
+//     a bound), all segments of that tensor are gone through once more with clamps (scale_map), still side by side;
 //  3. the scans run with zero points relative to the segment start.  For K that shifts every logit of a segment by one
 //     number, sum_c q_c * zp_c(start), for V it leaves out (sum of weights) * zp(start): both are put back
 //  4. when the partial softmax results of the segments are merged in shared memory.
 //
-// Only the appended token needs the encoder's exact state, and that comes from the tail.
-// @MEASURED@
+// Only the appended token needs the encoder's exact state, and that comes from the tail.  Steps 1 and 2 add about a third
+// to the work, so this pays only while a stream per warp pair leaves schedulers idle.
+//
+// Measured on a B200, one pair per stream (or the split head of adkv_narrow.cu) -> segments, 32 query heads: 4-bit, batch 4
+// x 2047 tokens 104 -> 48 us; batch 1 x 4000 tokens 195 -> 85 us; batch 8 x 2000 tokens 106 (92 with adkv_tailscan.cuh)
+// -> 88 us.  8 KV heads: 2-bit, batch 4 / 16 / 32 x 4000 tokens 286 / 305 / 307 -> 127 / 131 / 258 us, batch 32 x 32768
+// tokens 2436 -> 1948 us; 4-bit, batch 30 x 4000 tokens 336 -> 250 us.
 #include "adkv_host.h"
 
 #include "adkv_tailscan.cuh"
 
 namespace adkv {
 
-constexpr int kSegPairs = 8;      // segments per stream; 16 warps keep the four schedulers of an SM busy
 constexpr int kSegStages = 2;     // bulk-copy ring depth per warp
 constexpr int kPartFloats = 4 + kD;   // per (segment, head): maximum (log2 units), denominator, 2 pad, kD sums
 
-template <int BITS, int G>
+// NS: segments per stream
+template <int BITS, int G, int NS>
 struct SegShared {
-    alignas(128) uint8_t buf[2][kSegPairs][kSegStages * Tile<BITS>::BYTES];
-    alignas(16) float red[kSegPairs][G == 1 ? kRedFloats : G * 8 * 36];
-    alignas(16) float2 wts[kSegPairs][G * kTileTok];
-    alignas(16) float4 slow[kSegPairs][2 * 32];          // one head: constants of the K scans' guarded bodies
+    alignas(128) uint8_t buf[2][NS][kSegStages * Tile<BITS>::BYTES];
+    alignas(16) float red[NS][G == 1 ? kRedFloats : G * 8 * 36];
+    alignas(16) float2 wts[NS][G * kTileTok];
+    alignas(16) float4 slow[NS][2 * 32];          // one head: constants of the K scans' guarded bodies
     union {
-        alignas(16) float comp[2][kSegPairs][3][kD];     // steps 1 and 2: product, smallest and largest running product
-        alignas(16) float part[kSegPairs][G][kPartFloats];   // steps 3 and 4
+        alignas(16) float comp[2][NS][3][kD];     // steps 1 and 2: product, smallest and largest running product
+        alignas(16) float part[NS][G][kPartFloats];   // steps 3 and 4
     };
-    alignas(16) float init[2][kSegPairs][2][kD];         // zero point (relative) and scale at the segment starts
-    alignas(16) float zp_end[kSegPairs][kD];             // V: zero points after the segment, relative to its start
+    alignas(16) float init[2][NS][2][kD];         // zero point (relative) and scale at the segment starts
+    alignas(16) float zp_end[NS][kD];             // V: zero points after the segment, relative to its start
     alignas(16) float self_x[kD];                        // V: dequantised appended token
-    float z_end[kSegPairs][G];                           // K: sum_c q_c * zp_c after the segment, relative
+    float z_end[NS][G];                           // K: sum_c q_c * zp_c after the segment, relative
     float self_logit[G];
-    FusedShared<G> fs[kSegPairs];
-    uint64_t bar[2][kSegPairs][kSegStages];
+    int clamps[2];                                       // step 2: a segment of K / of V may have met a clamp
+    FusedShared<G> fs[NS];
+    uint64_t bar[2][NS][kSegStages];
 };
 
 template <int G>
@@ -103,6 +109,25 @@ struct SegSrc : SoftmaxSrc<G> {
 struct ScaleConst {
     f32x2 beta[2], tc[2];
 };
+
+// Interval that the scales at every fourth token (start and end included) have to lie in for the unclamped trajectory
+// between them to stay inside the bounds, for all four channels of a lane: at most four updates after one of them and at
+// most four before the next, whichever says more (for 2-bit codes the latter: a scale falls by 2.5 % a token at most but
+// grows by 7.5 %, so the upper bound is 0.90 * smax instead of 0.75 * smax).
+__device__ __forceinline__ SafeRange block_range(const float (&beta)[4], const float (&target)[4], int bias, float smin, float smax)
+{
+    SafeRange r{0.f, INFINITY};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const float g0 = 1.f - beta[c] * target[c], g1 = g0 + beta[c] * float(bias);
+        const float gmn = fminf(fminf(g0, g1), 1.f), gmx = fmaxf(fmaxf(g0, g1), 1.f);
+        const float pmn = gmn * gmn * gmn * gmn, pmx = gmx * gmx * gmx * gmx;
+        r.lo = fmaxf(r.lo, gmn > 0.f ? fmaxf(smin, kEps) * fminf(__fdividef(1.f, pmn), pmx) * (1.f + 2e-5f) : INFINITY);
+        r.hi = fminf(r.hi, smax * fmaxf(__fdividef(1.f, pmx), pmn) * (1.f - 2e-5f));
+    }
+    if (!(r.lo <= r.hi)) { r.lo = INFINITY; r.hi = 0.f; }
+    return r;
+}
 
 // Step 1: product of the factors of `n_words` words of a stream and the extremes of the running product at every
 // fourth token (1 at the start included).  src: this lane's vector of the first word.
@@ -197,13 +222,13 @@ __device__ __noinline__ void scale_map(const uint4 *src, int n_words, const Scal
         *reinterpret_cast<ulonglong2 *>(comp + r * (kD / 4)) = make_ulonglong2(rows[r][0], rows[r][1]);
 }
 
-template <int BITS, int G>
-__global__ void __launch_bounds__(64 * kSegPairs, 1)
+template <int BITS, int G, int NS>
+__global__ void __launch_bounds__(64 * NS, 8 / NS)
     decode_attn_segments_kernel(KArgs ka, VArgs va, const float *__restrict__ mask, long long mask_stride_b, float scaling,
                                 const int *__restrict__ seq_lens)
 {
     extern __shared__ uint8_t smem_raw[];
-    SegShared<BITS, G> &sh = *reinterpret_cast<SegShared<BITS, G> *>(smem_raw);
+    SegShared<BITS, G, NS> &sh = *reinterpret_cast<SegShared<BITS, G, NS> *>(smem_raw);
     using C = Codec<BITS>;
     const int bh = blockIdx.x, b = bh / ka.Hkv, h = bh % ka.Hkv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -219,7 +244,8 @@ __global__ void __launch_bounds__(64 * kSegPairs, 1)
         ka.T = T;
         va.T = T;
     }
-    if (threadIdx.x < kSegPairs) {
+    if (threadIdx.x < 2) sh.clamps[threadIdx.x] = 0;
+    if (threadIdx.x < NS) {
         for (int r = 0; r < 2; ++r)
             for (int i = 0; i < kSegStages; ++i) mbar_init(&sh.bar[r][threadIdx.x][i], 1);
         sh.fs[threadIdx.x].init_barriers(1);
@@ -227,7 +253,7 @@ __global__ void __launch_bounds__(64 * kSegPairs, 1)
         mbar_init_fence();
     }
     const int T = ka.T, n_tiles = (T + kTileTok - 1) / kTileTok;
-    const int per_seg = (n_tiles + kSegPairs - 1) / kSegPairs * kTileTok;
+    const int per_seg = (n_tiles + NS - 1) / NS * kTileTok;
     const int t_begin = min(seg * per_seg, T), t_end = min(t_begin + per_seg, T);
     const ParamPtrs &p = role ? va.p : ka.p;
     const int c0 = 4 * lane;
@@ -237,12 +263,12 @@ __global__ void __launch_bounds__(64 * kSegPairs, 1)
 
     // 1. products of all segments that another one follows (those are whole tiles)
     ScaleConst sc;
-    SafeRange safe8, safe4;   // safe8: not used
+    SafeRange range;
     float s[4];
     const bool followed = t_end < T;
     {
         Chan ch[4];
-        load_chan4<BITS, true>(ch, safe8, p, poff, ka.smin, ka.smax);
+        load_chan4<BITS, true>(ch, range, p, poff, ka.smin, ka.smax);
         float be[4], tg[4], tc[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -251,7 +277,7 @@ __global__ void __launch_bounds__(64 * kSegPairs, 1)
             tc[c] = fmaf(-be[c], tg[c], 1.0f);
             s[c] = ch[c].s;
         }
-        safe4.template init<BITS, 4, 4>(be, tg, ka.smin, ka.smax);
+        range = block_range(be, tg, C::BIAS, ka.smin, ka.smax);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             sc.beta[q] = pk2(be[2 * q], be[2 * q + 1]);
@@ -275,20 +301,23 @@ __global__ void __launch_bounds__(64 * kSegPairs, 1)
         const float4 F = *reinterpret_cast<const float4 *>(&sh.comp[role][i][0][c0]);
         const float4 mn = *reinterpret_cast<const float4 *>(&sh.comp[role][i][1][c0]);
         const float4 mx = *reinterpret_cast<const float4 *>(&sh.comp[role][i][2][c0]);
-        const bool ok = s[0] * mn.x >= safe4.lo && s[1] * mn.y >= safe4.lo && s[2] * mn.z >= safe4.lo && s[3] * mn.w >= safe4.lo &&
-                        s[0] * mx.x <= safe4.hi && s[1] * mx.y <= safe4.hi && s[2] * mx.z <= safe4.hi && s[3] * mx.w <= safe4.hi;
+        const bool ok = s[0] * mn.x >= range.lo && s[1] * mn.y >= range.lo && s[2] * mn.z >= range.lo && s[3] * mn.w >= range.lo &&
+                        s[0] * mx.x <= range.hi && s[1] * mx.y <= range.hi && s[2] * mx.z <= range.hi && s[3] * mx.w <= range.hi;
         proven = __all_sync(kFull, ok);
         s[0] *= F.x; s[1] *= F.y; s[2] *= F.z; s[3] *= F.w;
     }
-    if (__syncthreads_or(!proven)) {
+    if (!proven && lane == 0) sh.clamps[role] = 1;
+    __syncthreads();
+    if (sh.clamps[0] | sh.clamps[1]) {
+        const bool redo = sh.clamps[role] != 0;
         const float4 lo = seg ? make_float4(ka.smin, ka.smin, ka.smin, ka.smin) : start;
         const float4 hi = seg ? make_float4(ka.smax, ka.smax, ka.smax, ka.smax) : start;
-        if (followed)
+        if (followed && redo)
             scale_map<BITS>(words, per_seg / C::TPW, sc, ka.smin, ka.smax, lo, hi,
                             reinterpret_cast<float4 *>(&sh.comp[role][seg][0][c0]));
         __syncthreads();
-        s[0] = start.x; s[1] = start.y; s[2] = start.z; s[3] = start.w;
-        for (int i = 0; i < seg && !empty; ++i) {
+        if (redo) { s[0] = start.x; s[1] = start.y; s[2] = start.z; s[3] = start.w; }
+        for (int i = 0; i < seg && redo && !empty; ++i) {
             const float4 F = *reinterpret_cast<const float4 *>(&sh.comp[role][i][0][c0]);
             const float4 l = *reinterpret_cast<const float4 *>(&sh.comp[role][i][1][c0]);
             const float4 u = *reinterpret_cast<const float4 *>(&sh.comp[role][i][2][c0]);
@@ -360,13 +389,13 @@ __global__ void __launch_bounds__(64 * kSegPairs, 1)
 
     // 4. merge: segment maxima shifted by the zero points K left out, sums completed with those V left out
     const float mk = mask_row ? mask_row[T] * 1.4426950408889634f : 0.f;
-    for (int i = threadIdx.x; i < G * kD; i += 64 * kSegPairs) {
+    for (int i = threadIdx.x; i < G * kD; i += 64 * NS) {
         const int g = i / kD, c = i % kD;
-        float m[kSegPairs], z = 0.f;
+        float m[NS], z = 0.f;
         const float v = fmaf(sh.self_logit[g], scale2, mk);
         float M = v;
 #pragma unroll
-        for (int j = 0; j < kSegPairs; ++j) {
+        for (int j = 0; j < NS; ++j) {
             m[j] = sh.part[j][g][0];
             if (m[j] != -INFINITY) m[j] = fmaf(z, scale2, m[j]);
             z += sh.z_end[j][g];
@@ -376,7 +405,7 @@ __global__ void __launch_bounds__(64 * kSegPairs, 1)
         const float w_self = dead ? 0.f : exp2f(v - M);
         float L = w_self, A = w_self * sh.self_x[c], zp = 0.f;
 #pragma unroll
-        for (int j = 0; j < kSegPairs; ++j) {
+        for (int j = 0; j < NS; ++j) {
             const float w = m[j] == -INFINITY ? 0.f : exp2f(m[j] - M);
             const float l = sh.part[j][g][1];
             L = fmaf(l, w, L);
@@ -393,17 +422,17 @@ using namespace adkv;
 
 ADKV_DEFINE_TU_STATUS(adkv_tu_status_segments)
 
-template <int BITS, int G>
+template <int BITS, int G, int NS>
 static int launch_segments(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b, float scaling, int B,
                            const int *seq_lens, cudaStream_t s)
 {
-    constexpr int bytes = int(sizeof(SegShared<BITS, G>));
+    constexpr int bytes = int(sizeof(SegShared<BITS, G, NS>));
     static_assert(bytes <= 227 * 1024, "shared memory of one CTA");
     // per device and process: cheap enough (a host-side call) to be made before every launch
-    const cudaError_t e = cudaFuncSetAttribute(decode_attn_segments_kernel<BITS, G>,
+    const cudaError_t e = cudaFuncSetAttribute(decode_attn_segments_kernel<BITS, G, NS>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return int(e);
-    decode_attn_segments_kernel<BITS, G><<<B * ka.Hkv, 64 * kSegPairs, bytes, s>>>(ka, va, mask, mask_stride_b, scaling, seq_lens);
+    decode_attn_segments_kernel<BITS, G, NS><<<B * ka.Hkv, 64 * NS, bytes, s>>>(ka, va, mask, mask_stride_b, scaling, seq_lens);
     return launch_status();
 }
 
@@ -411,13 +440,17 @@ static int launch_segments(const KArgs &ka, const VArgs &va, const float *mask, 
 ADKV_HIDDEN int adkv_segments_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b,
                                           float scaling, int B, int bits, const int *seq_lens, cudaStream_t s)
 {
+    // One stream per SM: sixteen warps each.  More: two CTAs of eight warps share an SM (two rounds of sixteen warps take
+    // as long as twice the time of 148 streams: batch 8 x 2000 tokens, 32 heads, 94 us against 88 us).
+    const bool wide = (long long)B * ka.Hkv <= 148;
     switch (bits * 16 + ka.Hq / ka.Hkv) {
-    case 4 * 16 + 1: return launch_segments<4, 1>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
-    case 4 * 16 + 2: return launch_segments<4, 2>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
-    case 4 * 16 + 4: return launch_segments<4, 4>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
-    case 2 * 16 + 1: return launch_segments<2, 1>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
-    case 2 * 16 + 2: return launch_segments<2, 2>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
-    case 2 * 16 + 4: return launch_segments<2, 4>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
+#define ADKV_SEG_CASE(BITS_, G_)                                                                                            \
+    case BITS_ * 16 + G_:                                                                                                   \
+        return wide ? launch_segments<BITS_, G_, 8>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s)                   \
+                    : launch_segments<BITS_, G_, 4>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
+        ADKV_SEG_CASE(4, 1) ADKV_SEG_CASE(4, 2) ADKV_SEG_CASE(4, 4)
+        ADKV_SEG_CASE(2, 1) ADKV_SEG_CASE(2, 2) ADKV_SEG_CASE(2, 4)
+#undef ADKV_SEG_CASE
     default: return ADKV_E_SHAPE;
     }
 }
