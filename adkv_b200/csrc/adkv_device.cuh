@@ -267,6 +267,10 @@ struct SafeRange {
         const float mx = fmaxf(fmaxf(fmaxf(ch[0].s, ch[1].s), ch[2].s), ch[3].s);
         return __all_sync(kFull, mn >= lo && mx <= hi);
     }
+    __device__ __forceinline__ bool holds(const Chan (&ch)[1]) const
+    {
+        return __all_sync(kFull, ch[0].s >= lo && ch[0].s <= hi);
+    }
     __device__ __forceinline__ bool holds(const Chan (&ch)[2]) const
     {
         return __all_sync(kFull, fminf(ch[0].s, ch[1].s) >= lo && fmaxf(ch[0].s, ch[1].s) <= hi);

@@ -78,6 +78,29 @@ __device__ __forceinline__ bool encode_group(const __half2 *xin /* 8 rows of kD/
     return doubt;
 }
 
+// The same for the one channel of a thread (launches with few streams, see launch_encode): every operation rounded as in
+// encode_group.  xin: 8 rows of kD.
+template <int BITS, bool GUARDED>
+__device__ __forceinline__ bool encode_group(const __half *xin, Chan (&ch)[1], uint32_t (&word)[1], float smin, float smax, f32x2)
+{
+    using C = Codec<BITS>;
+    constexpr float M = 12582912.f + float(C::BIAS);
+    Chan &c = ch[0];
+    bool doubt = !(c.s < 1e29f);
+    static_for<8>([&](auto jc) {
+        const float x = __half2float(xin[decltype(jc)::value * kD]);
+        const float ss = GUARDED ? fmaxf(c.s, kEps) : c.s;
+        float inv;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(ss));
+        const float v = fminf(fmaxf(__fmul_rn(__fsub_rn(x, c.zp), inv), C::qlo()), C::qhi());
+        const float t = __fadd_rn(v, M), q = __fsub_rn(t, M);
+        doubt |= !(fabsf(__fsub_rn(v, q)) < 0.5f - 4e-6f);
+        advance_canonical_g<GUARDED>(q, __fmul_rn(q, ss), c, smin, smax);
+        word[0] = __funnelshift_r(word[0], __float_as_uint(t), BITS);
+    });
+    return doubt;
+}
+
 // One tensor (K or V) of a launch; blockIdx.y selects it, so K and V of a layer are quantised side by side.
 struct EncTensor {
     uint32_t *cache;
@@ -96,40 +119,70 @@ struct EncBatch {
     EncTensor t[kEncMaxTensors];
 };
 
-// WIDE = false: head dim 128, all strides are compile-time constants.
-template <int BITS, bool WIDE>
-__global__ void __launch_bounds__(kEncThreads) encode_kernel(EncBatch batch, CkptSpec cs, int H, int T,
+// WIDE = false: head dim 128, all strides are compile-time constants.  CPT: channels per thread, 2 or 1.
+template <int CPT>
+struct EncIo;    // a thread's channels of a row: half inputs, packed words, float states
+template <>
+struct EncIo<2> {
+    using Half = __half2;
+    using Word = uint2;
+    using Float = float2;
+    __device__ static void get(float2 v, float (&o)[2]) { o[0] = v.x; o[1] = v.y; }
+    __device__ static void get(__half2 v, float (&o)[2]) { get(__half22float2(v), o); }
+    __device__ static void get(uint2 v, uint32_t (&o)[2]) { o[0] = v.x; o[1] = v.y; }
+    __device__ static uint2 word(const uint32_t (&w)[2]) { return make_uint2(w[0], w[1]); }
+    __device__ static float2 zp(const Chan (&c)[2]) { return make_float2(c[0].zp, c[1].zp); }
+    __device__ static float2 scale(const Chan (&c)[2]) { return make_float2(c[0].s, c[1].s); }
+};
+template <>
+struct EncIo<1> {
+    using Half = __half;
+    using Word = uint32_t;
+    using Float = float;
+    __device__ static void get(float v, float (&o)[1]) { o[0] = v; }
+    __device__ static void get(__half v, float (&o)[1]) { o[0] = __half2float(v); }
+    __device__ static void get(uint32_t v, uint32_t (&o)[1]) { o[0] = v; }
+    __device__ static uint32_t word(const uint32_t (&w)[1]) { return w[0]; }
+    __device__ static float zp(const Chan (&c)[1]) { return c[0].zp; }
+    __device__ static float scale(const Chan (&c)[1]) { return c[0].s; }
+};
+
+template <int BITS, bool WIDE, int CPT>
+__global__ void __launch_bounds__(kD / CPT) encode_kernel(EncBatch batch, CkptSpec cs, int H, int T,
                                                              int n_super_cap, int t_start, float smin, float smax)
 {
     using C = Codec<BITS>;
+    using Io = EncIo<CPT>;
+    using Half = typename Io::Half;
+    using Word = typename Io::Word;
+    using Float = typename Io::Float;
     const EncTensor &et = batch.t[blockIdx.y];
     uint32_t *__restrict__ cache = et.cache;
     const __half *__restrict__ x = et.x;
     const ParamPtrs p = et.p;
     float *__restrict__ tail = et.tail;
     const int D = WIDE ? cs.D : kD, S = WIDE ? D / kD : 1;
-    const int bh = blockIdx.x / S, h = bh % H, c0 = kD * (blockIdx.x % S) + 2 * threadIdx.x;   // c0: channel in the head
+    const int bh = blockIdx.x / S, h = bh % H, c0 = kD * (blockIdx.x % S) + CPT * threadIdx.x;   // c0: channel in the head
     const size_t po = size_t(h) * D + c0;
-    Chan ch[2];
-    float beta[2], target[2];
+    Chan ch[CPT];
+    float beta[CPT], target[CPT];
     {
-        const float2 al = __half22float2(*reinterpret_cast<const __half2 *>(p.alpha + po));
-        const float2 be = __half22float2(*reinterpret_cast<const __half2 *>(p.beta + po));
-        const float2 tg = __half22float2(*reinterpret_cast<const __half2 *>(p.target + po));
-        float2 zp, sc;
+        float al[CPT], zp[CPT], sc[CPT];
+        Io::get(*reinterpret_cast<const Half *>(p.alpha + po), al);
+        Io::get(*reinterpret_cast<const Half *>(p.beta + po), beta);
+        Io::get(*reinterpret_cast<const Half *>(p.target + po), target);
         if (t_start > 0) {
-            zp = *reinterpret_cast<const float2 *>(tail + size_t(bh) * 2 * D + c0);
-            sc = *reinterpret_cast<const float2 *>(tail + size_t(bh) * 2 * D + D + c0);
+            Io::get(*reinterpret_cast<const Float *>(tail + size_t(bh) * 2 * D + c0), zp);
+            Io::get(*reinterpret_cast<const Float *>(tail + size_t(bh) * 2 * D + D + c0), sc);
         } else {
-            zp = __half22float2(*reinterpret_cast<const __half2 *>(p.zp_init + po));
-            sc = __half22float2(*reinterpret_cast<const __half2 *>(p.scale_init + po));
+            Io::get(*reinterpret_cast<const Half *>(p.zp_init + po), zp);
+            Io::get(*reinterpret_cast<const Half *>(p.scale_init + po), sc);
         }
-        ch[0] = Chan{zp.x, sc.x, al.x, be.x, tg.x};
-        ch[1] = Chan{zp.y, sc.y, al.y, be.y, tg.y};
-        beta[0] = be.x; beta[1] = be.y; target[0] = tg.x; target[1] = tg.y;
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) ch[c] = Chan{zp[c], sc[c], al[c], beta[c], target[c]};
     }
     SafeRange safe;
-    safe.template init<BITS, 2>(beta, target, smin, smax);
+    safe.template init<BITS, CPT>(beta, target, smin, smax);
     const f32x2 one = opaque_ones2();
 
     __shared__ alignas(128) __half buf[kEncStages][32 * kD];
@@ -140,18 +193,18 @@ __global__ void __launch_bounds__(kEncThreads) encode_kernel(EncBatch batch, Ckp
     }
     __syncthreads();
 
-    uint2 *w = reinterpret_cast<uint2 *>(cache + size_t(bh) * n_super_cap * D + c0);       // stride D/2 per word row
-    const __half2 *xs = reinterpret_cast<const __half2 *>(x + size_t(bh) * T * D + c0);    // stride D/2 per token
-    const int RS = D / 2;          // row stride in global memory (uint2 words / half2 inputs)
-    constexpr int SRS = kD / 2;    // row stride of the staged slice in shared memory
+    Word *w = reinterpret_cast<Word *>(cache + size_t(bh) * n_super_cap * D + c0);   // stride RS per word row
+    const Half *xs = reinterpret_cast<const Half *>(x + size_t(bh) * T * D + c0);    // stride RS per token
+    const int RS = D / CPT;          // row stride in global memory (words / inputs of a thread)
+    constexpr int SRS = kD / CPT;    // row stride of the staged slice in shared memory
 
     // one token with a run-time field position, exactly rounded division (partial words, redone groups)
     // (the word is shifted, not indexed: see encode_group)
-    auto exact_token = [&](int t, uint32_t(&word)[2]) {
-        const float2 xv = __half22float2(xs[size_t(t - t_start) * RS]);
-        const float xa[2] = {xv.x, xv.y};
+    auto exact_token = [&](int t, uint32_t(&word)[CPT]) {
+        float xa[CPT];
+        Io::get(xs[size_t(t - t_start) * RS], xa);
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < CPT; ++c) {
             float rh;
             const float q = quantize<BITS>(xa[c], ch[c], rh);
             word[c] = __funnelshift_r(word[c], uint32_t(int(q) + C::BIAS), BITS);
@@ -166,8 +219,8 @@ __global__ void __launch_bounds__(kEncThreads) encode_kernel(EncBatch batch, Ckp
         if (t_reached == next_ckpt) {
             const int k = next_ckpt / cs.interval - 1;
             if (k < cs.n_ckpt_cap) {
-                *reinterpret_cast<float2 *>(ckpt + size_t(k) * 2 * D) = make_float2(ch[0].zp, ch[1].zp);
-                *reinterpret_cast<float2 *>(ckpt + size_t(k) * 2 * D + D) = make_float2(ch[0].s, ch[1].s);
+                *reinterpret_cast<Float *>(ckpt + size_t(k) * 2 * D) = Io::zp(ch);
+                *reinterpret_cast<Float *>(ckpt + size_t(k) * 2 * D + D) = Io::scale(ch);
             }
             next_ckpt += cs.interval;
         }
@@ -175,23 +228,25 @@ __global__ void __launch_bounds__(kEncThreads) encode_kernel(EncBatch batch, Ckp
 
     const int t_end = t_start + T;
     int t = t_start;
-    uint32_t word[2] = {0u, 0u};
+    uint32_t word[CPT] = {};
+    auto flush = [&](int at) {   // a word is complete
+        w[size_t(at / C::TPW) * RS] = Io::word(word);
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) word[c] = 0u;
+    };
     // a chunk that starts inside a word keeps the fields already there (moved to the top, where the shifting
     // assembly expects the tokens seen so far)
     if (t % C::TPW != 0 && t < t_end) {
-        const uint2 old = w[size_t(t / C::TPW) * RS];
+        Io::get(w[size_t(t / C::TPW) * RS], word);
         const int up = BITS * (C::TPW - t % C::TPW);
-        word[0] = old.x << up;
-        word[1] = old.y << up;
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) word[c] <<= up;
     }
     // tokens up to the next multiple of 8
     for (; t < t_end && t % 8 != 0; ++t) {
         exact_token(t, word);
         checkpoint(t + 1);
-        if ((t + 1) % C::TPW == 0) {
-            w[size_t(t / C::TPW) * RS] = make_uint2(word[0], word[1]);
-            word[0] = word[1] = 0u;
-        }
+        if ((t + 1) % C::TPW == 0) flush(t);
     }
     // Groups of 8 tokens.  The fp16 rows of the stream are contiguous, so they are staged through a
     // ring of 32-token tiles filled by bulk copies (1-D TMA, issued by thread 0) that run ahead of
@@ -224,23 +279,20 @@ __global__ void __launch_bounds__(kEncThreads) encode_kernel(EncBatch batch, Ckp
         const int ng = min(4, n_groups - 4 * i);
 #pragma unroll 1
         for (int g = 0; g < ng; ++g, t += 8) {
-            const __half2 *rows = reinterpret_cast<const __half2 *>(&buf[i % kEncStages][0]) + g * 8 * SRS + threadIdx.x;
-            const Chan saved[2] = {ch[0], ch[1]};
-            const uint32_t word_in[2] = {word[0], word[1]};
+            const Half *rows = reinterpret_cast<const Half *>(&buf[i % kEncStages][0]) + g * 8 * SRS + threadIdx.x;
+            Chan saved[CPT];
+            uint32_t word_in[CPT];
+#pragma unroll
+            for (int c = 0; c < CPT; ++c) { saved[c] = ch[c]; word_in[c] = word[c]; }
             const bool doubt = safe.holds(ch) ? encode_group<BITS, false>(rows, ch, word, smin, smax, one)
                                               : encode_group<BITS, true>(rows, ch, word, smin, smax, one);
             if (doubt) {   // rare, per thread: redo the group from the saved state with the exact quantiser
-                ch[0] = saved[0];
-                ch[1] = saved[1];
-                word[0] = word_in[0];
-                word[1] = word_in[1];
+#pragma unroll
+                for (int c = 0; c < CPT; ++c) { ch[c] = saved[c]; word[c] = word_in[c]; }
                 for (int j = 0; j < 8; ++j) exact_token(t + j, word);
             }
             checkpoint(t + 8);
-            if ((t + 8) % C::TPW == 0) {
-                w[size_t(t / C::TPW) * RS] = make_uint2(word[0], word[1]);
-                word[0] = word[1] = 0u;
-            }
+            if ((t + 8) % C::TPW == 0) flush(t);
         }
         __syncthreads();   // every thread is done with this stage
         if (threadIdx.x == 0 && i + kEncStages < n_tiles) issue(i + kEncStages);
@@ -252,11 +304,13 @@ __global__ void __launch_bounds__(kEncThreads) encode_kernel(EncBatch batch, Ckp
     }
     if (t % C::TPW != 0) {   // bring the tokens of the last, partial word down; its unused fields are zero
         const int down = BITS * (C::TPW - t % C::TPW);
-        w[size_t(t / C::TPW) * RS] = make_uint2(word[0] >> down, word[1] >> down);
+        #pragma unroll
+        for (int c = 0; c < CPT; ++c) word[c] >>= down;
+        w[size_t(t / C::TPW) * RS] = Io::word(word);
     }
     if (tail) {
-        *reinterpret_cast<float2 *>(tail + size_t(bh) * 2 * D + c0) = make_float2(ch[0].zp, ch[1].zp);
-        *reinterpret_cast<float2 *>(tail + size_t(bh) * 2 * D + D + c0) = make_float2(ch[0].s, ch[1].s);
+        *reinterpret_cast<Float *>(tail + size_t(bh) * 2 * D + c0) = Io::zp(ch);
+        *reinterpret_cast<Float *>(tail + size_t(bh) * 2 * D + D + c0) = Io::scale(ch);
     }
 }
 
@@ -392,12 +446,19 @@ static int launch_encode(const EncBatch &b, int n, int B, int H, int T, int D, i
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cs.D = D;
     const dim3 grid(B * H * (D / kD), n);
+    // One channel per thread while that leaves a warp scheduler at most two warps: a warp then has its scheduler (nearly)
+    // to itself and takes as long as its own instructions, of which one channel needs about half as many as a pair.
+    // Measured on a B200, K and V of 32 heads: 1 x 4000 tokens 251 -> 231 us, 2 x 2000 tokens 131 -> 121 us, 4 x 2000 tokens
+    // 137 -> 133 us.  With more streams the schedulers are busy and the packed pair needs fewer issue slots per channel.
+    const bool few = (long long)grid.x * grid.y * (kD / 32) <= 2 * 592;
     if (D == kD) {
-        if (bits == 4) encode_kernel<4, false><<<grid, kEncThreads, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
-        else encode_kernel<2, false><<<grid, kEncThreads, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
+        if (bits == 4 && few) encode_kernel<4, false, 1><<<grid, kD, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
+        else if (bits == 4) encode_kernel<4, false, 2><<<grid, kEncThreads, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
+        else if (few) encode_kernel<2, false, 1><<<grid, kD, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
+        else encode_kernel<2, false, 2><<<grid, kEncThreads, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
     } else {
-        if (bits == 4) encode_kernel<4, true><<<grid, kEncThreads, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
-        else encode_kernel<2, true><<<grid, kEncThreads, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
+        if (bits == 4) encode_kernel<4, true, 2><<<grid, kEncThreads, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
+        else encode_kernel<2, true, 2><<<grid, kEncThreads, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
     }
     return launch_status();
 }

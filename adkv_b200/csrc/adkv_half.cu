@@ -103,6 +103,7 @@ __global__ void __launch_bounds__(32 * kStreamsPerCta) forward_ov_half_kernel(VA
 #pragma unroll
     for (int g = 0; g < G; ++g) src.row[g] = attn + (size_t(b) * va.Hq + size_t(h) * G + g) * (va.T + 1);
     src.wts = wts[warp];
+    src.T = va.T;
     const Seg seg{0, va.T, true, nullptr, nullptr, 0};
     v_warp_h<BITS, G>(va, seg, b, h, lane, vbuf[warp], vbar[warp], wts[warp], src);
 }

@@ -22,18 +22,26 @@ struct GlobalLogitSink {
     __device__ __forceinline__ void finish(int) {}
 };
 
+// The weights of the next tile are fetched while the current one is replayed: with few streams a warp has its scheduler
+// to itself, and a load that is waited for at every tile (about 700 cycles against 1500 of replay) would be paid in full.
 template <int G, bool HALF_W = false>
 struct GlobalWeightSrc {
     const __half *row[G];   // attention weights of each q head of this stream: [T+1]
-    float2 *wts;   // every weight stored twice
-    __device__ __forceinline__ bool tile_weights(int i, int ntok, int lane, float (&)[G][4])
+    float2 *wts;            // every weight stored twice
+    int T;
+    __half next[G];
+    __device__ __forceinline__ void fetch(int i, int lane)
     {
+        const int t = i * kTileTok + lane;
 #pragma unroll
-        for (int g = 0; g < G; ++g)
-        {
-            const float wv = lane < ntok ? __half2float(row[g][i * kTileTok + lane]) : 0.f;
-            put_weight<HALF_W>(wts, g * kTileTok + lane, wv);
-        }
+        for (int g = 0; g < G; ++g) next[g] = t < T ? row[g][t] : __half(0.f);
+    }
+    __device__ __forceinline__ bool tile_weights(int i, int, int lane, float (&)[G][4])
+    {
+        if (i == 0) fetch(0, lane);
+#pragma unroll
+        for (int g = 0; g < G; ++g) put_weight<HALF_W>(wts, g * kTileTok + lane, __half2float(next[g]));
+        fetch(i + 1, lane);
         __syncwarp();
         return true;
     }

@@ -3,6 +3,7 @@
 #include "adkv_host.h"
 
 #include "adkv_io.cuh"
+#include "adkv_narrow.cuh"
 
 namespace adkv {
 
@@ -53,9 +54,41 @@ __global__ void __launch_bounds__(32 * kStreamsPerCta) forward_ov_kernel(VArgs v
 #pragma unroll
     for (int g = 0; g < G; ++g) src.row[g] = attn + (size_t(b) * va.Hq + size_t(h) * G + g) * (va.T + 1);
     src.wts = wts[warp];
+    src.T = va.T;
     const Seg seg{0, va.T, true, nullptr, nullptr, 0};
     v_warp<BITS, G, EXACT>(va, seg, b, h, lane, vbuf[warp], vbar[warp], wts[warp], src);
 }
+
+// forward_ov with few streams: two warps per stream, 64 channels each (adkv_narrow.cuh).  Output channels are independent,
+// so the two warps have nothing to exchange; what is repeated is the staging of the weights.
+template <int BITS, int G, bool EXACT>
+__global__ void __launch_bounds__(32 * kNarrowSlices) forward_ov_split_kernel(VArgs va, const __half *__restrict__ attn)
+{
+    constexpr int S = kNarrowSlices;
+    __shared__ alignas(128) uint8_t vbuf[S][kStages * NarrowTile<BITS>::BYTES];
+    __shared__ alignas(16) float2 wts[S][G * kTileTok];
+    __shared__ uint64_t vbar[S][kStages];
+    const int sl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (lane == 0) {
+        for (int i = 0; i < kStages; ++i) mbar_init(&vbar[sl][i], 1);
+        mbar_init_fence();
+    }
+    __syncthreads();
+    const int bh = blockIdx.x, b = bh / va.Hkv, h = bh % va.Hkv;
+    GlobalWeightSrc<G> src;
+#pragma unroll
+    for (int g = 0; g < G; ++g) src.row[g] = attn + (size_t(b) * va.Hq + size_t(h) * G + g) * (va.T + 1);
+    src.wts = wts[sl];
+    src.T = va.T;
+    const Seg seg{0, va.T, true, nullptr, nullptr, sl};
+    v_warp_n<BITS, G, EXACT ? kArithCanon : kArithFma>(va, seg, b, h, lane, vbuf[sl], vbar[sl], wts[sl], src);
+}
+
+// forward_ov splits a stream over two warps up to this many streams per launch: one per warp scheduler of the chip.
+// Measured on a B200, 4-bit, 32 heads, the whole qk -> torch softmax -> ov sequence: 1 x 1000 tokens 136 -> 124 us, 4 x 2000
+// tokens 247 -> 224 us, 16 x 1023 tokens 146 -> 140 us (with the weights fetched ahead, adkv_io.cuh, which alone takes
+// 32 x 1000 tokens from 183 to 177 us).  Above it the schedulers are busy and the split only repeats work.
+constexpr int kOvSplitMaxStreams = 592;
 
 }  // namespace adkv
 
@@ -106,6 +139,12 @@ int adkv_forward_ov(const void *attn, void *v_cache, const void *v_new, const ad
     const bool half = flags & ADKV_FLAG_HALF_STATE, exact = !(flags & ADKV_FLAG_FAST_REPLAY);
     if (D != kD) return adkv_wide_forward_ov(va, static_cast<const __half *>(attn), B, bits, half ? 2 : int(exact), s);
     if (half) return adkv_half_forward_ov(va, static_cast<const __half *>(attn), B, bits, s);
+    if (n_streams <= kOvSplitMaxStreams) {
+        ADKV_DISPATCH(bits, exact, Hq / Hkv,
+                      (forward_ov_split_kernel<BITS, G, EXACT><<<n_streams, 32 * kNarrowSlices, 0, s>>>(
+                          va, static_cast<const __half *>(attn))))
+        return launch_status();
+    }
     ADKV_DISPATCH(bits, exact, Hq / Hkv,
                   (forward_ov_kernel<BITS, G, EXACT><<<grid, 32 * kStreamsPerCta, 0, s>>>(
                       va, static_cast<const __half *>(attn), n_streams)))

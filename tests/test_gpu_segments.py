@@ -118,3 +118,41 @@ def test_layered_append_forms():
             assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
     with pytest.raises(RuntimeError, match="wrong shape"):
         gemv.append_kv_layers(ls, x[0, :, :, :2].contiguous(), x[1], T, SMIN, SMAX)
+
+
+@pytest.mark.parametrize("Hq,Hkv,T,bits", [(2, 2, 0, 4), (2, 2, 95, 4), (8, 2, 129, 2), (4, 2, 300, 4)])
+def test_two_streams_per_sm(Hq, Hkv, T, bits):
+    """160 streams: the eight-warp form of the segment kernel, against one warp pair per stream."""
+    B, D = 80, 128
+    case = make_case(900 + T, 2, Hq, Hkv, T, bits)
+    dk, dv, tk, tv, ok_, ov_, *_ = _prefill(case, T + 1)
+    rep = lambda t: dev(t).repeat(B // 2, *([1] * (t.dim() - 1)))
+    args = (rep(case["q"]), rep(dk), rep(dv), rep(case["k"][:, :, T:]), rep(case["v"][:, :, T:]), dev(case["kp"]), dev(case["vp"]),
+            T, 0.08, SMIN, SMAX)
+    kw = dict(bits=bits, k_tail=rep(tk), v_tail=rep(tv), tail_keep=True)
+    want = gemv.decode_attn(*args, **kw, split_channels=False)
+    got = gemv.decode_attn(*args, **kw)
+    _status_ok()
+    np.testing.assert_allclose(got.float().cpu().numpy(), want.float().cpu().numpy(), rtol=RTOL, atol=ATOL)
+    assert torch.equal(got[:2], got[-2:])
+
+
+@pytest.mark.parametrize("T,bits", [(1, 4), (33, 4), (70, 2)])
+def test_few_and_many_streams_agree(T, bits):
+    """Prefill (one or two channels per thread) and forward_ov (one or two warps per stream) choose by the number of streams;
+    bytes, states and outputs do not depend on it."""
+    B, H, D = 160, 4, 128
+    case = make_case(40 + T, 1, H, H, T, bits)
+    dk, dv, tk, tv, *_ = _prefill(case, T + 1)
+    rep = lambda t: dev(t).repeat(B, *([1] * (t.dim() - 1)))
+    mk, mv, mtk, mtv = torch.zeros_like(rep(dk)), torch.zeros_like(rep(dv)), torch.zeros_like(rep(tk)), torch.zeros_like(rep(tv))
+    kp, vp = dev(case["kp"]), dev(case["vp"])
+    gemv.encode_kv_pair(mk, rep(case["k"][:, :, :T]), kp, mv, rep(case["v"][:, :, :T]), vp, SMIN, SMAX, bits=bits, k_tail=mtk,
+                        v_tail=mtv)
+    for many, one in ((mk, dk), (mv, dv), (mtk, tk), (mtv, tv)):
+        assert torch.equal(many.view(torch.uint8), rep(one).view(torch.uint8))
+    w = torch.softmax(torch.randn(1, H, 1, T + 1, generator=torch.Generator().manual_seed(1)), -1).half()
+    one = gemv.forward_ov(dev(w), dv, dev(case["v"][:, :, T:]), *vp, SMIN, SMAX, bits=bits)
+    many = gemv.forward_ov(rep(w), mv, rep(case["v"][:, :, T:]), *vp, SMIN, SMAX, bits=bits)
+    assert torch.equal(many, rep(one)) and torch.equal(mv, rep(dv))
+    _status_ok()
