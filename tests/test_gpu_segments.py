@@ -151,7 +151,7 @@ def test_few_and_many_streams_agree(T, bits):
                         v_tail=mtv)
     for many, one in ((mk, dk), (mv, dv), (mtk, tk), (mtv, tv)):
         assert torch.equal(many.view(torch.uint8), rep(one).view(torch.uint8))
-    w = torch.softmax(torch.randn(1, H, 1, T + 1, generator=torch.Generator().manual_seed(1)), -1).half()
+    w = torch.softmax(torch.randn(1, H, T + 1, generator=torch.Generator().manual_seed(1)), -1).half()
     one = gemv.forward_ov(dev(w), dv, dev(case["v"][:, :, T:]), *vp, SMIN, SMAX, bits=bits)
     many = gemv.forward_ov(rep(w), mv, rep(case["v"][:, :, T:]), *vp, SMIN, SMAX, bits=bits)
     assert torch.equal(many, rep(one)) and torch.equal(mv, rep(dv))
