@@ -2,7 +2,7 @@
 // and the reference interface each one replaces.
 #include "adkv_host.h"
 
-#include "adkv_tailscan.cuh"
+#include "adkv_softmax.cuh"
 
 namespace adkv {
 
@@ -64,47 +64,6 @@ __global__ void __launch_bounds__(64) decode_attn_kernel(KArgs ka, VArgs va, con
     }
 }
 
-// The same step next to tail states in the contracted arithmetic, one query head per KV head (adkv_tailscan.cuh).
-template <int BITS>
-__global__ void __launch_bounds__(64, 1) decode_attn_tail_kernel(KArgs ka, VArgs va, const float *__restrict__ mask,
-                                                                 long long mask_stride_b, float scaling,
-                                                                 const int *__restrict__ seq_lens)
-{
-    __shared__ alignas(128) uint8_t kbuf[kTailStages * Tile<BITS>::BYTES];
-    __shared__ alignas(128) uint8_t vbuf[kTailStages * Tile<BITS>::BYTES];
-    __shared__ alignas(16) float red[kRedFloats];
-    __shared__ alignas(16) float4 wts[kTileTok];
-    __shared__ alignas(16) float4 slow[2][2 * 32];
-    __shared__ FusedShared<1> fs;
-    __shared__ uint64_t kbar[kTailStages], vbar[kTailStages];
-
-    const int bh = blockIdx.x, b = bh / ka.Hkv, h = bh % ka.Hkv;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (seq_lens) {   // as in decode_attn_kernel
-        const int T = seq_lens[b];
-        if (T < 0 || T / Codec<BITS>::TPW >= ka.n_super_cap) {
-            if (threadIdx.x == 0) atomicExch(&g_status, kStatCapacity);
-            return;
-        }
-        ka.T = T;
-        va.T = T;
-    }
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < kTailStages; ++i) { mbar_init(&kbar[i], 1); mbar_init(&vbar[i], 1); }
-        fs.init_barriers(1);
-        mbar_init_fence();
-    }
-    __syncthreads();
-    if (warp == 0) {
-        RingSink<1> sink{&fs, 0, 0};
-        const Seg seg{0, ka.T, true, nullptr, nullptr, 0};
-        k_tail_warp<BITS, kTailStages, true>(ka, seg, b, h, lane, kbuf, kbar, red, slow[0], sink);
-    } else {
-        TailSoftmax src{&fs, wts, mask ? mask + size_t(b) * mask_stride_b : nullptr, scaling * 1.4426950408889634f, -INFINITY, 0.f};
-        v_tail_warp<BITS, kTailStages>(va, b, h, lane, vbuf, vbar, slow[1], src);
-    }
-}
-
 }  // namespace adkv
 
 using namespace adkv;
@@ -127,9 +86,9 @@ ADKV_HIDDEN int adkv_wide_decode_attn(const KArgs &ka, const VArgs &va, const fl
 ADKV_DEFINE_TU_STATUS(adkv_tu_status_fused)
 
 // Token segments of a stream side by side (adkv_segments.cu), next to tail states: up to two streams per SM.  Measured on
-// a B200 there (256 streams): 88 us against 92 us with one pair per stream for one query head per KV head, 258 us against
+// a B200 there (256 streams): 88 us against 106 us with one pair per stream for one query head per KV head, 258 us against
 // 307 us for four.  From three streams per SM on the schedulers are busy without segments (12 x 32 streams of 2000
-// tokens, two rounds of segments: 137 us against 131 us).
+// tokens, two rounds of segments: 137 us against 143 us).
 constexpr long long kSegmentsMaxStreams = 296;
 
 static bool use_segments(const KArgs &ka, int B, bool exact, unsigned flags)
@@ -142,13 +101,6 @@ static bool use_segments(const KArgs &ka, int B, bool exact, unsigned flags)
 static int launch_decode(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b, float scaling, int B,
                          int bits, bool exact, const int *seq_lens, cudaStream_t s)
 {
-    if (ka.tail && !exact && ka.Hq == ka.Hkv) {
-        if (bits == 4)
-            decode_attn_tail_kernel<4><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling, seq_lens);
-        else
-            decode_attn_tail_kernel<2><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling, seq_lens);
-        return launch_status();
-    }
     ADKV_DISPATCH(bits, exact, ka.Hq / ka.Hkv,
                   (decode_attn_kernel<BITS, G, ARITH><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling,
                                                                                seq_lens)))

@@ -22,8 +22,7 @@
 // to the work, so this pays only while a stream per warp pair leaves schedulers idle.
 //
 // Measured on a B200, one pair per stream (or the split head of adkv_narrow.cu) -> segments, 32 query heads: 4-bit, batch 4
-// x 2047 tokens 104 -> 48 us; batch 1 x 4000 tokens 195 -> 85 us; batch 8 x 2000 tokens 106 (92 with adkv_tailscan.cuh)
-// -> 88 us.  8 KV heads: 2-bit, batch 4 / 16 / 32 x 4000 tokens 286 / 305 / 307 -> 127 / 131 / 258 us, batch 32 x 32768
+// x 2047 tokens 104 -> 48 us; batch 1 x 4000 tokens 195 -> 85 us; batch 8 x 2000 tokens 106 -> 88 us.  8 KV heads: 2-bit, batch 4 / 16 / 32 x 4000 tokens 286 / 305 / 307 -> 127 / 131 / 258 us, batch 32 x 32768
 // tokens 2436 -> 1948 us; 4-bit, batch 30 x 4000 tokens 336 -> 250 us.
 #include "adkv_host.h"
 

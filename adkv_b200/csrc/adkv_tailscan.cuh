@@ -1,29 +1,25 @@
-// Scans of the decode step next to a persisted tail state (contracted arithmetic, head dim 128, one query head per KV
+// K scan of the decode step next to a persisted tail state (contracted arithmetic, head dim 128, one query head per KV
 // head).
 //
 // The tail supplies the state the appended token is quantised with, so a replay only has to feed the two attention
 // sums.  What bounds it is instruction issue: a packed fp32 instruction holds the issue port for two cycles, and the
-// contracted recurrence as written (adkv_decode.cuh) needs seven of them per channel pair and token.  Three identities
+// contracted recurrence as written (adkv_decode.cuh) needs seven of them per channel pair and token.  Two identities
 // leave 5.25:
 //
 //  * Scale.  s' = s * (tc + beta*|q|) with tc = 1 - beta*target.  With s = tc^k * u inside a block of four tokens
 //    (k = 0..3), u' = u + (beta/tc) * |q*u|: one multiply-add on the product q*u that the value needs anyway.  The
-//    powers tc^k are folded into constants (K) or into one accumulator per position (V); once per block u is scaled
+//    powers tc^k are folded into the query; once per block u is scaled
 //    back by tc^4.
 //  * K.  The logit needs the zero points only as z_t = sum_c q_c * zp_c(t), a running sum over tokens like zp itself:
 //    each lane carries its share of z in ONE register pair instead of a zero point per channel.
-//  * V.  zp_t = zp_T - alpha * sum_{u >= t} q_u*s_u, and zp_T is known before the scan: it is the tail.  Hence
-//    sum_t w_t*zp_t = zp_T * W - alpha * sum_u P_u*q_u*s_u with the running sums P_u = w_0 + .. + w_u, which the online
-//    softmax forms anyway (its denominator): no zero point is replayed.
 //
 // Clamp and eps guard are left out where eight worst-case updates cannot reach a bound, else where four cannot (on the
 // benchmark data the eight-token test fails for 7 % of the 4-bit chunks and 16 % of the 2-bit ones, the four-token test
 // for none); only what is left runs guarded.
 //
-// Measured on a B200, 4-bit, 32 heads, against decode_attn_kernel: batch 128 x 4096 tokens 1340 us (1473), batch 24 x
-// 1531 tokens with mask 131 us (152), ragged batch 48 of up to 3000 tokens 303 us (352).  With two and four query heads
-// the first identity alone remains and the longer constants cost what it gains (2480 us against 2436 us at batch 32 x 8
-// KV heads x 32768 tokens, 2-bit), so those keep decode_attn_kernel.
+// Used inside the segments of adkv_segments.cu, where it is as exact against 64 bits as the recurrence as written.  Over a
+// whole stream it is not (2.66e-4 instead of 2.47e-4 at 8192 tokens, 2-bit), so launches with one warp pair per stream
+// keep decode_attn_kernel although this scan would take 1.33 ms instead of 1.47 ms at batch 128 x 4096 tokens.
 #pragma once
 #include "adkv_softmax.cuh"
 
@@ -424,246 +420,6 @@ __device__ __forceinline__ void k_tail_warp(const KArgs &a, const Seg &seg, int 
         upk2(st.z, lo, hi);
         sink.end_share(lo + hi, lane);
     }
-}
-
-// ------------------------------------------------------------------------------------------ V side
-
-struct VTailState {
-    f32x2 s[2];
-    f32x2 acc[2], accp[2];     // sum w*q*s and sum P*q*s of the positions with power 0
-};
-
-// Up to eight tokens, one head (see k_tail_slow).  wts: (w, w, P, P) per token.
-template <int BITS>
-__device__ __noinline__ VTailState v_tail_slow(uint4 w, VTailState st, const float4 *slow, const float4 *wts, int count,
-                                               SafeRange safe4, float smin, float smax)
-{
-    float be[4], tc[4];
-    load_slow_consts(slow, be, tc);
-    PairFields<BITS> fc;
-    fc.init();
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half, count -= 4, wts += 4) {
-        const uint32_t grp[4] = {w.x, w.y, w.z, w.w};
-        if (count >= 4 && tail_safe(safe4, st.s)) {
-            static_for<4>([&](auto kc) {
-                constexpr int k = decltype(kc)::value;
-                const ulonglong2 wp = *reinterpret_cast<const ulonglong2 *>(wts + k);
-#pragma unroll
-                for (int p = 0; p < 2; ++p) {
-                    const f32x2 q2 = fc.template code2<k>(grp[2 * p], grp[2 * p + 1]);
-                    const f32x2 r = mul2(q2, st.s[p]);
-                    st.acc[p] = fma2(wp.x, r, st.acc[p]);
-                    st.accp[p] = fma2(wp.y, r, st.accp[p]);
-                    st.s[p] = mul2(st.s[p], fma2(pk2(be[2 * p], be[2 * p + 1]), abs2(q2), pk2(tc[2 * p], tc[2 * p + 1])));
-                }
-            });
-        } else {
-            float s[4];
-            upk2(st.s[0], s[0], s[1]);
-            upk2(st.s[1], s[2], s[3]);
-#pragma unroll 1
-            for (int j = 0; j < 4 && j < count; ++j) {
-                const ulonglong2 wp = *reinterpret_cast<const ulonglong2 *>(wts + j);
-                float rh[4];
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    rh[c] = guarded_scale_step(code_f_rt<BITS>(grp[c], j), s[c], be[c], tc[c], smin, smax);
-#pragma unroll
-                for (int p = 0; p < 2; ++p) {
-                    const f32x2 r = pk2(rh[2 * p], rh[2 * p + 1]);
-                    st.acc[p] = fma2(wp.x, r, st.acc[p]);
-                    st.accp[p] = fma2(wp.y, r, st.accp[p]);
-                }
-            }
-            st.s[0] = pk2(s[0], s[1]);
-            st.s[1] = pk2(s[2], s[3]);
-        }
-        shift_words(w, 4 * BITS);
-    }
-    return st;
-}
-
-// Four tokens without guards, one head: one accumulator pair per position of the block.
-template <int BITS>
-__device__ __forceinline__ void v_tail_block(const uint32_t (&grp)[4], const PairFields<BITS> &fc, f32x2 (&s)[2],
-                                             const f32x2 (&bp)[2], const f32x2 (&e4)[2], const float4 *wts,
-                                             f32x2 (&acc)[4][2], f32x2 (&accp)[4][2])
-{
-    static_for<4>([&](auto kc) {
-        constexpr int k = decltype(kc)::value;
-        const ulonglong2 wp = *reinterpret_cast<const ulonglong2 *>(wts + k);
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            const f32x2 r = mul2(fc.template code2<k>(grp[2 * p], grp[2 * p + 1]), s[p]);
-            acc[k][p] = fma2(wp.x, r, acc[k][p]);
-            accp[k][p] = fma2(wp.y, r, accp[k][p]);
-            s[p] = fma2(bp[p], abs2(r), s[p]);
-        }
-    });
-#pragma unroll
-    for (int p = 0; p < 2; ++p) s[p] = mul2(s[p], e4[p]);
-}
-
-// ------------------------------------------------------------------------------------------ V warp
-
-// Online softmax of a V warp.  Weights of a tile: (w, w, P, P) per token, P the running sum of the weights.
-struct TailSoftmax {
-    FusedShared<1> *sh;
-    float4 *wts;           // [kTileTok]
-    const float *mask;     // row of this batch or nullptr
-    float scale2;          // scaling * log2(e)
-    float m, l;            // running maximum (log2 units), sum of the weights so far
-
-    __device__ __forceinline__ static float redux_max(float v)
-    {
-        float r;
-        asm("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-        return r;
-    }
-    // Fills the weights of tile i; corr is what the accumulators have to be scaled with (warp-uniform).
-    __device__ __forceinline__ bool tile(int i, int ntok, int lane, float &corr)
-    {
-        const int slot = unsigned(i) % kLogitSlots;
-        const float mk = (mask && lane < ntok) ? mask[i * kTileTok + lane] * 1.4426950408889634f : 0.f;
-        if (!mbar_wait_short(&sh->lfull[slot], (unsigned(i) / kLogitSlots) & 1, kStatLFullWait)) return false;
-        const float x = sh->lring[slot][0][0][lane];
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sh->lempty[slot]);
-        const float v = lane < ntok ? fmaf(x, scale2, mk) : -INFINITY;
-        const float m_new = fmaxf(m, redux_max(v));
-        const bool dead = m_new == -INFINITY;
-        corr = dead ? 1.f : exp2f(m - m_new);
-        const float w = dead ? 0.f : exp2f(v - m_new);
-        m = m_new;
-        float P = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float y = __shfl_up_sync(kFull, P, o);
-            if (lane >= o) P += y;
-        }
-        P = fmaf(l, corr, P);
-        l = __shfl_sync(kFull, P, 31);
-        wts[lane] = make_float4(w, w, P, P);
-        __syncwarp();
-        return true;
-    }
-    // weight of the appended token, whose logit is the single entry of tile n_tiles
-    __device__ __forceinline__ bool self(int n_tiles, int T, float (&out)[4], float &w_self)
-    {
-        const int slot = unsigned(n_tiles) % kLogitSlots;
-        if (!mbar_wait_short(&sh->lfull[slot], (unsigned(n_tiles) / kLogitSlots) & 1, kStatLFullWait)) return false;
-        const float mk = mask ? mask[T] * 1.4426950408889634f : 0.f;
-        const float v = fmaf(sh->lring[slot][0][0][0], scale2, mk);
-        const float m_new = fmaxf(m, v);
-        const bool dead = m_new == -INFINITY;
-        const float corr = dead ? 1.f : exp2f(m - m_new);
-        w_self = dead ? 0.f : exp2f(v - m_new);
-        l = fmaf(l, corr, w_self);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) out[c] *= corr;
-        m = m_new;
-        return true;
-    }
-};
-
-// The whole stream of (b, h); writes the normalised output.
-template <int BITS, int STAGES>
-__device__ __forceinline__ void v_tail_warp(const VArgs &a, int b, int h, int lane, uint8_t *ring_buf, uint64_t *ring_bar,
-                                            float4 *slow, TailSoftmax &src)
-{
-    using C = Codec<BITS>;
-    const int bh = b * a.Hkv + h, c0 = 4 * lane;
-    const size_t poff = size_t(h) * kD + c0;
-    uint8_t *stream = a.cache + size_t(bh) * a.n_super_cap * kD * 4;
-    StreamRing<BITS, STAGES> ring{ring_buf, ring_bar, stream, (a.T + kTileTok - 1) / kTileTok, a.T, kStatVWait, kD * 4};
-    ring.prologue(lane);
-    PairFields<BITS> fc;
-    fc.init();
-    slow += lane;
-    float *tail = a.tail + size_t(bh) * 2 * kD;
-    TailChan t;
-    load_tail_chan<BITS>(t, a.p, poff, nullptr, c0, a.smin, a.smax, slow);
-    f32x2 s[2] = {t.s[0], t.s[1]}, acc[4][2], accp[4][2];
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-        for (int p = 0; p < 2; ++p) acc[k][p] = accp[k][p] = 0ull;
-    const auto slow_chunk = [&](const uint4 &w, int tok, int count) {
-        VTailState st;
-#pragma unroll
-        for (int p = 0; p < 2; ++p) { st.s[p] = s[p]; st.acc[p] = acc[0][p]; st.accp[p] = accp[0][p]; }
-        st = v_tail_slow<BITS>(w, st, slow, src.wts + tok, count, t.safe4, a.smin, a.smax);
-#pragma unroll
-        for (int p = 0; p < 2; ++p) { s[p] = st.s[p]; acc[0][p] = st.acc[p]; accp[0][p] = st.accp[p]; }
-    };
-    const auto chunk = [&](const uint4 &w, int tok) {
-        if (tail_safe(t.safe, s)) {
-            const float4 *wt = src.wts + tok;
-            uint32_t grp[4] = {w.x, w.y, w.z, w.w};
-            v_tail_block<BITS>(grp, fc, s, t.bp, t.e[3], wt, acc, accp);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) grp[c] >>= 4 * BITS;
-            v_tail_block<BITS>(grp, fc, s, t.bp, t.e[3], wt + 4, acc, accp);
-        } else {
-            slow_chunk(w, tok, 8);
-        }
-    };
-    bool ok = true;
-    int i = 0;
-    for (; i < ring.n_tiles; ++i) {
-        const int ntok = min(kTileTok, a.T - i * kTileTok);
-        float corr;
-        if (!(ok = src.tile(i, ntok, lane, corr))) break;
-        if (corr != 1.f) {       // warp-uniform; rare once the running maximum has settled
-            const f32x2 f = pk2(corr, corr);
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-#pragma unroll
-                for (int p = 0; p < 2; ++p) {
-                    acc[k][p] = mul2(acc[k][p], f);
-                    accp[k][p] = mul2(accp[k][p], f);
-                }
-        }
-        if (!(ok = ring.wait_short(i))) break;
-        const uint4 *tile = ring.tile(i, lane);
-        if (ntok == kTileTok) walk_full_tile<BITS>(tile, chunk);
-        else walk_tile<BITS>(tile, ntok, slow_chunk);
-        if ((i + 1) % kDriftTiles == 0) correct_drift(s, t.drift);
-        ring.release_and_refill(i, lane);   // also orders this tile's reads of wts before the next fill
-    }
-    if (!ok) {
-        ring.drain(i);
-        return;
-    }
-    // sum_k tc^k * (acc_k - alpha * accp_k) + W * zp_T; the constants are loaded again rather than kept
-    float out[4];
-    load_tail_chan<BITS>(t, a.p, poff, nullptr, c0, a.smin, a.smax, slow);
-    const f32x2 minus = pk2(-1.f, -1.f);
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-        const f32x2 nal = mul2(t.alpha[p], minus);
-        f32x2 sum = fma2(nal, accp[0][p], acc[0][p]);
-#pragma unroll
-        for (int k = 1; k < 4; ++k) sum = fma2(t.e[k - 1][p], fma2(nal, accp[k][p], acc[k][p]), sum);
-        upk2(sum, out[2 * p], out[2 * p + 1]);
-    }
-    if (a.T > 0) {
-        const float4 zp = *reinterpret_cast<const float4 *>(tail + c0);
-        out[0] = fmaf(src.l, zp.x, out[0]);
-        out[1] = fmaf(src.l, zp.y, out[1]);
-        out[2] = fmaf(src.l, zp.z, out[2]);
-        out[3] = fmaf(src.l, zp.w, out[3]);
-    }
-    float w_self, xh[4];
-    if (!src.self(ring.n_tiles, a.T, out, w_self)) return;
-    append_from_tail<BITS>(a.p, poff, tail, a.tail_keep, a.x_new + size_t(bh) * kD + c0,
-                           reinterpret_cast<uint4 *>(stream + size_t(a.T / C::TPW) * (kD * 4)) + lane, a.T, a.smin, a.smax,
-                           c0, xh);
-    const float inv = 1.0f / src.l;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) out[c] = fmaf(w_self, xh[c], out[c]) * inv;
-    store_half4(a.out + size_t(bh) * kD + c0, out);
 }
 
 }  // namespace adkv

@@ -186,7 +186,6 @@ int adkv_forward_ov(const void *attn, void *v_cache, const void *v_new, const ad
  *          previous decode step left it -- the new token is quantised from the tail (bit-identical to the
  *          encoder, in O(1)), the tail advances to the state after token T, and the replay of tokens [0, T)
  *          only feeds the attention sums, so ADKV_FLAG_FAST_REPLAY then costs no exactness of the stored codes.
- *          The tails must be those of the T cached tokens: the replay of V takes its zero points from them.
  *          Not available with ADKV_FLAG_HALF_STATE (ADKV_E_FLAGS): that arithmetic is the encoder's own. */
 int adkv_decode_attn(const void *q, void *k_cache, void *v_cache, const void *k_new, const void *v_new,
                      const adkv_params *kp, const adkv_params *vp, void *k_tail, void *v_tail,
