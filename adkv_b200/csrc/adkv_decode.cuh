@@ -77,10 +77,6 @@ struct StreamRing {
     {
         return mbar_wait_bounded(&bar[unsigned(i) % STAGES], (unsigned(i) / STAGES) & 1, wait_code);
     }
-    __device__ __forceinline__ bool wait_short(int i) const
-    {
-        return mbar_wait_short(&bar[unsigned(i) % STAGES], (unsigned(i) / STAGES) & 1, wait_code);
-    }
     __device__ __forceinline__ const uint4 *tile(int i, int lane) const
     {
         return reinterpret_cast<const uint4 *>(buf + (unsigned(i) % STAGES) * Tile<BITS>::BYTES) + lane;

@@ -232,12 +232,12 @@ __device__ __forceinline__ f32x2 replay_step2(f32x2 q2, f32x2 &zp, f32x2 &s, con
     return xh;
 }
 
-// Interval of scales from which STEPS (8 or 4) further updates cannot leave [max(smin, eps), smax]: inside it the
+// Interval of scales from which 8 further updates cannot leave [max(smin, eps), smax]: inside it the
 // clamp and the eps guard are the identity and the unguarded step gives bit-identical results.
 // One conservative interval per lane (intersection over its channels).
 struct SafeRange {
     float lo, hi;
-    template <int BITS, int N, int STEPS = 8>
+    template <int BITS, int N>
     __device__ __forceinline__ void init(const float (&beta)[N], const float (&target)[N], float smin, float smax)
     {
         lo = 0.f;
@@ -247,10 +247,9 @@ struct SafeRange {
             const float g0 = 1.f - beta[c] * target[c];                      // |q| = 0
             const float g1 = g0 + beta[c] * float(Codec<BITS>::BIAS);        // |q| = largest code magnitude
             const float gmn = fminf(fminf(g0, g1), 1.f), gmx = fmaxf(fmaxf(g0, g1), 1.f);
-            float pmn = gmn * gmn, pmx = gmx * gmx;                          // STEPS-th powers
-            pmn *= pmn;
-            pmx *= pmx;
-            if (STEPS == 8) { pmn *= pmn; pmx *= pmx; }
+            float pmn = gmn * gmn, pmx = gmx * gmx;                          // 8th powers
+            pmn *= pmn; pmn *= pmn;
+            pmx *= pmx; pmx *= pmx;
             // approximate division (2 ulp) is far inside the 2e-5 margin that keeps the interval conservative
             const float l = gmn > 0.f ? __fdividef(fmaxf(smin, kEps), pmn * (1.f - 2e-5f)) : INFINITY;
             const float h = __fdividef(smax, pmx * (1.f + 2e-5f));
@@ -413,16 +412,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
     ok = __all_sync(kFull, ok);
     if (!ok && (threadIdx.x & 31) == 0) atomicExch(&g_status, code);
     return ok;
-}
-
-// The same with the polling out of line: a scan that waits twice per tile keeps a test and a vote in its loop.
-static __device__ __noinline__ bool mbar_wait_slow(uint64_t *bar, uint32_t parity, int code)
-{
-    return mbar_wait_bounded(bar, parity, code);
-}
-__device__ __forceinline__ bool mbar_wait_short(uint64_t *bar, uint32_t parity, int code)
-{
-    return __all_sync(kFull, mbar_try_wait(bar, parity)) || mbar_wait_slow(bar, parity, code);
 }
 
 // Global -> shared bulk copy completing on an mbarrier.  dst, src 16-byte aligned, bytes % 16 == 0.

@@ -26,7 +26,7 @@
 // tokens 2436 -> 1948 us; 4-bit, batch 30 x 4000 tokens 336 -> 250 us.
 #include "adkv_host.h"
 
-#include "adkv_tailscan.cuh"
+#include "adkv_softmax.cuh"
 
 namespace adkv {
 
@@ -37,9 +37,8 @@ constexpr int kPartFloats = 4 + kD;   // per (segment, head): maximum (log2 unit
 template <int BITS, int G, int NS>
 struct SegShared {
     alignas(128) uint8_t buf[2][NS][kSegStages * Tile<BITS>::BYTES];
-    alignas(16) float red[NS][G == 1 ? kRedFloats : G * 8 * 36];
+    alignas(16) float red[NS][G * 8 * 36];
     alignas(16) float2 wts[NS][G * kTileTok];
-    alignas(16) float4 slow[NS][2 * 32];          // one head: constants of the K scans' guarded bodies
     union {
         alignas(16) float comp[2][NS][3][kD];     // steps 1 and 2: product, smallest and largest running product
         alignas(16) float part[NS][G][kPartFloats];   // steps 3 and 4
@@ -58,17 +57,14 @@ template <int G>
 struct SegSink : RingSink<G> {
     float *z_end;
     bool done;
-    __device__ __forceinline__ void end_share(float share, int lane, int g = 0)
-    {
-        done = true;
-        const float z = warp_sum(share);
-        if (lane == 0) z_end[g] = z;
-    }
     __device__ __forceinline__ void end_state(const Chan (&ch)[4], const float (&qv)[G][4], int lane)
     {
+        done = true;
 #pragma unroll
-        for (int g = 0; g < G; ++g)
-            end_share(fmaf(qv[g][3], ch[3].zp, fmaf(qv[g][2], ch[2].zp, fmaf(qv[g][1], ch[1].zp, qv[g][0] * ch[0].zp))), lane, g);
+        for (int g = 0; g < G; ++g) {
+            const float z = warp_sum(fmaf(qv[g][3], ch[3].zp, fmaf(qv[g][2], ch[2].zp, fmaf(qv[g][1], ch[1].zp, qv[g][0] * ch[0].zp))));
+            if (lane == 0) z_end[g] = z;
+        }
     }
 };
 
@@ -104,6 +100,18 @@ struct SegSrc : SoftmaxSrc<G> {
     }
 };
 
+// Quantise the new token of this lane's channels from the tail (see append_new_token).
+template <int BITS>
+__device__ __forceinline__ void append_from_tail(const ParamPtrs &p, size_t poff, float *tail, bool tail_keep,
+                                                 const __half *x_new, uint4 *slot, int T, float smin, float smax,
+                                                 int c0, float (&xh)[4])
+{
+    Chan ch[4];
+    SafeRange unused;
+    load_chan4<BITS, true>(ch, unused, p, poff, smin, smax);
+    append_new_token<BITS, kArithCanon>(ch, p, poff, tail, tail_keep, x_new, slot, T, smin, smax, nullptr, c0, kD, xh);
+}
+
 // Scales of four channels and what advances them (contracted constants: ch[].tc = 1 - beta * target).
 struct ScaleConst {
     f32x2 beta[2], tc[2];
@@ -130,6 +138,11 @@ __device__ __forceinline__ SafeRange block_range(const float (&beta)[4], const f
 
 // Step 1: product of the factors of `n_words` words of a stream and the extremes of the running product at every
 // fourth token (1 at the start included).  src: this lane's vector of the first word.
+//
+// The state that a segment starts with must not carry more rounding than a scan from the start of the stream would have
+// brought to it, so two factors at a time are multiplied without rounding, as a sum of two numbers, and the running
+// product is rounded every second token.  (A rounded product of factors will not do: factors take a handful of values, so
+// its rounding repeats and adds up, 7e-5 over 8192 tokens instead of 8e-6.)
 template <int BITS>
 __device__ __forceinline__ void scale_product(const uint4 *src, int n_words, const ScaleConst &sc, float (&F)[4],
                                               float (&mn)[4], float (&mx)[4])
@@ -137,6 +150,7 @@ __device__ __forceinline__ void scale_product(const uint4 *src, int n_words, con
     constexpr int kAhead = 4;
     FieldConsts<BITS> fc;
     fc.init();
+    const f32x2 minus = pk2(-1.f, -1.f);
     f32x2 f2[2] = {pk2(1.f, 1.f), pk2(1.f, 1.f)};
 #pragma unroll
     for (int c = 0; c < 4; ++c) mn[c] = mx[c] = 1.f;
@@ -152,12 +166,14 @@ __device__ __forceinline__ void scale_product(const uint4 *src, int n_words, con
             if (wd + i < n_words) {
 #pragma unroll 1
                 for (int blk = 0; blk < Codec<BITS>::TPW / 4; ++blk) {
-                    static_for<4>([&](auto kc) {
-                        constexpr int k = decltype(kc)::value;
+                    static_for<2>([&](auto hc) {
+                        constexpr int k = 2 * decltype(hc)::value;
 #pragma unroll
                         for (int p = 0; p < 2; ++p) {
-                            const f32x2 q2 = fc.template code2<k>(grp[2 * p], grp[2 * p + 1]);
-                            f2[p] = mul2(f2[p], fma2(sc.beta[p], abs2(q2), sc.tc[p]));
+                            const f32x2 a = fma2(sc.beta[p], abs2(fc.template code2<k>(grp[2 * p], grp[2 * p + 1])), sc.tc[p]);
+                            const f32x2 b = fma2(sc.beta[p], abs2(fc.template code2<k + 1>(grp[2 * p], grp[2 * p + 1])), sc.tc[p]);
+                            const f32x2 ab = mul2(a, b), rest = fma2(a, b, mul2(ab, minus));   // a * b == ab + rest
+                            f2[p] = fma2(f2[p], ab, mul2(f2[p], rest));
                         }
                     });
                     upk2(f2[0], F[0], F[1]);
@@ -174,19 +190,21 @@ __device__ __forceinline__ void scale_product(const uint4 *src, int n_words, con
     }
     upk2(f2[0], F[0], F[1]);
     upk2(f2[1], F[2], F[3]);
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+        if (F[c] != F[c]) F[c] = mx[c] = INFINITY;   // past the range of fp32 the sum above is infinity minus infinity
 }
 
 // Step 2 where a clamp may have acted.  The composition of the clamped steps is again a clamped scaling: a state x inside
-// the bounds ends as clamp(F * x, lo, hi), where F is the product of the factors and lo and hi are what the two bounds
-// themselves end as.  (A factor below zero sends every state to the same bound: then lo == hi.)  lo, hi: in the states to
-// start from -- the bounds, or twice the state itself where it is known and may lie outside them.
+// the bounds ends as clamp(F * x, lo, hi), where F is the product of the factors (step 1) and lo and hi are what the two
+// bounds themselves end as.  (A factor below zero sends every state to the same bound: then lo == hi.)  lo, hi: in the
+// states to start from -- the bounds, or twice the state itself where it is known and may lie outside them.  ends: [2].
 template <int BITS>
 __device__ __noinline__ void scale_map(const uint4 *src, int n_words, const ScaleConst &sc, float smin, float smax, float4 lo4,
-                                       float4 hi4, float4 *comp)
+                                       float4 hi4, float4 *ends)
 {
     FieldConsts<BITS> fc;
     fc.init();
-    f32x2 F[2] = {pk2(1.f, 1.f), pk2(1.f, 1.f)};
     f32x2 lo[2] = {pk2(lo4.x, lo4.y), pk2(lo4.z, lo4.w)}, hi[2] = {pk2(hi4.x, hi4.y), pk2(hi4.z, hi4.w)};
     const auto clamped = [&](f32x2 v) {
         float a, b;
@@ -205,7 +223,6 @@ __device__ __noinline__ void scale_map(const uint4 *src, int n_words, const Scal
 #pragma unroll
                 for (int p = 0; p < 2; ++p) {
                     const f32x2 f = fma2(sc.beta[p], abs2(fc.template code2<k>(grp[2 * p], grp[2 * p + 1])), sc.tc[p]);
-                    F[p] = mul2(F[p], f);
                     lo[p] = clamped(mul2(lo[p], f));
                     hi[p] = clamped(mul2(hi[p], f));
                 }
@@ -215,10 +232,8 @@ __device__ __noinline__ void scale_map(const uint4 *src, int n_words, const Scal
         }
         w = next;
     }
-    const f32x2 *rows[3] = {F, lo, hi};
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-        *reinterpret_cast<ulonglong2 *>(comp + r * (kD / 4)) = make_ulonglong2(rows[r][0], rows[r][1]);
+    *reinterpret_cast<ulonglong2 *>(ends) = make_ulonglong2(lo[0], lo[1]);
+    *reinterpret_cast<ulonglong2 *>(ends + kD / 4) = make_ulonglong2(hi[0], hi[1]);
 }
 
 template <int BITS, int G, int NS>
@@ -313,7 +328,7 @@ __global__ void __launch_bounds__(64 * NS, 8 / NS)
         const float4 hi = seg ? make_float4(ka.smax, ka.smax, ka.smax, ka.smax) : start;
         if (followed && redo)
             scale_map<BITS>(words, per_seg / C::TPW, sc, ka.smin, ka.smax, lo, hi,
-                            reinterpret_cast<float4 *>(&sh.comp[role][seg][0][c0]));
+                            reinterpret_cast<float4 *>(&sh.comp[role][seg][1][c0]));
         __syncthreads();
         if (redo) { s[0] = start.x; s[1] = start.y; s[2] = start.z; s[3] = start.w; }
         for (int i = 0; i < seg && redo && !empty; ++i) {
@@ -348,10 +363,7 @@ __global__ void __launch_bounds__(64 * NS, 8 / NS)
         sink.sl = 0;
         sink.z_end = sh.z_end[seg];
         sink.done = false;
-        if constexpr (G == 1)
-            k_tail_warp<BITS, kSegStages, false>(ka, sg, b, h, lane, sh.buf[0][seg], sh.bar[0][seg], sh.red[seg], sh.slow[seg], sink);
-        else
-            k_warp<BITS, G, kArithFma, SegSink<G>, kSegStages>(ka, sg, b, h, lane, sh.buf[0][seg], sh.bar[0][seg], sh.red[seg], sink);
+        k_warp<BITS, G, kArithFma, SegSink<G>, kSegStages>(ka, sg, b, h, lane, sh.buf[0][seg], sh.bar[0][seg], sh.red[seg], sink);
         if (last && sink.done) {
             float xh[4];
             append(ka.p, ka.tail, ka.tail_keep, ka.x_new, ka.cache, xh);

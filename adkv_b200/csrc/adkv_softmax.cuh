@@ -31,13 +31,6 @@ struct RingSink {
         slot = i % kLogitSlots;
         return mbar_wait_bounded(&sh->lempty[slot], ((i / kLogitSlots) & 1) ^ 1, kStatLEmptyWait);
     }
-    __device__ __forceinline__ bool begin_tile_short(int i)
-    {
-        slot = unsigned(i) % kLogitSlots;
-        return mbar_wait_short(&sh->lempty[slot], ((unsigned(i) / kLogitSlots) & 1) ^ 1, kStatLEmptyWait);
-    }
-    // logit of one token, every lane its own (head, token)
-    __device__ __forceinline__ void put(int g, int tok, float v) { sh->lring[slot][sl][g][tok] = v; }
     __device__ __forceinline__ void put8(int, int g, int tok, float v, int lane)
     {
         if (lane < 8) sh->lring[slot][sl][g][tok + lane] = v;
