@@ -85,16 +85,26 @@ ADKV_HIDDEN int adkv_wide_decode_attn(const KArgs &ka, const VArgs &va, const fl
 
 ADKV_DEFINE_TU_STATUS(adkv_tu_status_fused)
 
-// Token segments of a stream side by side (adkv_segments.cu), next to tail states: up to two streams per SM.  Measured on
-// a B200 there (256 streams): 88 us against 106 us with one pair per stream for one query head per KV head, 258 us against
-// 307 us for four.  From three streams per SM on the schedulers are busy without segments (12 x 32 streams of 2000
-// tokens, two rounds of segments: 137 us against 143 us).
-constexpr long long kSegmentsMaxStreams = 296;
+// Token segments of a stream side by side (adkv_segments.cu), next to tail states: up to one stream per SM and from 128
+// tokens on (max_tokens: the tokens of every sequence, or what the cache can hold of them where the lengths are on the
+// device).  Device time on a B200, caches rotated through more than L2 holds, the split head of adkv_narrow.cu -> segments,
+// where no scale meets a clamp / where one channel of every head rests at a bound:
+//    4-bit, 32 heads            128 streams x 2000 tokens   100 ->  50 us / 187 ->  87 us
+//    4-bit, 32 heads             32 streams x 8000 tokens   376 -> 176 us / 728 -> 322 us
+//    2-bit, 32 on 8 KV heads    128 streams x 2000 tokens   159 ->  75 us / 193 -> 104 us
+//    2-bit, 32 on 16 KV heads   144 streams x 128 tokens   12.0 -> 12.0 us / 14.8 -> 14.0 us
+// Below 128 tokens set-up and merge are not made up for (2-bit, 128 streams x 96 tokens: 8.4 -> 8.9 us); device-side
+// lengths may lie there, and cost a microsecond up to 64 tokens (64 streams x 64 tokens: 8.6 -> 9.3 us, x 96 tokens: 10.0
+// -> 9.4 us, x 256 tokens: 17.2 -> 12.3 us).  With more than one stream per SM the extra work has no idle schedulers to go
+// to: 256 streams x 8000 tokens with four segments each, 2-bit, 442 -> 378 us / 478 -> 655 us, with eight KV heads 595 ->
+// 522 us / 646 -> 788 us.
+constexpr long long kSegmentsMaxStreams = 148;
+constexpr int kSegmentsMinTokens = 128;
 
-static bool use_segments(const KArgs &ka, int B, bool exact, unsigned flags)
+static bool use_segments(const KArgs &ka, int B, int max_tokens, bool exact, unsigned flags)
 {
     return ka.tail && !exact && !(flags & (ADKV_FLAG_SPLIT_CHANNELS | ADKV_FLAG_NO_SPLIT_CHANNELS)) &&
-           ka.Hq / ka.Hkv <= 4 && (long long)B * ka.Hkv <= kSegmentsMaxStreams;
+           ka.Hq / ka.Hkv <= 4 && (long long)B * ka.Hkv <= kSegmentsMaxStreams && max_tokens >= kSegmentsMinTokens;
 }
 
 // One CTA per stream.
@@ -136,7 +146,7 @@ int adkv_decode_attn(const void *q, void *k_cache, void *v_cache, const void *k_
                                      half ? 2 : int(exact), s);
     if (half)
         return adkv_half_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, nullptr, s);
-    if (use_segments(ka, B, exact, flags))
+    if (use_segments(ka, B, T, exact, flags))
         return adkv_segments_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, nullptr, s);
     // Very few streams: split every head over two warp pairs (adkv_narrow.cu).
     const bool split = (flags & ADKV_FLAG_SPLIT_CHANNELS) ||
@@ -170,7 +180,7 @@ int adkv_decode_attn_varlen(const void *q, void *k_cache, void *v_cache, const v
     if (flags & ADKV_FLAG_HALF_STATE)
         return adkv_half_decode_attn(ka, va, nullptr, 0, scaling, B, bits, static_cast<const int *>(seq_lens), s);
     const bool exact = !(flags & ADKV_FLAG_FAST_REPLAY);
-    if (use_segments(ka, B, exact, flags))
+    if (use_segments(ka, B, min(n_super_cap, 1 << 20) * (32 / bits) - 1, exact, flags))
         return adkv_segments_decode_attn(ka, va, nullptr, 0, scaling, B, bits, static_cast<const int *>(seq_lens), s);
     return launch_decode(ka, va, nullptr, 0, scaling, B, bits, exact, static_cast<const int *>(seq_lens), s);
 }

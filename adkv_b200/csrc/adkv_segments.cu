@@ -1,7 +1,7 @@
 // Part of libadkv_b200.so (sm_100a).  See include/adkv_b200.h for the contract of every entry point.
 //
 // Fused decode step for launches with few (batch, kv head) streams, next to tail states: the token axis of every stream
-// is cut into NS segments that run side by side in ONE CTA, a K and a V warp each.  Reached through
+// is cut into eight segments that run side by side in ONE CTA, a K and a V warp each.  Reached through
 // adkv_decode_attn and adkv_decode_attn_varlen.
 //
 // What bounds a step with few streams is one warp's dependent instruction stream: a K/V pair walks its stream at about
@@ -9,32 +9,34 @@
 // per-token overhead in each.  The token axis looks serial, but the scale recurrence s' = clamp(s * (tc + beta*|q|)) is a
 // running product of factors that depend on the codes alone, and the zero point a running sum, so:
 //
-//  1. every warp forms the product F of the factors of its segment and the extremes of its running product (half the
-//     arithmetic of a scan, no clamps);
+//  1. every warp forms the product F of the factors of its segment and the extremes of its running product (about half
+//     the arithmetic of a scan, no clamps);
 //  2. the states at the segment starts follow from the products of the segments before.  If some segment, from the state
-//     it really starts with, may have met a clamp (rarely: the extremes, widened by the worst case of four tokens, reach
-//     a bound), all segments of that tensor are gone through once more with clamps (scale_map), still side by side;
-//  3. the scans run with zero points relative to the segment start.  For K that shifts every logit of a segment by one
-//     number, sum_c q_c * zp_c(start), for V it leaves out (sum of weights) * zp(start): both are put back
+//     it really starts with, may have met a clamp (the extremes, widened by the worst case of four tokens, reach a
+//     bound), what becomes of the two bounds is formed for all segments of that tensor as well (scale_map), still side by
+//     side;
+//  3. the scans run as in adkv_decode.cuh, with zero points relative to the segment start.  For K that shifts every logit
+//     of a segment by one number, sum_c q_c * zp_c(start), for V it leaves out (sum of weights) * zp(start): both are put
+//     back
 //  4. when the partial softmax results of the segments are merged in shared memory.
 //
-// Only the appended token needs the encoder's exact state, and that comes from the tail.  Steps 1 and 2 add about a third
-// to the work, so this pays only while a stream per warp pair leaves schedulers idle.
+// Only the appended token needs the encoder's exact state, and that comes from the tail.  Against 64 bits a logit is off
+// by 0.75 to 0.83 times what it is off after one scan over the whole stream (root mean square of 3840 to 9600 logits each,
+// 1500 to 4096 tokens, 4 and 2 bits), because the segments start from less rounding.
 //
-// Measured on a B200, one pair per stream (or the split head of adkv_narrow.cu) -> segments, 32 query heads: 4-bit, batch 4
-// x 2047 tokens 104 -> 48 us; batch 1 x 4000 tokens 195 -> 85 us; batch 8 x 2000 tokens 106 -> 88 us.  8 KV heads: 2-bit, batch 4 / 16 / 32 x 4000 tokens 286 / 305 / 307 -> 127 / 131 / 258 us, batch 32 x 32768
-// tokens 2436 -> 1948 us; 4-bit, batch 30 x 4000 tokens 336 -> 250 us.
+// Steps 1 and 2 add a third to the work, two thirds where a clamp is met, so this pays only while a stream per warp pair
+// leaves schedulers idle: see use_segments in adkv_fused.cu.
 #include "adkv_host.h"
 
 #include "adkv_softmax.cuh"
 
 namespace adkv {
 
+constexpr int NS = 8;             // segments per stream
 constexpr int kSegStages = 2;     // bulk-copy ring depth per warp
 constexpr int kPartFloats = 4 + kD;   // per (segment, head): maximum (log2 units), denominator, 2 pad, kD sums
 
-// NS: segments per stream
-template <int BITS, int G, int NS>
+template <int BITS, int G>
 struct SegShared {
     alignas(128) uint8_t buf[2][NS][kSegStages * Tile<BITS>::BYTES];
     alignas(16) float red[NS][G * 8 * 36];
@@ -236,13 +238,13 @@ __device__ __noinline__ void scale_map(const uint4 *src, int n_words, const Scal
     *reinterpret_cast<ulonglong2 *>(ends + kD / 4) = make_ulonglong2(hi[0], hi[1]);
 }
 
-template <int BITS, int G, int NS>
-__global__ void __launch_bounds__(64 * NS, 8 / NS)
+template <int BITS, int G>
+__global__ void __launch_bounds__(64 * NS)
     decode_attn_segments_kernel(KArgs ka, VArgs va, const float *__restrict__ mask, long long mask_stride_b, float scaling,
                                 const int *__restrict__ seq_lens)
 {
     extern __shared__ uint8_t smem_raw[];
-    SegShared<BITS, G, NS> &sh = *reinterpret_cast<SegShared<BITS, G, NS> *>(smem_raw);
+    SegShared<BITS, G> &sh = *reinterpret_cast<SegShared<BITS, G> *>(smem_raw);
     using C = Codec<BITS>;
     const int bh = blockIdx.x, b = bh / ka.Hkv, h = bh % ka.Hkv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -278,9 +280,9 @@ __global__ void __launch_bounds__(64 * NS, 8 / NS)
     // 1. products of all segments that another one follows (those are whole tiles)
     ScaleConst sc;
     SafeRange range;
-    float s[4];
+    float s[4] = {};
     const bool followed = t_end < T;
-    {
+    if (per_seg < T) {
         Chan ch[4];
         load_chan4<BITS, true>(ch, range, p, poff, ka.smin, ka.smax);
         float be[4], tg[4], tc[4];
@@ -433,17 +435,17 @@ using namespace adkv;
 
 ADKV_DEFINE_TU_STATUS(adkv_tu_status_segments)
 
-template <int BITS, int G, int NS>
+template <int BITS, int G>
 static int launch_segments(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b, float scaling, int B,
                            const int *seq_lens, cudaStream_t s)
 {
-    constexpr int bytes = int(sizeof(SegShared<BITS, G, NS>));
+    constexpr int bytes = int(sizeof(SegShared<BITS, G>));
     static_assert(bytes <= 227 * 1024, "shared memory of one CTA");
     // per device and process: cheap enough (a host-side call) to be made before every launch
-    const cudaError_t e = cudaFuncSetAttribute(decode_attn_segments_kernel<BITS, G, NS>,
+    const cudaError_t e = cudaFuncSetAttribute(decode_attn_segments_kernel<BITS, G>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return int(e);
-    decode_attn_segments_kernel<BITS, G, NS><<<B * ka.Hkv, 64 * NS, bytes, s>>>(ka, va, mask, mask_stride_b, scaling, seq_lens);
+    decode_attn_segments_kernel<BITS, G><<<B * ka.Hkv, 64 * NS, bytes, s>>>(ka, va, mask, mask_stride_b, scaling, seq_lens);
     return launch_status();
 }
 
@@ -451,14 +453,10 @@ static int launch_segments(const KArgs &ka, const VArgs &va, const float *mask, 
 ADKV_HIDDEN int adkv_segments_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b,
                                           float scaling, int B, int bits, const int *seq_lens, cudaStream_t s)
 {
-    // One stream per SM: sixteen warps each.  More: two CTAs of eight warps share an SM (two rounds of sixteen warps take
-    // as long as twice the time of 148 streams: batch 8 x 2000 tokens, 32 heads, 94 us against 88 us).
-    const bool wide = (long long)B * ka.Hkv <= 148;
     switch (bits * 16 + ka.Hq / ka.Hkv) {
 #define ADKV_SEG_CASE(BITS_, G_)                                                                                            \
     case BITS_ * 16 + G_:                                                                                                   \
-        return wide ? launch_segments<BITS_, G_, 8>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s)                   \
-                    : launch_segments<BITS_, G_, 4>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
+        return launch_segments<BITS_, G_>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
         ADKV_SEG_CASE(4, 1) ADKV_SEG_CASE(4, 2) ADKV_SEG_CASE(4, 4)
         ADKV_SEG_CASE(2, 1) ADKV_SEG_CASE(2, 2) ADKV_SEG_CASE(2, 4)
 #undef ADKV_SEG_CASE

@@ -1,5 +1,6 @@
-"""Decode steps next to tail states against the oracle, over token segments (launches with few streams) and with one
-warp pair per stream.  Needs a B200.
+"""Decode steps next to tail states against the oracle and against 64 bits, over token segments (up to 148 streams of 128
+tokens and more, any device-side length) and with one warp pair per stream; prefill and append by number of streams.  Needs
+a B200.
 
 Sizes are the edges of the split: no token, fewer tiles than segments, whole tiles, one token more or less; scales that
 never clamp, clamp at one bound, at both, and start outside the bounds.
@@ -38,6 +39,7 @@ def _clamping(case, kind):
 @pytest.mark.parametrize("B,Hq,Hkv,T,bits", [
     (1, 2, 2, 0, 4), (1, 2, 2, 1, 2), (2, 2, 2, 31, 4), (1, 4, 2, 32, 4), (1, 4, 1, 33, 2), (2, 2, 2, 255, 4), (1, 2, 1, 256, 2),
     (1, 2, 2, 257, 4), (1, 8, 2, 290, 2), (1, 2, 2, 777, 2), (2, 4, 2, 1031, 4),
+    (1, 2, 2, 127, 4), (1, 4, 2, 128, 2), (1, 2, 2, 129, 4), (1, 8, 2, 225, 4),
 ])
 def test_against_oracle(B, Hq, Hkv, T, bits, clamp, split):
     case = make_case(500 + T, B, Hq, Hkv, T, bits)
@@ -86,6 +88,35 @@ def test_segments_varlen(bits):
                                   SMAX, bits=bits, k_tail=tk, v_tail=tv)
     _status_ok()
     np.testing.assert_allclose(got.float().cpu().numpy(), want.float().cpu().numpy(), rtol=RTOL, atol=ATOL)
+
+
+@pytest.mark.parametrize("Hq,Hkv,bits", [(2, 2, 4), (8, 2, 2)])
+def test_segments_varlen_short(Hq, Hkv, bits):
+    """Sequences from one token to a few tiles, and one past the capacity, in caches with room for 700: one tile is
+    one segment.  The sequence that does not fit is reported and left alone."""
+    lens, D = [1, 32, 33, 95, 96, 97, 128, 129, 224, 225, 700], 128
+    B, cap = len(lens), 700
+    case = make_case(78, B, Hq, Hkv, cap, bits)
+    dk = torch.zeros(orc.cache_shape(B, Hkv, orc.n_super_for(cap, bits), D), dtype=torch.uint8, device="cuda")
+    dv = torch.zeros_like(dk)
+    tk = torch.zeros(B, Hkv, 2, D, device="cuda")
+    tv = torch.zeros_like(tk)
+    kp, vp = dev(case["kp"]), dev(case["vp"])
+    for b, n in enumerate(lens):
+        gemv.encode_kv_pair(dk[b:b + 1], dev(case["k"][b:b + 1, :, :n]), kp, dv[b:b + 1], dev(case["v"][b:b + 1, :, :n]), vp,
+                            SMIN, SMAX, bits=bits, k_tail=tk[b:b + 1], v_tail=tv[b:b + 1])
+    lens[-1] = dk.shape[2] * (32 // bits)
+    kn, vn, q = dev(case["k"][:, :, -1:]), dev(case["v"][:, :, -1:]), dev(case["q"])
+    before = [t.clone() for t in (dk, dv, tk, tv)]
+    want = torch.cat([gemv.decode_attn(q[b:b + 1], dk[b:b + 1].clone(), dv[b:b + 1].clone(), kn[b:b + 1], vn[b:b + 1], kp, vp, n,
+                                       0.09, SMIN, SMAX, bits=bits, k_tail=tk[b:b + 1], v_tail=tv[b:b + 1], tail_keep=True,
+                                       split_channels=False) for b, n in enumerate(lens[:-1])])
+    got = gemv.decode_attn_varlen(q, dk, dv, kn, vn, kp, vp, torch.tensor(lens, dtype=torch.int32, device="cuda"), 0.09, SMIN,
+                                  SMAX, bits=bits, k_tail=tk, v_tail=tv)
+    assert gemv.device_status() == 6 and gemv.device_status() == 0
+    np.testing.assert_allclose(got[:-1].float().cpu().numpy(), want.float().cpu().numpy(), rtol=RTOL, atol=ATOL)
+    for t, old in zip((dk, dv, tk, tv), before):
+        assert torch.equal(t[-1], old[-1])
 
 
 def test_product_past_the_range_of_fp32():
@@ -144,7 +175,7 @@ def test_layered_append_forms():
 
 @pytest.mark.parametrize("Hq,Hkv,T,bits", [(2, 2, 0, 4), (2, 2, 95, 4), (8, 2, 129, 2), (4, 2, 300, 4)])
 def test_two_streams_per_sm(Hq, Hkv, T, bits):
-    """160 streams: the eight-warp form of the segment kernel, against one warp pair per stream."""
+    """160 streams, more than the segments take: what the library picks, against one warp pair per stream."""
     B, D = 80, 128
     case = make_case(900 + T, 2, Hq, Hkv, T, bits)
     dk, dv, tk, tv, ok_, ov_, *_ = _prefill(case, T + 1)
