@@ -119,6 +119,29 @@ def test_segments_varlen_short(Hq, Hkv, bits):
         assert torch.equal(t[-1], old[-1])
 
 
+@pytest.mark.parametrize("Hq,T,bits", [(2, 300, 4), (8, 531, 2)])
+def test_masked_segments(Hq, T, bits):
+    """Additive masks that leave out whole segments, every cached token, and everything; the lowest fp32 and fp16 values
+    as well as minus infinity."""
+    case = make_case(610, 1, Hq, 2, T, bits)
+    dk, dv, tk, tv, *_ = _prefill(case, T + 1)
+    args = (dev(case["q"]), dk, dv, dev(case["k"][:, :, T:]), dev(case["v"][:, :, T:]), dev(case["kp"]), dev(case["vp"]), T, 0.08,
+            SMIN, SMAX)
+    kw = dict(bits=bits, k_tail=tk, v_tail=tv, tail_keep=True)
+    for low in (-float("inf"), torch.finfo(torch.float32).min, torch.finfo(torch.float16).min):
+        for out in (slice(0, T // 2), slice(T // 4, T), slice(0, T), slice(0, T + 1)):
+            mask = torch.zeros(1, T + 1, device="cuda")
+            mask[:, out] = low
+            want = gemv.decode_attn(*args, **kw, mask=mask, split_channels=False)
+            got = gemv.decode_attn(*args, **kw, mask=mask)
+            if out == slice(0, T + 1) and low > -1e5:    # scores near -94500 are an fp32 unit of 2**-7 apart, and are
+                rtol = atol = 2e-2                       # rounded twice: weights to 2 * 2**-7 * ln 2
+            else:
+                rtol, atol = RTOL, ATOL
+            np.testing.assert_allclose(got.float().cpu().numpy(), want.float().cpu().numpy(), rtol=rtol, atol=atol)
+    _status_ok()
+
+
 def test_product_past_the_range_of_fp32():
     """Factors far above 1 and no lower bound: the product of a segment's factors overflows, its scales end at the upper
     bound."""
@@ -285,3 +308,26 @@ def test_logit_error_is_that_of_a_whole_scan(B, T, bits, pinned):
     Sums of 192 to 384 squared errors each; segments start from less rounding, which leaves 0.6 to 0.85 of the whole scan's."""
     segments, whole = _logit_errors(B, T, bits, pinned, (None, False))
     assert segments <= whole, (segments, whole)
+
+
+@pytest.mark.parametrize("T,bits", [(70, 4), (161, 2)])
+def test_checkpoints_of_few_and_many_streams(T, bits):
+    """Checkpoints, codes and tails of a prefill with a channel pair per thread (more than 296 (stream, tensor) pairs) are
+    those of the one-channel form, bit for bit; started inside a word as well as at the front."""
+    B, H, D, S = 80, 2, 128, 32
+    case = make_case(50 + T, 1, H, H, T, bits)
+    kp, vp = dev(case["kp"]), dev(case["vp"])
+
+    def prefill(n):
+        rep = lambda t: dev(t).repeat(n, 1, 1, 1)
+        kc = torch.zeros(orc.cache_shape(n, H, orc.n_super_for(T, bits), D), dtype=torch.uint8, device="cuda")
+        vc, kt, vt = torch.zeros_like(kc), torch.zeros(n, H, 2, D, device="cuda"), torch.zeros(n, H, 2, D, device="cuda")
+        kk, vk = gemv.alloc_ckpt(n, H, D, T, S, "cuda"), gemv.alloc_ckpt(n, H, D, T, S, "cuda")
+        for lo, hi in ((0, 37), (37, T)):
+            gemv.encode_kv_pair(kc, rep(case["k"][:, :, lo:hi]), kp, vc, rep(case["v"][:, :, lo:hi]), vp, SMIN, SMAX, bits=bits,
+                                t_start=lo, k_tail=kt, v_tail=vt, k_ckpt=kk, v_ckpt=vk, ckpt_interval=S)
+        return kc, vc, kt, vt, kk, vk
+
+    for many, one in zip(prefill(B), prefill(1)):
+        assert torch.equal(many.view(torch.uint8), one.repeat(B, *([1] * (one.dim() - 1))).view(torch.uint8))
+    assert float(one[:, :, -1, 1].min()) > 0.0      # the last checkpoint is written
