@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kD / CPT) encode_kernel(EncBatch batch, CkptSp
     }
     if (t % C::TPW != 0) {   // bring the tokens of the last, partial word down; its unused fields are zero
         const int down = BITS * (C::TPW - t % C::TPW);
-        #pragma unroll
+#pragma unroll
         for (int c = 0; c < CPT; ++c) word[c] >>= down;
         w[size_t(t / C::TPW) * RS] = Io::word(word);
     }
@@ -324,7 +324,7 @@ struct AppendBatch {
 // A step moves 26 bytes a channel, so it is bound by the latency of one round of loads and by how many threads the chip
 // takes in at once: half the threads and twice the bytes per load of one channel per thread (append_kernel).  All
 // tensors of 32 layers in one launch instead of four: 41 us -> 21.5 us a call at 32 layers x batch 16 x 32 heads, 2-bit,
-// one B200 (82 MB of tails, words and tokens that cannot be left out: 17 us at the measured copy bandwidth).
+// one B200 (109 MB of tails, words and tokens that cannot be left out: 17 us at the measured copy bandwidth).
 // Wider accesses need the alignment that append_aligned checks; what fails it takes append_kernel.
 template <int BITS, class Batch>
 __global__ void __launch_bounds__(kD) append_pair_kernel(const __grid_constant__ Batch batch, CkptSpec cs, int H, int n_slices,
@@ -450,7 +450,7 @@ static int launch_encode(const EncBatch &b, int n, int B, int H, int T, int D, i
     // to itself and takes as long as its own instructions, of which one channel needs about half as many as a pair.
     // Measured on a B200, K and V of 32 heads: 1 x 4000 tokens 251 -> 231 us, 2 x 2000 tokens 131 -> 121 us, 4 x 2000 tokens
     // 137 -> 133 us.  With more streams the schedulers are busy and the packed pair needs fewer issue slots per channel.
-    const bool few = (long long)grid.x * grid.y * (kD / 32) <= 2 * 592;
+    const bool few = (long long)grid.x * grid.y * (kD / 32) <= 2 * kSchedulers;
     if (D == kD) {
         if (bits == 4 && few) encode_kernel<4, false, 1><<<grid, kD, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
         else if (bits == 4) encode_kernel<4, false, 2><<<grid, kEncThreads, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);

@@ -98,7 +98,7 @@ ADKV_DEFINE_TU_STATUS(adkv_tu_status_fused)
 // -> 9.4 us, x 256 tokens: 17.2 -> 12.3 us).  With more than one stream per SM the extra work has no idle schedulers to go
 // to: 256 streams x 8000 tokens with four segments each, 2-bit, 442 -> 378 us / 478 -> 655 us, with eight KV heads 595 ->
 // 522 us / 646 -> 788 us.
-constexpr long long kSegmentsMaxStreams = 148;
+constexpr long long kSegmentsMaxStreams = kSMs;
 constexpr int kSegmentsMinTokens = 128;
 
 static bool use_segments(const KArgs &ka, int B, int max_tokens, bool exact, unsigned flags)

@@ -7,6 +7,8 @@
 
 namespace adkv {
 
+constexpr int kSMs = 148, kSchedulers = 4 * kSMs;   // B200: what the choice of a kernel by number of streams counts in
+
 static inline ParamPtrs to_ptrs(const adkv_params *p)
 {
     return ParamPtrs{static_cast<const __half *>(p->zp_init), static_cast<const __half *>(p->scale_init),

@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(32 * kNarrowSlices) forward_ov_split_kernel(VA
 // Measured on a B200, 4-bit, 32 heads, the whole qk -> torch softmax -> ov sequence: 1 x 1000 tokens 136 -> 124 us, 4 x 2000
 // tokens 247 -> 224 us, 16 x 1023 tokens 146 -> 140 us (with the weights fetched ahead, adkv_io.cuh, which alone takes
 // 32 x 1000 tokens from 183 to 177 us).  Above it the schedulers are busy and the split only repeats work.
-constexpr int kOvSplitMaxStreams = 592;
+constexpr int kOvSplitMaxStreams = kSchedulers;
 
 }  // namespace adkv
 

@@ -486,9 +486,10 @@ def decode_attn(q, k_cache, v_cache, k_new, v_new, k_params, v_params, T: int, s
     processed in independent segments; ``scratch`` (uint8/any dtype, at least :func:`decode_scratch_bytes`) is
     allocated per call when not given.
 
-    ``split_channels``: None lets the library choose between one warp per tensor and stream and a head split
-    over two warp pairs (launches with few streams); True / False force one (head dim 128, fp32 arithmetic,
-    no checkpoints)."""
+    ``split_channels``: None lets the library choose between one warp per tensor and stream, a head split over two
+    warp pairs (launches with few streams) and, next to tails with the contracted replay, a token axis split over eight
+    warp pairs (up to 148 streams of 128 tokens or more).  True / False force the second / the first (head dim 128,
+    fp32 arithmetic, no checkpoints)."""
     _require(q.dtype == torch.float16, "q must be float16")
     _require(k_new.dtype == torch.float16 and v_new.dtype == torch.float16, "k_new / v_new must be float16")
     B, Hkv, n_super_cap, D = _cache_dims(k_cache, "k_cache")

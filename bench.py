@@ -889,7 +889,10 @@ def run_ours(args, w, name):
                                     "over_32_layers": seqs_job * args.steps / (total_ms * 1e-3) / 32},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_source": peak_src, "frac_of_8TBps_nominal": achieved / 8000.0,
-                         "traffic": NCU_TRAFFIC_BYTES.get(name) if world == 1 else None, "kernel": "fused decode step",
+                         "traffic": NCU_TRAFFIC_BYTES.get(name) if world == 1 else None,
+                         # what the traffic was captured from; other layouts take shards of few streams and checkpoints
+                         "kernel": "decode_attn_kernel" if w["B"] * w["Hkv"] > 160 and not args.ckpt_interval and not half
+                         else "fused decode step",
                          "algorithmic_bytes_per_launch": bytes_rank, "avg_launch_ms": avg_launch_ms,
                          "median_launch_ms": statistics.median(per_launch_ms)},
             "clocks": sampler.summary(t_wall0, t_wall1),

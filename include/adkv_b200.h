@@ -67,11 +67,19 @@ extern "C" {
  * of advancing it over that token.  The call can then be repeated with the same T (the appended code overwrites
  * itself): benchmarks that time one step over and over, and callers that may still reject the token. */
 #define ADKV_FLAG_TAIL_KEEP 4u
-/* adkv_decode_attn, head dim 128, fp32 arithmetic: how the channels of a head are laid over warps.  By default the
- * library decides from the number of (batch, kv head) streams of the call: a launch with very few streams (about
- * one per SM or fewer) splits every head over two K warps and two V warps so that the GPU has more warps to
- * interleave; larger launches keep one warp per tensor and stream, which needs fewer instructions in all.  Results agree up to the summation order of the logits.  These two flags force one
- * or the other (tests, tuning); with both set, SPLIT wins. */
+/* adkv_decode_attn, head dim 128, fp32 arithmetic: how a (batch, kv head) stream is laid over warps.  By default the
+ * library decides from the number of streams and tokens of the call:
+ *   - token segments: next to tail states, with the contracted replay and up to four query heads per KV head, up to 148
+ *     streams (one per SM) of 128 tokens or more are cut along the token axis over eight K and eight V warps;
+ *   - split heads: otherwise, up to 160 streams have the channels of a head split over two K and two V warps;
+ *   - whole heads: everything else keeps one warp per tensor and stream, which needs the fewest instructions in all.
+ * Next to tail states appended codes and tails do not depend on the layout, bit for bit.  Outputs of split and whole
+ * heads agree up to the summation order of the logits; token segments start from products of the scale factors before
+ * them and merge partial softmax sums, and stay as close to exact arithmetic as a whole head does.
+ * SPLIT forces split heads, NO_SPLIT whole heads (tests, tuning; with both set, SPLIT wins); either one rules out token
+ * segments, and nothing forces those.  adkv_decode_attn_varlen has no split heads: up to 148 streams of a cache with room
+ * for 128 tokens or more take token segments under the same conditions, the rest, and calls with either flag, whole
+ * heads. */
 #define ADKV_FLAG_SPLIT_CHANNELS 8u
 #define ADKV_FLAG_NO_SPLIT_CHANNELS 16u
 /* Self-test of the failure path of adkv_decode_attn_ckpt (no counterpart in the reference): the K warps return at
@@ -136,7 +144,8 @@ typedef struct adkv_layer_kv {
 } adkv_layer_kv;
 
 /* adkv_encode_kv / adkv_append_kv for several layers at once: `layers` is a HOST array of n_layers descriptors, all
- * layers share shapes, bits and clamp bounds, and K and V of up to 8 layers go into one launch.  No counterpart in the
+ * layers share shapes, bits and clamp bounds, and K and V of up to 8 layers (encode) or 32 (append; 8 where a pointer
+ * is aligned only to its type) go into one launch.  No counterpart in the
  * reference, which quantises one tensor per call (src/adkv/hf/llama_adkv.py:144-153).  For callers that hold the
  * fp16 K/V of many layers at once -- converting an existing fp16 cache, or appending the token of a step to every
  * layer's cache after the layers have run: the quantiser is bound by its token-sequential chain and by launch
