@@ -84,11 +84,12 @@ __global__ void __launch_bounds__(32 * kNarrowSlices) forward_ov_split_kernel(VA
     v_warp_n<BITS, G, EXACT ? kArithCanon : kArithFma>(va, seg, b, h, lane, vbuf[sl], vbar[sl], wts[sl], src);
 }
 
-// forward_ov splits a stream over two warps up to this many streams per launch: one per warp scheduler of the chip.
-// Measured on a B200, 4-bit, 32 heads, the whole qk -> torch softmax -> ov sequence: 1 x 1000 tokens 136 -> 124 us, 4 x 2000
-// tokens 247 -> 224 us, 16 x 1023 tokens 146 -> 140 us (with the weights fetched ahead, adkv_io.cuh, which alone takes
-// 32 x 1000 tokens from 183 to 177 us).  Above it the schedulers are busy and the split only repeats work.
-constexpr int kOvSplitMaxStreams = kSchedulers;
+// forward_ov splits a stream over two warps while each of them has a scheduler to itself: up to 296 streams.  Measured on
+// a B200, 4-bit, 32 heads, 1000 tokens, canonical replay where no scale meets a clamp / where one channel of every head
+// rests at a bound; contracted replay, the same:
+//    256 streams, one warp without the weights fetched ahead -> two warps   50.2 -> 40.9 / 63.3 -> 53.1;  44.1 -> 38.7 / 53.6 -> 50.5 us
+//    512 streams, one warp with the weights fetched ahead -> two warps      49.1 -> 49.9 / 61.5 -> 69.2;  41.5 -> 45.9 / 51.7 -> 64.3 us
+constexpr int kOvSplitMaxStreams = kSchedulers / 2;
 
 }  // namespace adkv
 
