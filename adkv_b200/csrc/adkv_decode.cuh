@@ -99,12 +99,22 @@ struct StreamRing {
 
 // ---------------------------------------------------------------------------------- K side
 
+// Tokens between two sums over the lanes (reduce_lanes): rows of per-lane partial dot products that a K warp keeps, RT
+// below.  Sixteen halve the number of sums and save a shuffle in each; forward_qk and the narrow kernel, where a K warp
+// has its scheduler to itself, take them (the three calls of a step at 512 streams x 1023 tokens 128.0 -> 122.3 us, narrow
+// heads at 256 streams x 4096 tokens 232 -> 228 us).  The fused kernels keep eight: the larger transpose and another
+// register allocation cost them more (4096 streams x 4096 tokens 1469 -> 1480 us, 512 streams x 2000 tokens with four
+// query heads 220 -> 230 us).  Eight query heads have no room for sixteen rows each.
+template <int G>
+constexpr int kRedTok = G > 4 ? 8 : 16;
+constexpr int kRedRow = kD / 4 + 4;   // floats a row: 32 partial sums and 4 of padding, so that 16-byte loads of 8 rows meet 32 banks
+
 // Replay 8 tokens (fields 0..7 of the 4 words in `w`; the caller shifts the second half of a 16-token
-// word down) and leave the per-lane partial dot products of head g, token j in red[(g*8 + j)*36 + lane].
+// word down) and leave the per-lane partial dot products of head g, token j in red[(g*RT + j)*kRedRow + lane].
 // The two halves of 4 tokens run through ONE body in a two-trip loop, which halves the straight-line
 // code (with several query heads per KV head the unrolled body no longer fitted the instruction
 // cache).  `count`: valid fields when PARTIAL (the others are stored as zero).
-template <int BITS, int G, bool EXACT, bool PARTIAL, bool GUARDED>
+template <int BITS, int G, bool EXACT, bool PARTIAL, int RT>
 __device__ __forceinline__ void k_chunk(const uint4 &w, const FieldConsts<BITS> &fc, Chan (&ch)[4],
                                         const float (&qv)[G][4], float *red, int lane, int count, float smin,
                                         float smax)
@@ -120,7 +130,7 @@ __device__ __forceinline__ void k_chunk(const uint4 &w, const FieldConsts<BITS> 
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const float q = fc.template code<k>(grp[c]);
-                    const float xh = replay_step<EXACT, GUARDED>(q, ch[c], smin, smax);
+                    const float xh = replay_step<EXACT, true>(q, ch[c], smin, smax);
 #pragma unroll
                     for (int g = 0; g < G; ++g) part[g] = c == 0 ? qv[g][0] * xh : fmaf(qv[g][c], xh, part[g]);
                 }
@@ -129,19 +139,20 @@ __device__ __forceinline__ void k_chunk(const uint4 &w, const FieldConsts<BITS> 
                 for (int g = 0; g < G; ++g) part[g] = 0.f;
             }
 #pragma unroll
-            for (int g = 0; g < G; ++g) red[(g * 8 + 4 * half + k) * 36 + lane] = part[g];
+            for (int g = 0; g < G; ++g) red[(g * RT + 4 * half + k) * kRedRow + lane] = part[g];
         });
 #pragma unroll
         for (int c = 0; c < 4; ++c) grp[c] >>= 4 * BITS;
     }
 }
 
-// The unguarded, full 8-token case of k_chunk on channel pairs (packed fp32): identical results for the
+// The full 8-token case of k_chunk on channel pairs (packed fp32), without the eps guard, and without the clamps unless
+// CLAMP: identical results for the
 // state; the per-lane partial dot product is summed in a different order (pairs first).
-template <int BITS, int G, bool EXACT>
+template <int BITS, int G, bool EXACT, bool CLAMP, int RT>
 __device__ __forceinline__ void k_chunk2(const uint4 &w, const FieldConsts<BITS> &fc, Chan (&ch)[4],
                                          const PairConst (&pc)[2], f32x2 one, const f32x2 (&qv2)[G][2], float *red,
-                                         int lane)
+                                         int lane, float smin, float smax)
 {
     uint32_t grp[4] = {w.x, w.y, w.z, w.w};
     f32x2 zp[2] = {pk2(ch[0].zp, ch[1].zp), pk2(ch[2].zp, ch[3].zp)};
@@ -154,7 +165,7 @@ __device__ __forceinline__ void k_chunk2(const uint4 &w, const FieldConsts<BITS>
 #pragma unroll
             for (int p = 0; p < 2; ++p) {
                 const f32x2 q2 = fc.template code2<k>(grp[2 * p], grp[2 * p + 1]);
-                const f32x2 xh = replay_step2<EXACT>(q2, zp[p], s[p], pc[p], one);
+                const f32x2 xh = replay_step2<EXACT, CLAMP>(q2, zp[p], s[p], pc[p], one, smin, smax);
 #pragma unroll
                 for (int g = 0; g < G; ++g) part[g] = p == 0 ? mul2(qv2[g][0], xh) : fma2(qv2[g][1], xh, part[g]);
             }
@@ -162,7 +173,7 @@ __device__ __forceinline__ void k_chunk2(const uint4 &w, const FieldConsts<BITS>
             for (int g = 0; g < G; ++g) {
                 float a, b;
                 upk2(part[g], a, b);
-                red[(g * 8 + 4 * half + k) * 36 + lane] = a + b;
+                red[(g * RT + 4 * half + k) * kRedRow + lane] = a + b;
             }
         });
 #pragma unroll
@@ -174,22 +185,33 @@ __device__ __forceinline__ void k_chunk2(const uint4 &w, const FieldConsts<BITS>
     upk2(s[1], ch[2].s, ch[3].s);
 }
 
-// Sum the partials left by k_chunk over the 32 lanes: each lane reads 8 lanes' values of one token
-// (two 16-byte loads from the padded transpose) and two shuffles finish the job; afterwards lane l
-// (every lane, replicated over l>>3) holds the full sum for token (l & 7) of head g.
-// red: float [G][8][36] of this warp.
-template <int G>
-__device__ __forceinline__ void reduce8(const float *red, int lane, float (&sum)[G])
+// Sum the partials left by k_chunk over the 32 lanes: each lane adds up RT of the partial sums of one token (16-byte loads
+// from the padded transpose) and log2(32 / RT) shuffles finish the job; afterwards lane l (every lane, replicated over
+// l / RT) holds the full sum for token l % RT of head g.
+// red: float [G][RT][kRedRow] of this warp.
+template <int G, int RT>
+__device__ __forceinline__ void reduce_lanes(const float *red, int lane, float (&sum)[G])
 {
     __syncwarp();
-    const int row = lane & 7, cb = (lane >> 3) * 8;
+    constexpr int N = RT / 4;   // 16-byte loads of a lane
+    const float *at = red + (lane % RT) * kRedRow + (lane / RT) * RT;
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-        const float4 a = *reinterpret_cast<const float4 *>(&red[(g * 8 + row) * 36 + cb]);
-        const float4 b = *reinterpret_cast<const float4 *>(&red[(g * 8 + row) * 36 + cb + 4]);
-        float s = ((a.x + a.y) + (a.z + a.w)) + ((b.x + b.y) + (b.z + b.w));
-        s += __shfl_xor_sync(kFull, s, 8);
-        s += __shfl_xor_sync(kFull, s, 16);
+        f32x2 v[N];
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const ulonglong2 r = *reinterpret_cast<const ulonglong2 *>(at + g * RT * kRedRow + 4 * i);
+            v[i] = add2(r.x, r.y);
+        }
+#pragma unroll
+        for (int n = N / 2; n > 0; n /= 2)
+#pragma unroll
+            for (int i = 0; i < n; ++i) v[i] = add2(v[i], v[i + n]);
+        float a, b;
+        upk2(v[0], a, b);
+        float s = a + b;
+#pragma unroll
+        for (int o = RT; o < 32; o *= 2) s += __shfl_xor_sync(kFull, s, o);
         sum[g] = s;
     }
     __syncwarp();
@@ -294,15 +316,47 @@ template <int G>
 struct QueryRegs {
     float v[G][4];
 };
-template <int BITS, int G, bool EXACT>
+template <int BITS, int G, bool EXACT, int RT>
 __device__ __noinline__ Chan4 k_chunk_guarded(uint4 w, Chan4 st, QueryRegs<G> q, float *red, int lane, int count,
                                               float smin, float smax)
 {
     FieldConsts<BITS> fc;
     fc.init();
-    k_chunk<BITS, G, EXACT, true, true>(w, fc, st.c, q.v, red, lane, count, smin, smax);
+    k_chunk<BITS, G, EXACT, true, RT>(w, fc, st.c, q.v, red, lane, count, smin, smax);
     return st;
 }
+
+// The packed body with clamps as a function call, for the kernels that keep the rare bodies out of line.
+template <int G>
+struct QueryPairs {
+    f32x2 v[G][2];
+};
+struct PairConsts {
+    PairConst c[2];
+};
+template <int BITS, int G, bool EXACT, int RT>
+__device__ __noinline__ Chan4 k_chunk_clamped(uint4 w, Chan4 st, PairConsts pc, QueryPairs<G> q, float *red, int lane, float smin,
+                                              float smax)
+{
+    FieldConsts<BITS> fc;
+    fc.init();
+    k_chunk2<BITS, G, EXACT, true, RT>(w, fc, st.c, pc.c, opaque_ones2(), q.v, red, lane, smin, smax);
+    return st;
+}
+
+// The eps guard is the identity on a scale that is not below eps, and after one update no scale is below smin: with smin
+// at eps or above, and initial scales too, only the clamps are left of the guards (a NaN does not count as above).
+__device__ __forceinline__ bool no_eps_guard(const Chan (&ch)[4], float smin)
+{
+    return __all_sync(kFull, smin >= kEps && ch[0].s >= kEps && ch[1].s >= kEps && ch[2].s >= kEps && ch[3].s >= kEps);
+}
+
+// Whether chunks that may meet a clamp bound, but not the eps guard, take the packed body with clamps; otherwise the scalar
+// body.  Measured on a B200, scalar -> packed: one query head per KV head 4096 x 4096 tokens 1474 -> 1445 us (6 % of the
+// chunks), 4096 x 128 72.7 -> 63.8 us, 2048 x 1000 with a channel per head at a bound 317 -> 227 us; four heads 512 x 2000
+// 220 -> 231 us, two heads 1024 x 2000 300 -> 302 us (a third body next to unrolled heads costs registers everywhere).
+template <int G>
+constexpr bool kPackedClamps = G == 1;
 
 // A sink or source may want the state a scan without append ended in (end_state is optional): the segment kernel does.
 template <class S, int G>
@@ -318,17 +372,18 @@ __device__ __forceinline__ void src_end_state(S &, const Chan (&)[4], int, long)
 
 // Sink interface (duck-typed):
 //   bool begin_tile(int i)            wait for room; false = bounded wait gave up
-//   void put8(int i, int g, int tok_in_tile, float v, int lane)   called by lanes 0..7 with tok = base + lane
+//   void put<N>(int i, int g, int base, float v, int lane)   lanes 0 .. N-1 hold the logits of tokens base + lane of the tile;
+//                                     those past the last token of a stream are anything and have to be dropped
 //   void end_tile(int i, int lane)
 //   void put_self(int g, float v)     lane 0
 //   void finish(int lane)
-template <int BITS, int G, int ARITH, class Sink, int STAGES = kStages, bool WIDE = false, bool OUTLINE = false>
+template <int BITS, int G, int ARITH, class Sink, int STAGES = kStages, bool WIDE = false, bool OUTLINE = false, int RT = 8>
 __device__ __forceinline__ void k_warp(const KArgs &a, const Seg &seg, int b, int h, int lane, uint8_t *ring_buf,
                                        uint64_t *ring_bar, float *red, Sink &sink)
 {
     using C = Codec<BITS>;
     constexpr bool EXACT = ARITH == kArithCanon;
-    const int bh = b * a.Hkv + h;
+        const int bh = b * a.Hkv + h;
     const int D = WIDE ? a.D : kD, slice = WIDE ? seg.slice : 0;
     const int c0 = kD * slice + 4 * lane;      // first of this lane's 4 channels within the head
     const uint32_t row_stride = uint32_t(D) * 4;
@@ -357,9 +412,31 @@ __device__ __forceinline__ void k_warp(const KArgs &a, const Seg &seg, int b, in
     }
 
 
-    auto guarded = [&](const uint4 &w, int count, auto partial_tag) {
+    const bool tame = no_eps_guard(ch, a.smin);
+    // some scale may meet a clamp bound within the eight tokens
+    auto clamped = [&](const uint4 &w, float *rows) {
+        if constexpr (!kPackedClamps<G>) {
+        } else if constexpr (!OUTLINE) {
+            k_chunk2<BITS, G, EXACT, true, RT>(w, fc, ch, pc, one, qv2, rows, lane, a.smin, a.smax);
+        } else {
+            Chan4 st;
+            QueryPairs<G> qp;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) st.c[c] = ch[c];
+#pragma unroll
+            for (int g = 0; g < G; ++g) { qp.v[g][0] = qv2[g][0]; qp.v[g][1] = qv2[g][1]; }
+            st = k_chunk_clamped<BITS, G, EXACT, RT>(w, st, PairConsts{{pc[0], pc[1]}}, qp, rows, lane, a.smin, a.smax);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                ch[c].zp = st.c[c].zp;
+                ch[c].s = st.c[c].s;
+            }
+        }
+    };
+    // the last tokens of a stream, and scales that the eps guard may act on
+    auto guarded = [&](const uint4 &w, float *rows, int count, auto partial) {
         if constexpr (!OUTLINE) {
-            k_chunk<BITS, G, EXACT, decltype(partial_tag)::value, true>(w, fc, ch, qv, red, lane, count, a.smin, a.smax);
+            k_chunk<BITS, G, EXACT, decltype(partial)::value, RT>(w, fc, ch, qv, rows, lane, count, a.smin, a.smax);
         } else {
             Chan4 st;
             QueryRegs<G> qr;
@@ -369,7 +446,7 @@ __device__ __forceinline__ void k_warp(const KArgs &a, const Seg &seg, int b, in
             for (int g = 0; g < G; ++g)
 #pragma unroll
                 for (int c = 0; c < 4; ++c) qr.v[g][c] = qv[g][c];
-            st = k_chunk_guarded<BITS, G, EXACT>(w, st, qr, red, lane, count, a.smin, a.smax);
+            st = k_chunk_guarded<BITS, G, EXACT, RT>(w, st, qr, rows, lane, count, a.smin, a.smax);
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 ch[c].zp = st.c[c].zp;
@@ -385,7 +462,12 @@ __device__ __forceinline__ void k_warp(const KArgs &a, const Seg &seg, int b, in
         if (!(ok = sink.begin_tile(i))) break;
         const uint4 *tile = ring.tile(i, lane);
         const int ntok = min(kTileTok, n_tok - i * kTileTok);
-        float sum[G];
+        const auto logits = [&](int base) {
+            float sum[G];
+            reduce_lanes<G, RT>(red, lane, sum);
+#pragma unroll
+            for (int g = 0; g < G; ++g) sink.template put<RT>(i, g, base, sum[g], lane);
+        };
         if (ntok == kTileTok) {
             // not unrolled over the words of the tile: the loop body must stay resident in the
             // instruction cache while K and V warps of many streams interleave
@@ -395,11 +477,12 @@ __device__ __forceinline__ void k_warp(const KArgs &a, const Seg &seg, int b, in
                 const uint4 w_next = tile[min(wd + 1, Tile<BITS>::WORDS - 1) * (kD / 4)];
 #pragma unroll 1
                 for (int c8 = 0; c8 < C::TPW / 8; ++c8) {
-                    if (safe.holds(ch)) k_chunk2<BITS, G, EXACT>(w, fc, ch, pc, one, qv2, red, lane);
-                    else guarded(w, 8, std::false_type{});
-                    reduce8<G>(red, lane, sum);
-#pragma unroll
-                    for (int g = 0; g < G; ++g) sink.put8(i, g, wd * C::TPW + c8 * 8, sum[g], lane);
+                    const int t = wd * C::TPW + c8 * 8;
+                    float *rows = red + t % RT * kRedRow;
+                    if (safe.holds(ch)) k_chunk2<BITS, G, EXACT, false, RT>(w, fc, ch, pc, one, qv2, rows, lane, a.smin, a.smax);
+                    else if (kPackedClamps<G> && tame) clamped(w, rows);
+                    else guarded(w, rows, 8, std::bool_constant<kPackedClamps<G>>{});   // a body less where this is rare
+                    if ((t + 8) % RT == 0) logits(t + 8 - RT);
                     if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
                 }
                 w = w_next;
@@ -408,13 +491,11 @@ __device__ __forceinline__ void k_warp(const KArgs &a, const Seg &seg, int b, in
 #pragma unroll 1
             for (int wd = 0; wd * C::TPW < ntok; ++wd) {
                 uint4 w = tile[wd * (kD / 4)];
-                const int count = ntok - wd * C::TPW;   // valid fields in this word (may exceed TPW)
 #pragma unroll 1
-                for (int c8 = 0; c8 < C::TPW / 8 && c8 * 8 < count; ++c8) {
-                    guarded(w, count - c8 * 8, std::true_type{});
-                    reduce8<G>(red, lane, sum);
-#pragma unroll
-                    for (int g = 0; g < G; ++g) sink.put8(i, g, wd * C::TPW + c8 * 8, sum[g], lane);
+                for (int c8 = 0; c8 < C::TPW / 8 && wd * C::TPW + c8 * 8 < ntok; ++c8) {
+                    const int t = wd * C::TPW + c8 * 8;
+                    guarded(w, red + t % RT * kRedRow, ntok - t, std::true_type{});
+                    if ((t + 8) % RT == 0 || t + 8 >= ntok) logits(t / RT * RT);
                     if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
                 }
             }
@@ -452,7 +533,7 @@ __device__ __forceinline__ void k_warp(const KArgs &a, const Seg &seg, int b, in
 
 // ---------------------------------------------------------------------------------- V side
 
-template <int BITS, int G, bool EXACT, bool PARTIAL, bool GUARDED>
+template <int BITS, int G, bool EXACT, bool PARTIAL>
 __device__ __forceinline__ void v_chunk(const uint4 &w, const FieldConsts<BITS> &fc, Chan (&ch)[4],
                                         const float2 *wts /* [G][32] smem, each weight twice */, int tok0,
                                         float (&acc)[G][4], int count, float smin, float smax)
@@ -473,7 +554,7 @@ __device__ __forceinline__ void v_chunk(const uint4 &w, const FieldConsts<BITS> 
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
                     const float q = fc.template code<k>(grp[c]);
-                    const float xh = replay_step<EXACT, GUARDED>(q, ch[c], smin, smax);
+                    const float xh = replay_step<EXACT, true>(q, ch[c], smin, smax);
 #pragma unroll
                     for (int g = 0; g < G; ++g) acc[g][c] = fmaf(wt[g][k], xh, acc[g][c]);
                 }
@@ -484,12 +565,12 @@ __device__ __forceinline__ void v_chunk(const uint4 &w, const FieldConsts<BITS> 
     }
 }
 
-// The unguarded, full 8-token case of v_chunk on channel pairs (packed fp32).  `wts2` holds every weight
+// The full 8-token case of v_chunk on channel pairs (packed fp32), guards as in k_chunk2.  `wts2` holds every weight
 // twice ([G][32] float2) so that one 8-byte load yields the packed multiplier.
-template <int BITS, int G, bool EXACT>
+template <int BITS, int G, bool EXACT, bool CLAMP>
 __device__ __forceinline__ void v_chunk2(const uint4 &w, const FieldConsts<BITS> &fc, Chan (&ch)[4],
                                          const PairConst (&pc)[2], f32x2 one, const float2 *wts2, int tok0,
-                                         float (&acc)[G][4])
+                                         float (&acc)[G][4], float smin, float smax)
 {
     uint32_t grp[4] = {w.x, w.y, w.z, w.w};
     f32x2 zp[2] = {pk2(ch[0].zp, ch[1].zp), pk2(ch[2].zp, ch[3].zp)};
@@ -514,7 +595,7 @@ __device__ __forceinline__ void v_chunk2(const uint4 &w, const FieldConsts<BITS>
 #pragma unroll
             for (int p = 0; p < 2; ++p) {
                 const f32x2 q2 = fc.template code2<k>(grp[2 * p], grp[2 * p + 1]);
-                const f32x2 xh = replay_step2<EXACT>(q2, zp[p], s[p], pc[p], one);
+                const f32x2 xh = replay_step2<EXACT, CLAMP>(q2, zp[p], s[p], pc[p], one, smin, smax);
 #pragma unroll
                 for (int g = 0; g < G; ++g) acc2[g][p] = fma2(wt[g][k], xh, acc2[g][p]);
             }
@@ -572,7 +653,17 @@ __device__ __noinline__ VState<G> v_chunk_guarded(uint4 w, VState<G> st, const f
 {
     FieldConsts<BITS> fc;
     fc.init();
-    v_chunk<BITS, G, EXACT, true, true>(w, fc, st.c, wts, tok0, st.acc, count, smin, smax);
+    v_chunk<BITS, G, EXACT, true>(w, fc, st.c, wts, tok0, st.acc, count, smin, smax);
+    return st;
+}
+
+template <int BITS, int G, bool EXACT>
+__device__ __noinline__ VState<G> v_chunk_clamped(uint4 w, VState<G> st, PairConsts pc, const float2 *wts, int tok0, float smin,
+                                                  float smax)
+{
+    FieldConsts<BITS> fc;
+    fc.init();
+    v_chunk2<BITS, G, EXACT, true>(w, fc, st.c, pc.c, opaque_ones2(), wts, tok0, st.acc, smin, smax);
     return st;
 }
 
@@ -607,28 +698,37 @@ __device__ __forceinline__ void v_warp(const VArgs &a, const Seg &seg, int b, in
         for (int c = 0; c < 4; ++c) acc[g][c] = 0.f;
 
 
-    auto guarded = [&](const uint4 &w, int tok0, int count, auto partial_tag) {
-        if constexpr (!OUTLINE) {
-            v_chunk<BITS, G, EXACT, decltype(partial_tag)::value, true>(w, fc, ch, wts, tok0, acc, count, a.smin, a.smax);
-        } else {
-            VState<G> st;
+    const bool tame = no_eps_guard(ch, a.smin);
+    const auto out_of_line = [&](auto &&body) {   // body: state -> state after the chunk
+        VState<G> st;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) st.c[c] = ch[c];
+        for (int c = 0; c < 4; ++c) st.c[c] = ch[c];
 #pragma unroll
-            for (int g = 0; g < G; ++g)
+        for (int g = 0; g < G; ++g)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) st.acc[g][c] = acc[g][c];
-            st = v_chunk_guarded<BITS, G, EXACT>(w, st, wts, tok0, count, a.smin, a.smax);
+            for (int c = 0; c < 4; ++c) st.acc[g][c] = acc[g][c];
+        st = body(st);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                ch[c].zp = st.c[c].zp;
-                ch[c].s = st.c[c].s;
-            }
-#pragma unroll
-            for (int g = 0; g < G; ++g)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[g][c] = st.acc[g][c];
+        for (int c = 0; c < 4; ++c) {
+            ch[c].zp = st.c[c].zp;
+            ch[c].s = st.c[c].s;
         }
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[g][c] = st.acc[g][c];
+    };
+    // as in k_warp
+    auto clamped = [&](const uint4 &w, int tok0) {
+        if constexpr (!kPackedClamps<G>) {
+        } else if constexpr (!OUTLINE) v_chunk2<BITS, G, EXACT, true>(w, fc, ch, pc, one, wts, tok0, acc, a.smin, a.smax);
+        else out_of_line([&](const VState<G> &st) {
+            return v_chunk_clamped<BITS, G, EXACT>(w, st, PairConsts{{pc[0], pc[1]}}, wts, tok0, a.smin, a.smax);
+        });
+    };
+    auto guarded = [&](const uint4 &w, int tok0, int count, auto partial) {
+        if constexpr (!OUTLINE) v_chunk<BITS, G, EXACT, decltype(partial)::value>(w, fc, ch, wts, tok0, acc, count, a.smin, a.smax);
+        else out_of_line([&](const VState<G> &st) { return v_chunk_guarded<BITS, G, EXACT>(w, st, wts, tok0, count, a.smin, a.smax); });
     };
 
     bool ok = true;
@@ -646,8 +746,9 @@ __device__ __forceinline__ void v_warp(const VArgs &a, const Seg &seg, int b, in
 #pragma unroll 1
                 for (int c8 = 0; c8 < C::TPW / 8; ++c8) {
                     const int tok0 = wd * C::TPW + c8 * 8;
-                    if (safe.holds(ch)) v_chunk2<BITS, G, EXACT>(w, fc, ch, pc, one, wts, tok0, acc);
-                    else guarded(w, tok0, 8, std::false_type{});
+                    if (safe.holds(ch)) v_chunk2<BITS, G, EXACT, false>(w, fc, ch, pc, one, wts, tok0, acc, a.smin, a.smax);
+                    else if (kPackedClamps<G> && tame) clamped(w, tok0);
+                    else guarded(w, tok0, 8, std::bool_constant<kPackedClamps<G>>{});
                     if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
                 }
                 w = w_next;

@@ -214,10 +214,10 @@ __device__ __forceinline__ void make_pair_consts(const Chan (&ch)[4], PairConst 
     }
 }
 
-// Unguarded decoder step on a channel pair: same operations, same order, same roundings as
-// replay_step<EXACT, false> on each element.
-template <bool EXACT>
-__device__ __forceinline__ f32x2 replay_step2(f32x2 q2, f32x2 &zp, f32x2 &s, const PairConst &c, f32x2 one)
+// Decoder step on a channel pair without the eps guard: same operations, same order, same roundings as
+// replay_step<EXACT, false> on each element; with CLAMP the scale is clamped as by replay_step<EXACT, true>.
+template <bool EXACT, bool CLAMP>
+__device__ __forceinline__ f32x2 replay_step2(f32x2 q2, f32x2 &zp, f32x2 &s, const PairConst &c, f32x2 one, float smin, float smax)
 {
     const f32x2 rh = mul2(q2, s);
     const f32x2 xh = add_product2(rh, one, zp);
@@ -228,6 +228,11 @@ __device__ __forceinline__ f32x2 replay_step2(f32x2 q2, f32x2 &zp, f32x2 &s, con
     } else {
         zp = fma2(c.alpha, rh, zp);
         s = mul2(s, fma2(c.beta, aq, c.tc));
+    }
+    if (CLAMP) {
+        float lo, hi;
+        upk2(s, lo, hi);
+        s = pk2(fminf(fmaxf(lo, smin), smax), fminf(fmaxf(hi, smin), smax));
     }
     return xh;
 }

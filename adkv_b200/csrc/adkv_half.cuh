@@ -198,7 +198,7 @@ __device__ __forceinline__ void k_chunk_h(const uint4 &w, HPair (&hp)[2], const 
 
 // Sum the partials left by k_chunk_h over the 32 lanes and the two halves (fp16, as the reference's butterfly
 // does).  Afterwards lane l (every lane, replicated over l>>3) holds the sum for token (l & 7) of head g as a
-// float: the contract of reduce8.
+// float: the contract of reduce_lanes for 8 tokens.
 template <int G>
 __device__ __forceinline__ void reduce8_h(const uint32_t *red, int lane, float (&sum)[G])
 {
@@ -260,7 +260,7 @@ __device__ __forceinline__ void k_warp_h(const KArgs &a, const Seg &seg, int b, 
                     k_chunk_h<BITS, G, false>(w, hp, qv, red, lane, 8);
                     reduce8_h<G>(red, lane, sum);
 #pragma unroll
-                    for (int g = 0; g < G; ++g) sink.put8(i, g, wd * C::TPW + c8 * 8, sum[g], lane);
+                    for (int g = 0; g < G; ++g) sink.template put<8>(i, g, wd * C::TPW + c8 * 8, sum[g], lane);
                     if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
                 }
                 w = w_next;
@@ -275,7 +275,7 @@ __device__ __forceinline__ void k_warp_h(const KArgs &a, const Seg &seg, int b, 
                     k_chunk_h<BITS, G, true>(w, hp, qv, red, lane, count - c8 * 8);
                     reduce8_h<G>(red, lane, sum);
 #pragma unroll
-                    for (int g = 0; g < G; ++g) sink.put8(i, g, wd * C::TPW + c8 * 8, sum[g], lane);
+                    for (int g = 0; g < G; ++g) sink.template put<8>(i, g, wd * C::TPW + c8 * 8, sum[g], lane);
                     if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
                 }
             }

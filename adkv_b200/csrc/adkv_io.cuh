@@ -12,10 +12,11 @@ struct GlobalLogitSink {
     __half *row[G];   // logits row of each q head of this stream: [T+1]
     int T;
     __device__ __forceinline__ bool begin_tile(int) { return true; }
-    __device__ __forceinline__ void put8(int i, int g, int tok, float v, int lane)
+    template <int N>
+    __device__ __forceinline__ void put(int i, int g, int tok, float v, int lane)
     {
         const int t = i * kTileTok + tok + lane;
-        if (lane < 8 && t < T) row[g][t] = __float2half_rn(v);
+        if (lane < N && t < T) row[g][t] = __float2half_rn(v);
     }
     __device__ __forceinline__ void end_tile(int, int) {}
     __device__ __forceinline__ void put_self(int g, float v) { row[g][T] = __float2half_rn(v); }

@@ -16,7 +16,7 @@ __global__ void __launch_bounds__(64 * kNarrowSlices) decode_attn_narrow_kernel(
     constexpr int S = kNarrowSlices;
     __shared__ alignas(128) uint8_t kbuf[S][kStages * NarrowTile<BITS>::BYTES];
     __shared__ alignas(128) uint8_t vbuf[S][kStages * NarrowTile<BITS>::BYTES];
-    __shared__ alignas(16) float red[S][G * 8 * 36];
+    __shared__ alignas(16) float red[S][G * kRedTok<G> * kRedRow];
     __shared__ alignas(16) float2 wts[S][G * kTileTok];
     __shared__ FusedShared<G, S> fs;
     __shared__ uint64_t kbar[S][kStages], vbar[S][kStages];

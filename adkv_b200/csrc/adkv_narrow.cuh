@@ -166,12 +166,12 @@ __device__ __forceinline__ void k_chunk_n2(const uint2 &w, const FieldConsts<BIT
         static_for<4>([&](auto kc) {
             constexpr int k = decltype(kc)::value;
             const f32x2 q2 = fc.template code2<k>(ga, gb);
-            const f32x2 xh = replay_step2<EXACT>(q2, zp, s, pc, one);
+            const f32x2 xh = replay_step2<EXACT, false>(q2, zp, s, pc, one, 0.f, 0.f);
 #pragma unroll
             for (int g = 0; g < G; ++g) {
                 float a, b;
                 upk2(mul2(qv2[g], xh), a, b);
-                red[(g * 8 + 4 * half + k) * 36 + lane] = a + b;
+                red[(g * kRedTok<G> + 4 * half + k) * kRedRow + lane] = a + b;
             }
         });
         ga >>= 4 * BITS;
@@ -201,7 +201,7 @@ __device__ __forceinline__ void k_chunk_n(const uint2 &w, Chan (&ch)[2], const f
             }
         }
 #pragma unroll
-        for (int g = 0; g < G; ++g) red[(g * 8 + j) * 36 + lane] = part[g];
+        for (int g = 0; g < G; ++g) red[(g * kRedTok<G> + j) * kRedRow + lane] = part[g];
     }
 }
 
@@ -246,20 +246,21 @@ __device__ __forceinline__ void k_warp_n(const KArgs &a, const Seg &seg, int b, 
         if (!(ok = sink.begin_tile(i))) break;
         const uint2 *tile = ring.tile(i, lane);
         const int ntok = min(kTileTok, n_tok - i * kTileTok);
-        float sum[G];
+        constexpr int RT = kRedTok<G>;
+        uint2 w;
 #pragma unroll 1
-        for (int wd = 0; wd * C::TPW < ntok; ++wd) {
-            uint2 w = tile[wd * (kNarrowCh / 2)];
-            const int count = ntok - wd * C::TPW;   // valid fields in this word (may exceed TPW)
-#pragma unroll 1
-            for (int c8 = 0; c8 < C::TPW / 8 && c8 * 8 < count; ++c8) {
-                if (count - c8 * 8 >= 8 && safe.holds(ch)) k_chunk_n2<BITS, G, EXACT>(w, fc, ch, pc, one, qv2, red, lane);
-                else k_chunk_n<BITS, G, EXACT>(w, ch, qv, red, lane, count - c8 * 8, a.smin, a.smax);
-                reduce8<G>(red, lane, sum);
+        for (int t = 0; t < ntok; t += 8) {
+            if (C::TPW == 8 || t % 16 == 0) w = tile[t / C::TPW * (kNarrowCh / 2)];
+            float *rows = red + t % RT * kRedRow;
+            if (ntok - t >= 8 && safe.holds(ch)) k_chunk_n2<BITS, G, EXACT>(w, fc, ch, pc, one, qv2, rows, lane);
+            else k_chunk_n<BITS, G, EXACT>(w, ch, qv, rows, lane, ntok - t, a.smin, a.smax);
+            if ((t + 8) % RT == 0 || t + 8 >= ntok) {
+                float sum[G];
+                reduce_lanes<G, RT>(red, lane, sum);
 #pragma unroll
-                for (int g = 0; g < G; ++g) sink.put8(i, g, wd * C::TPW + c8 * 8, sum[g], lane);
-                if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; }
+                for (int g = 0; g < G; ++g) sink.template put<RT>(i, g, t / RT * RT, sum[g], lane);
             }
+            if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; }
         }
         sink.end_tile(i, lane);
         ring.release_and_refill(i, lane);
@@ -306,7 +307,7 @@ __device__ __forceinline__ void v_chunk_n2(const uint2 &w, const FieldConsts<BIT
         static_for<4>([&](auto kc) {
             constexpr int k = decltype(kc)::value;
             const f32x2 q2 = fc.template code2<k>(ga, gb);
-            const f32x2 xh = replay_step2<EXACT>(q2, zp, s, pc, one);
+            const f32x2 xh = replay_step2<EXACT, false>(q2, zp, s, pc, one, 0.f, 0.f);
 #pragma unroll
             for (int g = 0; g < G; ++g) acc2[g] = fma2(wt[g][k], xh, acc2[g]);
         });

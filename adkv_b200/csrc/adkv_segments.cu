@@ -39,7 +39,7 @@ constexpr int kPartFloats = 4 + kD;   // per (segment, head): maximum (log2 unit
 template <int BITS, int G>
 struct SegShared {
     alignas(128) uint8_t buf[2][NS][kSegStages * Tile<BITS>::BYTES];
-    alignas(16) float red[NS][G * 8 * 36];
+    alignas(16) float red[NS][G * 8 * kRedRow];
     alignas(16) float2 wts[NS][G * kTileTok];
     union {
         alignas(16) float comp[2][NS][3][kD];     // steps 1 and 2: product, smallest and largest running product

@@ -31,9 +31,10 @@ struct RingSink {
         slot = i % kLogitSlots;
         return mbar_wait_bounded(&sh->lempty[slot], ((i / kLogitSlots) & 1) ^ 1, kStatLEmptyWait);
     }
-    __device__ __forceinline__ void put8(int, int g, int tok, float v, int lane)
+    template <int N>
+    __device__ __forceinline__ void put(int, int g, int tok, float v, int lane)
     {
-        if (lane < 8) sh->lring[slot][sl][g][tok + lane] = v;
+        if (lane < N) sh->lring[slot][sl][g][tok + lane] = v;
     }
     __device__ __forceinline__ void end_tile(int, int lane)
     {

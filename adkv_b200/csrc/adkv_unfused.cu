@@ -15,7 +15,7 @@ __global__ void __launch_bounds__(32 * kStreamsPerCta) forward_qk_kernel(KArgs k
                                                                          int n_streams)
 {
     __shared__ alignas(128) uint8_t kbuf[kStreamsPerCta][kStages * Tile<BITS>::BYTES];
-    __shared__ alignas(16) float red[kStreamsPerCta][G * 8 * 36];
+    __shared__ alignas(16) float red[kStreamsPerCta][G * kRedTok<G> * kRedRow];
     __shared__ uint64_t kbar[kStreamsPerCta][kStages];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane == 0) {
@@ -31,7 +31,8 @@ __global__ void __launch_bounds__(32 * kStreamsPerCta) forward_qk_kernel(KArgs k
     for (int g = 0; g < G; ++g) sink.row[g] = logits + (size_t(b) * ka.Hq + size_t(h) * G + g) * (ka.T + 1);
     sink.T = ka.T;
     const Seg seg{0, ka.T, true, nullptr, nullptr, 0};
-    k_warp<BITS, G, EXACT>(ka, seg, b, h, lane, kbuf[warp], kbar[warp], red[warp], sink);
+    k_warp<BITS, G, EXACT, GlobalLogitSink<G>, kStages, false, false, kRedTok<G>>(ka, seg, b, h, lane, kbuf[warp], kbar[warp],
+                                                                                    red[warp], sink);
 }
 
 template <int BITS, int G, bool EXACT>

@@ -25,7 +25,7 @@ __global__ void __launch_bounds__(64 * S) decode_attn_wide_kernel(KArgs ka, VArg
     constexpr int ST = WideCfg<S>::STAGES;
     __shared__ alignas(128) uint8_t kbuf[S][ST * Tile<BITS>::BYTES];
     __shared__ alignas(128) uint8_t vbuf[S][ST * Tile<BITS>::BYTES];
-    __shared__ alignas(16) float red[S][G * 8 * 36];
+    __shared__ alignas(16) float red[S][G * 8 * kRedRow];
     __shared__ alignas(16) float2 wts[S][G * kTileTok];
     __shared__ FusedShared<G, S> fs;
     __shared__ uint64_t kbar[S][ST], vbar[S][ST];
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(32 * S) forward_qk_wide_kernel(KArgs ka, __hal
 {
     constexpr int ST = WideCfg<S>::STAGES;
     __shared__ alignas(128) uint8_t kbuf[S][ST * Tile<BITS>::BYTES];
-    __shared__ alignas(16) float red[S][G * 8 * 36];
+    __shared__ alignas(16) float red[S][G * 8 * kRedRow];
     __shared__ FusedShared<G, S> fs;
     __shared__ uint64_t kbar[S][ST];
     const int bh = blockIdx.x, b = bh / ka.Hkv, h = bh % ka.Hkv;
