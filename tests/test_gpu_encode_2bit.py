@@ -1,0 +1,68 @@
+"""2-bit prefill of few streams (codes from comparisons) against the oracle and against the quotient form that launches with
+many streams take, bit for bit.  Needs a B200."""
+import numpy as np
+import pytest
+import torch
+
+from adkv_b200 import gemv, synth
+from oracle import adkv_oracle as orc
+from tests.util import SMAX, SMIN, np_params
+
+pytestmark = pytest.mark.gpu
+
+H, D, MANY = 2, 128, 80      # 80 sequences x 2 heads x K and V: 320 streams, past the 296 that count as few
+
+
+def _inputs(T, special):
+    g = torch.Generator().manual_seed(T)
+    p = [t.clone() for t in synth.gen_params(5, H, D, 2)]
+    x = torch.randn(1, H, T, D, generator=g)
+    x[..., ::9] *= 20
+    # frozen states: quotients that are multiples of a half, and the fp16 numbers next to them
+    p[2][:, ::4] = 0
+    p[3][:, ::4] = 0
+    p[1][:, ::4] = torch.rand(H, D // 4, generator=g).half() * 2 + 0.1
+    k = torch.randint(-5, 6, (1, H, T, D // 4), generator=g) * 0.5
+    near = (p[1][:, None, ::4].float() * k).half().contiguous()
+    step = torch.randint(-1, 2, near.shape, generator=g).to(torch.int16)
+    x = x.half()
+    x[..., ::4] = torch.where(near == 0, near, (near.view(torch.int16) + step).view(torch.float16))
+    p[4][:, 3::16] = 100.0       # scales that rest at the lower bound
+    if special:
+        x[0, 0, ::3, 1] = float("nan")
+        x[0, 0, ::5, 2] = float("inf")
+        x[0, 1, ::5, 2] = -float("inf")
+        p[0][:, 5] = -0.0        # zero points of -0, moved by nothing while the codes are 0
+        x[..., 5] = 0.0
+        p[2][0, 6] = float("inf")
+        p[3][:, 7] = 60.0        # scales from one bound to the other within a token
+        p[1][:, 10] = 0.0        # initial scale under the eps guard
+    return x, tuple(p)
+
+
+def _encode(x, p, B, smin, smax, t_start=0):
+    xs = x.cuda().expand(B, -1, -1, -1).contiguous()
+    T = x.shape[2]
+    pc = tuple(t.cuda() for t in p)
+    kc, vc = (torch.zeros(B, H, gemv.n_super_for(T, 2), D // 4, 4, 4, dtype=torch.uint8, device="cuda") for _ in range(2))
+    kt, vt = (torch.zeros(B, H, 2, D, device="cuda") for _ in range(2))
+    for a, b in ((0, t_start), (t_start, T)):
+        if a < b:
+            gemv.encode_kv_pair(kc, xs[:, :, a:b], pc, vc, xs[:, :, a:b], pc, smin, smax, bits=2, k_tail=kt, v_tail=vt, t_start=a)
+    assert torch.equal(kc, vc) and torch.equal(kt.view(torch.int32), vt.view(torch.int32))
+    return kc, kt
+
+
+@pytest.mark.parametrize("T,t_start", [(7, 0), (8, 0), (9, 0), (16, 0), (33, 0), (777, 0), (100, 13)])
+@pytest.mark.parametrize("special,smin,smax", [(False, SMIN, SMAX), (True, SMIN, SMAX), (True, 0.0, 1e30)])
+def test_few_streams(T, t_start, special, smin, smax):
+    x, p = _inputs(T, special)
+    kc, kt = _encode(x, p, 1, smin, smax, t_start)
+    mc, mt = _encode(x, p, MANY, smin, smax, t_start)
+    assert torch.equal(kc[0], mc[0]) and torch.equal(mc[0], mc[MANY - 1])
+    assert torch.equal(kt[0].view(torch.int32), mt[0].view(torch.int32))
+    if not special:
+        want = np.zeros(kc.shape, np.uint8)
+        _, st = orc.encode_kv(want, x.numpy(), np_params(p), 2, smin, smax)
+        assert np.array_equal(kc.cpu().numpy(), want)
+        assert np.array_equal(kt.cpu().numpy(), np.stack([st.zp, st.s], axis=2).astype(np.float32))
