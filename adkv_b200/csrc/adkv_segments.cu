@@ -92,7 +92,7 @@ struct SegSrc : SoftmaxSrc<G> {
     {
 #pragma unroll
         for (int g = 0; g < G; ++g)
-            put(c0, g, this->m[g], this->l[g], make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]));
+            put(c0, g, this->m[g], this->denominator(g), make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]));
     }
     // a bounded wait gave up: the merged output of these heads becomes NaN
     __device__ __forceinline__ void give_up(int c0) const

@@ -66,7 +66,7 @@ struct SoftmaxSrc {
     float scale2;          // scaling * log2(e)
     int n_tiles;           // tiles of this segment
     int t_begin;           // first token of this segment (mask index of local token 0)
-    float m[G], l[G];
+    float m[G], l[G];      // maximum (the same in all lanes) and this lane's share of the denominator (see denominator)
 
     __device__ __forceinline__ void init()
     {
@@ -80,7 +80,7 @@ struct SoftmaxSrc {
         const bool dead = (m_new == -INFINITY);
         const float corr = dead ? 1.f : exp2f(m[g] - m_new);
         const float pw = dead ? 0.f : exp2f(v - m_new);
-        l[g] = fmaf(l[g], corr, warp_sum(pw));
+        l[g] = fmaf(l[g], corr, pw);
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[g][c] *= corr;
         m[g] = m_new;
@@ -125,7 +125,7 @@ struct SoftmaxSrc {
             const bool dead = (m_new == -INFINITY);
             const float corr = dead ? 1.f : exp2f(m[g] - m_new);
             const float pw = dead ? 0.f : exp2f(v - m_new);
-            l[g] = fmaf(l[g], corr, pw);
+            l[g] = fmaf(l[g], corr, lane == 0 ? pw : 0.f);
 #pragma unroll
             for (int c = 0; c < 4; ++c) acc[g][c] *= corr;
             m[g] = m_new;
@@ -133,7 +133,9 @@ struct SoftmaxSrc {
         }
         return true;
     }
-    __device__ __forceinline__ float norm(int g) const { return l[g]; }
+    // Summed over the lanes once per stream: a sum per tile would put five shuffles in a row before its weights.
+    __device__ __forceinline__ float denominator(int g) const { return warp_sum(l[g]); }
+    __device__ __forceinline__ float norm(int g) const { return denominator(g); }
     __device__ __forceinline__ void store(const VArgs &a, int b, int h, int c0, const float (&acc)[G][4]) const
     {
         store_normalised<G>(*this, a, b, h, c0, acc);

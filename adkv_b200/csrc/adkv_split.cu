@@ -24,9 +24,10 @@ struct PartialSrc : SoftmaxSrc<G, 1, HALF_W> {
     {
 #pragma unroll
         for (int g = 0; g < G; ++g) {
+            const float l = this->denominator(g);
             if (c0 == 0) {
                 part[g * kPartStride] = this->m[g];
-                part[g * kPartStride + 1] = this->l[g];
+                part[g * kPartStride + 1] = l;
             }
             *reinterpret_cast<float4 *>(part + g * kPartStride + 4 + c0) =
                 make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
