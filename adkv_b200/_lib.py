@@ -6,6 +6,7 @@ with instructions instead of silently computing something else.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 
 from . import build as _build
@@ -105,6 +106,25 @@ def load() -> ctypes.CDLL:
         raise RuntimeError("libadkv_b200.so ABI version mismatch; rebuild it")
     _lib = lib
     return lib
+
+
+_host = None
+
+
+def host():
+    """The native host module of ``gemv.decode_attn``, bound to the loaded library."""
+    global _host
+    if _host is None:
+        lib = load()
+        if not os.path.exists(_build.HOST_LIB):
+            raise RuntimeError(f"{_build.HOST_LIB} is missing: build it with `python -m adkv_b200.build`.")
+        import torch  # noqa: F401  (the module links against torch's libraries)
+        spec = importlib.util.spec_from_file_location("_adkv_pyhost", _build.HOST_LIB)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        mod.bind(ctypes.cast(lib.adkv_decode_attn, c_void_p).value)
+        _host = mod
+    return _host
 
 
 def strerror(code: int) -> str:

@@ -1,20 +1,24 @@
-"""Build the C-ABI shared library ``adkv_b200/lib/libadkv_b200.so`` for sm_100a with nvcc.
+"""Build the C-ABI shared library ``adkv_b200/lib/libadkv_b200.so`` for sm_100a with nvcc, and the host module of gemv.py.
 
 The library has no dependency on torch or Python: plain ``extern "C"`` entry points declared in
-``include/adkv_b200.h``.  It is built in-tree so that it travels with the source snapshot.
+``include/adkv_b200.h``; the host module ``_adkv_pyhost.so`` checks torch tensors and calls it.  It is built in-tree so that it travels with the source snapshot.
 """
 from __future__ import annotations
 
+import importlib.util
 import os
 import shutil
 from concurrent.futures import ThreadPoolExecutor
 import subprocess
 import sys
+import sysconfig
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB_DIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIB_DIR, "libadkv_b200.so")
+HOST_LIB = os.path.join(LIB_DIR, "_adkv_pyhost.so")   # argument checks of gemv.decode_attn, against torch's headers
+HOST_SOURCE = os.path.join(CSRC, "adkv_pyhost.cpp")
 SOURCES = ["adkv_capi.cu", "adkv_encode.cu", "adkv_fused.cu", "adkv_unfused.cu", "adkv_split.cu", "adkv_wide.cu",
            "adkv_half.cu", "adkv_narrow.cu", "adkv_segments.cu"]
 HEADERS = ["adkv_device.cuh", "adkv_decode.cuh", "adkv_softmax.cuh", "adkv_half.cuh", "adkv_io.cuh", "adkv_host.h",
@@ -34,11 +38,24 @@ def _nvcc() -> str:
 
 
 def is_stale() -> bool:
-    if not os.path.exists(LIB):
+    if not os.path.exists(LIB) or not os.path.exists(HOST_LIB):
         return True
-    t = os.path.getmtime(LIB)
-    deps = [os.path.join(CSRC, f) for f in SOURCES + HEADERS] + [os.path.abspath(__file__)]
+    t = min(os.path.getmtime(LIB), os.path.getmtime(HOST_LIB))
+    deps = [os.path.join(CSRC, f) for f in SOURCES + HEADERS] + [HOST_SOURCE, os.path.abspath(__file__)]
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def build_host(verbose: bool = False) -> str:
+    torch_dir = importlib.util.find_spec("torch").submodule_search_locations[0]
+    inc = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
+           sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")]
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", HOST_SOURCE, "-o", HOST_LIB]
+    cmd += ["-I" + d for d in inc] + ["-L" + os.path.join(torch_dir, "lib")]
+    cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    subprocess.check_call(cmd)
+    return HOST_LIB
 
 
 def build(force: bool = False, verbose: bool = False, extra: list[str] | None = None) -> str:
@@ -63,6 +80,7 @@ def build(force: bool = False, verbose: bool = False, extra: list[str] | None = 
     if verbose:
         print(" ".join(link), flush=True)
     subprocess.check_call(link)
+    build_host(verbose)
     return LIB
 
 

@@ -490,6 +490,14 @@ def decode_attn(q, k_cache, v_cache, k_new, v_new, k_params, v_params, T: int, s
     warp pairs (launches with few streams) and, next to tails with the contracted replay, a token axis split over eight
     warp pairs (up to 148 streams of 128 tokens or more).  True / False force the second / the first (head dim 128,
     fp32 arithmetic, no checkpoints)."""
+    if mask is None and not ckpt_interval:      # plain contiguous tensors: checked and called in native code
+        done = _lib.host().decode(q, k_cache, v_cache, k_new, v_new, k_params, v_params, T, scaling, scale_min, scale_max, bits,
+                                  out, k_tail, v_tail,
+                                  _lib.flags(_fast_default(fast, k_tail), half_state, tail_keep, split_channels))
+        if done is not None:
+            if isinstance(done, int):
+                _lib.check(done, "decode_attn")
+            return done
     _require(q.dtype == torch.float16, "q must be float16")
     _require(k_new.dtype == torch.float16 and v_new.dtype == torch.float16, "k_new / v_new must be float16")
     B, Hkv, n_super_cap, D = _cache_dims(k_cache, "k_cache")
