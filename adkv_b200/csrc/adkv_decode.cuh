@@ -1,7 +1,7 @@
 // Decode-side scans over one (batch, kv head) stream of the packed cache.
 //
 // One warp owns a tensor (K or V) of a stream; lane l owns channels 4l..4l+3, i.e. one 16-byte
-// vector of every supergroup.  The stream is brought into shared memory in tiles of 32 tokens
+// vector of every supergroup.  The stream is brought into shared memory in tiles of 32 or 64 tokens
 // by non-multicast bulk copies (1-D TMA) that complete on mbarriers; each warp runs its own
 // ring, issued by its lane 0, so no other warp can stall it.
 //
@@ -18,7 +18,8 @@
 
 namespace adkv {
 
-constexpr int kTileTok = 32;   // tokens per tile
+constexpr int kTileTok = 32;   // tokens per tile where a kernel does not choose its own (template parameter TOK below); checkpoint
+                               // intervals and token segments are multiples of it
 constexpr int kStages = 3;     // bulk-copy ring depth per warp
 constexpr int kLogitSlots = 4; // logits ring depth (fused kernel)
 
@@ -30,17 +31,18 @@ constexpr int kLogitSlots = 4; // logits ring depth (fused kernel)
 // the canonical state the appended token is quantised with.
 constexpr int kArithFma = 0, kArithCanon = 1;
 
-template <int BITS>
+template <int BITS, int TOK = kTileTok>
 struct Tile {
-    static constexpr int WORDS = kTileTok / Codec<BITS>::TPW;   // words per channel per tile
+    static constexpr int WORDS = TOK / Codec<BITS>::TPW;   // words per channel per tile
     static constexpr int BYTES = WORDS * kD * 4;                // 4-bit: 2048, 2-bit: 1024
 };
 
 // Per-warp bulk-copy ring over the words of one stream.
 // WIDE = false: head dim 128, the stream is contiguous and its geometry is known at compile time (keeps the
 // 128-wide kernels free of the registers and branches the strided case needs).
-template <int BITS, int STAGES = kStages, bool WIDE = false>
+template <int BITS, int STAGES = kStages, bool WIDE = false, int TOK = kTileTok>
 struct StreamRing {
+    using T_ = Tile<BITS, TOK>;
     uint8_t *buf;           // STAGES * Tile::BYTES, 128-byte aligned
     uint64_t *bar;          // STAGES barriers
     const uint8_t *src;     // first word row of this warp's 128-channel slice of the stream
@@ -50,7 +52,7 @@ struct StreamRing {
 
     __device__ __forceinline__ uint32_t tile_bytes(int i) const
     {
-        const int ntok = min(kTileTok, T - i * kTileTok);
+        const int ntok = min(TOK, T - i * TOK);
         const int words = (ntok + Codec<BITS>::TPW - 1) / Codec<BITS>::TPW;
         return uint32_t(words) * kD * 4;
     }
@@ -61,11 +63,11 @@ struct StreamRing {
         const uint32_t bytes = tile_bytes(i);
         mbar_expect_tx(&bar[st], bytes);
         if (!WIDE || row_stride == kD * 4) {
-            bulk_load(buf + st * Tile<BITS>::BYTES, src + size_t(i) * Tile<BITS>::BYTES, bytes, &bar[st]);
+            bulk_load(buf + st * T_::BYTES, src + size_t(i) * T_::BYTES, bytes, &bar[st]);
         } else {   // head_dim > 128: the slice's 512-byte rows are strided, one copy per row
-            const uint8_t *row = src + size_t(i) * Tile<BITS>::WORDS * row_stride;
+            const uint8_t *row = src + size_t(i) * T_::WORDS * row_stride;
             for (uint32_t off = 0; off < bytes; off += kD * 4, row += row_stride)
-                bulk_load(buf + st * Tile<BITS>::BYTES + off, row, kD * 4, &bar[st]);
+                bulk_load(buf + st * T_::BYTES + off, row, kD * 4, &bar[st]);
         }
     }
     __device__ __forceinline__ void prologue(int lane) const
@@ -79,7 +81,7 @@ struct StreamRing {
     }
     __device__ __forceinline__ const uint4 *tile(int i, int lane) const
     {
-        return reinterpret_cast<const uint4 *>(buf + (unsigned(i) % STAGES) * Tile<BITS>::BYTES) + lane;
+        return reinterpret_cast<const uint4 *>(buf + (unsigned(i) % STAGES) * T_::BYTES) + lane;
     }
     // all lanes, after the tile has been consumed
     __device__ __forceinline__ void release_and_refill(int i, int lane) const
@@ -377,7 +379,8 @@ __device__ __forceinline__ void src_end_state(S &, const Chan (&)[4], int, long)
 //   void end_tile(int i, int lane)
 //   void put_self(int g, float v)     lane 0
 //   void finish(int lane)
-template <int BITS, int G, int ARITH, class Sink, int STAGES = kStages, bool WIDE = false, bool OUTLINE = false, int RT = 8>
+template <int BITS, int G, int ARITH, class Sink, int STAGES = kStages, bool WIDE = false, bool OUTLINE = false, int RT = 8,
+          int TOK = kTileTok>
 __device__ __forceinline__ void k_warp(const KArgs &a, const Seg &seg, int b, int h, int lane, uint8_t *ring_buf,
                                        uint64_t *ring_bar, float *red, Sink &sink)
 {
@@ -389,8 +392,8 @@ __device__ __forceinline__ void k_warp(const KArgs &a, const Seg &seg, int b, in
     const uint32_t row_stride = uint32_t(D) * 4;
     uint8_t *stream = a.cache + (size_t(bh) * a.n_super_cap * D + size_t(kD) * slice) * 4;
     const int n_tok = seg.t_end - seg.t_begin;
-    StreamRing<BITS, STAGES, WIDE> ring{ring_buf, ring_bar, stream + size_t(seg.t_begin / C::TPW) * row_stride,
-                          (n_tok + kTileTok - 1) / kTileTok, n_tok, kStatKWait, row_stride};
+    StreamRing<BITS, STAGES, WIDE, TOK> ring{ring_buf, ring_bar, stream + size_t(seg.t_begin / C::TPW) * row_stride,
+                          (n_tok + TOK - 1) / TOK, n_tok, kStatKWait, row_stride};
     ring.prologue(lane);   // first: the copies of the first tiles fly while the parameters below are loaded
     Chan ch[4];
     SafeRange safe;
@@ -461,45 +464,41 @@ __device__ __forceinline__ void k_warp(const KArgs &a, const Seg &seg, int b, in
         if (!(ok = ring.wait(i))) break;
         if (!(ok = sink.begin_tile(i))) break;
         const uint4 *tile = ring.tile(i, lane);
-        const int ntok = min(kTileTok, n_tok - i * kTileTok);
+        const int ntok = min(TOK, n_tok - i * TOK);
         const auto logits = [&](int base) {
             float sum[G];
             reduce_lanes<G, RT>(red, lane, sum);
 #pragma unroll
             for (int g = 0; g < G; ++g) sink.template put<RT>(i, g, base, sum[g], lane);
         };
-        if (ntok == kTileTok) {
-            // not unrolled over the words of the tile: the loop body must stay resident in the
-            // instruction cache while K and V warps of many streams interleave
-            uint4 w = tile[0];
+        // whole words; not unrolled over the words of the tile: the loop body must stay resident in the
+        // instruction cache while K and V warps of many streams interleave
+        const int full = ntok / C::TPW;
+        uint4 w = tile[0];
 #pragma unroll 1
-            for (int wd = 0; wd < Tile<BITS>::WORDS; ++wd) {
-                const uint4 w_next = tile[min(wd + 1, Tile<BITS>::WORDS - 1) * (kD / 4)];
+        for (int wd = 0; wd < full; ++wd) {
+            const uint4 w_next = tile[min(wd + 1, Tile<BITS, TOK>::WORDS - 1) * (kD / 4)];
 #pragma unroll 1
-                for (int c8 = 0; c8 < C::TPW / 8; ++c8) {
-                    const int t = wd * C::TPW + c8 * 8;
-                    float *rows = red + t % RT * kRedRow;
-                    if (safe.holds(ch)) k_chunk2<BITS, G, EXACT, false, RT>(w, fc, ch, pc, one, qv2, rows, lane, a.smin, a.smax);
-                    else if (kPackedClamps<G> && tame) clamped(w, rows);
-                    else guarded(w, rows, 8, std::bool_constant<kPackedClamps<G>>{});   // a body less where this is rare
-                    if ((t + 8) % RT == 0) logits(t + 8 - RT);
-                    if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
-                }
-                w = w_next;
+            for (int c8 = 0; c8 < C::TPW / 8; ++c8) {
+                const int t = wd * C::TPW + c8 * 8;
+                float *rows = red + t % RT * kRedRow;
+                if (safe.holds(ch)) k_chunk2<BITS, G, EXACT, false, RT>(w, fc, ch, pc, one, qv2, rows, lane, a.smin, a.smax);
+                else if (kPackedClamps<G> && tame) clamped(w, rows);
+                else guarded(w, rows, 8, std::bool_constant<kPackedClamps<G>>{});   // a body less where this is rare
+                if ((t + 8) % RT == 0) logits(t + 8 - RT);
+                if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
             }
-        } else {
-#pragma unroll 1
-            for (int wd = 0; wd * C::TPW < ntok; ++wd) {
-                uint4 w = tile[wd * (kD / 4)];
-#pragma unroll 1
-                for (int c8 = 0; c8 < C::TPW / 8 && wd * C::TPW + c8 * 8 < ntok; ++c8) {
-                    const int t = wd * C::TPW + c8 * 8;
-                    guarded(w, red + t % RT * kRedRow, ntok - t, std::true_type{});
-                    if ((t + 8) % RT == 0 || t + 8 >= ntok) logits(t / RT * RT);
-                    if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
-                }
-            }
+            w = w_next;
         }
+        // the tokens of the stream's last, partial word
+        int t = full * C::TPW;
+#pragma unroll 1
+        for (; t < ntok; t += 8) {
+            guarded(w, red + t % RT * kRedRow, ntok - t, std::true_type{});
+            if ((t + 8) % RT == 0) logits(t + 8 - RT);
+            if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
+        }
+        if (t % RT != 0) logits(t / RT * RT);
         sink.end_tile(i, lane);
         ring.release_and_refill(i, lane);
     }
@@ -533,7 +532,7 @@ __device__ __forceinline__ void k_warp(const KArgs &a, const Seg &seg, int b, in
 
 // ---------------------------------------------------------------------------------- V side
 
-template <int BITS, int G, bool EXACT, bool PARTIAL>
+template <int BITS, int G, bool EXACT, bool PARTIAL, int TOK>
 __device__ __forceinline__ void v_chunk(const uint4 &w, const FieldConsts<BITS> &fc, Chan (&ch)[4],
                                         const float2 *wts /* [G][32] smem, each weight twice */, int tok0,
                                         float (&acc)[G][4], int count, float smin, float smax)
@@ -546,7 +545,7 @@ __device__ __forceinline__ void v_chunk(const uint4 &w, const FieldConsts<BITS> 
 #pragma unroll
         for (int g = 0; g < G; ++g) {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) wt[g][k] = wts[g * kTileTok + tok0 + 4 * half + k].x;
+            for (int k = 0; k < 4; ++k) wt[g][k] = wts[g * TOK + tok0 + 4 * half + k].x;
         }
         static_for<4>([&](auto kc) {
             constexpr int k = decltype(kc)::value;
@@ -567,7 +566,7 @@ __device__ __forceinline__ void v_chunk(const uint4 &w, const FieldConsts<BITS> 
 
 // The full 8-token case of v_chunk on channel pairs (packed fp32), guards as in k_chunk2.  `wts2` holds every weight
 // twice ([G][32] float2) so that one 8-byte load yields the packed multiplier.
-template <int BITS, int G, bool EXACT, bool CLAMP>
+template <int BITS, int G, bool EXACT, bool CLAMP, int TOK>
 __device__ __forceinline__ void v_chunk2(const uint4 &w, const FieldConsts<BITS> &fc, Chan (&ch)[4],
                                          const PairConst (&pc)[2], f32x2 one, const float2 *wts2, int tok0,
                                          float (&acc)[G][4], float smin, float smax)
@@ -586,8 +585,8 @@ __device__ __forceinline__ void v_chunk2(const uint4 &w, const FieldConsts<BITS>
         f32x2 wt[G][4];
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-            const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(wts2 + g * kTileTok + tok0 + 4 * half);
-            const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(wts2 + g * kTileTok + tok0 + 4 * half + 2);
+            const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(wts2 + g * TOK + tok0 + 4 * half);
+            const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(wts2 + g * TOK + tok0 + 4 * half + 2);
             wt[g][0] = a.x; wt[g][1] = a.y; wt[g][2] = b.x; wt[g][3] = b.y;
         }
         static_for<4>([&](auto kc) {
@@ -647,27 +646,28 @@ struct VState {
     Chan c[4];
     float acc[G][4];
 };
-template <int BITS, int G, bool EXACT>
+template <int BITS, int G, bool EXACT, int TOK>
 __device__ __noinline__ VState<G> v_chunk_guarded(uint4 w, VState<G> st, const float2 *wts, int tok0, int count,
                                                   float smin, float smax)
 {
     FieldConsts<BITS> fc;
     fc.init();
-    v_chunk<BITS, G, EXACT, true>(w, fc, st.c, wts, tok0, st.acc, count, smin, smax);
+    v_chunk<BITS, G, EXACT, true, TOK>(w, fc, st.c, wts, tok0, st.acc, count, smin, smax);
     return st;
 }
 
-template <int BITS, int G, bool EXACT>
+template <int BITS, int G, bool EXACT, int TOK>
 __device__ __noinline__ VState<G> v_chunk_clamped(uint4 w, VState<G> st, PairConsts pc, const float2 *wts, int tok0, float smin,
                                                   float smax)
 {
     FieldConsts<BITS> fc;
     fc.init();
-    v_chunk2<BITS, G, EXACT, true>(w, fc, st.c, pc.c, opaque_ones2(), wts, tok0, st.acc, smin, smax);
+    v_chunk2<BITS, G, EXACT, true, TOK>(w, fc, st.c, pc.c, opaque_ones2(), wts, tok0, st.acc, smin, smax);
     return st;
 }
 
-template <int BITS, int G, int ARITH, class Src, int STAGES = kStages, bool WIDE = false, bool OUTLINE = false>
+template <int BITS, int G, int ARITH, class Src, int STAGES = kStages, bool WIDE = false, bool OUTLINE = false,
+          int TOK = kTileTok>
 __device__ __forceinline__ void v_warp(const VArgs &a, const Seg &seg, int b, int h, int lane, uint8_t *ring_buf,
                                        uint64_t *ring_bar, const float2 *wts, Src &src)
 {
@@ -679,8 +679,8 @@ __device__ __forceinline__ void v_warp(const VArgs &a, const Seg &seg, int b, in
     const uint32_t row_stride = uint32_t(D) * 4;
     uint8_t *stream = a.cache + (size_t(bh) * a.n_super_cap * D + size_t(kD) * slice) * 4;
     const int n_tok = seg.t_end - seg.t_begin;
-    StreamRing<BITS, STAGES, WIDE> ring{ring_buf, ring_bar, stream + size_t(seg.t_begin / C::TPW) * row_stride,
-                          (n_tok + kTileTok - 1) / kTileTok, n_tok, kStatVWait, row_stride};
+    StreamRing<BITS, STAGES, WIDE, TOK> ring{ring_buf, ring_bar, stream + size_t(seg.t_begin / C::TPW) * row_stride,
+                          (n_tok + TOK - 1) / TOK, n_tok, kStatVWait, row_stride};
     ring.prologue(lane);   // first: the copies of the first tiles fly while the parameters below are loaded
     Chan ch[4];
     SafeRange safe;
@@ -721,49 +721,42 @@ __device__ __forceinline__ void v_warp(const VArgs &a, const Seg &seg, int b, in
     // as in k_warp
     auto clamped = [&](const uint4 &w, int tok0) {
         if constexpr (!kPackedClamps<G>) {
-        } else if constexpr (!OUTLINE) v_chunk2<BITS, G, EXACT, true>(w, fc, ch, pc, one, wts, tok0, acc, a.smin, a.smax);
+        } else if constexpr (!OUTLINE) v_chunk2<BITS, G, EXACT, true, TOK>(w, fc, ch, pc, one, wts, tok0, acc, a.smin, a.smax);
         else out_of_line([&](const VState<G> &st) {
-            return v_chunk_clamped<BITS, G, EXACT>(w, st, PairConsts{{pc[0], pc[1]}}, wts, tok0, a.smin, a.smax);
+            return v_chunk_clamped<BITS, G, EXACT, TOK>(w, st, PairConsts{{pc[0], pc[1]}}, wts, tok0, a.smin, a.smax);
         });
     };
     auto guarded = [&](const uint4 &w, int tok0, int count, auto partial) {
-        if constexpr (!OUTLINE) v_chunk<BITS, G, EXACT, decltype(partial)::value>(w, fc, ch, wts, tok0, acc, count, a.smin, a.smax);
-        else out_of_line([&](const VState<G> &st) { return v_chunk_guarded<BITS, G, EXACT>(w, st, wts, tok0, count, a.smin, a.smax); });
+        if constexpr (!OUTLINE) v_chunk<BITS, G, EXACT, decltype(partial)::value, TOK>(w, fc, ch, wts, tok0, acc, count, a.smin, a.smax);
+        else out_of_line([&](const VState<G> &st) { return v_chunk_guarded<BITS, G, EXACT, TOK>(w, st, wts, tok0, count, a.smin, a.smax); });
     };
 
     bool ok = true;
     int i = 0;
     for (; i < ring.n_tiles; ++i) {
-        const int ntok = min(kTileTok, n_tok - i * kTileTok);
+        const int ntok = min(TOK, n_tok - i * TOK);
         if (!(ok = src.tile_weights(i, ntok, lane, acc))) break;
         if (!(ok = ring.wait(i))) break;
         const uint4 *tile = ring.tile(i, lane);
-        if (ntok == kTileTok) {
-            uint4 w = tile[0];
+        const int full = ntok / C::TPW;   // as in k_warp
+        uint4 w = tile[0];
 #pragma unroll 1
-            for (int wd = 0; wd < Tile<BITS>::WORDS; ++wd) {
-                const uint4 w_next = tile[min(wd + 1, Tile<BITS>::WORDS - 1) * (kD / 4)];
+        for (int wd = 0; wd < full; ++wd) {
+            const uint4 w_next = tile[min(wd + 1, Tile<BITS, TOK>::WORDS - 1) * (kD / 4)];
 #pragma unroll 1
-                for (int c8 = 0; c8 < C::TPW / 8; ++c8) {
-                    const int tok0 = wd * C::TPW + c8 * 8;
-                    if (safe.holds(ch)) v_chunk2<BITS, G, EXACT, false>(w, fc, ch, pc, one, wts, tok0, acc, a.smin, a.smax);
-                    else if (kPackedClamps<G> && tame) clamped(w, tok0);
-                    else guarded(w, tok0, 8, std::bool_constant<kPackedClamps<G>>{});
-                    if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
-                }
-                w = w_next;
+            for (int c8 = 0; c8 < C::TPW / 8; ++c8) {
+                const int tok0 = wd * C::TPW + c8 * 8;
+                if (safe.holds(ch)) v_chunk2<BITS, G, EXACT, false, TOK>(w, fc, ch, pc, one, wts, tok0, acc, a.smin, a.smax);
+                else if (kPackedClamps<G> && tame) clamped(w, tok0);
+                else guarded(w, tok0, 8, std::bool_constant<kPackedClamps<G>>{});
+                if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
             }
-        } else {
+            w = w_next;
+        }
 #pragma unroll 1
-            for (int wd = 0; wd * C::TPW < ntok; ++wd) {
-                uint4 w = tile[wd * (kD / 4)];
-                const int count = ntok - wd * C::TPW;
-#pragma unroll 1
-                for (int c8 = 0; c8 < C::TPW / 8 && c8 * 8 < count; ++c8) {
-                    guarded(w, wd * C::TPW + c8 * 8, count - c8 * 8, std::true_type{});
-                    if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
-                }
-            }
+        for (int t = full * C::TPW; t < ntok; t += 8) {
+            guarded(w, t, ntok - t, std::true_type{});
+            if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
         }
         ring.release_and_refill(i, lane);   // also orders this tile's reads of wts before the next fill
     }

@@ -17,6 +17,9 @@ constexpr int kEncStages = 2;   // 32-token (8 KB) tiles of fp16 input in flight
                                 // which is what a launch over several layers needs (8 layers: 0.645 ms per layer with 2
                                 // stages, 0.688 ms with 3); K and V of one layer are 6.9 CTAs per SM either way (0.86 ms)
 
+// A clamped quotient within 4e-6 of a rounding boundary: cannot tell which way the exact one rounds.
+constexpr float kClear = 0.5f - 4e-6f;
+
 // Eight tokens for the two channels of a thread,
 // speculative quantiser (see quantize_spec) on the channel pair with packed fp32 arithmetic: half the
 // issue slots for the adds and multiplies, every element rounded exactly as by the scalar instruction.
@@ -31,6 +34,7 @@ __device__ __forceinline__ bool encode_group(const __half2 *xin /* 8 rows of kD/
     using C = Codec<BITS>;
     constexpr float M = 12582912.f + float(C::BIAS);   // 1.5 * 2^23 + BIAS: the low bits of (v + M) are code + BIAS
     bool doubt = !(ch[0].s < 1e29f) || !(ch[1].s < 1e29f);   // reciprocal would flush to zero
+    float worst = 0.f;   // largest distance of a clamped quotient from its code
     f32x2 zp = pk2(ch[0].zp, ch[1].zp), s = pk2(ch[0].s, ch[1].s);
     const f32x2 alpha = pk2(ch[0].alpha, ch[1].alpha), beta = pk2(ch[0].beta, ch[1].beta);
     const f32x2 neg_t = pk2(-ch[0].tc, -ch[1].tc), m2 = pk2(M, M);
@@ -55,8 +59,8 @@ __device__ __forceinline__ bool encode_group(const __half2 *xin /* 8 rows of kD/
         const f32x2 q = sub2(t, m2);
         float d0, d1;
         upk2(sub2(vc, q), d0, d1);
-        // clamped quotient within 4e-6 of a rounding boundary: cannot tell which way the exact one rounds
-        doubt |= !(fabsf(d0) < 0.5f - 4e-6f) || !(fabsf(d1) < 0.5f - 4e-6f);
+        if (BITS == 4) worst = fmaxf(fmaxf(worst, fabsf(d0)), fabsf(d1));   // one three-input instruction; not faster for 2 bits
+        else doubt |= !(fabsf(d0) < kClear) || !(fabsf(d1) < kClear);
         const f32x2 rh = mul2(q, ss);
         uint32_t t0, t1;
         asm("mov.b64 {%0, %1}, %2;" : "=r"(t0), "=r"(t1) : "l"(t));
@@ -75,7 +79,7 @@ __device__ __forceinline__ bool encode_group(const __half2 *xin /* 8 rows of kD/
     });
     upk2(zp, ch[0].zp, ch[1].zp);
     upk2(s, ch[0].s, ch[1].s);
-    return doubt;
+    return doubt || !(worst < kClear);
 }
 
 // Eight tokens of one 2-bit channel, without a quotient.  clamp(rint(r / s), -2, 1) asks on which side of -1.5, -0.5 and 0.5
@@ -126,7 +130,8 @@ __device__ __forceinline__ bool encode_group(const __half *xin, Chan (&ch)[1], u
     constexpr float M = 12582912.f + float(C::BIAS);
     Chan &c = ch[0];
     if constexpr (BITS == 2) return encode_group_compare<GUARDED>(xin, c, word[0], smin, smax);
-    bool doubt = !(c.s < 1e29f);
+    const bool doubt = !(c.s < 1e29f);
+    float worst = 0.f;
     static_for<8>([&](auto jc) {
         const float x = __half2float(xin[decltype(jc)::value * kD]);
         const float ss = GUARDED ? fmaxf(c.s, kEps) : c.s;
@@ -134,11 +139,11 @@ __device__ __forceinline__ bool encode_group(const __half *xin, Chan (&ch)[1], u
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(ss));
         const float v = fminf(fmaxf(__fmul_rn(__fsub_rn(x, c.zp), inv), C::qlo()), C::qhi());
         const float t = __fadd_rn(v, M), q = __fsub_rn(t, M);
-        doubt |= !(fabsf(__fsub_rn(v, q)) < 0.5f - 4e-6f);
+        worst = fmaxf(worst, fabsf(__fsub_rn(v, q)));
         advance_canonical_g<GUARDED>(q, __fmul_rn(q, ss), c, smin, smax);
         word[0] = __funnelshift_r(word[0], __float_as_uint(t), BITS);
     });
-    return doubt;
+    return doubt || !(worst < kClear);
 }
 
 // One tensor (K or V) of a launch; blockIdx.y selects it, so K and V of a layer are quantised side by side.
@@ -486,11 +491,11 @@ static int launch_encode(const EncBatch &b, int n, int B, int H, int T, int D, i
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cs.D = D;
     const dim3 grid(B * H * (D / kD), n);
-    // One channel per thread while that leaves a warp scheduler at most two warps: a warp then has its scheduler (nearly)
+    // One channel per thread while that leaves a warp scheduler at most three warps: a warp then has its scheduler (nearly)
     // to itself and takes as long as its own instructions, of which one channel needs about half as many as a pair.
     // Measured on a B200, K and V of 32 heads: 1 x 4000 tokens 251 -> 231 us, 2 x 2000 tokens 131 -> 121 us, 4 x 2000 tokens
-    // 137 -> 133 us.  With more streams the schedulers are busy and the packed pair needs fewer issue slots per channel.
-    const bool few = (long long)grid.x * grid.y * (kD / 32) <= 2 * kSchedulers;
+    // 137 -> 133 us, 6 x 3000 tokens 213 -> 199 us (2-bit 224 -> 212 us), but 8 x 2000 tokens 148 -> 155 us.  With more streams the schedulers are busy and the packed pair needs fewer issue slots per channel.
+    const bool few = (long long)grid.x * grid.y * (kD / 32) <= 3 * kSchedulers;
     if (D == kD) {
         if (bits == 4 && few) encode_kernel<4, false, 1><<<grid, kD, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
         else if (bits == 4) encode_kernel<4, false, 2><<<grid, kEncThreads, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);

@@ -9,6 +9,13 @@ namespace adkv {
 // =========================================================================================
 // Fused decode step: one CTA per (batch, kv head); warp 0 scans K, warp 1 scans V.
 
+// Tokens per tile, and tiles in flight per warp.  Every tile costs two waits, the hand-over of its logits, a step of the online
+// softmax with its shuffles, and a refill: a few hundred instructions and, for a warp that has its scheduler to itself, about
+// a thousand cycles.  Tiles of 32 (three stages) -> 64 (two), device time on a B200: 2-bit, 256 streams of four heads x 32768
+// tokens 2359 -> 2183 us, 4-bit x 2000 tokens 162 -> 134 us; 4096 streams x 4096 tokens 1442 -> 1411 us, 256 x 2000 98 -> 91 us,
+// 768 x 1531 143 -> 136 us.  Tiles of 128 give 1 % at 2-bit codes and lose 6 % at 200 tokens.
+constexpr int kFusedTok = 64, kFusedStages = 2;
+
 // Whether the guarded chunk bodies of this instantiation are function calls (see k_chunk_guarded).  Measured on a
 // B200 against the inline form, streams of 32 heads x 128: 4-bit codes with one query head per KV head gain 13 % at
 // 128-token contexts and lose nothing elsewhere; 2-bit codes gain 17 % there but lose 7 % in the canonical replay and
@@ -50,12 +57,12 @@ __global__ void __launch_bounds__(64) decode_attn_kernel(KArgs ka, VArgs va, con
                                                          long long mask_stride_b, float scaling,
                                                          const int *__restrict__ seq_lens, int n_rank)
 {
-    __shared__ alignas(128) uint8_t kbuf[kStages * Tile<BITS>::BYTES];
-    __shared__ alignas(128) uint8_t vbuf[kStages * Tile<BITS>::BYTES];
+    __shared__ alignas(128) uint8_t kbuf[kFusedStages * Tile<BITS, kFusedTok>::BYTES];
+    __shared__ alignas(128) uint8_t vbuf[kFusedStages * Tile<BITS, kFusedTok>::BYTES];
     __shared__ alignas(16) float red[G * 8 * kRedRow];
-    __shared__ alignas(16) float2 wts[G * kTileTok];
-    __shared__ FusedShared<G> fs;
-    __shared__ uint64_t kbar[kStages], vbar[kStages];
+    __shared__ alignas(16) float2 wts[G * kFusedTok];
+    __shared__ FusedShared<G, 1, kFusedTok> fs;
+    __shared__ uint64_t kbar[kFusedStages], vbar[kFusedStages];
 
     int b = blockIdx.x / ka.Hkv;
     const int h = blockIdx.x % ka.Hkv;
@@ -73,25 +80,25 @@ __global__ void __launch_bounds__(64) decode_attn_kernel(KArgs ka, VArgs va, con
         va.T = T;
     }
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kStages; ++i) { mbar_init(&kbar[i], 1); mbar_init(&vbar[i], 1); }
+        for (int i = 0; i < kFusedStages; ++i) { mbar_init(&kbar[i], 1); mbar_init(&vbar[i], 1); }
         fs.init_barriers(1);
         mbar_init_fence();
     }
     __syncthreads();
     const Seg seg{0, ka.T, true, nullptr, nullptr, 0};
     if (warp == 0) {
-        RingSink<G> sink{&fs, 0, 0};
-        k_warp<BITS, G, ARITH, RingSink<G>, kStages, false, kOutOfLineGuarded<BITS, G>>(ka, seg, b, h, lane, kbuf, kbar, red, sink);
+        RingSink<G, 1, kFusedTok> sink{&fs, 0, 0};
+        k_warp<BITS, G, ARITH, RingSink<G, 1, kFusedTok>, kFusedStages, false, kOutOfLineGuarded<BITS, G>, 8, kFusedTok>(ka, seg, b, h, lane, kbuf, kbar, red, sink);
     } else {
-        SoftmaxSrc<G> src;
+        SoftmaxSrc<G, 1, false, kFusedTok> src;
         src.sh = &fs;
         src.wts = wts;
         src.mask = mask ? mask + size_t(b) * mask_stride_b : nullptr;
         src.scale2 = scaling * 1.4426950408889634f;
-        src.n_tiles = (va.T + kTileTok - 1) / kTileTok;
+        src.n_tiles = (va.T + kFusedTok - 1) / kFusedTok;
         src.t_begin = 0;
         src.init();
-        v_warp<BITS, G, ARITH, SoftmaxSrc<G>, kStages, false, kOutOfLineGuarded<BITS, G>>(va, seg, b, h, lane, vbuf, vbar, wts, src);
+        v_warp<BITS, G, ARITH, SoftmaxSrc<G, 1, false, kFusedTok>, kFusedStages, false, kOutOfLineGuarded<BITS, G>, kFusedTok>(va, seg, b, h, lane, vbuf, vbar, wts, src);
     }
 }
 

@@ -7,7 +7,7 @@ namespace adkv {
 
 constexpr int kStreamsPerCta = 2;   // unfused kernels: 2 streams per CTA, one warp each
 
-template <int G>
+template <int G, int TOK = kTileTok>
 struct GlobalLogitSink {
     __half *row[G];   // logits row of each q head of this stream: [T+1]
     int T;
@@ -15,7 +15,7 @@ struct GlobalLogitSink {
     template <int N>
     __device__ __forceinline__ void put(int i, int g, int tok, float v, int lane)
     {
-        const int t = i * kTileTok + tok + lane;
+        const int t = i * TOK + tok + lane;
         if (lane < N && t < T) row[g][t] = __float2half_rn(v);
     }
     __device__ __forceinline__ void end_tile(int, int) {}

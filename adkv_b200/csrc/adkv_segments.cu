@@ -34,13 +34,17 @@ namespace adkv {
 
 constexpr int NS = 8;             // segments per stream
 constexpr int kSegStages = 2;     // bulk-copy ring depth per warp
+// tokens per tile: see kFusedTok; shorter tiles where 64 tokens of 16 warps do not fit the shared memory
+template <int BITS, int G>
+constexpr int kSegTok = BITS == 4 && G == 4 ? kTileTok : 64;
 constexpr int kPartFloats = 4 + kD;   // per (segment, head): maximum (log2 units), denominator, 2 pad, kD sums
 
 template <int BITS, int G>
 struct SegShared {
-    alignas(128) uint8_t buf[2][NS][kSegStages * Tile<BITS>::BYTES];
+    static constexpr int TOK = kSegTok<BITS, G>;
+    alignas(128) uint8_t buf[2][NS][kSegStages * Tile<BITS, TOK>::BYTES];
     alignas(16) float red[NS][G * 8 * kRedRow];
-    alignas(16) float2 wts[NS][G * kTileTok];
+    alignas(16) float2 wts[NS][G * TOK];
     union {
         alignas(16) float comp[2][NS][3][kD];     // steps 1 and 2: product, smallest and largest running product
         alignas(16) float part[NS][G][kPartFloats];   // steps 3 and 4
@@ -51,12 +55,12 @@ struct SegShared {
     float z_end[NS][G];                           // K: sum_c q_c * zp_c after the segment, relative
     float self_logit[G];
     int clamps[2];                                       // step 2: a segment of K / of V may have met a clamp
-    FusedShared<G> fs[NS];
+    FusedShared<G, 1, TOK> fs[NS];
     uint64_t bar[2][NS][kSegStages];
 };
 
-template <int G>
-struct SegSink : RingSink<G> {
+template <int G, int TOK>
+struct SegSink : RingSink<G, 1, TOK> {
     float *z_end;
     bool done;
     __device__ __forceinline__ void end_state(const Chan (&ch)[4], const float (&qv)[G][4], int lane)
@@ -70,8 +74,8 @@ struct SegSink : RingSink<G> {
     }
 };
 
-template <int G>
-struct SegSrc : SoftmaxSrc<G> {
+template <int G, int TOK>
+struct SegSrc : SoftmaxSrc<G, 1, false, TOK> {
     float *part;       // [G][kPartFloats] of this segment
     float *zp_end;
     bool done;
@@ -246,6 +250,7 @@ __global__ void __launch_bounds__(64 * NS)
     extern __shared__ uint8_t smem_raw[];
     SegShared<BITS, G> &sh = *reinterpret_cast<SegShared<BITS, G> *>(smem_raw);
     using C = Codec<BITS>;
+    constexpr int TOK = kSegTok<BITS, G>;
     const int bh = blockIdx.x, b = bh / ka.Hkv, h = bh % ka.Hkv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // Warps go to the four schedulers round robin: a pair of warps is the K and the V warp of one segment, and the order
@@ -359,13 +364,13 @@ __global__ void __launch_bounds__(64 * NS)
     // The appended token goes into the word behind the last cached one: only the warps that read that word may write it.
     const bool last = t_end == T && (seg == 0 || t_begin < T);
     if (role == 0) {
-        SegSink<G> sink;
+        SegSink<G, TOK> sink;
         sink.sh = &sh.fs[seg];
         sink.slot = 0;
         sink.sl = 0;
         sink.z_end = sh.z_end[seg];
         sink.done = false;
-        k_warp<BITS, G, kArithFma, SegSink<G>, kSegStages>(ka, sg, b, h, lane, sh.buf[0][seg], sh.bar[0][seg], sh.red[seg], sink);
+        k_warp<BITS, G, kArithFma, SegSink<G, TOK>, kSegStages, false, false, 8, TOK>(ka, sg, b, h, lane, sh.buf[0][seg], sh.bar[0][seg], sh.red[seg], sink);
         if (last && sink.done) {
             float xh[4];
             append(ka.p, ka.tail, ka.tail_keep, ka.x_new, ka.cache, xh);
@@ -380,18 +385,18 @@ __global__ void __launch_bounds__(64 * NS)
             }
         }
     } else {
-        SegSrc<G> src;
+        SegSrc<G, TOK> src;
         src.sh = &sh.fs[seg];
         src.wts = sh.wts[seg];
         src.mask = mask_row;
         src.scale2 = scale2;
-        src.n_tiles = (t_end - t_begin + kTileTok - 1) / kTileTok;
+        src.n_tiles = (t_end - t_begin + TOK - 1) / TOK;
         src.t_begin = t_begin;
         src.part = &sh.part[seg][0][0];
         src.zp_end = sh.zp_end[seg];
         src.done = false;
         src.init();
-        v_warp<BITS, G, kArithFma, SegSrc<G>, kSegStages>(va, sg, b, h, lane, sh.buf[1][seg], sh.bar[1][seg], sh.wts[seg], src);
+        v_warp<BITS, G, kArithFma, SegSrc<G, TOK>, kSegStages, false, false, TOK>(va, sg, b, h, lane, sh.buf[1][seg], sh.bar[1][seg], sh.wts[seg], src);
         if (last && src.done) {
             float xh[4];
             append(va.p, va.tail, va.tail_keep, va.x_new, va.cache, xh);

@@ -8,9 +8,9 @@ namespace adkv {
 // S = number of 128-channel slices of the head (head_dim / 128): each slice has its own K warp, which
 // contributes a partial logit, and its own V warp, which sums the S partials.  The full barrier of a slot
 // therefore collects S arrivals (one per K warp) and the empty barrier S arrivals (one per V warp).
-template <int G, int S = 1>
+template <int G, int S = 1, int TOK = kTileTok>
 struct FusedShared {
-    float lring[kLogitSlots][S][G][kTileTok];
+    float lring[kLogitSlots][S][G][TOK];
     uint64_t lfull[kLogitSlots], lempty[kLogitSlots];
     __device__ __forceinline__ void init_barriers(int n_consumers)
     {
@@ -21,9 +21,9 @@ struct FusedShared {
     }
 };
 
-template <int G, int S = 1>
+template <int G, int S = 1, int TOK = kTileTok>
 struct RingSink {
-    FusedShared<G, S> *sh;
+    FusedShared<G, S, TOK> *sh;
     int slot;
     int sl;      // this K warp's slice
     __device__ __forceinline__ bool begin_tile(int i)
@@ -58,10 +58,11 @@ __device__ __forceinline__ void put_weight(float2 *wts, int idx, float w)
     }
 }
 
-template <int G, int S = 1, bool HALF_W = false>
+template <int G, int S = 1, bool HALF_W = false, int TOK = kTileTok>
 struct SoftmaxSrc {
-    FusedShared<G, S> *sh;
-    float2 *wts;           // [G][32], every weight stored twice (packed multiplier for a channel pair)
+    static constexpr int TPL = TOK / 32;   // tokens of a tile that a lane weighs: lane, lane + 32
+    FusedShared<G, S, TOK> *sh;
+    float2 *wts;           // [G][TOK], every weight stored twice (packed multiplier for a channel pair)
     const float *mask;     // row of this batch or nullptr
     float scale2;          // scaling * log2(e)
     int n_tiles;           // tiles of this segment
@@ -73,38 +74,51 @@ struct SoftmaxSrc {
 #pragma unroll
         for (int g = 0; g < G; ++g) { m[g] = -INFINITY; l[g] = 0.f; }
     }
-    // online-softmax update of head g with this lane's logit v (already in log2 units, -inf if invalid)
-    __device__ __forceinline__ float update(int g, float v, float (&acc)[G][4])
+    // online-softmax update of head g with this lane's logits v (already in log2 units, -inf if invalid): v becomes the weights
+    __device__ __forceinline__ void update(int g, float (&v)[TPL], float (&acc)[G][4])
     {
-        const float m_new = fmaxf(m[g], warp_max(v));
+        float top = v[0];
+#pragma unroll
+        for (int k = 1; k < TPL; ++k) top = fmaxf(top, v[k]);
+        const float m_new = fmaxf(m[g], warp_max(top));
         const bool dead = (m_new == -INFINITY);
         const float corr = dead ? 1.f : exp2f(m[g] - m_new);
-        const float pw = dead ? 0.f : exp2f(v - m_new);
-        l[g] = fmaf(l[g], corr, pw);
+        l[g] *= corr;
+#pragma unroll
+        for (int k = 0; k < TPL; ++k) {
+            v[k] = dead ? 0.f : exp2f(v[k] - m_new);
+            l[g] += v[k];
+        }
 #pragma unroll
         for (int c = 0; c < 4; ++c) acc[g][c] *= corr;
         m[g] = m_new;
-        return pw;
     }
     __device__ __forceinline__ bool tile_weights(int i, int ntok, int lane, float (&acc)[G][4])
     {
         const int slot = i % kLogitSlots;
-        const float mk = (mask && lane < ntok) ? mask[t_begin + i * kTileTok + lane] * 1.4426950408889634f : 0.f;
+        float mk[TPL];
+#pragma unroll
+        for (int k = 0; k < TPL; ++k)
+            mk[k] = (mask && lane + 32 * k < ntok) ? mask[t_begin + i * TOK + lane + 32 * k] * 1.4426950408889634f : 0.f;
         if (!mbar_wait_bounded(&sh->lfull[slot], (i / kLogitSlots) & 1, kStatLFullWait)) return false;
-        float x[G];
+        float x[G][TPL];
 #pragma unroll
-        for (int g = 0; g < G; ++g) {
-            x[g] = sh->lring[slot][0][g][lane];
+        for (int g = 0; g < G; ++g)
 #pragma unroll
-            for (int k = 1; k < S; ++k) x[g] += sh->lring[slot][k][g][lane];
-        }
+            for (int k = 0; k < TPL; ++k) {
+                x[g][k] = sh->lring[slot][0][g][lane + 32 * k];
+#pragma unroll
+                for (int j = 1; j < S; ++j) x[g][k] += sh->lring[slot][j][g][lane + 32 * k];
+            }
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh->lempty[slot]);
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-            const float v = lane < ntok ? fmaf(x[g], scale2, mk) : -INFINITY;
-            const float pw = update(g, v, acc);
-            put_weight<HALF_W>(wts, g * kTileTok + lane, pw);
+#pragma unroll
+            for (int k = 0; k < TPL; ++k) x[g][k] = lane + 32 * k < ntok ? fmaf(x[g][k], scale2, mk[k]) : -INFINITY;
+            update(g, x[g], acc);
+#pragma unroll
+            for (int k = 0; k < TPL; ++k) put_weight<HALF_W>(wts, g * TOK + lane + 32 * k, x[g][k]);
         }
         __syncwarp();
         return true;

@@ -17,8 +17,14 @@ namespace adkv {
 
 constexpr int kPartStride = 4 + kD;   // floats per (stream, segment, head): max (log2 units), denominator, 2 pad, kD sums
 
+// tokens per tile; the fp16-state scans know tiles of kTileTok only
+template <bool HALF>
+constexpr int kSplitTok = HALF ? kTileTok : 64;
+template <bool HALF>
+constexpr int kSplitStages = HALF ? kStages : 2;
+
 template <int G, bool HALF_W>
-struct PartialSrc : SoftmaxSrc<G, 1, HALF_W> {
+struct PartialSrc : SoftmaxSrc<G, 1, HALF_W, kSplitTok<HALF_W>> {
     float *part;   // [G][kPartStride] of this (stream, segment)
     __device__ __forceinline__ void store(const VArgs &, int, int, int c0, const float (&acc)[G][4]) const
     {
@@ -65,18 +71,19 @@ __global__ void __launch_bounds__(64) decode_attn_split_kernel(KArgs ka, VArgs v
                                                                long long mask_stride_b, float scaling, CkptArgs ck,
                                                                float *__restrict__ scratch)
 {
-    __shared__ alignas(128) uint8_t kbuf[kStages * Tile<BITS>::BYTES];
-    __shared__ alignas(128) uint8_t vbuf[kStages * Tile<BITS>::BYTES];
+    constexpr int TOK = kSplitTok<MODE == kModeHalf>, ST = kSplitStages<MODE == kModeHalf>;
+    __shared__ alignas(128) uint8_t kbuf[ST * Tile<BITS, TOK>::BYTES];
+    __shared__ alignas(128) uint8_t vbuf[ST * Tile<BITS, TOK>::BYTES];
     __shared__ alignas(16) float red[G * 8 * kRedRow];
-    __shared__ alignas(16) float2 wts[G * kTileTok];
-    __shared__ FusedShared<G> fs;
-    __shared__ uint64_t kbar[kStages], vbar[kStages];
+    __shared__ alignas(16) float2 wts[G * TOK];
+    __shared__ FusedShared<G, 1, TOK> fs;
+    __shared__ uint64_t kbar[ST], vbar[ST];
 
     const int bh = blockIdx.x, b = bh / ka.Hkv, h = bh % ka.Hkv;
     const int j = blockIdx.y, n_seg = gridDim.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kStages; ++i) { mbar_init(&kbar[i], 1); mbar_init(&vbar[i], 1); }
+        for (int i = 0; i < ST; ++i) { mbar_init(&kbar[i], 1); mbar_init(&vbar[i], 1); }
         fs.init_barriers(1);
         mbar_init_fence();
     }
@@ -95,8 +102,8 @@ __global__ void __launch_bounds__(64) decode_attn_split_kernel(KArgs ka, VArgs v
         if (ck.mute_k) return;
         seg.init = j ? ck.k_ckpt + (stream_ckpt + j - 1) * 2 * kD : nullptr;
         seg.ckpt_out = write_ckpt ? ck.k_ckpt + out_idx * 2 * kD : nullptr;
-        RingSink<G> sink{&fs, 0, 0};
-        k_scan<BITS, G, MODE, RingSink<G>, kStages, false, kOutOfLineGuardedSegments<BITS, G>>(ka, seg, b, h, lane, kbuf, kbar, red, sink);
+        RingSink<G, 1, TOK> sink{&fs, 0, 0};
+        k_scan<BITS, G, MODE, RingSink<G, 1, TOK>, ST, false, kOutOfLineGuardedSegments<BITS, G>, TOK>(ka, seg, b, h, lane, kbuf, kbar, red, sink);
     } else {
         seg.init = j ? ck.v_ckpt + (stream_ckpt + j - 1) * 2 * kD : nullptr;
         seg.ckpt_out = write_ckpt ? ck.v_ckpt + out_idx * 2 * kD : nullptr;
@@ -105,11 +112,11 @@ __global__ void __launch_bounds__(64) decode_attn_split_kernel(KArgs ka, VArgs v
         src.wts = wts;
         src.mask = mask ? mask + size_t(b) * mask_stride_b : nullptr;
         src.scale2 = scaling * 1.4426950408889634f;
-        src.n_tiles = (seg.t_end - seg.t_begin + kTileTok - 1) / kTileTok;
+        src.n_tiles = (seg.t_end - seg.t_begin + TOK - 1) / TOK;
         src.t_begin = seg.t_begin;
         src.part = scratch + (size_t(bh) * n_seg + j) * G * kPartStride;
         src.init();
-        v_scan<BITS, G, MODE, PartialSrc<G, MODE == kModeHalf>, kStages, false, kOutOfLineGuardedSegments<BITS, G>>(va, seg, b, h, lane, vbuf, vbar, wts, src);
+        v_scan<BITS, G, MODE, PartialSrc<G, MODE == kModeHalf>, ST, false, kOutOfLineGuardedSegments<BITS, G>, TOK>(va, seg, b, h, lane, vbuf, vbar, wts, src);
     }
 }
 
