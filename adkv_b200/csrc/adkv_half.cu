@@ -11,17 +11,19 @@ namespace adkv {
 
 // =========================================================================================
 // Fused decode step, as decode_attn_kernel: one CTA per (batch, kv head); warp 0 scans K, warp 1 scans V.
-template <int BITS, int G>
+// TOK: tokens per tile, 64 (two stages) or 32 (three), see adkv_half_decode_attn.
+template <int BITS, int G, int TOK>
 __global__ void __launch_bounds__(64) decode_attn_half_kernel(KArgs ka, VArgs va, const float *__restrict__ mask,
                                                               long long mask_stride_b, float scaling,
                                                               const int *__restrict__ seq_lens)
 {
-    __shared__ alignas(128) uint8_t kbuf[kStages * Tile<BITS>::BYTES];
-    __shared__ alignas(128) uint8_t vbuf[kStages * Tile<BITS>::BYTES];
+    constexpr int ST = TOK == 64 ? 2 : 3;
+    __shared__ alignas(128) uint8_t kbuf[ST * Tile<BITS, TOK>::BYTES];
+    __shared__ alignas(128) uint8_t vbuf[ST * Tile<BITS, TOK>::BYTES];
     __shared__ alignas(16) float red[G * 8 * 36];
-    __shared__ alignas(16) float2 wts[G * kTileTok];
-    __shared__ FusedShared<G> fs;
-    __shared__ uint64_t kbar[kStages], vbar[kStages];
+    __shared__ alignas(16) float2 wts[G * TOK];
+    __shared__ FusedShared<G, 1, TOK> fs;
+    __shared__ uint64_t kbar[ST], vbar[ST];
 
     const int bh = blockIdx.x, b = bh / ka.Hkv, h = bh % ka.Hkv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -35,25 +37,25 @@ __global__ void __launch_bounds__(64) decode_attn_half_kernel(KArgs ka, VArgs va
         va.T = T;
     }
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kStages; ++i) { mbar_init(&kbar[i], 1); mbar_init(&vbar[i], 1); }
+        for (int i = 0; i < ST; ++i) { mbar_init(&kbar[i], 1); mbar_init(&vbar[i], 1); }
         fs.init_barriers(1);
         mbar_init_fence();
     }
     __syncthreads();
     const Seg seg{0, ka.T, true, nullptr, nullptr, 0};
     if (warp == 0) {
-        RingSink<G> sink{&fs, 0, 0};
-        k_warp_h<BITS, G>(ka, seg, b, h, lane, kbuf, kbar, red, sink);
+        RingSink<G, 1, TOK> sink{&fs, 0, 0};
+        k_warp_h<BITS, G, RingSink<G, 1, TOK>, ST, false, TOK>(ka, seg, b, h, lane, kbuf, kbar, red, sink);
     } else {
-        SoftmaxSrc<G, 1, true> src;
+        SoftmaxSrc<G, 1, true, TOK> src;
         src.sh = &fs;
         src.wts = wts;
         src.mask = mask ? mask + size_t(b) * mask_stride_b : nullptr;
         src.scale2 = scaling * 1.4426950408889634f;
-        src.n_tiles = (va.T + kTileTok - 1) / kTileTok;
+        src.n_tiles = (va.T + TOK - 1) / TOK;
         src.t_begin = 0;
         src.init();
-        v_warp_h<BITS, G>(va, seg, b, h, lane, vbuf, vbar, wts, src);
+        v_warp_h<BITS, G, SoftmaxSrc<G, 1, true, TOK>, ST, false, TOK>(va, seg, b, h, lane, vbuf, vbar, wts, src);
     }
 }
 
@@ -358,9 +360,18 @@ ADKV_HIDDEN int adkv_half_decode_attn(const KArgs &ka, const VArgs &va, const fl
                                       float scaling, int B, int bits, const int *seq_lens, cudaStream_t s)
 {
     if (ka.D != kD) return ADKV_E_FLAGS;
+    // Tiles of 64 tokens (see kFusedTok in adkv_fused.cu) while all CTAs fit the chip at once with the 19 KB that they take,
+    // eleven per SM: 128 streams x 1000 tokens 44.2 -> 39.3 us, 512 x 2000 113.5 -> 104.7 us, 1056 x 777 76.5 -> 73.7 us on a
+    // B200.  Beyond, fifteen CTAs with tiles of 32 hide more: 2048 streams x 2048 tokens 300 us against 323 us.
+    if ((long long)B * ka.Hkv <= 11 * kSMs) {
+        ADKV_DISPATCH_H(bits, ka.Hq / ka.Hkv,
+                        (decode_attn_half_kernel<BITS, G, 64><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling,
+                                                                                       seq_lens)))
+        return launch_status();
+    }
     ADKV_DISPATCH_H(bits, ka.Hq / ka.Hkv,
-                    (decode_attn_half_kernel<BITS, G><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling,
-                                                                               seq_lens)))
+                    (decode_attn_half_kernel<BITS, G, 32><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling,
+                                                                                   seq_lens)))
     return launch_status();
 }
 

@@ -216,7 +216,7 @@ __device__ __forceinline__ void reduce8_h(const uint32_t *red, int lane, float (
     __syncwarp();
 }
 
-template <int BITS, int G, class Sink, int STAGES = kStages, bool WIDE = false>
+template <int BITS, int G, class Sink, int STAGES = kStages, bool WIDE = false, int TOK = kTileTok>
 __device__ __forceinline__ void k_warp_h(const KArgs &a, const Seg &seg, int b, int h, int lane, uint8_t *ring_buf,
                                          uint64_t *ring_bar, float *red_f, Sink &sink)
 {
@@ -238,8 +238,8 @@ __device__ __forceinline__ void k_warp_h(const KArgs &a, const Seg &seg, int b, 
     const uint32_t row_stride = uint32_t(D) * 4;
     uint8_t *stream = a.cache + (size_t(bh) * a.n_super_cap * D + size_t(kD) * slice) * 4;
     const int n_tok = seg.t_end - seg.t_begin;
-    StreamRing<BITS, STAGES, WIDE> ring{ring_buf, ring_bar, stream + size_t(seg.t_begin / C::TPW) * row_stride,
-                                  (n_tok + kTileTok - 1) / kTileTok, n_tok, kStatKWait, row_stride};
+    StreamRing<BITS, STAGES, WIDE, TOK> ring{ring_buf, ring_bar, stream + size_t(seg.t_begin / C::TPW) * row_stride,
+                                  (n_tok + TOK - 1) / TOK, n_tok, kStatKWait, row_stride};
     ring.prologue(lane);
 
     bool ok = true;
@@ -248,37 +248,30 @@ __device__ __forceinline__ void k_warp_h(const KArgs &a, const Seg &seg, int b, 
         if (!(ok = ring.wait(i))) break;
         if (!(ok = sink.begin_tile(i))) break;
         const uint4 *tile = ring.tile(i, lane);
-        const int ntok = min(kTileTok, n_tok - i * kTileTok);
+        const int ntok = min(TOK, n_tok - i * TOK);
         float sum[G];
-        if (ntok == kTileTok) {
-            uint4 w = tile[0];
+        const int full = ntok / C::TPW;   // whole words
+        uint4 w = tile[0];
 #pragma unroll 1
-            for (int wd = 0; wd < Tile<BITS>::WORDS; ++wd) {
-                const uint4 w_next = tile[min(wd + 1, Tile<BITS>::WORDS - 1) * (kD / 4)];
+        for (int wd = 0; wd < full; ++wd) {
+            const uint4 w_next = tile[min(wd + 1, Tile<BITS, TOK>::WORDS - 1) * (kD / 4)];
 #pragma unroll 1
-                for (int c8 = 0; c8 < C::TPW / 8; ++c8) {
-                    k_chunk_h<BITS, G, false>(w, hp, qv, red, lane, 8);
-                    reduce8_h<G>(red, lane, sum);
+            for (int c8 = 0; c8 < C::TPW / 8; ++c8) {
+                k_chunk_h<BITS, G, false>(w, hp, qv, red, lane, 8);
+                reduce8_h<G>(red, lane, sum);
 #pragma unroll
-                    for (int g = 0; g < G; ++g) sink.template put<8>(i, g, wd * C::TPW + c8 * 8, sum[g], lane);
-                    if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
-                }
-                w = w_next;
+                for (int g = 0; g < G; ++g) sink.template put<8>(i, g, wd * C::TPW + c8 * 8, sum[g], lane);
+                if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
             }
-        } else {
+            w = w_next;
+        }
 #pragma unroll 1
-            for (int wd = 0; wd * C::TPW < ntok; ++wd) {
-                uint4 w = tile[wd * (kD / 4)];
-                const int count = ntok - wd * C::TPW;
-#pragma unroll 1
-                for (int c8 = 0; c8 < C::TPW / 8 && c8 * 8 < count; ++c8) {
-                    k_chunk_h<BITS, G, true>(w, hp, qv, red, lane, count - c8 * 8);
-                    reduce8_h<G>(red, lane, sum);
+        for (int t = full * C::TPW; t < ntok; t += 8) {   // the tokens of the stream's last, partial word
+            k_chunk_h<BITS, G, true>(w, hp, qv, red, lane, ntok - t);
+            reduce8_h<G>(red, lane, sum);
 #pragma unroll
-                    for (int g = 0; g < G; ++g) sink.template put<8>(i, g, wd * C::TPW + c8 * 8, sum[g], lane);
-                    if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
-                }
-            }
+            for (int g = 0; g < G; ++g) sink.template put<8>(i, g, t, sum[g], lane);
+            if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
         }
         sink.end_tile(i, lane);
         ring.release_and_refill(i, lane);
@@ -330,7 +323,7 @@ __device__ __forceinline__ void k_warp_h(const KArgs &a, const Seg &seg, int b, 
 // 8 tokens for the lane's two channel pairs: weight * value accumulated in fp16 over the 8 tokens, then added
 // to the fp32 accumulators (the reference accumulates all tokens in fp16, gemv.cu:1087).  wts: [G][32] fp16
 // pairs (w, w), written by a source with HALF_W set.
-template <int BITS, int G, bool PARTIAL>
+template <int BITS, int G, bool PARTIAL, int TOK>
 __device__ __forceinline__ void v_chunk_h(const uint4 &w, HPair (&hp)[2], const uint32_t *wts, int tok0,
                                           float (&acc)[G][4], int count)
 {
@@ -339,8 +332,8 @@ __device__ __forceinline__ void v_chunk_h(const uint4 &w, HPair (&hp)[2], const 
     h2 wt[G][8];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-        const uint4 a = *reinterpret_cast<const uint4 *>(wts + g * kTileTok + tok0);
-        const uint4 b = *reinterpret_cast<const uint4 *>(wts + g * kTileTok + tok0 + 4);
+        const uint4 a = *reinterpret_cast<const uint4 *>(wts + g * TOK + tok0);
+        const uint4 b = *reinterpret_cast<const uint4 *>(wts + g * TOK + tok0 + 4);
         wt[g][0] = a.x; wt[g][1] = a.y; wt[g][2] = a.z; wt[g][3] = a.w;
         wt[g][4] = b.x; wt[g][5] = b.y; wt[g][6] = b.z; wt[g][7] = b.w;
     }
@@ -370,7 +363,7 @@ __device__ __forceinline__ void v_chunk_h(const uint4 &w, HPair (&hp)[2], const 
     }
 }
 
-template <int BITS, int G, class Src, int STAGES = kStages, bool WIDE = false>
+template <int BITS, int G, class Src, int STAGES = kStages, bool WIDE = false, int TOK = kTileTok>
 __device__ __forceinline__ void v_warp_h(const VArgs &a, const Seg &seg, int b, int h, int lane, uint8_t *ring_buf,
                                          uint64_t *ring_bar, const float2 *wts_f2, Src &src)
 {
@@ -391,40 +384,33 @@ __device__ __forceinline__ void v_warp_h(const VArgs &a, const Seg &seg, int b, 
     const uint32_t row_stride = uint32_t(D) * 4;
     uint8_t *stream = a.cache + (size_t(bh) * a.n_super_cap * D + size_t(kD) * slice) * 4;
     const int n_tok = seg.t_end - seg.t_begin;
-    StreamRing<BITS, STAGES, WIDE> ring{ring_buf, ring_bar, stream + size_t(seg.t_begin / C::TPW) * row_stride,
-                                  (n_tok + kTileTok - 1) / kTileTok, n_tok, kStatVWait, row_stride};
+    StreamRing<BITS, STAGES, WIDE, TOK> ring{ring_buf, ring_bar, stream + size_t(seg.t_begin / C::TPW) * row_stride,
+                                  (n_tok + TOK - 1) / TOK, n_tok, kStatVWait, row_stride};
     ring.prologue(lane);
 
     bool ok = true;
     int i = 0;
     for (; i < ring.n_tiles; ++i) {
-        const int ntok = min(kTileTok, n_tok - i * kTileTok);
+        const int ntok = min(TOK, n_tok - i * TOK);
         if (!(ok = src.tile_weights(i, ntok, lane, acc))) break;
         if (!(ok = ring.wait(i))) break;
         const uint4 *tile = ring.tile(i, lane);
-        if (ntok == kTileTok) {
-            uint4 w = tile[0];
+        const int full = ntok / C::TPW;
+        uint4 w = tile[0];
 #pragma unroll 1
-            for (int wd = 0; wd < Tile<BITS>::WORDS; ++wd) {
-                const uint4 w_next = tile[min(wd + 1, Tile<BITS>::WORDS - 1) * (kD / 4)];
+        for (int wd = 0; wd < full; ++wd) {
+            const uint4 w_next = tile[min(wd + 1, Tile<BITS, TOK>::WORDS - 1) * (kD / 4)];
 #pragma unroll 1
-                for (int c8 = 0; c8 < C::TPW / 8; ++c8) {
-                    v_chunk_h<BITS, G, false>(w, hp, wts, wd * C::TPW + c8 * 8, acc, 8);
-                    if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
-                }
-                w = w_next;
+            for (int c8 = 0; c8 < C::TPW / 8; ++c8) {
+                v_chunk_h<BITS, G, false, TOK>(w, hp, wts, wd * C::TPW + c8 * 8, acc, 8);
+                if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
             }
-        } else {
+            w = w_next;
+        }
 #pragma unroll 1
-            for (int wd = 0; wd * C::TPW < ntok; ++wd) {
-                uint4 w = tile[wd * (kD / 4)];
-                const int count = ntok - wd * C::TPW;
-#pragma unroll 1
-                for (int c8 = 0; c8 < C::TPW / 8 && c8 * 8 < count; ++c8) {
-                    v_chunk_h<BITS, G, true>(w, hp, wts, wd * C::TPW + c8 * 8, acc, count - c8 * 8);
-                    if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
-                }
-            }
+        for (int t = full * C::TPW; t < ntok; t += 8) {
+            v_chunk_h<BITS, G, true, TOK>(w, hp, wts, t, acc, ntok - t);
+            if (C::TPW == 16) { w.x >>= 16; w.y >>= 16; w.z >>= 16; w.w >>= 16; }
         }
         ring.release_and_refill(i, lane);
     }
@@ -475,7 +461,7 @@ template <int BITS, int G, int MODE, class Sink, int ST = kStages, bool WIDE = f
 __device__ __forceinline__ void k_scan(const KArgs &a, const Seg &seg, int b, int h, int lane, uint8_t *buf, uint64_t *bar,
                                        float *red, Sink &sink)
 {
-    if constexpr (MODE == kModeHalf) k_warp_h<BITS, G, Sink, ST, WIDE>(a, seg, b, h, lane, buf, bar, red, sink);
+    if constexpr (MODE == kModeHalf) k_warp_h<BITS, G, Sink, ST, WIDE, TOK>(a, seg, b, h, lane, buf, bar, red, sink);
     else k_warp<BITS, G, MODE, Sink, ST, WIDE, OUTLINE, 8, TOK>(a, seg, b, h, lane, buf, bar, red, sink);
 }
 
@@ -483,7 +469,7 @@ template <int BITS, int G, int MODE, class Src, int ST = kStages, bool WIDE = fa
 __device__ __forceinline__ void v_scan(const VArgs &a, const Seg &seg, int b, int h, int lane, uint8_t *buf, uint64_t *bar,
                                        const float2 *wts, Src &src)
 {
-    if constexpr (MODE == kModeHalf) v_warp_h<BITS, G, Src, ST, WIDE>(a, seg, b, h, lane, buf, bar, wts, src);
+    if constexpr (MODE == kModeHalf) v_warp_h<BITS, G, Src, ST, WIDE, TOK>(a, seg, b, h, lane, buf, bar, wts, src);
     else v_warp<BITS, G, MODE, Src, ST, WIDE, OUTLINE, TOK>(a, seg, b, h, lane, buf, bar, wts, src);
 }
 

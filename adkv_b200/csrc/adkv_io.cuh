@@ -25,23 +25,29 @@ struct GlobalLogitSink {
 
 // The weights of the next tile are fetched while the current one is replayed: with few streams a warp has its scheduler
 // to itself, and a load that is waited for at every tile (about 700 cycles against 1500 of replay) would be paid in full.
-template <int G, bool HALF_W = false>
+template <int G, bool HALF_W = false, int TOK = kTileTok>
 struct GlobalWeightSrc {
+    static constexpr int TPL = TOK / 32;   // weights of a tile that a lane brings
     const __half *row[G];   // attention weights of each q head of this stream: [T+1]
     float2 *wts;            // every weight stored twice
     int T;
-    __half next[G];
+    __half next[G][TPL];
     __device__ __forceinline__ void fetch(int i, int lane)
     {
-        const int t = i * kTileTok + lane;
 #pragma unroll
-        for (int g = 0; g < G; ++g) next[g] = t < T ? row[g][t] : __half(0.f);
+        for (int k = 0; k < TPL; ++k) {
+            const int t = i * TOK + lane + 32 * k;
+#pragma unroll
+            for (int g = 0; g < G; ++g) next[g][k] = t < T ? row[g][t] : __half(0.f);
+        }
     }
     __device__ __forceinline__ bool tile_weights(int i, int, int lane, float (&)[G][4])
     {
         if (i == 0) fetch(0, lane);
 #pragma unroll
-        for (int g = 0; g < G; ++g) put_weight<HALF_W>(wts, g * kTileTok + lane, __half2float(next[g]));
+        for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int k = 0; k < TPL; ++k) put_weight<HALF_W>(wts, g * TOK + lane + 32 * k, __half2float(next[g][k]));
         fetch(i + 1, lane);
         __syncwarp();
         return true;

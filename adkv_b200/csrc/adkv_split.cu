@@ -17,11 +17,12 @@ namespace adkv {
 
 constexpr int kPartStride = 4 + kD;   // floats per (stream, segment, head): max (log2 units), denominator, 2 pad, kD sums
 
-// tokens per tile; the fp16-state scans know tiles of kTileTok only
+// Tokens per tile and stages: see kFusedTok (adkv_fused.cu).  The fp16-state kernel keeps tiles of 32 and with them more CTAs on
+// an SM (see adkv_half_decode_attn).
 template <bool HALF>
-constexpr int kSplitTok = HALF ? kTileTok : 64;
+constexpr int kSplitTok = HALF ? 32 : 64;
 template <bool HALF>
-constexpr int kSplitStages = HALF ? kStages : 2;
+constexpr int kSplitStages = HALF ? 3 : 2;
 
 template <int G, bool HALF_W>
 struct PartialSrc : SoftmaxSrc<G, 1, HALF_W, kSplitTok<HALF_W>> {
