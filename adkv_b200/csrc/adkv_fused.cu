@@ -106,10 +106,12 @@ __global__ void __launch_bounds__(64) decode_attn_kernel(KArgs ka, VArgs va, con
 
 using namespace adkv;
 
-// adkv_decode_attn splits the channels of a head over two warp pairs up to this many (batch, kv head) streams per
-// launch: measured on a B200 (4096 tokens, 4-bit) the split is no slower only while there is at most about one
-// stream per SM (128 streams: 200 us either way); from 256 streams on the whole-head kernel is faster (512 streams:
-// 274 us against 324 us), because the split costs a quarter more instructions and both are then bound by issue.
+// adkv_decode_attn splits the channels of a head over two warp pairs up to one (batch, kv head) stream per SM, and up to 160
+// streams while the set-up counts: a short stream is loaded and appended by more warps, a long one pays the sums, votes and
+// rings of twice as many.  Device time on a B200, 160 streams next to tails, split -> whole head: 4-bit 150 tokens 13.0 -> 13.2
+// us, 2000 tokens 110 -> 91 us; 2-bit with four heads 16.4 -> 18.4 us, 163 -> 142 us; canonical replay, 2-bit, 100 tokens 10.8 ->
+// 11.6 us, 2000 tokens 139 -> 108 us.
+constexpr int kSplitChannelsMaxTokens = 200;
 constexpr long long kSplitChannelsMaxStreams = 160;
 
 ADKV_HIDDEN int adkv_half_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b,
@@ -189,7 +191,8 @@ int adkv_decode_attn(const void *q, void *k_cache, void *v_cache, const void *k_
         return adkv_segments_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, nullptr, s);
     // Very few streams: split every head over two warp pairs (adkv_narrow.cu).
     const bool split = (flags & ADKV_FLAG_SPLIT_CHANNELS) ||
-                       (!(flags & ADKV_FLAG_NO_SPLIT_CHANNELS) && (long long)B * Hkv <= kSplitChannelsMaxStreams);
+                       (!(flags & ADKV_FLAG_NO_SPLIT_CHANNELS) &&
+                        ((long long)B * Hkv <= kSMs || ((long long)B * Hkv <= kSplitChannelsMaxStreams && T < kSplitChannelsMaxTokens)));
     if (split)
         return adkv_narrow_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, exact, s);
     return launch_decode(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, exact, nullptr, s);
