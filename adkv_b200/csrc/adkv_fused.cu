@@ -110,8 +110,8 @@ using namespace adkv;
 // streams while the set-up counts: a short stream is loaded and appended by more warps, a long one pays the sums, votes and
 // rings of twice as many.  Device time on a B200, 160 streams next to tails, split -> whole head: 4-bit 150 tokens 13.0 -> 13.2
 // us, 2000 tokens 110 -> 91 us; 2-bit with four heads 16.4 -> 18.4 us, 163 -> 142 us; canonical replay, 2-bit, 100 tokens 10.8 ->
-// 11.6 us, 2000 tokens 139 -> 108 us.
-constexpr int kSplitChannelsMaxTokens = 200;
+// 11.6 us, 210 tokens with four heads 23.3 -> 24.4 us, 2000 tokens 139 -> 108 us.
+constexpr int kSplitChannelsMaxTokens = 256;
 constexpr long long kSplitChannelsMaxStreams = 160;
 
 ADKV_HIDDEN int adkv_half_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b,

@@ -71,7 +71,7 @@ extern "C" {
  * library decides from the number of streams and tokens of the call:
  *   - token segments: next to tail states, with the contracted replay and up to four query heads per KV head, up to 148
  *     streams (one per SM) of 128 tokens or more are cut along the token axis over eight K and eight V warps;
- *   - split heads: otherwise, up to 148 streams (160 of fewer than 200 tokens) have the channels of a head split over two K
+ *   - split heads: otherwise, up to 148 streams (160 of fewer than 256 tokens) have the channels of a head split over two K
  *     and two V warps;
  *   - whole heads: everything else keeps one warp per tensor and stream, which needs the fewest instructions in all.
  * Next to tail states appended codes and tails do not depend on the layout, bit for bit.  Outputs of split and whole
