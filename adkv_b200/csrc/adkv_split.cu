@@ -122,9 +122,14 @@ __global__ void __launch_bounds__(64) decode_attn_split_kernel(KArgs ka, VArgs v
 }
 
 // out[b, hq, c] = sum_j acc_j[c] * 2^(m_j - M) / sum_j l_j * 2^(m_j - M),  M = max_j m_j.
+// Bound by the latency of its loads, a few hundred nanoseconds each: the maxima and denominators of all segments are read side
+// by side, a segment per thread, and the sums eight segments at a time.  One after the other, the merge was up to a sixth of the
+// step (one B200, whole step): 128 heads x 32 segments 112.8 -> 109.3 us, 32 x 63 49.9 -> 42.5 us, 64 x 39 56.8 -> 51.9 us; with few
+// segments of many heads the barriers cost a little, 512 x 4 59.8 -> 61.0 us.
 __global__ void __launch_bounds__(kD) merge_partials_kernel(const float *__restrict__ scratch, __half *__restrict__ out,
                                                             int Hq, int Hkv, int n_seg)
 {
+    __shared__ float w[kD], part_max[kD / 32], part_sum[kD / 32];
     const int bhq = blockIdx.x, b = bhq / Hq, hq = bhq % Hq, G = Hq / Hkv, h = hq / G, g = hq % G;
     const int c = threadIdx.x;
     // Launched as a programmatic dependent of the segment kernel (its launch latency is paid while that kernel
@@ -134,14 +139,29 @@ __global__ void __launch_bounds__(kD) merge_partials_kernel(const float *__restr
     const float *base = scratch + (size_t(b * Hkv + h) * n_seg * G + g) * kPartStride;
     const size_t seg_stride = size_t(G) * kPartStride;
     float M = -INFINITY;
-    for (int j = 0; j < n_seg; ++j) M = fmaxf(M, base[j * seg_stride]);
+    for (int j = c; j < n_seg; j += kD) M = fmaxf(M, base[j * seg_stride]);
+    M = warp_max(M);
+    if (c % 32 == 0) part_max[c / 32] = M;
+    __syncthreads();
+    M = fmaxf(fmaxf(part_max[0], part_max[1]), fmaxf(part_max[2], part_max[3]));
     float L = 0.f, A = 0.f;
-    for (int j = 0; j < n_seg; ++j) {
-        const float m = base[j * seg_stride];
-        const float w = (m == -INFINITY) ? 0.f : exp2f(m - M);
-        L = fmaf(base[j * seg_stride + 1], w, L);
-        A = fmaf(base[j * seg_stride + 4 + c], w, A);
+    for (int j0 = 0; j0 < n_seg; j0 += kD) {
+        const int n = min(kD, n_seg - j0);
+        if (c < n) {
+            const float2 ml = *reinterpret_cast<const float2 *>(base + (j0 + c) * seg_stride);
+            w[c] = ml.x == -INFINITY ? 0.f : exp2f(ml.x - M);
+            L = fmaf(ml.y, w[c], L);
+        }
+        __syncthreads();
+        const float *acc = base + j0 * seg_stride + 4 + c;
+#pragma unroll 8
+        for (int j = 0; j < n; ++j) A = fmaf(acc[j * seg_stride], w[j], A);
+        __syncthreads();
     }
+    L = warp_sum(L);
+    if (c % 32 == 0) part_sum[c / 32] = L;
+    __syncthreads();
+    L = (part_sum[0] + part_sum[1]) + (part_sum[2] + part_sum[3]);
     out[size_t(bhq) * kD + c] = __float2half_rn(A / L);
 }
 
