@@ -346,11 +346,12 @@ __device__ __noinline__ Chan4 k_chunk_clamped(uint4 w, Chan4 st, PairConsts pc, 
     return st;
 }
 
-// The eps guard is the identity on a scale that is not below eps, and after one update no scale is below smin: with smin
-// at eps or above, and initial scales too, only the clamps are left of the guards (a NaN does not count as above).
-__device__ __forceinline__ bool no_eps_guard(const Chan (&ch)[4], float smin)
+// The eps guard is the identity on a scale that is not below eps, and after one update no scale is below the smaller of the
+// bounds (smax is applied last, and may be below smin): with both at eps or above, and initial scales too, only the clamps
+// are left of the guards (a NaN does not count as above).
+__device__ __forceinline__ bool no_eps_guard(const Chan (&ch)[4], float smin, float smax)
 {
-    return __all_sync(kFull, smin >= kEps && ch[0].s >= kEps && ch[1].s >= kEps && ch[2].s >= kEps && ch[3].s >= kEps);
+    return __all_sync(kFull, smin >= kEps && smax >= kEps && ch[0].s >= kEps && ch[1].s >= kEps && ch[2].s >= kEps && ch[3].s >= kEps);
 }
 
 // Whether chunks that may meet a clamp bound, but not the eps guard, take the packed body with clamps; otherwise the scalar
@@ -415,7 +416,7 @@ __device__ __forceinline__ void k_warp(const KArgs &a, const Seg &seg, int b, in
     }
 
 
-    const bool tame = no_eps_guard(ch, a.smin);
+    const bool tame = no_eps_guard(ch, a.smin, a.smax);
     // some scale may meet a clamp bound within the eight tokens
     auto clamped = [&](const uint4 &w, float *rows) {
         if constexpr (!kPackedClamps<G>) {
@@ -698,7 +699,7 @@ __device__ __forceinline__ void v_warp(const VArgs &a, const Seg &seg, int b, in
         for (int c = 0; c < 4; ++c) acc[g][c] = 0.f;
 
 
-    const bool tame = no_eps_guard(ch, a.smin);
+    const bool tame = no_eps_guard(ch, a.smin, a.smax);
     const auto out_of_line = [&](auto &&body) {   // body: state -> state after the chunk
         VState<G> st;
 #pragma unroll
