@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes
 import importlib.util
 import os
+import warnings
 
 from . import build as _build
 
@@ -111,19 +112,29 @@ def load() -> ctypes.CDLL:
 _host = None
 
 
+def _load_host():
+    if _build.HOST_LIB is None or not os.path.exists(_build.HOST_LIB):
+        raise ImportError(f"{_build.HOST_LIB} is missing: build it with `python -m adkv_b200.build`")
+    import torch  # noqa: F401  (the module links against torch's libraries)
+    spec = importlib.util.spec_from_file_location("_adkv_pyhost", _build.HOST_LIB)
+    mod = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(mod)
+    mod.bind(ctypes.cast(load().adkv_decode_attn, c_void_p).value)
+    return mod
+
+
 def host():
-    """The native host module of ``gemv.decode_attn``, bound to the loaded library."""
+    """The native host module of ``gemv.decode_attn``, bound to the loaded library; False where it does not load (the
+    Python code does the same with more time per call), decided by the first call."""
     global _host
     if _host is None:
-        lib = load()
-        if not os.path.exists(_build.HOST_LIB):
-            raise RuntimeError(f"{_build.HOST_LIB} is missing: build it with `python -m adkv_b200.build`.")
-        import torch  # noqa: F401  (the module links against torch's libraries)
-        spec = importlib.util.spec_from_file_location("_adkv_pyhost", _build.HOST_LIB)
-        mod = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(mod)
-        mod.bind(ctypes.cast(lib.adkv_decode_attn, c_void_p).value)
-        _host = mod
+        try:
+            _host = _load_host()
+        except (ImportError, OSError) as e:
+            warnings.warn(f"adkv_b200: argument checks stay in Python: {e}", RuntimeWarning, stacklevel=3)
+            _host = False
+        except RuntimeError:    # no kernels either: what needs them says so
+            return False
     return _host
 
 

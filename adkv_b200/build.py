@@ -1,11 +1,13 @@
 """Build the C-ABI shared library ``adkv_b200/lib/libadkv_b200.so`` for sm_100a with nvcc, and the host module of gemv.py.
 
 The library has no dependency on torch or Python: plain ``extern "C"`` entry points declared in
-``include/adkv_b200.h``; the host module ``_adkv_pyhost.so`` checks torch tensors and calls it.  It is built in-tree so that it travels with the source snapshot.
+``include/adkv_b200.h``.  The host module checks torch tensors and calls it; it is bound to the torch and Python it was built
+with, which its file name says, and ``gemv.py`` does without it where it is missing.  Both are built in-tree so that they
+travel with the source snapshot.
 """
 from __future__ import annotations
 
-import importlib.util
+import importlib.metadata
 import os
 import shutil
 from concurrent.futures import ThreadPoolExecutor
@@ -17,7 +19,17 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB_DIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIB_DIR, "libadkv_b200.so")
-HOST_LIB = os.path.join(LIB_DIR, "_adkv_pyhost.so")   # argument checks of gemv.decode_attn, against torch's headers
+
+def _host_lib() -> str | None:
+    """Argument checks of gemv.decode_attn, compiled against the headers of the installed torch (None without one)."""
+    try:
+        torch_version = importlib.metadata.version("torch")
+    except importlib.metadata.PackageNotFoundError:
+        return None
+    return os.path.join(LIB_DIR, f"_adkv_pyhost-torch{torch_version}{sysconfig.get_config_var('EXT_SUFFIX')}")
+
+
+HOST_LIB = _host_lib()
 HOST_SOURCE = os.path.join(CSRC, "adkv_pyhost.cpp")
 SOURCES = ["adkv_capi.cu", "adkv_encode.cu", "adkv_fused.cu", "adkv_unfused.cu", "adkv_split.cu", "adkv_wide.cu",
            "adkv_half.cu", "adkv_narrow.cu", "adkv_segments.cu"]
@@ -37,19 +49,26 @@ def _nvcc() -> str:
     return exe
 
 
+def _older(path: str, deps: list[str]) -> bool:
+    return not os.path.exists(path) or any(os.path.getmtime(d) > os.path.getmtime(path) for d in deps)
+
+
 def is_stale() -> bool:
-    if not os.path.exists(LIB) or not os.path.exists(HOST_LIB):
-        return True
-    t = min(os.path.getmtime(LIB), os.path.getmtime(HOST_LIB))
-    deps = [os.path.join(CSRC, f) for f in SOURCES + HEADERS] + [HOST_SOURCE, os.path.abspath(__file__)]
-    return any(os.path.getmtime(d) > t for d in deps)
+    return _older(LIB, [os.path.join(CSRC, f) for f in SOURCES + HEADERS] + [os.path.abspath(__file__)])
+
+
+def host_is_stale() -> bool:
+    header = os.path.join(CSRC, HEADERS[-1])
+    return HOST_LIB is not None and _older(HOST_LIB, [HOST_SOURCE, header, os.path.abspath(__file__)])
 
 
 def build_host(verbose: bool = False) -> str:
-    torch_dir = importlib.util.find_spec("torch").submodule_search_locations[0]
+    import torch
+    torch_dir = os.path.dirname(os.path.abspath(torch.__file__))
     inc = [os.path.join(torch_dir, "include"), os.path.join(torch_dir, "include", "torch", "csrc", "api", "include"),
            sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))), "include")]
-    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", HOST_SOURCE, "-o", HOST_LIB]
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", HOST_SOURCE, "-o", HOST_LIB]
     cmd += ["-I" + d for d in inc] + ["-L" + os.path.join(torch_dir, "lib")]
     cmd += ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
     if verbose:
@@ -59,8 +78,17 @@ def build_host(verbose: bool = False) -> str:
 
 
 def build(force: bool = False, verbose: bool = False, extra: list[str] | None = None) -> str:
-    if not force and not is_stale():
-        return LIB
+    if force or is_stale():
+        _build_library(verbose, extra)
+    if HOST_LIB is not None and (force or host_is_stale()):
+        try:
+            build_host(verbose)
+        except (ImportError, OSError, subprocess.CalledProcessError) as e:   # the library does not need it
+            print(f"host module not built, gemv.decode_attn checks its arguments in Python: {e}", file=sys.stderr)
+    return LIB
+
+
+def _build_library(verbose: bool, extra: list[str] | None) -> None:
     os.makedirs(LIB_DIR, exist_ok=True)
     os.makedirs(OBJ_DIR, exist_ok=True)
     nvcc = _nvcc()
@@ -80,8 +108,6 @@ def build(force: bool = False, verbose: bool = False, extra: list[str] | None = 
     if verbose:
         print(" ".join(link), flush=True)
     subprocess.check_call(link)
-    build_host(verbose)
-    return LIB
 
 
 if __name__ == "__main__":

@@ -490,10 +490,10 @@ def decode_attn(q, k_cache, v_cache, k_new, v_new, k_params, v_params, T: int, s
     warp pairs (launches with few streams) and, next to tails with the contracted replay, a token axis split over eight
     warp pairs (up to 148 streams of 128 tokens or more).  True / False force the second / the first (head dim 128,
     fp32 arithmetic, no checkpoints)."""
-    if mask is None and not ckpt_interval:      # plain contiguous tensors: checked and called in native code
-        done = _lib.host().decode(q, k_cache, v_cache, k_new, v_new, k_params, v_params, T, scaling, scale_min, scale_max, bits,
-                                  out, k_tail, v_tail,
-                                  _lib.flags(_fast_default(fast, k_tail), half_state, tail_keep, split_channels))
+    native = mask is None and not ckpt_interval and _lib.host()
+    if native:                                  # plain contiguous tensors: checked and called in native code
+        done = native.decode(q, k_cache, v_cache, k_new, v_new, k_params, v_params, T, scaling, scale_min, scale_max, bits, out, k_tail, v_tail,
+                             _lib.flags(_fast_default(fast, k_tail), half_state, tail_keep, split_channels))
         if done is not None:
             if isinstance(done, int):
                 _lib.check(done, "decode_attn")

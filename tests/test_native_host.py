@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from adkv_b200 import _lib, gemv, synth
+from adkv_b200 import _lib, build, gemv, synth
 from tests.util import SMAX, SMIN
 
 B, H, D, T, BITS = 2, 2, 128, 40, 4
@@ -76,3 +76,46 @@ def test_what_the_native_path_leaves_alone():
     assert got.shape == (B, H, D)
     with pytest.raises(RuntimeError, match="group size"):                   # the library's refusals keep their text
         gemv.decode_attn(torch.zeros(B, 3 * H, 1, D, dtype=torch.float16, device="cuda"), *base[1:], bits=BITS)
+
+
+@pytest.fixture
+def no_host_module(monkeypatch):
+    monkeypatch.setattr(build, "HOST_LIB", build.HOST_LIB + ".missing")
+    monkeypatch.setattr(_lib, "_host", None)
+    with pytest.warns(RuntimeWarning, match="argument checks stay in Python"):
+        assert not _lib.host()
+
+
+def test_without_the_host_module(no_host_module):
+    """The Python path takes every call, its refusals included; only the first call says so."""
+    args = _args("cpu")
+    with pytest.raises(RuntimeError, match="k_cache must be a CUDA tensor"):
+        gemv.decode_attn(*args)
+
+
+def test_refusals_come_before_missing_kernels(monkeypatch):
+    def missing():
+        raise RuntimeError("libadkv_b200.so is missing")
+    monkeypatch.setattr(_lib, "load", missing)
+    monkeypatch.setattr(_lib, "_host", None)
+    with pytest.raises(RuntimeError, match="q must be float16"):
+        args = _args("cpu")
+        gemv.decode_attn(args[0].float(), *args[1:])
+
+
+def test_build_goes_on_without_the_host_module(monkeypatch, tmp_path, capsys):
+    """A torch of another version or Python asks for another file; a compiler that is missing costs the host module only."""
+    assert torch.__version__ in build.HOST_LIB and build.HOST_LIB.endswith(".so")
+    monkeypatch.setattr(build, "HOST_LIB", str(tmp_path / "other_torch.so"))
+    monkeypatch.setattr(build, "HOST_SOURCE", str(tmp_path / "missing.cpp"))
+    monkeypatch.setattr(build, "is_stale", lambda: False)
+    monkeypatch.setattr(build, "host_is_stale", lambda: True)
+    assert build.build() == build.LIB
+    assert "host module not built" in capsys.readouterr().err
+
+
+@pytest.mark.gpu
+def test_results_without_the_host_module(request):
+    want = gemv.decode_attn(*_args("cuda"), bits=BITS)
+    request.getfixturevalue("no_host_module")
+    assert torch.equal(gemv.decode_attn(*_args("cuda"), bits=BITS), want)
