@@ -107,29 +107,37 @@ PyObject *decode(PyObject *, PyObject *const *a, Py_ssize_t n)
                 tail[i] = t->data_ptr();
             }
         }
-        at::Tensor out;
+        void *const stream = c10::cuda::getCurrentCUDAStream(dev.index).stream();
+        const void *const qp = q->data_ptr();
+        void *const kcp = kc->data_ptr(), *const vcp = vc->data_ptr();
+        // Everything that may fail comes before the launch, the Python object of the result too: a step that has been
+        // launched must not be left to the Python code, which would launch it again.
+        void *op;
+        PyObject *result;
         if (a[12] == Py_None) {
-            out = at::empty({B, Hq, D}, kc->options().dtype(at::kHalf));
+            const at::Tensor out = at::empty({B, Hq, D}, kc->options().dtype(at::kHalf));
             if (!out.is_cuda() || !out.has_storage()) Py_RETURN_NONE;
+            op = out.data_ptr();
+            result = THPVariable_Wrap(out);
+            if (!result) {
+                PyErr_Clear();
+                Py_RETURN_NONE;
+            }
         } else {
             const at::Tensor *t = dev.tensor(a[12], at::kHalf);
             if (!t || t->dim() != 3 || t->size(0) != B || t->size(1) != Hq || t->size(2) != D) Py_RETURN_NONE;
-            out = *t;
+            op = t->data_ptr();
+            result = a[12];
+            Py_INCREF(result);
         }
-        void *const stream = c10::cuda::getCurrentCUDAStream(dev.index).stream();
-        const void *const qp = q->data_ptr();
-        void *const kcp = kc->data_ptr(), *const vcp = vc->data_ptr(), *const op = out.data_ptr();
         int rc;
         Py_BEGIN_ALLOW_THREADS
         rc = g_decode(qp, kcp, vcp, kn, vn, &kp, &vp, tail[0], tail[1], nullptr, 0, op, int(B), int(Hq), int(Hkv), T, int(D),
                       int(cap), bits, scaling, smin, smax, unsigned(flags), stream);
         Py_END_ALLOW_THREADS
-        if (rc) return PyLong_FromLong(rc);
-        if (a[12] != Py_None) {
-            Py_INCREF(a[12]);
-            return a[12];
-        }
-        return THPVariable_Wrap(out);
+        if (!rc) return result;
+        Py_DECREF(result);
+        return PyLong_FromLong(rc);
     } catch (...) {   // out of memory and the like: the Python code meets it again and raises what it raises
         PyErr_Clear();
         Py_RETURN_NONE;

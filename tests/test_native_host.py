@@ -1,5 +1,8 @@
 """The native host path of ``gemv.decode_attn``: what it takes over equals the Python path, what it does not take over is left
 alone and refused or converted as before."""
+import ctypes
+import gc
+
 import numpy as np
 import pytest
 import torch
@@ -119,3 +122,66 @@ def test_results_without_the_host_module(request):
     want = gemv.decode_attn(*_args("cuda"), bits=BITS)
     request.getfixturevalue("no_host_module")
     assert torch.equal(gemv.decode_attn(*_args("cuda"), bits=BITS), want)
+
+
+def _step(native, Hq=H, out=None, **kw):
+    args = _args("cuda")
+    args[0] = torch.randn(B, Hq, 1, D, generator=torch.Generator().manual_seed(5)).half().cuda().requires_grad_()
+    kt, vt = (None, None) if kw.get("half_state") else _tails()
+    q = args[0] if native else args[0].as_subclass(type("T2", (torch.Tensor,), {}))
+    got = gemv.decode_attn(q, *args[1:], bits=BITS, out=out, k_tail=kt, v_tail=vt, **kw)
+    assert not got.requires_grad
+    return [got, args[1], args[2]] + ([] if kt is None else [kt, vt])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kw", [dict(Hq=4 * H), dict(half_state=True), dict(tail_keep=True), dict(split_channels=True, fast=False)])
+def test_options_equal_the_python_path(kw):
+    for a, b in zip(_step(True, **kw), _step(False, **kw)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.gpu
+def test_side_stream_and_capture():
+    """The native path launches on the current stream: a side stream sees its own inputs, a capture records the step."""
+    want = _step(False, tail_keep=True)
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        got = _step(True, tail_keep=True)
+        args, (kt, vt) = _args("cuda"), _tails()
+    s.synchronize()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    ref = gemv.decode_attn(*args, bits=BITS, k_tail=kt, v_tail=vt, tail_keep=True).clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = gemv.decode_attn(*args, bits=BITS, k_tail=kt, v_tail=vt, tail_keep=True)
+    out.zero_()
+    graph.replay()
+    assert torch.equal(out, ref)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rc", [0, -3])
+def test_one_launch_a_step(rc):
+    """Nothing that may fail is left to be done once the step is launched (the Python path would launch it again): the result's
+    Python object is there when the library is called."""
+    seen = []
+
+    @ctypes.CFUNCTYPE(ctypes.c_int, *_lib.SIGNATURES["adkv_decode_attn"])
+    def launch(*a):
+        seen.append(any(type(o) is torch.Tensor and o.is_cuda and o.data_ptr() == a[11] for o in gc.get_objects()))
+        return rc
+
+    args = _args("cuda")
+    host = _lib.host()
+    host.bind(ctypes.cast(launch, ctypes.c_void_p).value)
+    try:
+        if rc:
+            with pytest.raises(RuntimeError, match="decode_attn"):
+                gemv.decode_attn(*args, bits=BITS)
+        else:
+            assert gemv.decode_attn(*args, bits=BITS).shape == (B, H, D)
+    finally:
+        host.bind(ctypes.cast(_lib.load().adkv_decode_attn, ctypes.c_void_p).value)
+    assert seen == [True]
