@@ -1,5 +1,5 @@
-"""2-bit prefill of few streams (codes from comparisons) against the oracle and against the quotient form that launches with
-many streams take, bit for bit.  Needs a B200."""
+"""2-bit prefill of few streams (codes from comparisons) against exact fp32 division in numpy and against the quotient form that
+launches with many streams take, bit for bit.  Needs a B200."""
 import numpy as np
 import pytest
 import torch
@@ -10,7 +10,7 @@ from tests.util import SMAX, SMIN, np_params
 
 pytestmark = pytest.mark.gpu
 
-H, D, MANY = 2, 128, 80      # 80 sequences x 2 heads x K and V: 320 streams, past the 296 that count as few
+H, D, MANY = 2, 128, 160     # 160 sequences x 2 heads x K and V: 640 streams, well past the 444 that count as few
 
 
 def _inputs(T, special):
@@ -53,6 +53,21 @@ def _encode(x, p, B, smin, smax, t_start=0):
     return kc, kt
 
 
+def _reference(x, p, smin, smax):
+    """Codes and final state by numpy's fp32 division; minimum and maximum as on the device, where a NaN gives the other operand."""
+    zp, s, alpha, beta, target = (np.broadcast_to(a.astype(np.float32), (1, H, D)) for a in np_params(p))
+    lo, hi = np.float32(smin), np.float32(smax)
+    codes = np.empty(x.shape, np.int8)
+    with np.errstate(all="ignore"):
+        for t in range(x.shape[2]):
+            ss = np.fmax(s, np.float32(1e-8))
+            q = np.fmin(np.fmax(np.rint((x[:, :, t] - zp) / ss), np.float32(-2)), np.float32(1))
+            codes[:, :, t] = q.astype(np.int8)
+            zp = zp + alpha * (q * ss)
+            s = np.fmin(np.fmax(s + s * beta * (np.abs(q) - target), lo), hi)
+    return codes, np.stack([zp, s], axis=2)
+
+
 @pytest.mark.parametrize("T,t_start", [(7, 0), (8, 0), (9, 0), (16, 0), (33, 0), (777, 0), (100, 13)])
 @pytest.mark.parametrize("special,smin,smax", [(False, SMIN, SMAX), (True, SMIN, SMAX), (True, 0.0, 1e30)])
 def test_few_streams(T, t_start, special, smin, smax):
@@ -61,8 +76,10 @@ def test_few_streams(T, t_start, special, smin, smax):
     mc, mt = _encode(x, p, MANY, smin, smax, t_start)
     assert torch.equal(kc[0], mc[0]) and torch.equal(mc[0], mc[MANY - 1])
     assert torch.equal(kt[0].view(torch.int32), mt[0].view(torch.int32))
+    codes, tail = _reference(x.float().numpy(), p, smin, smax)
+    assert np.array_equal(kc.cpu().numpy(), orc.pack_codes(codes, 2, kc.shape[2]))
+    assert np.array_equal(kt.cpu().numpy(), tail, equal_nan=True)
     if not special:
         want = np.zeros(kc.shape, np.uint8)
-        _, st = orc.encode_kv(want, x.numpy(), np_params(p), 2, smin, smax)
+        orc.encode_kv(want, x.numpy(), np_params(p), 2, smin, smax)
         assert np.array_equal(kc.cpu().numpy(), want)
-        assert np.array_equal(kt.cpu().numpy(), np.stack([st.zp, st.s], axis=2).astype(np.float32))

@@ -198,7 +198,7 @@ def test_layered_append_forms():
 
 @pytest.mark.parametrize("Hq,Hkv,T,bits", [(2, 2, 0, 4), (2, 2, 95, 4), (8, 2, 129, 2), (4, 2, 300, 4)])
 def test_two_streams_per_sm(Hq, Hkv, T, bits):
-    """160 streams, more than the segments take: what the library picks, against one warp pair per stream."""
+    """160 streams, more than the segments take: what the library picks and split heads, against one warp pair per stream."""
     B, D = 80, 128
     case = make_case(900 + T, 2, Hq, Hkv, T, bits)
     dk, dv, tk, tv, ok_, ov_, *_ = _prefill(case, T + 1)
@@ -207,10 +207,11 @@ def test_two_streams_per_sm(Hq, Hkv, T, bits):
             T, 0.08, SMIN, SMAX)
     kw = dict(bits=bits, k_tail=rep(tk), v_tail=rep(tv), tail_keep=True)
     want = gemv.decode_attn(*args, **kw, split_channels=False)
-    got = gemv.decode_attn(*args, **kw)
-    _status_ok()
-    np.testing.assert_allclose(got.float().cpu().numpy(), want.float().cpu().numpy(), rtol=RTOL, atol=ATOL)
-    assert torch.equal(got[:2], got[-2:])
+    for split in (None, True):
+        got = gemv.decode_attn(*args, **kw, split_channels=split)
+        _status_ok()
+        np.testing.assert_allclose(got.float().cpu().numpy(), want.float().cpu().numpy(), rtol=RTOL, atol=ATOL)
+        assert torch.equal(got[:2], got[-2:])
 
 
 @pytest.mark.parametrize("T,bits", [(1, 4), (33, 4), (70, 2)])
@@ -312,9 +313,9 @@ def test_logit_error_is_that_of_a_whole_scan(B, T, bits, pinned):
 
 @pytest.mark.parametrize("T,bits", [(70, 4), (161, 2)])
 def test_checkpoints_of_few_and_many_streams(T, bits):
-    """Checkpoints, codes and tails of a prefill with a channel pair per thread (more than 296 (stream, tensor) pairs) are
+    """Checkpoints, codes and tails of a prefill with a channel pair per thread (more than 444 (stream, tensor) pairs) are
     those of the one-channel form, bit for bit; started inside a word as well as at the front."""
-    B, H, D, S = 80, 2, 128, 32
+    B, H, D, S = 160, 2, 128, 32
     case = make_case(50 + T, 1, H, H, T, bits)
     kp, vp = dev(case["kp"]), dev(case["vp"])
 
