@@ -63,6 +63,37 @@ def test_checkpointed_generation_matches_plain(bits, Hq, Hkv, T0, steps, S):
         assert np.array_equal(got[:, :, k, 1].view(np.uint32), s_.view(np.uint32)), k
 
 
+@pytest.mark.parametrize("T,G,bits", [(32, 1, 4), (255, 2, 4), (256, 1, 2), (287, 1, 4), (4095, 1, 4), (4096, 4, 2), (8300, 1, 4)])
+def test_merge_of_many_segments(T, G, bits):
+    """1 to 260 segments of 32 tokens, the merge of few of them, of up to 128 at once and of several rounds; whole segments
+    masked out, the first 128 of 260 among them.  Against the unsplit step and the oracle."""
+    B, Hkv, D, S = 2, 2, 128, 32
+    case = make_case(700 + T, B, G * Hkv, Hkv, T, bits)
+    kp, vp = dev(case["kp"]), dev(case["vp"])
+    kc, vc = (torch.zeros(orc.cache_shape(B, Hkv, orc.n_super_for(T + 1, bits), D), dtype=torch.uint8, device="cuda") for _ in range(2))
+    ck = [gemv.alloc_ckpt(B, Hkv, D, T + 1, S, "cuda") for _ in range(2)]
+    gemv.encode_kv_pair(kc, dev(case["k"][:, :, :T]), kp, vc, dev(case["v"][:, :, :T]), vp, SMIN, SMAX, bits=bits, k_ckpt=ck[0],
+                        v_ckpt=ck[1], ckpt_interval=S)
+    mask = torch.zeros(B, T + 1)
+    mask[0, :T - T // 32 // 2 * 32] = -float("inf")
+    mask[1].view(-1)[: T // 96 * 96].view(-1, 96)[:, 64:] = -float("inf")      # every third segment
+    if T > 8000:
+        mask[1, :128 * 32] = -float("inf")
+    new = (dev(case["k"][:, :, T:]), dev(case["v"][:, :, T:]))
+    wk, wv = kc.cpu().numpy(), vc.cpu().numpy()
+    want = orc.decode_attn(case["q"][:, :, 0].numpy(), wk, wv, new[0][:, :, 0].cpu().numpy(), new[1][:, :, 0].cpu().numpy(),
+                           np_params(case["kp"]), np_params(case["vp"]), T, 0.07, mask=mask[:, None].numpy(), bits=bits,
+                           scale_min=SMIN, scale_max=SMAX)
+    outs = []
+    for kw in (dict(k_ckpt=ck[0], v_ckpt=ck[1], ckpt_interval=S), dict(split_channels=False)):
+        a, b = kc.clone(), vc.clone()
+        outs.append(gemv.decode_attn(dev(case["q"]), a, b, *new, kp, vp, T, 0.07, SMIN, SMAX, bits=bits, mask=dev(mask), **kw).float())
+        np.testing.assert_allclose(outs[-1].cpu().numpy(), want, rtol=RTOL, atol=ATOL)
+        assert np.array_equal(a.cpu().numpy(), wk) and np.array_equal(b.cpu().numpy(), wv)
+    torch.testing.assert_close(outs[0], outs[1], rtol=RTOL, atol=ATOL)
+    assert gemv.device_status() == 0
+
+
 def test_checkpointed_append_and_errors():
     B, H, D, T, S, bits = 1, 2, 128, 95, 32, 4
     x = synth.gen_kv(9, B, H, T + 2, D)

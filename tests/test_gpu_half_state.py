@@ -179,6 +179,41 @@ def test_fused_decode_against_numpy_restatement(B, Hq, Hkv, T, bits):
     assert gemv.device_status() == 0
 
 
+@pytest.mark.parametrize("varlen", [False, True])
+@pytest.mark.parametrize("G,T,bits", [(1, 131, 4), (1, 64, 2), (4, 77, 4), (4, 203, 2), (8, 33, 4)])
+def test_more_streams_than_fit_the_chip(G, T, bits, varlen):
+    """Past the streams that the launch with 64-token tiles is for (at most 1628): tiles of 32 tokens, ragged ends, masks and
+    device-side lengths.  Three sequences, repeated, against the numpy restatement and the same sequences alone."""
+    n, Hkv, rep = 3, 2, 280
+    k, v, kp, vp, kc, vc = _prefilled(1300 + T, n, Hkv, T, bits)
+    q = synth.gen_q(1301 + T, n, G * Hkv, D).cuda()
+    kn, vn = k[:, :, T:].contiguous(), v[:, :, T:].contiguous()
+    mask = torch.zeros(n, T + 1)
+    if not varlen:
+        mask[0, : T // 3] = -1e4
+    okc, ovc = kc.cpu().numpy().copy(), vc.cpu().numpy().copy()
+    want, _ = orh.decode_attn(q[:, :, 0].cpu().numpy(), okc, ovc, kn[:, :, 0].cpu().numpy(), vn[:, :, 0].cpu().numpy(), np16(kp),
+                              np16(vp), T, D ** -0.5, bits, mask=mask.numpy())
+    outs = []
+    for r in (1, rep):
+        m = lambda t: t.repeat(r, *([1] * (t.dim() - 1)))
+        a, b = m(kc), m(vc)
+        args = (m(q), a, b, m(kn), m(vn), kp, vp)
+        if varlen:
+            lens = torch.full((n * r,), T, dtype=torch.int32, device="cuda")
+            got = gemv.decode_attn_varlen(*args, lens, D ** -0.5, SMIN, SMAX, bits=bits, half_state=True)
+        else:
+            got = gemv.decode_attn(*args, T, D ** -0.5, SMIN, SMAX, bits=bits, half_state=True, mask=m(mask).cuda())
+        assert torch.equal(got, m(got[:n])) and torch.equal(a, m(a[:n])) and torch.equal(b, m(b[:n]))
+        assert np.array_equal(a[:n].cpu().numpy(), okc) and np.array_equal(b[:n].cpu().numpy(), ovc)
+        outs.append(got[:n].float().cpu().numpy())
+        # logits are summed in fp16 over the 128 channels (as in the reference's kernel): tolerance of that sum
+        np.testing.assert_allclose(outs[-1], want, rtol=2e-2, atol=2e-2 * max(1.0, np.abs(want).max()))
+    # the same logits, summed by tiles of other lengths in fp32
+    np.testing.assert_allclose(outs[0], outs[1], rtol=5e-3, atol=5e-3 * max(1.0, np.abs(want).max()))
+    assert gemv.device_status() == 0
+
+
 @pytest.mark.parametrize("bits", [4, 2])
 def test_trio_against_numpy_restatement(bits):
     B, Hq, Hkv, T = 2, 4, 2, 75
