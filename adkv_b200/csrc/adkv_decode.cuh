@@ -351,7 +351,8 @@ __device__ __noinline__ Chan4 k_chunk_clamped(uint4 w, Chan4 st, PairConsts pc, 
 // are left of the guards (a NaN does not count as above).
 __device__ __forceinline__ bool no_eps_guard(const Chan (&ch)[4], float smin, float smax)
 {
-    return __all_sync(kFull, smin >= kEps && smax >= kEps && ch[0].s >= kEps && ch[1].s >= kEps && ch[2].s >= kEps && ch[3].s >= kEps);
+    return smin >= kEps && smax >= kEps &&
+           __all_sync(kFull, ch[0].s >= kEps && ch[1].s >= kEps && ch[2].s >= kEps && ch[3].s >= kEps);
 }
 
 // Whether chunks that may meet a clamp bound, but not the eps guard, take the packed body with clamps; otherwise the scalar
