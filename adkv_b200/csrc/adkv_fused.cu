@@ -28,17 +28,24 @@ constexpr bool kOutOfLineGuarded = BITS == 4 && G == 1;
 // in the order of the batch an SM may hold several long streams while its neighbours run dry.  Measured on a B200, lengths
 // spread evenly between a twentieth of the longest and the longest, order of the batch -> longest first, 32 heads:
 //    4-bit, 48 sequences x 3000 tokens 324 -> 252 us; 24 x 2000 154 -> 131 us; 2-bit, 8 KV heads, 96 x 3000 372 -> 304 us
-// Every CTA ranks the lengths for itself, in shared memory: B * B / 64 comparisons a thread.  For caches of a few hundred
-// tokens that can be more than it gains (2-bit, 96 x 200 tokens: 59.4 -> 62.4 us, measured with a costlier count), and more than 128 sequences fill the chip
-// several times over, so that its scheduler evens them out.
-constexpr int kRankMax = 128, kRankMinTokens = 512;
-__device__ __forceinline__ int longest_first(const int *__restrict__ seq_lens, int B, int r, int *key /* [kRankMax + 1] shared */)
+// Every CTA ranks the lengths for itself, in shared memory: B * B / 64 comparisons a thread.  With many CTAs to an SM and no sequence
+// of a few hundred tokens that is more than it gains, however large the cache: 128 sequences of 150 to 200 tokens in a cache for
+// 4096, 4-bit, 32 heads, 101 us in the order of the batch, 112 us ranked; 2-bit, 8 KV heads, 48 sequences 30.3 us against 28.2 us
+// ranked.  More than 128 sequences fill the chip several times over, so that its scheduler evens them out.
+// A call, not inlined, and no early return: either would change the registers of the scans behind it (up to 5 % of a step).
+constexpr int kRankMax = 128, kRankMinTokens = 512, kRankAlways = 8 * kSMs;
+__device__ __noinline__ int longest_first(const int *__restrict__ seq_lens, int B, int r, int *key /* [kRankMax + 1] shared */)
 {
     // length and index in one number, all different; lengths that no cache holds fall together at either end
-    for (int i = threadIdx.x; i < kRankMax; i += 64)
-        key[i] = i < B ? min(max(seq_lens[i], 0), 1 << 23) * kRankMax + (kRankMax - 1 - i) : -1;
-    __syncthreads();
-    for (int b = threadIdx.x; b < B; b += 64) {
+    bool any_long = false;
+    for (int i = threadIdx.x; i < kRankMax; i += 64) {
+        const int len = i < B ? min(max(seq_lens[i], 0), 1 << 23) : 0;
+        any_long |= len >= kRankMinTokens;
+        key[i] = i < B ? len * kRankMax + (kRankMax - 1 - i) : -1;
+    }
+    if (threadIdx.x == 0) key[kRankMax] = r;
+    const int n = __syncthreads_or(any_long || gridDim.x <= kRankAlways) ? B : 0;
+    for (int b = threadIdx.x; b < n; b += 64) {
         const int mine = key[b];
         int before = 0;
         for (int i = 0; i < B; i += 4) {

@@ -8,17 +8,19 @@ from tests.util import SMAX, SMIN
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("B,Hkv,cap", [(2, 80, 520), (50, 3, 512), (65, 3, 512), (128, 2, 512), (129, 2, 512)])
-def test_ranked_lengths(B, Hkv, cap):
-    """More than 148 streams, 512 tokens and more: up to 128 sequences are ranked.  Equal lengths, empty sequences and full
-    caches among them; every sequence as the dense call with one warp per tensor gives it (the same scan: bit-equal)."""
+@pytest.mark.parametrize("B,Hkv,cap,room", [(2, 80, 520, 520), (50, 3, 512, 512), (65, 3, 512, 512), (128, 2, 512, 512),
+                                            (129, 2, 512, 512), (60, 3, 512, 4000), (60, 3, 513, 4000)])
+def test_ranked_lengths(B, Hkv, cap, room):
+    """More than 148 streams, 512 tokens and more: up to 128 sequences are ranked, unless all are shorter.  Equal lengths, empty
+    sequences and full caches among them; every sequence as the dense call with one warp per tensor gives it (the same scan:
+    bit-equal)."""
     D, bits = 128, 4
     g = torch.Generator().manual_seed(B)
     lens = torch.randint(0, cap, (B,), generator=g)
     lens[::7] = lens[0]
     lens[1], lens[B - 1] = 0, cap - 1
     kp, vp = synth.gen_params(3, Hkv, D, bits, device="cuda"), synth.gen_params(4, Hkv, D, bits, device="cuda")
-    shape = (B, Hkv, gemv.n_super_for(cap, bits), D // 4, 4, 4)
+    shape = (B, Hkv, gemv.n_super_for(room, bits), D // 4, 4, 4)
     kc, vc = (torch.randint(0, 256, shape, dtype=torch.uint8, generator=g).cuda() for _ in range(2))
     kt, vt = (torch.rand(B, Hkv, 2, D, generator=g).cuda() + 0.1 for _ in range(2))
     q, kn, vn = (torch.randn(B, Hkv, 1, D, generator=g).half().cuda() for _ in range(3))
