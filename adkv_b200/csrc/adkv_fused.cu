@@ -13,8 +13,10 @@ namespace adkv {
 // softmax with its shuffles, and a refill: a few hundred instructions and, for a warp that has its scheduler to itself, about
 // a thousand cycles.  Tiles of 32 (three stages) -> 64 (two), device time on a B200: 2-bit, 256 streams of four heads x 32768
 // tokens 2359 -> 2183 us, 4-bit x 2000 tokens 162 -> 134 us; 4096 streams x 4096 tokens 1442 -> 1411 us, 256 x 2000 98 -> 91 us,
-// 768 x 1531 143 -> 136 us.  Tiles of 128 give 1 % at 2-bit codes and lose 6 % at 200 tokens.
-constexpr int kFusedTok = 64, kFusedStages = 2;
+// 768 x 1531 143 -> 136 us.  Tiles of 128 give 1 % at 2-bit codes and lose 6 % at 200 tokens.  Where the longer tiles are the
+// slower ones: see short_tiles.
+template <int TOK>
+constexpr int kFusedStages = TOK == 64 ? 2 : 3;
 
 // Whether the guarded chunk bodies of this instantiation are function calls (see k_chunk_guarded).  Measured on a
 // B200 against the inline form, streams of 32 heads x 128: 4-bit codes with one query head per KV head gain 13 % at
@@ -58,18 +60,19 @@ __device__ __noinline__ int longest_first(const int *__restrict__ seq_lens, int 
     return key[kRankMax];
 }
 
-// n_rank: number of sequences if the CTAs take them longest first, 0 if in the order of the batch.
-template <int BITS, int G, int ARITH>
+// n_rank: number of sequences if the CTAs may take them longest first, 0 if in the order of the batch.
+template <int BITS, int G, int ARITH, int TOK>
 __global__ void __launch_bounds__(64) decode_attn_kernel(KArgs ka, VArgs va, const float *__restrict__ mask,
                                                          long long mask_stride_b, float scaling,
                                                          const int *__restrict__ seq_lens, int n_rank)
 {
-    __shared__ alignas(128) uint8_t kbuf[kFusedStages * Tile<BITS, kFusedTok>::BYTES];
-    __shared__ alignas(128) uint8_t vbuf[kFusedStages * Tile<BITS, kFusedTok>::BYTES];
+    constexpr int ST = kFusedStages<TOK>;
+    __shared__ alignas(128) uint8_t kbuf[ST * Tile<BITS, TOK>::BYTES];
+    __shared__ alignas(128) uint8_t vbuf[ST * Tile<BITS, TOK>::BYTES];
     __shared__ alignas(16) float red[G * 8 * kRedRow];
-    __shared__ alignas(16) float2 wts[G * kFusedTok];
-    __shared__ FusedShared<G, 1, kFusedTok> fs;
-    __shared__ uint64_t kbar[kFusedStages], vbar[kFusedStages];
+    __shared__ alignas(16) float2 wts[G * TOK];
+    __shared__ FusedShared<G, 1, TOK> fs;
+    __shared__ uint64_t kbar[ST], vbar[ST];
 
     int b = blockIdx.x / ka.Hkv;
     const int h = blockIdx.x % ka.Hkv;
@@ -87,25 +90,27 @@ __global__ void __launch_bounds__(64) decode_attn_kernel(KArgs ka, VArgs va, con
         va.T = T;
     }
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kFusedStages; ++i) { mbar_init(&kbar[i], 1); mbar_init(&vbar[i], 1); }
+        for (int i = 0; i < ST; ++i) { mbar_init(&kbar[i], 1); mbar_init(&vbar[i], 1); }
         fs.init_barriers(1);
         mbar_init_fence();
     }
     __syncthreads();
     const Seg seg{0, ka.T, true, nullptr, nullptr, 0};
     if (warp == 0) {
-        RingSink<G, 1, kFusedTok> sink{&fs, 0, 0};
-        k_warp<BITS, G, ARITH, RingSink<G, 1, kFusedTok>, kFusedStages, false, kOutOfLineGuarded<BITS, G>, 8, kFusedTok>(ka, seg, b, h, lane, kbuf, kbar, red, sink);
+        RingSink<G, 1, TOK> sink{&fs, 0, 0};
+        k_warp<BITS, G, ARITH, RingSink<G, 1, TOK>, ST, false, kOutOfLineGuarded<BITS, G>, 8, TOK>(ka, seg, b, h, lane, kbuf, kbar,
+                                                                                                   red, sink);
     } else {
-        SoftmaxSrc<G, 1, false, kFusedTok> src;
+        SoftmaxSrc<G, 1, false, TOK> src;
         src.sh = &fs;
         src.wts = wts;
         src.mask = mask ? mask + size_t(b) * mask_stride_b : nullptr;
         src.scale2 = scaling * 1.4426950408889634f;
-        src.n_tiles = (va.T + kFusedTok - 1) / kFusedTok;
+        src.n_tiles = (va.T + TOK - 1) / TOK;
         src.t_begin = 0;
         src.init();
-        v_warp<BITS, G, ARITH, SoftmaxSrc<G, 1, false, kFusedTok>, kFusedStages, false, kOutOfLineGuarded<BITS, G>, kFusedTok>(va, seg, b, h, lane, vbuf, vbar, wts, src);
+        v_warp<BITS, G, ARITH, SoftmaxSrc<G, 1, false, TOK>, ST, false, kOutOfLineGuarded<BITS, G>, TOK>(va, seg, b, h, lane, vbuf,
+                                                                                                         vbar, wts, src);
     }
 }
 
@@ -154,14 +159,43 @@ static bool use_segments(const KArgs &ka, int B, int max_tokens, bool exact, uns
            ka.Hq / ka.Hkv <= 4 && (long long)B * ka.Hkv <= kSegmentsMaxStreams && max_tokens >= kSegmentsMinTokens;
 }
 
+// Whether a launch of whole heads takes tiles of 32 tokens (three stages) instead of 64 (two).  V starts when K is through its
+// first tile, so a stream of one or a few tiles is walked by one warp after the other; with few CTAs on an SM nothing fills that
+// gap.  With eight query heads 64 tokens also take 38 KB of shared memory (4-bit), so that fewer CTAs fit an SM than its
+// registers allow; long streams make up for it.  Device time on a B200, next to tails, 64 -> 32 tokens:
+//    up to 64 tokens      256 streams, 2-bit, four heads 12.1 -> 10.7 us; 600 streams, 4-bit 12.4 -> 11.4 us; but 4096 streams, 4-bit,
+//                         four heads 60 -> 62 us
+//    up to 255 tokens     600 streams x 150, 4-bit 20.7 -> 19.9 us, 2-bit, four heads 31.9 -> 29.6 us; 256 x 200, 2-bit, two heads,
+//                         canonical replay 20.0 -> 19.3 us; but 256 x 200, 4-bit, two heads 17.0 -> 17.6 us; 600 x 150, 4-bit, four heads
+//                         31.2 -> 32.1 us; 4096 x 200, 2-bit, four heads 141 -> 151 us
+//    eight heads          4-bit, 4096 x 150 287 -> 246 us, 4096 x 1000 964 -> 916 us, 600 x 300 72.0 -> 68.6 us, but 1200 x 1000 342 ->
+//                         354 us, 150 x 1000 100 -> 103 us;
+//                         2-bit, 600 x 200 55.9 -> 51.9 us, 4096 x 150 167 -> 158 us, but 4096 x 300 486 -> 505 us
+// Up to one stream per SM only calls with device-side lengths or split_channels = False come here; they keep 64.
+// T: the tokens of every sequence, or what the cache can hold of them where the lengths are on the device.
+static bool short_tiles(int bits, int G, long long streams, int T)
+{
+    const bool many = streams > 8 * kSMs;
+    if (G == 8) return T < (bits == 4 ? (streams > 16 * kSMs ? 1024 : 512) : (many ? 192 : 256));
+    if (many || streams <= kSMs || (bits == 4 && G == 4)) return false;
+    if (T <= 64) return true;
+    return T < 256 && (bits == 4 ? streams > 2 * kSMs : G > 1);
+}
+
 // One CTA per stream.
 static int launch_decode(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b, float scaling, int B,
-                         int bits, bool exact, const int *seq_lens, cudaStream_t s)
+                         int max_tokens, int bits, bool exact, const int *seq_lens, cudaStream_t s)
 {
     const int n_rank = seq_lens && B <= kRankMax && ka.n_super_cap >= kRankMinTokens * bits / 32 ? B : 0;
+    if (short_tiles(bits, ka.Hq / ka.Hkv, (long long)B * ka.Hkv, max_tokens)) {
+        ADKV_DISPATCH(bits, exact, ka.Hq / ka.Hkv,
+                      (decode_attn_kernel<BITS, G, ARITH, 32><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling,
+                                                                                       seq_lens, n_rank)))
+        return launch_status();
+    }
     ADKV_DISPATCH(bits, exact, ka.Hq / ka.Hkv,
-                  (decode_attn_kernel<BITS, G, ARITH><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling,
-                                                                               seq_lens, n_rank)))
+                  (decode_attn_kernel<BITS, G, ARITH, 64><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling,
+                                                                                   seq_lens, n_rank)))
     return launch_status();
 }
 
@@ -202,7 +236,7 @@ int adkv_decode_attn(const void *q, void *k_cache, void *v_cache, const void *k_
                         ((long long)B * Hkv <= kSMs || ((long long)B * Hkv <= kSplitChannelsMaxStreams && T < kSplitChannelsMaxTokens)));
     if (split)
         return adkv_narrow_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, exact, s);
-    return launch_decode(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, exact, nullptr, s);
+    return launch_decode(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, T, bits, exact, nullptr, s);
 }
 
 int adkv_decode_attn_varlen(const void *q, void *k_cache, void *v_cache, const void *k_new, const void *v_new,
@@ -229,9 +263,10 @@ int adkv_decode_attn_varlen(const void *q, void *k_cache, void *v_cache, const v
     if (flags & ADKV_FLAG_HALF_STATE)
         return adkv_half_decode_attn(ka, va, nullptr, 0, scaling, B, bits, static_cast<const int *>(seq_lens), s);
     const bool exact = !(flags & ADKV_FLAG_FAST_REPLAY);
-    if (use_segments(ka, B, min(n_super_cap, 1 << 20) * (32 / bits) - 1, exact, flags))
+    const int room = min(n_super_cap, 1 << 20) * (32 / bits) - 1;
+    if (use_segments(ka, B, room, exact, flags))
         return adkv_segments_decode_attn(ka, va, nullptr, 0, scaling, B, bits, static_cast<const int *>(seq_lens), s);
-    return launch_decode(ka, va, nullptr, 0, scaling, B, bits, exact, static_cast<const int *>(seq_lens), s);
+    return launch_decode(ka, va, nullptr, 0, scaling, B, room, bits, exact, static_cast<const int *>(seq_lens), s);
 }
 
 }  // extern "C"

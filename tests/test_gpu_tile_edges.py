@@ -71,3 +71,30 @@ def test_ov_many_streams(B):
     for b in (0, B // 2, B - 1):
         want = orc.forward_ov(w[b:b + 1].double().numpy(), ov_.copy(), vn.numpy(), np_params(case["vp"]), bits, SMIN, SMAX)
         np.testing.assert_allclose(out[b:b + 1].float().cpu().numpy(), want, rtol=RTOL, atol=ATOL)
+
+
+# up to one stream per SM, one to two, two to eight, more: the lines at which tiles of 32 tokens begin
+BY_SIZE = [(4, 1, 37, 64), (4, 1, 40, 64), (4, 1, 40, 65), (4, 1, 80, 65), (4, 2, 80, 255), (4, 2, 80, 256), (4, 4, 80, 64), (2, 1, 80, 64), (2, 1, 80, 65),
+           (2, 2, 40, 255), (2, 4, 80, 255), (2, 4, 80, 256), (4, 1, 320, 64), (2, 4, 320, 130), (4, 8, 2, 511), (4, 8, 2, 512),
+           (4, 8, 320, 1023), (4, 8, 320, 1024), (2, 8, 2, 255), (2, 8, 2, 256), (2, 8, 320, 191), (2, 8, 320, 192)]
+
+
+@pytest.mark.parametrize("bits,G,n,T", BY_SIZE)
+def test_tiles_by_size(bits, G, n, T):
+    """Whole-head steps on either side of each line, canonical and contracted; n copies of two sequences."""
+    B, Hkv = 2, 2
+    case = make_case(1200 + T, B, G * Hkv, Hkv, T, bits)
+    dk, dv, tk, tv, ok_, ov_, *_ = _prefill(case, T + 1)
+    kn, vn = case["k"][:, :, T], case["v"][:, :, T]
+    wk, wv = ok_.copy(), ov_.copy()
+    want = orc.decode_attn(case["q"][:, :, 0].numpy(), wk, wv, kn.numpy(), vn.numpy(), np_params(case["kp"]), np_params(case["vp"]), T,
+                           0.07, bits=bits, scale_min=SMIN, scale_max=SMAX)
+    rep = lambda t: dev(t).repeat(n, *([1] * (t.dim() - 1)))
+    for kw in (dict(k_tail=rep(tk), v_tail=rep(tv), tail_keep=True), dict()):
+        a, b = rep(dk), rep(dv)
+        got = gemv.decode_attn(rep(case["q"]), a, b, rep(kn[:, :, None]), rep(vn[:, :, None]), dev(case["kp"]), dev(case["vp"]), T, 0.07,
+                               SMIN, SMAX, bits=bits, split_channels=False, **kw)
+        np.testing.assert_allclose(got[:B].float().cpu().numpy(), want, rtol=RTOL, atol=ATOL)
+        assert torch.equal(got, rep(got[:B])) and torch.equal(a, rep(a[:B])) and torch.equal(b, rep(b[:B]))
+        assert np.array_equal(a[:B].cpu().numpy(), wk) and np.array_equal(b[:B].cpu().numpy(), wv)
+    _status_ok()
