@@ -131,7 +131,7 @@ ADKV_HIDDEN int adkv_half_decode_attn(const KArgs &ka, const VArgs &va, const fl
 ADKV_HIDDEN int adkv_narrow_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b,
                                         float scaling, int B, int bits, bool exact, cudaStream_t s);
 ADKV_HIDDEN int adkv_segments_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b,
-                                          float scaling, int B, int bits, const int *seq_lens, cudaStream_t s);
+                                          float scaling, int B, int max_tokens, int bits, const int *seq_lens, cudaStream_t s);
 ADKV_HIDDEN int adkv_wide_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b,
                                       float scaling, int B, int bits, int mode, cudaStream_t s);
 
@@ -229,7 +229,7 @@ int adkv_decode_attn(const void *q, void *k_cache, void *v_cache, const void *k_
     if (half)
         return adkv_half_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, nullptr, s);
     if (use_segments(ka, B, T, exact, flags))
-        return adkv_segments_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, nullptr, s);
+        return adkv_segments_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, T, bits, nullptr, s);
     // Very few streams: split every head over two warp pairs (adkv_narrow.cu).
     const bool split = (flags & ADKV_FLAG_SPLIT_CHANNELS) ||
                        (!(flags & ADKV_FLAG_NO_SPLIT_CHANNELS) &&
@@ -265,7 +265,7 @@ int adkv_decode_attn_varlen(const void *q, void *k_cache, void *v_cache, const v
     const bool exact = !(flags & ADKV_FLAG_FAST_REPLAY);
     const int room = min(n_super_cap, 1 << 20) * (32 / bits) - 1;
     if (use_segments(ka, B, room, exact, flags))
-        return adkv_segments_decode_attn(ka, va, nullptr, 0, scaling, B, bits, static_cast<const int *>(seq_lens), s);
+        return adkv_segments_decode_attn(ka, va, nullptr, 0, scaling, B, room, bits, static_cast<const int *>(seq_lens), s);
     return launch_decode(ka, va, nullptr, 0, scaling, B, room, bits, exact, static_cast<const int *>(seq_lens), s);
 }
 

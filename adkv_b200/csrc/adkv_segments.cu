@@ -34,14 +34,18 @@ namespace adkv {
 
 constexpr int NS = 8;             // segments per stream
 constexpr int kSegStages = 2;     // bulk-copy ring depth per warp
-// tokens per tile: see kFusedTok; shorter tiles where 64 tokens of 16 warps do not fit the shared memory
+// Tokens per tile (TOK), 64 as in adkv_fused.cu, but 32 where 64 tokens of 16 warps do not fit the shared memory, and for segments
+// of one such tile, where V would wait until K is through: 300 tokens, device time on a B200, 64 -> 32: 4-bit, two heads, 8
+// streams 16.6 -> 15.5 us, 2-bit, 64 streams, two heads 16.8 -> 15.8 us, four heads 19.2 -> 18.7 us.  Segments have 64 tokens
+// from 257 to 512 tokens of a stream; with four heads 500 tokens are back where 64 is no slower (2-bit, 128 streams 24.1 -> 25.1 us).
 template <int BITS, int G>
-constexpr int kSegTok = BITS == 4 && G == 4 ? kTileTok : 64;
+constexpr bool kSegLongTiles = !(BITS == 4 && G == 4);
+template <int G>
+constexpr int kSegShortTokens = G == 4 ? 384 : 512;
 constexpr int kPartFloats = 4 + kD;   // per (segment, head): maximum (log2 units), denominator, 2 pad, kD sums
 
-template <int BITS, int G>
+template <int BITS, int G, int TOK>
 struct SegShared {
-    static constexpr int TOK = kSegTok<BITS, G>;
     alignas(128) uint8_t buf[2][NS][kSegStages * Tile<BITS, TOK>::BYTES];
     alignas(16) float red[NS][G * 8 * kRedRow];
     alignas(16) float2 wts[NS][G * TOK];
@@ -242,15 +246,14 @@ __device__ __noinline__ void scale_map(const uint4 *src, int n_words, const Scal
     *reinterpret_cast<ulonglong2 *>(ends + kD / 4) = make_ulonglong2(hi[0], hi[1]);
 }
 
-template <int BITS, int G>
+template <int BITS, int G, int TOK>
 __global__ void __launch_bounds__(64 * NS)
     decode_attn_segments_kernel(KArgs ka, VArgs va, const float *__restrict__ mask, long long mask_stride_b, float scaling,
                                 const int *__restrict__ seq_lens)
 {
     extern __shared__ uint8_t smem_raw[];
-    SegShared<BITS, G> &sh = *reinterpret_cast<SegShared<BITS, G> *>(smem_raw);
+    SegShared<BITS, G, TOK> &sh = *reinterpret_cast<SegShared<BITS, G, TOK> *>(smem_raw);
     using C = Codec<BITS>;
-    constexpr int TOK = kSegTok<BITS, G>;
     const int bh = blockIdx.x, b = bh / ka.Hkv, h = bh % ka.Hkv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // Warps go to the four schedulers round robin: a pair of warps is the K and the V warp of one segment, and the order
@@ -440,28 +443,32 @@ using namespace adkv;
 
 ADKV_DEFINE_TU_STATUS(adkv_tu_status_segments)
 
-template <int BITS, int G>
+template <int BITS, int G, int TOK>
 static int launch_segments(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b, float scaling, int B,
                            const int *seq_lens, cudaStream_t s)
 {
-    constexpr int bytes = int(sizeof(SegShared<BITS, G>));
+    constexpr int bytes = int(sizeof(SegShared<BITS, G, TOK>));
     static_assert(bytes <= 227 * 1024, "shared memory of one CTA");
     // per device and process: cheap enough (a host-side call) to be made before every launch
-    const cudaError_t e = cudaFuncSetAttribute(decode_attn_segments_kernel<BITS, G>,
+    const cudaError_t e = cudaFuncSetAttribute(decode_attn_segments_kernel<BITS, G, TOK>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return int(e);
-    decode_attn_segments_kernel<BITS, G><<<B * ka.Hkv, 64 * NS, bytes, s>>>(ka, va, mask, mask_stride_b, scaling, seq_lens);
+    decode_attn_segments_kernel<BITS, G, TOK><<<B * ka.Hkv, 64 * NS, bytes, s>>>(ka, va, mask, mask_stride_b, scaling, seq_lens);
     return launch_status();
 }
 
 // Arguments checked by the caller (head dim 128, fp32 arithmetic, contracted, tail states present, Hq / Hkv at most 4).
+// max_tokens: as in use_segments (adkv_fused.cu).
 ADKV_HIDDEN int adkv_segments_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b,
-                                          float scaling, int B, int bits, const int *seq_lens, cudaStream_t s)
+                                          float scaling, int B, int max_tokens, int bits, const int *seq_lens, cudaStream_t s)
 {
     switch (bits * 16 + ka.Hq / ka.Hkv) {
 #define ADKV_SEG_CASE(BITS_, G_)                                                                                            \
     case BITS_ * 16 + G_:                                                                                                   \
-        return launch_segments<BITS_, G_>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
+        if constexpr (kSegLongTiles<BITS_, G_>)                                                                             \
+            if (max_tokens > kSegShortTokens<G_>)                                                                           \
+                return launch_segments<BITS_, G_, 64>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);                \
+        return launch_segments<BITS_, G_, 32>(ka, va, mask, mask_stride_b, scaling, B, seq_lens, s);
         ADKV_SEG_CASE(4, 1) ADKV_SEG_CASE(4, 2) ADKV_SEG_CASE(4, 4)
         ADKV_SEG_CASE(2, 1) ADKV_SEG_CASE(2, 2) ADKV_SEG_CASE(2, 4)
 #undef ADKV_SEG_CASE
