@@ -17,15 +17,15 @@ namespace adkv {
 
 constexpr int kPartStride = 4 + kD;   // floats per (stream, segment, head): max (log2 units), denominator, 2 pad, kD sums
 
-// Tokens per tile and stages: see kFusedTok (adkv_fused.cu).  The fp16-state kernel keeps tiles of 32 and with them more CTAs on
-// an SM (see adkv_half_decode_attn).
-template <bool HALF>
-constexpr int kSplitTok = HALF ? 32 : 64;
-template <bool HALF>
-constexpr int kSplitStages = HALF ? 3 : 2;
+// Tokens per tile (TOK), 64 in two stages or 32 in three, see kFusedStages (adkv_fused.cu).  The fp16-state kernel keeps 32 and with
+// it more CTAs on an SM (see adkv_half_decode_attn), and so do 4-bit codes with eight query heads, where 64 take 38 KB of shared
+// memory, up to intervals of 512.  Device time on a B200, 64 -> 32 tokens: intervals of 128, 512 streams x 2000 tokens 311 -> 275 us,
+// 128 x 8000 305 -> 269 us; of 512, 512 x 2000 262 -> 248 us; of 1024, 8 x 2000 100 -> 103 us; 2-bit, of 128, 512 x 2000 317 -> 353 us.
+template <int TOK>
+constexpr int kSplitStages = TOK == 64 ? 2 : 3;
 
-template <int G, bool HALF_W>
-struct PartialSrc : SoftmaxSrc<G, 1, HALF_W, kSplitTok<HALF_W>> {
+template <int G, bool HALF_W, int TOK>
+struct PartialSrc : SoftmaxSrc<G, 1, HALF_W, TOK> {
     float *part;   // [G][kPartStride] of this (stream, segment)
     __device__ __forceinline__ void store(const VArgs &, int, int, int c0, const float (&acc)[G][4]) const
     {
@@ -67,12 +67,12 @@ struct CkptArgs {
 template <int BITS, int G>
 constexpr bool kOutOfLineGuardedSegments = BITS == 4 && G == 1;
 
-template <int BITS, int G, int MODE>
+template <int BITS, int G, int MODE, int TOK>
 __global__ void __launch_bounds__(64) decode_attn_split_kernel(KArgs ka, VArgs va, const float *__restrict__ mask,
                                                                long long mask_stride_b, float scaling, CkptArgs ck,
                                                                float *__restrict__ scratch)
 {
-    constexpr int TOK = kSplitTok<MODE == kModeHalf>, ST = kSplitStages<MODE == kModeHalf>;
+    constexpr int ST = kSplitStages<TOK>;
     __shared__ alignas(128) uint8_t kbuf[ST * Tile<BITS, TOK>::BYTES];
     __shared__ alignas(128) uint8_t vbuf[ST * Tile<BITS, TOK>::BYTES];
     __shared__ alignas(16) float red[G * 8 * kRedRow];
@@ -104,11 +104,13 @@ __global__ void __launch_bounds__(64) decode_attn_split_kernel(KArgs ka, VArgs v
         seg.init = j ? ck.k_ckpt + (stream_ckpt + j - 1) * 2 * kD : nullptr;
         seg.ckpt_out = write_ckpt ? ck.k_ckpt + out_idx * 2 * kD : nullptr;
         RingSink<G, 1, TOK> sink{&fs, 0, 0};
-        k_scan<BITS, G, MODE, RingSink<G, 1, TOK>, ST, false, kOutOfLineGuardedSegments<BITS, G>, TOK>(ka, seg, b, h, lane, kbuf, kbar, red, sink);
+        k_scan<BITS, G, MODE, RingSink<G, 1, TOK>, ST, false, kOutOfLineGuardedSegments<BITS, G>, TOK>(ka, seg, b, h, lane, kbuf, kbar,
+                                                                                                       red, sink);
     } else {
         seg.init = j ? ck.v_ckpt + (stream_ckpt + j - 1) * 2 * kD : nullptr;
         seg.ckpt_out = write_ckpt ? ck.v_ckpt + out_idx * 2 * kD : nullptr;
-        PartialSrc<G, MODE == kModeHalf> src;
+        using Src = PartialSrc<G, MODE == kModeHalf, TOK>;
+        Src src;
         src.sh = &fs;
         src.wts = wts;
         src.mask = mask ? mask + size_t(b) * mask_stride_b : nullptr;
@@ -117,7 +119,7 @@ __global__ void __launch_bounds__(64) decode_attn_split_kernel(KArgs ka, VArgs v
         src.t_begin = seg.t_begin;
         src.part = scratch + (size_t(bh) * n_seg + j) * G * kPartStride;
         src.init();
-        v_scan<BITS, G, MODE, PartialSrc<G, MODE == kModeHalf>, ST, false, kOutOfLineGuardedSegments<BITS, G>, TOK>(va, seg, b, h, lane, vbuf, vbar, wts, src);
+        v_scan<BITS, G, MODE, Src, ST, false, kOutOfLineGuardedSegments<BITS, G>, TOK>(va, seg, b, h, lane, vbuf, vbar, wts, src);
     }
 }
 
@@ -262,12 +264,15 @@ int adkv_decode_attn_ckpt(const void *q, void *k_cache, void *v_cache, const voi
     const dim3 grid(B * Hkv, n_seg);
     if (flags & ADKV_FLAG_HALF_STATE) {
         ADKV_DISPATCH_H(bits, Hq / Hkv,
-                        (decode_attn_split_kernel<BITS, G, kModeHalf><<<grid, 64, 0, s>>>(
+                        (decode_attn_split_kernel<BITS, G, kModeHalf, 32><<<grid, 64, 0, s>>>(
                           ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, ck,
                           static_cast<float *>(scratch))))
+    } else if (bits == 4 && Hq / Hkv == 8 && interval <= 512) {
+        const auto kernel = exact ? decode_attn_split_kernel<4, 8, kArithCanon, 32> : decode_attn_split_kernel<4, 8, kArithFma, 32>;
+        kernel<<<grid, 64, 0, s>>>(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, ck, static_cast<float *>(scratch));
     } else {
         ADKV_DISPATCH(bits, exact, Hq / Hkv,
-                      (decode_attn_split_kernel<BITS, G, ARITH><<<grid, 64, 0, s>>>(
+                      (decode_attn_split_kernel<BITS, G, ARITH, 64><<<grid, 64, 0, s>>>(
                           ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, ck,
                           static_cast<float *>(scratch))))
     }

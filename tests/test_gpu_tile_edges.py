@@ -114,3 +114,22 @@ def test_segments_by_size(bits, G, T):
     np.testing.assert_allclose(got.float().cpu().numpy(), want, rtol=RTOL, atol=ATOL)
     assert np.array_equal(dk.cpu().numpy(), ok_) and np.array_equal(dv.cpu().numpy(), ov_)
     _status_ok()
+
+
+@pytest.mark.parametrize("interval", [512, 544])
+@pytest.mark.parametrize("bits", [4, 2])
+def test_eight_heads_over_checkpoints(bits, interval):
+    B, Hkv, G, T = 2, 2, 8, 1100
+    case = make_case(1400, B, G * Hkv, Hkv, T, bits)
+    ck = [gemv.alloc_ckpt(B, Hkv, 128, T + 1, interval, "cuda") for _ in range(2)]
+    dk, dv, tk, tv, ok_, ov_, *_ = _prefill(case, T + 1, k_ckpt=ck[0], v_ckpt=ck[1], ckpt_interval=interval)
+    kn, vn = case["k"][:, :, T], case["v"][:, :, T]
+    want = orc.decode_attn(case["q"][:, :, 0].numpy(), ok_, ov_, kn.numpy(), vn.numpy(), np_params(case["kp"]), np_params(case["vp"]), T,
+                           0.07, bits=bits, scale_min=SMIN, scale_max=SMAX)
+    for kw in (dict(k_tail=tk, v_tail=tv, tail_keep=True), dict()):
+        a, b = dk.clone(), dv.clone()
+        got = gemv.decode_attn(dev(case["q"]), a, b, dev(kn[:, :, None]), dev(vn[:, :, None]), dev(case["kp"]), dev(case["vp"]), T, 0.07,
+                               SMIN, SMAX, bits=bits, k_ckpt=ck[0], v_ckpt=ck[1], ckpt_interval=interval, **kw)
+        np.testing.assert_allclose(got.float().cpu().numpy(), want, rtol=RTOL, atol=ATOL)
+        assert np.array_equal(a.cpu().numpy(), ok_) and np.array_equal(b.cpu().numpy(), ov_)
+    _status_ok()
