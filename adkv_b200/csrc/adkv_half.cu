@@ -356,20 +356,30 @@ using namespace adkv;
 
 ADKV_DEFINE_TU_STATUS(adkv_tu_status_half)
 
+// Tiles of 32 tokens (three stages) instead of 64 (two; see kFusedStages in adkv_fused.cu), device time on a B200.  Tiles of 64 pay up
+// to about eleven CTAs an SM, which is all that fit at once with one query head and 4 bits (19 KB): 128 streams x 1000 tokens 44.2 ->
+// 39.3 us, 512 x 2000 113.5 -> 104.7 us, 1056 x 777 76.5 -> 73.7 us, but 2048 x 2048 300 -> 323 us.  With more heads fewer fit, and the line
+// is no lower: eight heads, 2-bit, 1600 x 1000 323 -> 312 us; two heads, 1600 x 300 53.2 -> 50.9 us.
+// Below 256 tokens V waits too long for its first tile (see short_tiles in adkv_fused.cu), 64 -> 32: 600 x 150 tokens, four heads 25.0 ->
+// 23.3 us, 2-bit 16.9 -> 15.2 us, eight heads 1600 x 30 30.4 -> 24.7 us; with 2-bit codes and one head on few streams too, 8 x 150 tokens
+// 10.2 -> 9.6 us, but 4-bit, 8 x 100 tokens 7.4 -> 7.6 us.
+static bool short_tiles_half(int bits, int G, long long streams, int max_tokens)
+{
+    return streams > 11 * kSMs || (max_tokens < 256 && (streams > 2 * kSMs || (bits == 2 && G == 1)));
+}
+
 ADKV_HIDDEN int adkv_half_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b,
                                       float scaling, int B, int bits, const int *seq_lens, cudaStream_t s)
 {
     if (ka.D != kD) return ADKV_E_FLAGS;
-    // Tiles of 64 tokens (see kFusedTok in adkv_fused.cu) while all CTAs fit the chip at once with the 19 KB that they take,
-    // eleven per SM: 128 streams x 1000 tokens 44.2 -> 39.3 us, 512 x 2000 113.5 -> 104.7 us, 1056 x 777 76.5 -> 73.7 us on a
-    // B200.  Beyond, fifteen CTAs with tiles of 32 hide more: 2048 streams x 2048 tokens 300 us against 323 us.
-    if ((long long)B * ka.Hkv <= 11 * kSMs) {
-        ADKV_DISPATCH_H(bits, ka.Hq / ka.Hkv,
+    const int n_heads = ka.Hq / ka.Hkv, max_tokens = seq_lens ? min(ka.n_super_cap, 1 << 20) * (32 / bits) - 1 : ka.T;
+    if (!short_tiles_half(bits, n_heads, (long long)B * ka.Hkv, max_tokens)) {
+        ADKV_DISPATCH_H(bits, n_heads,
                         (decode_attn_half_kernel<BITS, G, 64><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling,
                                                                                        seq_lens)))
         return launch_status();
     }
-    ADKV_DISPATCH_H(bits, ka.Hq / ka.Hkv,
+    ADKV_DISPATCH_H(bits, n_heads,
                     (decode_attn_half_kernel<BITS, G, 32><<<B * ka.Hkv, 64, 0, s>>>(ka, va, mask, mask_stride_b, scaling,
                                                                                    seq_lens)))
     return launch_status();
