@@ -10,22 +10,23 @@ namespace adkv {
 // =========================================================================================
 // Unfused entry points (the reference's two-kernel decode): 2 streams per CTA, one warp each.
 
-// Tokens per tile (see kFusedTok in adkv_fused.cu): the three calls at 512 streams x 1023 tokens 118.7 -> 108.7 us.  Eight query
-// heads leave no room for 64.
+// Tokens per tile (see kFusedStages in adkv_fused.cu): the three calls at 512 streams x 1023 tokens 118.7 -> 108.7 us.  Eight query
+// heads leave no room for 64, and three tiles of 32 in flight are the faster ones there: 2-bit, 64 streams x 1000 tokens 117 -> 115 us.
 template <int G>
 constexpr int kQkTok = G > 4 ? kTileTok : 64;
-constexpr int kQkStages = 2;
+template <int G>
+constexpr int kQkStages = G > 4 ? 3 : 2;
 
 template <int BITS, int G, bool EXACT>
 __global__ void __launch_bounds__(32 * kStreamsPerCta) forward_qk_kernel(KArgs ka, __half *__restrict__ logits,
                                                                          int n_streams)
 {
-    __shared__ alignas(128) uint8_t kbuf[kStreamsPerCta][kQkStages * Tile<BITS, kQkTok<G>>::BYTES];
+    __shared__ alignas(128) uint8_t kbuf[kStreamsPerCta][kQkStages<G> * Tile<BITS, kQkTok<G>>::BYTES];
     __shared__ alignas(16) float red[kStreamsPerCta][G * kRedTok<G> * kRedRow];
-    __shared__ uint64_t kbar[kStreamsPerCta][kQkStages];
+    __shared__ uint64_t kbar[kStreamsPerCta][kQkStages<G>];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane == 0) {
-        for (int i = 0; i < kQkStages; ++i) mbar_init(&kbar[warp][i], 1);
+        for (int i = 0; i < kQkStages<G>; ++i) mbar_init(&kbar[warp][i], 1);
         mbar_init_fence();
     }
     __syncthreads();
@@ -37,8 +38,8 @@ __global__ void __launch_bounds__(32 * kStreamsPerCta) forward_qk_kernel(KArgs k
     for (int g = 0; g < G; ++g) sink.row[g] = logits + (size_t(b) * ka.Hq + size_t(h) * G + g) * (ka.T + 1);
     sink.T = ka.T;
     const Seg seg{0, ka.T, true, nullptr, nullptr, 0};
-    k_warp<BITS, G, EXACT, GlobalLogitSink<G, kQkTok<G>>, kQkStages, false, false, kRedTok<G>, kQkTok<G>>(ka, seg, b, h, lane, kbuf[warp], kbar[warp],
-                                                                                    red[warp], sink);
+    k_warp<BITS, G, EXACT, GlobalLogitSink<G, kQkTok<G>>, kQkStages<G>, false, false, kRedTok<G>, kQkTok<G>>(ka, seg, b, h, lane, kbuf[warp],
+                                                                                                    kbar[warp], red[warp], sink);
 }
 
 // Tokens per tile, as for forward_qk: the three calls at 512 streams x 1023 tokens 106.6 -> 99.6 us, 2048 x 2000 530 -> 512 us.
