@@ -94,7 +94,8 @@ __device__ __forceinline__ bool encode_group(const __half2 *xin /* 8 rows of kD/
 // a subtraction, a comparison and two selections, instead of the reciprocal, clamps, roundings and products in a row.
 // One B200, K and V of 32 heads, device time with the quotient -> this: 1 x 777 tokens 50.0 -> 38.6 us, 2 x 2000 tokens 123 -> 94
 // us, 4 x 2000 tokens 131 -> 113 us, 1 x 60 tokens 8.2 -> 6.1 us.
-// Returns true where that does not hold: scales near overflow, alpha that is not finite, a zero point of -0.
+// Returns true where that does not hold: scales near overflow, which the range of the unguarded form leaves out even without an
+// upper bound, alpha that is not finite, a zero point of -0.
 template <bool GUARDED>
 __device__ __forceinline__ bool encode_group_compare(const __half *xin, Chan &c, uint32_t &word, float smin, float smax)
 {
@@ -227,7 +228,7 @@ __global__ void __launch_bounds__(kD / CPT) encode_kernel(EncBatch batch, CkptSp
         for (int c = 0; c < CPT; ++c) ch[c] = Chan{zp[c], sc[c], al[c], beta[c], target[c]};
     }
     SafeRange safe;
-    safe.template init<BITS, CPT>(beta, target, smin, smax);
+    safe.template init<BITS, CPT>(beta, target, smin, fminf(smax, 1e29f));   // 1e29: see encode_group_compare
     const f32x2 one = opaque_ones2();
 
     __shared__ alignas(128) __half buf[kEncStages][32 * kD];

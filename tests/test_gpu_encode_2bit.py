@@ -53,9 +53,11 @@ def _encode(x, p, B, smin, smax, t_start=0):
     return kc, kt
 
 
-def _reference(x, p, smin, smax):
+def _reference(x, p, smin, smax, state=None):
     """Codes and final state by numpy's fp32 division; minimum and maximum as on the device, where a NaN gives the other operand."""
     zp, s, alpha, beta, target = (np.broadcast_to(a.astype(np.float32), (1, H, D)) for a in np_params(p))
+    if state is not None:
+        zp, s = state
     lo, hi = np.float32(smin), np.float32(smax)
     codes = np.empty(x.shape, np.int8)
     with np.errstate(all="ignore"):
@@ -83,3 +85,21 @@ def test_few_streams(T, t_start, special, smin, smax):
         want = np.zeros(kc.shape, np.uint8)
         orc.encode_kv(want, x.numpy(), np_params(p), 2, smin, smax)
         assert np.array_equal(kc.cpu().numpy(), want)
+
+
+def test_scale_overflows_within_a_group():
+    """Without an upper bound a scale may grow from 3e28 to 2e38 within eight tokens: twice the scale overflows, and the zero point
+    with it, although alpha is 0."""
+    T = 8
+    p = [t.clone() for t in synth.gen_params(5, H, D, 2)]
+    p[2][:], p[3][:], p[4][:] = 0.0, 12.0, 0.0
+    x = torch.randn(1, H, T, D, generator=torch.Generator().manual_seed(1)).half()
+    start = [np.full((1, H, D), v, np.float32) for v in (3.3e38, 3.113e28)]
+    codes, tail = _reference(x.float().numpy(), tuple(p), 0.0, np.inf, start)
+    assert np.isnan(tail[:, :, 0]).all() and codes[:, :, -1].max() == -2
+    pc = tuple(t.cuda() for t in p)
+    kc, vc = (torch.zeros(1, H, 1, D // 4, 4, 4, dtype=torch.uint8, device="cuda") for _ in range(2))
+    kt, vt = (torch.from_numpy(np.stack(start, axis=2)).cuda() for _ in range(2))
+    gemv.encode_kv_pair(kc, x.cuda(), pc, vc, x.cuda(), pc, 0.0, float("inf"), bits=2, k_tail=kt, v_tail=vt, t_start=8)
+    assert np.array_equal(orc.unpack_codes(kc.cpu().numpy(), 16, 2)[:, :, 8:], codes)
+    assert np.array_equal(kt.cpu().numpy(), tail, equal_nan=True) and np.array_equal(vt.cpu().numpy(), tail, equal_nan=True)
