@@ -362,10 +362,13 @@ ADKV_DEFINE_TU_STATUS(adkv_tu_status_half)
 // is no lower: eight heads, 2-bit, 1600 x 1000 323 -> 312 us; two heads, 1600 x 300 53.2 -> 50.9 us.
 // Below 256 tokens V waits too long for its first tile (see short_tiles in adkv_fused.cu), 64 -> 32: 600 x 150 tokens, four heads 25.0 ->
 // 23.3 us, 2-bit 16.9 -> 15.2 us, eight heads 1600 x 30 30.4 -> 24.7 us; with 2-bit codes and one head on few streams too, 8 x 150 tokens
-// 10.2 -> 9.6 us, but 4-bit, 8 x 100 tokens 7.4 -> 7.6 us.
+// 10.2 -> 9.6 us, but 4-bit, 8 x 100 tokens 7.4 -> 7.6 us; with one or two heads not for more than eight CTAs an SM, 4-bit, 1600 x 100
+// tokens 18.9 -> 19.2 us, two heads 22.3 -> 22.9 us.
 static bool short_tiles_half(int bits, int G, long long streams, int max_tokens)
 {
-    return streams > 11 * kSMs || (max_tokens < 256 && (streams > 2 * kSMs || (bits == 2 && G == 1)));
+    if (streams > 11 * kSMs) return true;
+    if (max_tokens >= 256) return false;
+    return (bits == 2 && G == 1) || (streams > 2 * kSMs && (G > 2 || streams <= 8 * kSMs));
 }
 
 ADKV_HIDDEN int adkv_half_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b,

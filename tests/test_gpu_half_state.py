@@ -181,7 +181,8 @@ def test_fused_decode_against_numpy_restatement(B, Hq, Hkv, T, bits):
 
 @pytest.mark.parametrize("varlen", [False, True])
 @pytest.mark.parametrize("G,T,bits,rep", [(1, 131, 4, 280), (1, 64, 2, 280), (4, 77, 4, 280), (4, 203, 2, 280), (8, 33, 4, 280),
-                                          (1, 300, 4, 280), (8, 256, 4, 150), (4, 255, 4, 60), (4, 256, 4, 60), (1, 255, 2, 2)])
+                                          (1, 300, 4, 280), (8, 256, 4, 150), (4, 255, 4, 60), (4, 256, 4, 60), (1, 255, 2, 2),
+                                          (2, 100, 4, 197), (2, 100, 4, 198)])
 def test_more_streams_than_fit_the_chip(G, T, bits, rep, varlen):
     """Past the streams that the launch with 64-token tiles is for (at most 1628), and on either side of its other lines: tiles of
     32 tokens, ragged ends, masks and device-side lengths.  Three sequences, repeated, against the numpy restatement and the
