@@ -34,7 +34,7 @@ constexpr int kArithFma = 0, kArithCanon = 1;
 template <int BITS, int TOK = kTileTok>
 struct Tile {
     static constexpr int WORDS = TOK / Codec<BITS>::TPW;   // words per channel per tile
-    static constexpr int BYTES = WORDS * kD * 4;                // 4-bit: 2048, 2-bit: 1024
+    static constexpr int BYTES = WORDS * kD * 4;           // 32 tokens: 2048 (4-bit), 1024 (2-bit)
 };
 
 // Per-warp bulk-copy ring over the words of one stream.
@@ -388,7 +388,7 @@ __device__ __forceinline__ void k_warp(const KArgs &a, const Seg &seg, int b, in
 {
     using C = Codec<BITS>;
     constexpr bool EXACT = ARITH == kArithCanon;
-        const int bh = b * a.Hkv + h;
+    const int bh = b * a.Hkv + h;
     const int D = WIDE ? a.D : kD, slice = WIDE ? seg.slice : 0;
     const int c0 = kD * slice + 4 * lane;      // first of this lane's 4 channels within the head
     const uint32_t row_stride = uint32_t(D) * 4;
@@ -536,7 +536,7 @@ __device__ __forceinline__ void k_warp(const KArgs &a, const Seg &seg, int b, in
 
 template <int BITS, int G, bool EXACT, bool PARTIAL, int TOK>
 __device__ __forceinline__ void v_chunk(const uint4 &w, const FieldConsts<BITS> &fc, Chan (&ch)[4],
-                                        const float2 *wts /* [G][32] smem, each weight twice */, int tok0,
+                                        const float2 *wts /* [G][TOK] smem, each weight twice */, int tok0,
                                         float (&acc)[G][4], int count, float smin, float smax)
 {
     uint32_t grp[4] = {w.x, w.y, w.z, w.w};
@@ -567,7 +567,7 @@ __device__ __forceinline__ void v_chunk(const uint4 &w, const FieldConsts<BITS> 
 }
 
 // The full 8-token case of v_chunk on channel pairs (packed fp32), guards as in k_chunk2.  `wts2` holds every weight
-// twice ([G][32] float2) so that one 8-byte load yields the packed multiplier.
+// twice ([G][TOK] float2) so that one 8-byte load yields the packed multiplier.
 template <int BITS, int G, bool EXACT, bool CLAMP, int TOK>
 __device__ __forceinline__ void v_chunk2(const uint4 &w, const FieldConsts<BITS> &fc, Chan (&ch)[4],
                                          const PairConst (&pc)[2], f32x2 one, const float2 *wts2, int tok0,

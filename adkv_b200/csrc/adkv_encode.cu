@@ -495,7 +495,8 @@ static int launch_encode(const EncBatch &b, int n, int B, int H, int T, int D, i
     // One channel per thread while that leaves a warp scheduler at most three warps: a warp then has its scheduler (nearly)
     // to itself and takes as long as its own instructions, of which one channel needs about half as many as a pair.
     // Measured on a B200, K and V of 32 heads: 1 x 4000 tokens 251 -> 231 us, 2 x 2000 tokens 131 -> 121 us, 4 x 2000 tokens
-    // 137 -> 133 us, 6 x 3000 tokens 213 -> 199 us (2-bit 224 -> 212 us), but 8 x 2000 tokens 148 -> 155 us.  With more streams the schedulers are busy and the packed pair needs fewer issue slots per channel.
+    // 137 -> 133 us, 6 x 3000 tokens 213 -> 199 us (2-bit 224 -> 212 us), but 8 x 2000 tokens 148 -> 155 us.  With more streams the
+    // schedulers are busy and the packed pair needs fewer issue slots per channel.
     const bool few = (long long)grid.x * grid.y * (kD / 32) <= 3 * kSchedulers;
     if (D == kD) {
         if (bits == 4 && few) encode_kernel<4, false, 1><<<grid, kD, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);

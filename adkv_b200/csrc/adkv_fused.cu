@@ -120,9 +120,13 @@ using namespace adkv;
 
 // adkv_decode_attn splits the channels of a head over two warp pairs up to one (batch, kv head) stream per SM, and up to 160
 // streams while the set-up counts: a short stream is loaded and appended by more warps, a long one pays the sums, votes and
-// rings of twice as many.  Device time on a B200, 160 streams next to tails, split -> whole head: 4-bit 150 tokens 13.0 -> 13.2
-// us, 2000 tokens 110 -> 91 us; 2-bit with four heads 16.4 -> 18.4 us, 163 -> 142 us; canonical replay, 2-bit, 100 tokens 10.8 ->
-// 11.6 us, 210 tokens with four heads 23.3 -> 24.4 us, 2000 tokens 139 -> 108 us.
+// rings of twice as many.  Device time on a B200, split / whole head, us (in brackets: one channel of every head at a bound):
+//    148 streams, canonical replay    4-bit 100 tokens 10.1 / 11.5, 256 17.0 / 18.6, 2000 100 / 103 (183 / 131); with four heads 142 /
+//                                     152 (196 / 159); 2-bit 100 tokens 9.2 / 11.3, 256 20.7 / 18.5, 2000 129 / 108 (179 / 114)
+//    148 streams next to tails        4-bit 60 tokens 7.7 / 9.5, 100 9.9 / 10.5; 2-bit, four heads, 100 11.2 / 14.5; longer ones: segments
+//    160 streams next to tails        4-bit 100 tokens 10.4 / 10.5, 256 18.2 / 16.6, 2000 110 / 89; 2-bit, four heads, 100 12.9 / 13.8, 256
+//                                     24.1 / 24.4, 2000 160 / 140
+// Without segments, long 2-bit streams of one head and streams with scales at a bound would be better off whole below 148, too.
 constexpr int kSplitChannelsMaxTokens = 256;
 constexpr long long kSplitChannelsMaxStreams = 160;
 
@@ -139,12 +143,12 @@ ADKV_DEFINE_TU_STATUS(adkv_tu_status_fused)
 
 // Token segments of a stream side by side (adkv_segments.cu), next to tail states: up to one stream per SM and from 128
 // tokens on (max_tokens: the tokens of every sequence, or what the cache can hold of them where the lengths are on the
-// device).  Device time on a B200, caches rotated through more than L2 holds, the split head of adkv_narrow.cu -> segments,
-// where no scale meets a clamp / where one channel of every head rests at a bound:
-//    4-bit, 32 heads            128 streams x 2000 tokens   100 ->  50 us / 187 ->  87 us
-//    4-bit, 32 heads             32 streams x 8000 tokens   376 -> 176 us / 728 -> 322 us
-//    2-bit, 32 on 8 KV heads    128 streams x 2000 tokens   159 ->  75 us / 193 -> 104 us
-//    2-bit, 32 on 16 KV heads   144 streams x 128 tokens   12.0 -> 12.0 us / 14.8 -> 14.0 us
+// device).  Device time on a B200, the split head of adkv_narrow.cu / whole head / segments, where no scale meets a clamp and,
+// in brackets, where one channel of every head rests at a bound:
+//    4-bit                 128 streams x 256 tokens 16.4 / 16.7 / 12.4 us, x 2000 93 / 89 / 49 us (179 / 109 / 80 us)
+//    2-bit, four heads     128 streams x 256 tokens 22.0 / 24.4 / 16.0 us, x 2000 141 / 140 / 73 us (185 / 146 / 102 us)
+// Measured with tiles of 32 tokens everywhere, split head -> segments: 32 streams x 8000 tokens, 4-bit, 376 -> 176 us (728 -> 322 us);
+// 144 x 128, 2-bit, two heads, 12.0 -> 12.0 us (14.8 -> 14.0 us).
 // Below 128 tokens set-up and merge are not made up for (2-bit, 128 streams x 96 tokens: 8.4 -> 8.9 us); device-side
 // lengths may lie there, and cost a microsecond up to 64 tokens (64 streams x 64 tokens: 8.6 -> 9.3 us, x 96 tokens: 10.0
 // -> 9.4 us, x 256 tokens: 17.2 -> 12.3 us).  With more than one stream per SM the extra work has no idle schedulers to go

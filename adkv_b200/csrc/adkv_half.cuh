@@ -321,7 +321,7 @@ __device__ __forceinline__ void k_warp_h(const KArgs &a, const Seg &seg, int b, 
 // ---------------------------------------------------------------------------------- V side
 
 // 8 tokens for the lane's two channel pairs: weight * value accumulated in fp16 over the 8 tokens, then added
-// to the fp32 accumulators (the reference accumulates all tokens in fp16, gemv.cu:1087).  wts: [G][32] fp16
+// to the fp32 accumulators (the reference accumulates all tokens in fp16, gemv.cu:1087).  wts: [G][TOK] fp16
 // pairs (w, w), written by a source with HALF_W set.
 template <int BITS, int G, bool PARTIAL, int TOK>
 __device__ __forceinline__ void v_chunk_h(const uint4 &w, HPair (&hp)[2], const uint32_t *wts, int tok0,

@@ -45,7 +45,7 @@ struct RingSink {
     __device__ __forceinline__ void finish(int lane) { end_tile(0, lane); }
 };
 
-// Weights of a tile for the V warp: [G][32] float2 (w, w), or with HALF_W [G][32] fp16 pairs (w, w) in the first
+// Weights of a tile for the V warp: [G][TOK] float2 (w, w), or with HALF_W [G][TOK] fp16 pairs (w, w) in the first
 // half of the same array (the fp16-state kernels multiply in fp16x2).
 template <bool HALF_W>
 __device__ __forceinline__ void put_weight(float2 *wts, int idx, float w)

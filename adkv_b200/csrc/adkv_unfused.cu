@@ -96,10 +96,15 @@ __global__ void __launch_bounds__(32 * kNarrowSlices) forward_ov_split_kernel(VA
 }
 
 // forward_ov splits a stream over two warps while each of them has a scheduler to itself: up to 296 streams.  Measured on
-// a B200, 4-bit, 32 heads, 1000 tokens, canonical replay where no scale meets a clamp / where one channel of every head
-// rests at a bound; contracted replay, the same:
-//    256 streams, one warp without the weights fetched ahead -> two warps   50.2 -> 40.9 / 63.3 -> 53.1;  44.1 -> 38.7 / 53.6 -> 50.5 us
-//    512 streams, one warp with the weights fetched ahead -> two warps      49.1 -> 49.9 / 61.5 -> 69.2;  41.5 -> 45.9 / 51.7 -> 64.3 us
+// a B200, 1000 tokens, one warp (tiles of 64 tokens, weights fetched ahead) -> two, us, canonical replay where no scale meets a clamp /
+// where one channel of every head rests at a bound; contracted replay, the same:
+//    256 streams    4-bit 38.0 -> 41.5 / 41.2 -> 53.8; 34.4 -> 39.4 / 38.2 -> 50.9
+//                   four heads 55.6 -> 50.0 / 60.7 -> 64.5; 50.2 -> 48.6 / 55.3 -> 60.1
+//                   2-bit 51.2 -> 44.5 / 52.1 -> 53.0; 46.1 -> 42.8 / 47.9 -> 52.1
+//                   four heads 60.1 -> 58.0 / 65.2 -> 66.2; 55.9 -> 55.9 / 59.1 -> 63.2
+//    320 streams    4-bit 38.2 -> 49.7, four heads 55.9 -> 62.1; 2-bit 50.9 -> 54.7, four heads 60.1 -> 71.3 (canonical, no clamp)
+// Two warps are the better choice there for several heads and for 2-bit codes away from the bounds; 4-bit codes of one head are the
+// exception since one warp takes tiles of 64.
 constexpr int kOvSplitMaxStreams = kSchedulers / 2;
 
 }  // namespace adkv
