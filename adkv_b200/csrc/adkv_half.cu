@@ -11,7 +11,7 @@ namespace adkv {
 
 // =========================================================================================
 // Fused decode step, as decode_attn_kernel: one CTA per (batch, kv head); warp 0 scans K, warp 1 scans V.
-// TOK: tokens per tile, 64 (two stages) or 32 (three), see adkv_half_decode_attn.
+// TOK: tokens per tile, 64 (two stages) or 32 (three), see short_tiles_half.
 template <int BITS, int G, int TOK>
 __global__ void __launch_bounds__(64) decode_attn_half_kernel(KArgs ka, VArgs va, const float *__restrict__ mask,
                                                               long long mask_stride_b, float scaling,

@@ -18,7 +18,7 @@ namespace adkv {
 constexpr int kPartStride = 4 + kD;   // floats per (stream, segment, head): max (log2 units), denominator, 2 pad, kD sums
 
 // Tokens per tile (TOK), 64 in two stages or 32 in three, see kFusedStages (adkv_fused.cu).  The fp16-state kernel keeps 32 and with
-// it more CTAs on an SM (see adkv_half_decode_attn), and so do 4-bit codes with eight query heads, where 64 take 38 KB of shared
+// it more CTAs on an SM (see short_tiles_half), and so do 4-bit codes with eight query heads, where 64 take 38 KB of shared
 // memory, up to intervals of 512.  Device time on a B200, 64 -> 32 tokens: intervals of 128, 512 streams x 2000 tokens 311 -> 275 us,
 // 128 x 8000 305 -> 269 us; of 512, 512 x 2000 262 -> 248 us; of 1024, 8 x 2000 100 -> 103 us; 2-bit, of 128, 512 x 2000 317 -> 353 us.
 template <int TOK>
