@@ -32,9 +32,9 @@ def _host_lib() -> str | None:
 HOST_LIB = _host_lib()
 HOST_SOURCE = os.path.join(CSRC, "adkv_pyhost.cpp")
 SOURCES = ["adkv_capi.cu", "adkv_encode.cu", "adkv_fused.cu", "adkv_unfused.cu", "adkv_split.cu", "adkv_wide.cu",
-           "adkv_half.cu", "adkv_narrow.cu", "adkv_segments.cu"]
+           "adkv_half.cu", "adkv_narrow.cu", "adkv_segments.cu", "adkv_tensor.cu"]
 HEADERS = ["adkv_device.cuh", "adkv_decode.cuh", "adkv_softmax.cuh", "adkv_half.cuh", "adkv_io.cuh", "adkv_host.h",
-           "adkv_narrow.cuh",
+           "adkv_narrow.cuh", "adkv_tensor.cuh",
            os.path.join("..", "..", "include", "adkv_b200.h")]
 OBJ_DIR = os.path.join(PKG, "build")
 

@@ -10,6 +10,7 @@ ADKV_HIDDEN int adkv_tu_status_wide(int *out);
 ADKV_HIDDEN int adkv_tu_status_half(int *out);
 ADKV_HIDDEN int adkv_tu_status_narrow(int *out);
 ADKV_HIDDEN int adkv_tu_status_segments(int *out);
+ADKV_HIDDEN int adkv_tu_status_tensor(int *out);
 
 namespace adkv {
 
@@ -61,7 +62,7 @@ int adkv_device_status(int *status, void *stream)
     if (!status) return ADKV_E_NULL;
     const cudaError_t e = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return int(e);
-    int a = 0, b = 0, c = 0, d = 0, w = 0, t = 0, hf = 0, nr = 0, sg = 0;
+    int a = 0, b = 0, c = 0, d = 0, w = 0, t = 0, hf = 0, nr = 0, sg = 0, tn = 0;
     if (int rc = adkv_tu_status_fused(&a)) return rc;
     if (int rc = adkv_tu_status_unfused(&b)) return rc;
     if (int rc = adkv_tu_status_encode(&c)) return rc;
@@ -71,7 +72,9 @@ int adkv_device_status(int *status, void *stream)
     if (int rc = adkv_tu_status_half(&hf)) return rc;
     if (int rc = adkv_tu_status_narrow(&nr)) return rc;
     if (int rc = adkv_tu_status_segments(&sg)) return rc;
+    if (int rc = adkv_tu_status_tensor(&tn)) return rc;
     if (sg) nr = sg;
+    if (tn) nr = tn;
     *status = a ? a : (b ? b : (c ? c : (d ? d : (w ? w : (hf ? hf : (nr ? nr : t))))));
     return 0;
 }

@@ -302,6 +302,18 @@ __device__ __forceinline__ void append_new_token(Chan (&ch)[4], const ParamPtrs 
     if (ckpt_out) store_state(ckpt_out, ch, c0, D);
 }
 
+// Quantise the new token of this lane's channels from the tail (see append_new_token).
+template <int BITS>
+__device__ __forceinline__ void append_from_tail(const ParamPtrs &p, size_t poff, float *tail, bool tail_keep,
+                                                 const __half *x_new, uint4 *slot, int T, float smin, float smax,
+                                                 float *ckpt_out, int c0, float (&xh)[4])
+{
+    Chan ch[4];
+    SafeRange unused;
+    load_chan4<BITS, true>(ch, unused, p, poff, smin, smax);
+    append_new_token<BITS, kArithCanon>(ch, p, poff, tail, tail_keep, x_new, slot, T, smin, smax, ckpt_out, c0, kD, xh);
+}
+
 struct Chan4 {
     Chan c[4];
 };

@@ -25,41 +25,6 @@ constexpr int kFusedStages = TOK == 64 ? 2 : 3;
 template <int BITS, int G>
 constexpr bool kOutOfLineGuarded = BITS == 4 && G == 1;
 
-// Device-side lengths: the sequence that comes r-th when they are ordered by length, longest first (equal ones by index).
-// CTAs start in the order of their index, so the long streams start together and early and the short ones fill the gaps;
-// in the order of the batch an SM may hold several long streams while its neighbours run dry.  Measured on a B200, lengths
-// spread evenly between a twentieth of the longest and the longest, order of the batch -> longest first, 32 heads:
-//    4-bit, 48 sequences x 3000 tokens 324 -> 252 us; 24 x 2000 154 -> 131 us; 2-bit, 8 KV heads, 96 x 3000 372 -> 304 us
-// Every CTA ranks the lengths for itself, in shared memory: B * B / 64 comparisons a thread.  With many CTAs to an SM and no sequence
-// of a few hundred tokens that is more than it gains, however large the cache: 128 sequences of 150 to 200 tokens in a cache for
-// 4096, 4-bit, 32 heads, 101 us in the order of the batch, 112 us ranked; 2-bit, 8 KV heads, 48 sequences 30.3 us against 28.2 us
-// ranked.  More than 128 sequences fill the chip several times over, so that its scheduler evens them out.
-// A call, not inlined, and no early return: either would change the registers of the scans behind it (up to 5 % of a step).
-constexpr int kRankMax = 128, kRankMinTokens = 512, kRankAlways = 8 * kSMs;
-__device__ __noinline__ int longest_first(const int *__restrict__ seq_lens, int B, int r, int *key /* [kRankMax + 1] shared */)
-{
-    // length and index in one number, all different; lengths that no cache holds fall together at either end
-    bool any_long = false;
-    for (int i = threadIdx.x; i < kRankMax; i += 64) {
-        const int len = i < B ? min(max(seq_lens[i], 0), 1 << 23) : 0;
-        any_long |= len >= kRankMinTokens;
-        key[i] = i < B ? len * kRankMax + (kRankMax - 1 - i) : -1;
-    }
-    if (threadIdx.x == 0) key[kRankMax] = r;
-    const int n = __syncthreads_or(any_long || gridDim.x <= kRankAlways) ? B : 0;
-    for (int b = threadIdx.x; b < n; b += 64) {
-        const int mine = key[b];
-        int before = 0;
-        for (int i = 0; i < B; i += 4) {
-            const int4 v = *reinterpret_cast<const int4 *>(key + i);
-            before += (v.x > mine) + (v.y > mine) + (v.z > mine) + (v.w > mine);
-        }
-        if (before == r) key[kRankMax] = b;
-    }
-    __syncthreads();
-    return key[kRankMax];
-}
-
 // n_rank: number of sequences if the CTAs may take them longest first, 0 if in the order of the batch.
 template <int BITS, int G, int ARITH, int TOK>
 __global__ void __launch_bounds__(64) decode_attn_kernel(KArgs ka, VArgs va, const float *__restrict__ mask,
@@ -78,7 +43,7 @@ __global__ void __launch_bounds__(64) decode_attn_kernel(KArgs ka, VArgs va, con
     const int h = blockIdx.x % ka.Hkv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (seq_lens) {
-        if (n_rank) b = longest_first(seq_lens, n_rank, b, reinterpret_cast<int *>(red));
+        if (n_rank) b = longest_first<64>(seq_lens, n_rank, b, reinterpret_cast<int *>(red));
         // per-sequence token counts held on the device (ragged batches; also lets a captured launch be
         // replayed while the sequences grow).  The host could not check the capacity, so it is checked here.
         const int T = seq_lens[b];
@@ -139,6 +104,10 @@ ADKV_HIDDEN int adkv_segments_decode_attn(const KArgs &ka, const VArgs &va, cons
 ADKV_HIDDEN int adkv_wide_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b,
                                       float scaling, int B, int bits, int mode, cudaStream_t s);
 
+ADKV_HIDDEN int adkv_tensor_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b, float scaling,
+                                        int B, int bits, const int *seq_lens, int n_rank, const CkptArgs &ck, int n_seg,
+                                        float *scratch, cudaStream_t s);
+
 ADKV_DEFINE_TU_STATUS(adkv_tu_status_fused)
 
 // Token segments of a stream side by side (adkv_segments.cu), next to tail states: up to one stream per SM and from 128
@@ -161,6 +130,13 @@ static bool use_segments(const KArgs &ka, int B, int max_tokens, bool exact, uns
 {
     return ka.tail && !exact && !(flags & (ADKV_FLAG_SPLIT_CHANNELS | ADKV_FLAG_NO_SPLIT_CHANNELS)) &&
            ka.Hq / ka.Hkv <= 4 && (long long)B * ka.Hkv <= kSegmentsMaxStreams && max_tokens >= kSegmentsMinTokens;
+}
+
+static bool use_tensor(const KArgs &ka, int B, int bits, int max_tokens, bool device_lengths, bool exact, unsigned flags)
+{
+    const int G = ka.Hq / ka.Hkv;
+    return ka.tail && !exact && !(flags & (ADKV_FLAG_SPLIT_CHANNELS | ADKV_FLAG_NO_SPLIT_CHANNELS)) && tensor_can(G, ka.smin, ka.smax) &&
+           tensor_pays(bits, G, (long long)B * ka.Hkv, max_tokens, device_lengths);
 }
 
 // Whether a launch of whole heads takes tiles of 32 tokens (three stages) instead of 64 (two).  V starts when K is through its
@@ -232,6 +208,8 @@ int adkv_decode_attn(const void *q, void *k_cache, void *v_cache, const void *k_
                                      half ? 2 : int(exact), s);
     if (half)
         return adkv_half_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, nullptr, s);
+    if (use_tensor(ka, B, bits, T, false, exact, flags))
+        return adkv_tensor_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, nullptr, 0, CkptArgs{}, 1, nullptr, s);
     if (use_segments(ka, B, T, exact, flags))
         return adkv_segments_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, T, bits, nullptr, s);
     // Very few streams: split every head over two warp pairs (adkv_narrow.cu).
@@ -268,6 +246,9 @@ int adkv_decode_attn_varlen(const void *q, void *k_cache, void *v_cache, const v
         return adkv_half_decode_attn(ka, va, nullptr, 0, scaling, B, bits, static_cast<const int *>(seq_lens), s);
     const bool exact = !(flags & ADKV_FLAG_FAST_REPLAY);
     const int room = min(n_super_cap, 1 << 20) * (32 / bits) - 1;
+    if (use_tensor(ka, B, bits, room, true, exact, flags))
+        return adkv_tensor_decode_attn(ka, va, nullptr, 0, scaling, B, bits, static_cast<const int *>(seq_lens),
+                                       B <= kRankMax && n_super_cap >= kRankMinTokens * bits / 32 ? B : 0, CkptArgs{}, 1, nullptr, s);
     if (use_segments(ka, B, room, exact, flags))
         return adkv_segments_decode_attn(ka, va, nullptr, 0, scaling, B, room, bits, static_cast<const int *>(seq_lens), s);
     return launch_decode(ka, va, nullptr, 0, scaling, B, room, bits, exact, static_cast<const int *>(seq_lens), s);

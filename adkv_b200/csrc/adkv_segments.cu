@@ -110,18 +110,6 @@ struct SegSrc : SoftmaxSrc<G, 1, false, TOK> {
     }
 };
 
-// Quantise the new token of this lane's channels from the tail (see append_new_token).
-template <int BITS>
-__device__ __forceinline__ void append_from_tail(const ParamPtrs &p, size_t poff, float *tail, bool tail_keep,
-                                                 const __half *x_new, uint4 *slot, int T, float smin, float smax,
-                                                 int c0, float (&xh)[4])
-{
-    Chan ch[4];
-    SafeRange unused;
-    load_chan4<BITS, true>(ch, unused, p, poff, smin, smax);
-    append_new_token<BITS, kArithCanon>(ch, p, poff, tail, tail_keep, x_new, slot, T, smin, smax, nullptr, c0, kD, xh);
-}
-
 // Scales of four channels and what advances them (contracted constants: ch[].tc = 1 - beta * target).
 struct ScaleConst {
     f32x2 beta[2], tc[2];
@@ -362,7 +350,7 @@ __global__ void __launch_bounds__(64 * NS)
     const auto append = [&](const ParamPtrs &pp, float *tail, bool keep, const __half *x_new, uint8_t *cache, float (&xh)[4]) {
         append_from_tail<BITS>(pp, poff, tail + size_t(bh) * 2 * kD, keep, x_new + size_t(bh) * kD + c0,
                                reinterpret_cast<uint4 *>(cache + (size_t(bh) * ka.n_super_cap + T / C::TPW) * kD * 4) + lane,
-                               T, ka.smin, ka.smax, c0, xh);
+                               T, ka.smin, ka.smax, nullptr, c0, xh);
     };
     // The appended token goes into the word behind the last cached one: only the warps that read that word may write it.
     const bool last = t_end == T && (seg == 0 || t_begin < T);

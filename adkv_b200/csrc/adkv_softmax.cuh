@@ -156,4 +156,48 @@ struct SoftmaxSrc {
     }
 };
 
+constexpr int kPartStride = 4 + kD;   // floats per (stream, segment, head): max (log2 units), denominator, 2 pad, kD sums
+
+struct CkptArgs {
+    float *k_ckpt, *v_ckpt;   // [B*Hkv][n_ckpt_cap][2][kD]; entry k = state before token (k+1)*interval
+    int interval, n_ckpt_cap;
+    bool mute_k;              // self-test (ADKV_FLAG_SELFTEST_MUTE_K): the K warps do nothing, so every V warp's wait runs out
+};
+
+// Device-side lengths: the sequence that comes r-th when they are ordered by length, longest first (equal ones by index).
+// CTAs start in the order of their index, so the long streams start together and early and the short ones fill the gaps;
+// in the order of the batch an SM may hold several long streams while its neighbours run dry.  Measured on a B200, lengths
+// spread evenly between a twentieth of the longest and the longest, order of the batch -> longest first, 32 heads:
+//    4-bit, 48 sequences x 3000 tokens 324 -> 252 us; 24 x 2000 154 -> 131 us; 2-bit, 8 KV heads, 96 x 3000 372 -> 304 us
+// Every CTA ranks the lengths for itself, in shared memory: B * B / 64 comparisons a thread.  With many CTAs to an SM and no sequence
+// of a few hundred tokens that is more than it gains, however large the cache: 128 sequences of 150 to 200 tokens in a cache for
+// 4096, 4-bit, 32 heads, 101 us in the order of the batch, 112 us ranked; 2-bit, 8 KV heads, 48 sequences 30.3 us against 28.2 us
+// ranked.  More than 128 sequences fill the chip several times over, so that its scheduler evens them out.
+// A call, not inlined, and no early return: either would change the registers of the scans behind it (up to 5 % of a step).
+constexpr int kRankMax = 128, kRankMinTokens = 512, kRankAlways = 8 * 148 /* SMs */;
+template <int THREADS>
+__device__ __noinline__ int longest_first(const int *__restrict__ seq_lens, int B, int r, int *key /* [kRankMax + 1] shared */)
+{
+    // length and index in one number, all different; lengths that no cache holds fall together at either end
+    bool any_long = false;
+    for (int i = threadIdx.x; i < kRankMax; i += THREADS) {
+        const int len = i < B ? min(max(seq_lens[i], 0), 1 << 23) : 0;
+        any_long |= len >= kRankMinTokens;
+        key[i] = i < B ? len * kRankMax + (kRankMax - 1 - i) : -1;
+    }
+    if (threadIdx.x == 0) key[kRankMax] = r;
+    const int n = __syncthreads_or(any_long || gridDim.x <= kRankAlways) ? B : 0;
+    for (int b = threadIdx.x; b < n; b += THREADS) {
+        const int mine = key[b];
+        int before = 0;
+        for (int i = 0; i < B; i += 4) {
+            const int4 v = *reinterpret_cast<const int4 *>(key + i);
+            before += (v.x > mine) + (v.y > mine) + (v.z > mine) + (v.w > mine);
+        }
+        if (before == r) key[kRankMax] = b;
+    }
+    __syncthreads();
+    return key[kRankMax];
+}
+
 }  // namespace adkv

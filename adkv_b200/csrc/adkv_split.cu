@@ -15,8 +15,6 @@
 
 namespace adkv {
 
-constexpr int kPartStride = 4 + kD;   // floats per (stream, segment, head): max (log2 units), denominator, 2 pad, kD sums
-
 // Tokens per tile (TOK), 64 in two stages or 32 in three, see kFusedStages (adkv_fused.cu).  The fp16-state kernel keeps 32 and with
 // it more CTAs on an SM (see short_tiles_half), and so do 4-bit codes with eight query heads, where 64 take 38 KB of shared
 // memory, up to intervals of 512.  Device time on a B200, 64 -> 32 tokens: intervals of 128, 512 streams x 2000 tokens 311 -> 275 us,
@@ -54,12 +52,6 @@ struct PartialSrc : SoftmaxSrc<G, 1, HALF_W, TOK> {
             *reinterpret_cast<float4 *>(part + g * kPartStride + 4 + c0) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
     }
-};
-
-struct CkptArgs {
-    float *k_ckpt, *v_ckpt;   // [B*Hkv][n_ckpt_cap][2][kD]; entry k = state before token (k+1)*interval
-    int interval, n_ckpt_cap;
-    bool mute_k;              // self-test (ADKV_FLAG_SELFTEST_MUTE_K): the K warps do nothing, so every V warp's wait runs out
 };
 
 // Guarded chunk bodies as function calls (see k_chunk_guarded): measured 2-3 % faster for 4-bit codes with one query
@@ -201,6 +193,10 @@ __global__ void __launch_bounds__(kD) merge_few_kernel(const float *__restrict__
 
 using namespace adkv;
 
+ADKV_HIDDEN int adkv_tensor_decode_attn(const KArgs &ka, const VArgs &va, const float *mask, long long mask_stride_b, float scaling,
+                                        int B, int bits, const int *seq_lens, int n_rank, const CkptArgs &ck, int n_seg,
+                                        float *scratch, cudaStream_t s);
+
 ADKV_DEFINE_TU_STATUS(adkv_tu_status_split)
 
 // The merge follows the segment kernel on the same stream as its programmatic dependent: set up early, started
@@ -262,7 +258,12 @@ int adkv_decode_attn_ckpt(const void *q, void *k_cache, void *v_cache, const voi
     const int n_seg = T / interval + 1;
     if (n_seg > 65535) return ADKV_E_SHAPE;
     const dim3 grid(B * Hkv, n_seg);
-    if (flags & ADKV_FLAG_HALF_STATE) {
+    if (ka.tail && !exact && !ck.mute_k && tensor_can(Hq / Hkv, scale_min, scale_max) &&
+        tensor_pays(bits, Hq / Hkv, (long long)B * Hkv * n_seg, min(T, interval), false)) {
+        if (int rc = adkv_tensor_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, nullptr, 0, ck, n_seg,
+                                             static_cast<float *>(scratch), s))
+            return rc;
+    } else if (flags & ADKV_FLAG_HALF_STATE) {
         ADKV_DISPATCH_H(bits, Hq / Hkv,
                         (decode_attn_split_kernel<BITS, G, kModeHalf, 32><<<grid, 64, 0, s>>>(
                           ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, ck,

@@ -1,0 +1,135 @@
+"""Decode steps on the tensor cores (next to tail states, up to four query heads per KV head) against the oracle and the
+one-warp-per-tensor scan.  Sizes are the edges of the 64-token tiles and of the 16 tokens that a product of V takes, scales
+at and outside the clamp bounds, values near the ends of fp16, more streams than a round of the chip holds.  Needs a B200."""
+import numpy as np
+import pytest
+import torch
+
+from adkv_b200 import gemv
+from oracle import adkv_oracle as orc
+from tests.test_gpu_tail_state import ATOL, RTOL, _bits_equal, _oracle_tail, _prefill, _status_ok
+from tests.util import SMAX, SMIN, dev, make_case, np_params
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("Hq,bits", [(2, 4), (4, 2), (8, 4), (8, 2)])
+@pytest.mark.parametrize("T", [32, 33, 63, 64, 65, 79, 80, 81, 127, 128, 129, 193, 260])
+def test_tile_edges(T, Hq, bits, pinned):
+    case = make_case(1300 + T, 2, Hq, 2, T, bits)
+    if pinned:
+        for n in ("kp", "vp"):
+            case[n][4][:, 5] = 100.0          # its scale falls to scale_min and stays there
+    dk, dv, tk, tv, ok_, ov_, sk, sv = _prefill(case, T + 1)
+    kn, vn = case["k"][:, :, T], case["v"][:, :, T]
+    mask = torch.zeros(2, 1, 1, T + 1)
+    mask[1, 0, 0, :T // 2] = torch.finfo(torch.float16).min
+    for m in (mask, None):
+        ok2, ov2 = ok_.copy(), ov_.copy()
+        want = orc.decode_attn(case["q"][:, :, 0].numpy(), ok2, ov2, kn.numpy(), vn.numpy(), np_params(case["kp"]), np_params(case["vp"]),
+                               T, 0.08, mask=None if m is None else m[:, 0].numpy(), bits=bits, scale_min=SMIN, scale_max=SMAX)
+        got = gemv.decode_attn(dev(case["q"]), dk, dv, dev(kn[:, :, None]), dev(vn[:, :, None]), dev(case["kp"]), dev(case["vp"]), T,
+                               0.08, SMIN, SMAX, mask=None if m is None else dev(m), bits=bits, k_tail=tk, v_tail=tv, tail_keep=m is not None)
+        _status_ok()
+        np.testing.assert_allclose(got.float().cpu().numpy(), want, rtol=RTOL, atol=ATOL)
+        assert np.array_equal(dk.cpu().numpy(), ok2) and np.array_equal(dv.cpu().numpy(), ov2)
+    orc.append_token(ok_, kn.numpy(), sk, T, np_params(case["kp"]), bits, SMIN, SMAX)
+    orc.append_token(ov_, vn.numpy(), sv, T, np_params(case["vp"]), bits, SMIN, SMAX)
+    assert _bits_equal(tk, _oracle_tail(sk)) and _bits_equal(tv, _oracle_tail(sv))
+
+
+def _filled(case, B, H, T, smin, smax, bits, ckpt=0):
+    kp, vp = dev(case["kp"]), dev(case["vp"])
+    kc = torch.zeros(orc.cache_shape(B, H, orc.n_super_for(T + 1, bits), 128), dtype=torch.uint8, device="cuda")
+    vc = torch.zeros_like(kc)
+    kt, vt = torch.zeros(B, H, 2, 128, device="cuda"), torch.zeros(B, H, 2, 128, device="cuda")
+    extra = {}
+    if ckpt:
+        kk, vk = (gemv.alloc_ckpt(B, H, 128, T + 1, ckpt, "cuda") for _ in range(2))
+        extra = dict(k_ckpt=kk, v_ckpt=vk, ckpt_interval=ckpt)
+    gemv.encode_kv_pair(kc, dev(case["k"][:, :, :T]), kp, vc, dev(case["v"][:, :, :T]), vp, smin, smax, bits=bits, k_tail=kt, v_tail=vt,
+                        **extra)
+    args = (dev(case["q"]), kc, vc, dev(case["k"][:, :, T:]), dev(case["v"][:, :, T:]), kp, vp)
+    return args, dict(bits=bits, k_tail=kt, v_tail=vt, tail_keep=True), extra
+
+
+@pytest.mark.parametrize("T,interval,Hq,bits", [(127, 64, 4, 4), (128, 64, 8, 2), (191, 96, 2, 4), (300, 96, 8, 4), (255, 128, 2, 2), (95, 32, 4, 2)])
+def test_checkpoint_segments(T, interval, Hq, bits):
+    """Segments that end inside a tile, an empty last segment, and the checkpoint that the appended token completes."""
+    case = make_case(1500 + T, 2, Hq, 2, T, bits)
+    args, kw, ck = _filled(case, 2, 2, T, SMIN, SMAX, bits, interval)
+    want = gemv.decode_attn(*args, T, 0.08, SMIN, SMAX, **kw, split_channels=False)
+    kw["tail_keep"] = False
+    got = gemv.decode_attn(*args, T, 0.08, SMIN, SMAX, **kw, **ck)
+    _status_ok()
+    np.testing.assert_allclose(got.float().cpu().numpy(), want.float().cpu().numpy(), rtol=RTOL, atol=ATOL)
+    if (T + 1) % interval == 0:
+        n = (T + 1) // interval - 1
+        assert _bits_equal(ck["k_ckpt"][:, :, n], kw["k_tail"].cpu().numpy()) and _bits_equal(ck["v_ckpt"][:, :, n], kw["v_tail"].cpu().numpy())
+
+
+@pytest.mark.parametrize("kind", ["large", "small", "zero_start", "fast_zero_point", "zero_query", "large_query"])
+@pytest.mark.parametrize("Hq,bits", [(2, 2), (8, 4)])
+def test_ranges(Hq, bits, kind):
+    """Scales of thousands, of 1e-5, from zero; alpha above one; queries at either end: as the scan with fp32 sums gives it, in units of
+    the result."""
+    T, smin, smax, scaling = 150, SMIN, SMAX, 0.08
+    case = make_case(1700, 2, Hq, 2, T, bits)
+    k, v, q = case["k"], case["v"], case["q"]
+    for n in ("kp", "vp"):
+        zp, sc, al, be, tg = (t.clone() for t in case[n])
+        if kind == "large":
+            smax = 30000.0
+            sc[:, ::3] = 9000.0
+        elif kind == "small":
+            smin, smax = 1e-7, 1.0
+            sc[:] = 2e-5
+        elif kind == "zero_start":
+            sc[:, ::4] = 0.0
+        elif kind == "fast_zero_point":
+            al[:, ::5] = 1.5
+        case[n] = (zp, sc, al, be, tg)
+    if kind == "large":
+        case["k"], case["v"], scaling = (k.float().clamp(-100, 100) * 600).half(), (v.float().clamp(-100, 100) * 600).half(), 1e-5
+    elif kind == "small":
+        case["k"], case["v"], scaling = (k.float() * 2e-5).half(), (v.float() * 2e-5).half(), 2000.0
+    elif kind == "zero_query":
+        case["q"] = torch.zeros_like(q)
+    elif kind == "large_query":
+        case["q"], scaling = (q.float() * 10000).clamp(-60000, 60000).half(), 8e-6
+    args, kw, _ = _filled(case, 2, 2, T, smin, smax, bits)
+    want = gemv.decode_attn(*args, T, scaling, smin, smax, **kw, split_channels=False).float().cpu().numpy()
+    got = gemv.decode_attn(*args, T, scaling, smin, smax, **kw).float().cpu().numpy()
+    _status_ok()
+    assert np.isfinite(want).all()
+    np.testing.assert_allclose(got, want, rtol=RTOL, atol=ATOL * np.abs(want).max())
+
+
+@pytest.mark.parametrize("B,Hkv,Hq,T,bits", [(37, 8, 8, 260, 2), (40, 8, 32, 130, 4), (56, 8, 16, 300, 4), (93, 8, 32, 300, 2)])
+def test_more_streams_than_a_round(B, Hkv, Hq, T, bits):
+    """296, 320, 448 and 744 streams: two share an SM and its tensor memory, the others follow."""
+    case = make_case(1800 + T, 1, Hq, Hkv, T, bits)
+    (q, kc, vc, kn, vn, kp, vp), kw, _ = _filled(case, 1, Hkv, T, SMIN, SMAX, bits)
+    rep = lambda t: t.repeat(B, *([1] * (t.dim() - 1)))
+    want = gemv.decode_attn(q, kc, vc, kn, vn, kp, vp, T, 0.08, SMIN, SMAX, **kw, split_channels=False)
+    many = (rep(q), rep(kc), rep(vc), rep(kn), rep(vn), kp, vp)
+    kw.update(k_tail=rep(kw["k_tail"]), v_tail=rep(kw["v_tail"]))
+    got = gemv.decode_attn(*many, T, 0.08, SMIN, SMAX, **kw)
+    again = gemv.decode_attn_varlen(*many, torch.full((B,), T, dtype=torch.int32, device="cuda"), 0.08, SMIN, SMAX, **kw)
+    _status_ok()
+    for out in (got, again):
+        np.testing.assert_allclose(out[:1].float().cpu().numpy(), want.float().cpu().numpy(), rtol=RTOL, atol=ATOL)
+        assert torch.equal(out, rep(out[:1]))
+
+
+@pytest.mark.parametrize("smax", [1e6, float("inf")])
+@pytest.mark.parametrize("Hq,T,bits", [(2, 130, 4), (8, 300, 2), (4, 700, 4)])
+def test_no_upper_bound(Hq, T, bits, smax):
+    """Scales that may grow past what pairs of fp16 numbers hold: token segments, with fp32 values."""
+    case = make_case(1900 + T, 1, Hq, 2, T, bits)
+    args, kw, _ = _filled(case, 1, 2, T, SMIN, smax, bits)
+    want = gemv.decode_attn(*args, T, 0.08, SMIN, smax, **kw, split_channels=False)
+    got = gemv.decode_attn(*args, T, 0.08, SMIN, smax, **kw)
+    _status_ok()
+    np.testing.assert_allclose(got.float().cpu().numpy(), want.float().cpu().numpy(), rtol=RTOL, atol=ATOL)
