@@ -147,7 +147,7 @@ __device__ __forceinline__ bool encode_group(const __half *xin, Chan (&ch)[1], u
     return doubt || !(worst < kClear);
 }
 
-// One tensor (K or V) of a launch; blockIdx.y selects it, so K and V of a layer are quantised side by side.
+// One tensor (K or V) of a launch, which takes several, so that K and V of a layer are quantised side by side.
 struct EncTensor {
     uint32_t *cache;
     const __half *x;
@@ -193,22 +193,31 @@ struct EncIo<1> {
     __device__ static float scale(const Chan (&c)[1]) { return c[0].s; }
 };
 
-template <int BITS, bool WIDE, int CPT>
-__global__ void __launch_bounds__(kD / CPT) encode_kernel(EncBatch batch, CkptSpec cs, int H, int T,
+// A CTA takes one 128-channel slice (blockIdx.x) of one stream of one tensor (blockIdx.y).  PART: the launch is one of two that run side
+// by side (see launch_encode) and takes the slices from `first` on, n_slices per tensor.
+constexpr int kAlone = 0, kFirstPart = 1, kSecondPart = 2;
+template <int BITS, bool WIDE, int CPT, int PART = kAlone>
+__global__ void __launch_bounds__(kD / CPT) encode_kernel(EncBatch batch, CkptSpec cs, int first, int n_slices, int H, int T,
                                                              int n_super_cap, int t_start, float smin, float smax)
 {
+    if (PART == kFirstPart) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // the work that follows on the stream waits for the second part, so that one ends after the first
+    const auto leave = [] {
+        if (PART == kSecondPart) asm volatile("griddepcontrol.wait;" ::: "memory");
+    };
+    const int number = first + blockIdx.x, slice = PART == kAlone ? blockIdx.x : number % n_slices;
     using C = Codec<BITS>;
     using Io = EncIo<CPT>;
     using Half = typename Io::Half;
     using Word = typename Io::Word;
     using Float = typename Io::Float;
-    const EncTensor &et = batch.t[blockIdx.y];
+    const EncTensor &et = batch.t[PART == kAlone ? blockIdx.y : number / n_slices];
     uint32_t *__restrict__ cache = et.cache;
     const __half *__restrict__ x = et.x;
     const ParamPtrs p = et.p;
     float *__restrict__ tail = et.tail;
     const int D = WIDE ? cs.D : kD, S = WIDE ? D / kD : 1;
-    const int bh = blockIdx.x / S, h = bh % H, c0 = kD * (blockIdx.x % S) + CPT * threadIdx.x;   // c0: channel in the head
+    const int bh = slice / S, h = bh % H, c0 = kD * (slice % S) + CPT * threadIdx.x;   // c0: channel in the head
     const size_t po = size_t(h) * D + c0;
     Chan ch[CPT];
     float beta[CPT], target[CPT];
@@ -299,7 +308,7 @@ __global__ void __launch_bounds__(kD / CPT) encode_kernel(EncBatch batch, CkptSp
     // the quantiser by kEncStages - 1 tiles.
     const int n_groups = (t_end - t) / 8;
     const int n_tiles = (n_groups + 3) / 4;
-    const __half *src = x + (size_t(bh) * T + (t - t_start)) * D + kD * (blockIdx.x % S);
+    const __half *src = x + (size_t(bh) * T + (t - t_start)) * D + kD * (slice % S);
     auto issue = [&](int i) {
         const int rows = min(4, n_groups - 4 * i) * 8;
         const uint32_t bytes = uint32_t(rows) * kD * 2;
@@ -320,6 +329,7 @@ __global__ void __launch_bounds__(kD / CPT) encode_kernel(EncBatch batch, CkptSp
             // give up as one CTA; let copies already in flight land (bounded) before the memory is released
             for (int k = i; k < min(n_tiles, i + kEncStages); ++k)
                 if (!mbar_wait_bounded(&bar[k % kEncStages], (k / kEncStages) & 1, kStatDrain)) break;
+            leave();
             return;
         }
         const int ng = min(4, n_groups - 4 * i);
@@ -358,6 +368,7 @@ __global__ void __launch_bounds__(kD / CPT) encode_kernel(EncBatch batch, CkptSp
         *reinterpret_cast<Float *>(tail + size_t(bh) * 2 * D + c0) = Io::zp(ch);
         *reinterpret_cast<Float *>(tail + size_t(bh) * 2 * D + D + c0) = Io::scale(ch);
     }
+    leave();
 }
 
 // Tensors of one append launch over several layers: K and V of up to 32 (4.6 KB of kernel parameters).
@@ -486,27 +497,53 @@ static int ckpt_check(const void *k_ckpt, const void *v_ckpt, int interval, int 
     return 0;
 }
 
+// An odd number of two-warp CTAs on an SM leaves two of its schedulers a warp more than the other two, and all wait for those.  Then
+// the CTAs beyond the even number come as four warps of one channel a thread, one for each scheduler: two launches side by side
+// (the second is a programmatic dependent that starts as soon as the first is in place).  Device time on a B200, K and V of 32 heads, 4-bit,
+// one launch -> two: 16 x 8192 tokens (6.9 CTAs an SM) 856 -> 790 us, 15 x 4000 426 -> 392 us, 11 x 4000 (4.8) 346 -> 323 us, 19 x 2000 (8.2)
+// 262 -> 243 us, 16 x 256 34.8 -> 33.2 us; 2-bit 16 x 8192 852 -> 818 us, 14 x 2000 (6.1) 216 -> 206 us.  With more than one left over
+// for an SM the two do not come out even.  Returns the size of the first, 0 for one launch.
+static int side_by_side(long long grid, int T)
+{
+    const long long even = grid / (2 * kSMs) * (2 * kSMs), rest = grid - even;
+    return even >= 4 * kSMs && even <= 10 * kSMs && rest > 0 && rest <= kSMs && T >= 256 ? int(even) : 0;
+}
+
 static int launch_encode(const EncBatch &b, int n, int B, int H, int T, int D, int n_super_cap, int bits,
                          int t_start, float smin, float smax, void *stream, CkptSpec cs = CkptSpec{0, 0, 0})
 {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     cs.D = D;
-    const dim3 grid(B * H * (D / kD), n);
+    const int n_slices = B * H * (D / kD);
+    const long long grid = (long long)n_slices * n;
     // One channel per thread while that leaves a warp scheduler at most three warps: a warp then has its scheduler (nearly)
     // to itself and takes as long as its own instructions, of which one channel needs about half as many as a pair.
     // Measured on a B200, K and V of 32 heads: 1 x 4000 tokens 251 -> 231 us, 2 x 2000 tokens 131 -> 121 us, 4 x 2000 tokens
     // 137 -> 133 us, 6 x 3000 tokens 213 -> 199 us (2-bit 224 -> 212 us), but 8 x 2000 tokens 148 -> 155 us.  With more streams the
     // schedulers are busy and the packed pair needs fewer issue slots per channel.
-    const bool few = (long long)grid.x * grid.y * (kD / 32) <= 3 * kSchedulers;
-    if (D == kD) {
-        if (bits == 4 && few) encode_kernel<4, false, 1><<<grid, kD, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
-        else if (bits == 4) encode_kernel<4, false, 2><<<grid, kEncThreads, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
-        else if (few) encode_kernel<2, false, 1><<<grid, kD, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
-        else encode_kernel<2, false, 2><<<grid, kEncThreads, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
-    } else {
-        if (bits == 4) encode_kernel<4, true, 2><<<grid, kEncThreads, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
-        else encode_kernel<2, true, 2><<<grid, kEncThreads, 0, s>>>(b, cs, H, T, n_super_cap, t_start, smin, smax);
+    const bool few = grid * (kD / 32) <= 3 * kSchedulers;
+    const auto kernel = D == kD ? (bits == 4 ? (few ? encode_kernel<4, false, 1> : encode_kernel<4, false, 2>)
+                                             : (few ? encode_kernel<2, false, 1> : encode_kernel<2, false, 2>))
+                                : (bits == 4 ? encode_kernel<4, true, 2> : encode_kernel<2, true, 2>);
+    const int split = D == kD && !few ? side_by_side(grid, T) : 0;
+    if (split) {
+        const auto first = bits == 4 ? encode_kernel<4, false, 2, kFirstPart> : encode_kernel<2, false, 2, kFirstPart>;
+        const auto second = bits == 4 ? encode_kernel<4, false, 1, kSecondPart> : encode_kernel<2, false, 1, kSecondPart>;
+        first<<<split, kEncThreads, 0, s>>>(b, cs, 0, n_slices, H, T, n_super_cap, t_start, smin, smax);
+        if (int rc = launch_status()) return rc;
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(int(grid) - split);
+        cfg.blockDim = dim3(kD);
+        cfg.stream = s;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, second, b, cs, split, n_slices, H, T, n_super_cap, t_start, smin, smax);
+        return e == cudaSuccess ? launch_status() : int(e);
     }
+    kernel<<<dim3(n_slices, n), D == kD && few ? kD : kEncThreads, 0, s>>>(b, cs, 0, n_slices, H, T, n_super_cap, t_start, smin, smax);
     return launch_status();
 }
 
