@@ -20,8 +20,9 @@
 // e) and add the sums of V to the result; two issue the products and the copies of packed words.  All meet at mbarriers, two tiles
 // in flight.  What bounds it: issue and register reads of the scans, 10 cycles a value and scheduler with four warps, 13 with two
 // (measured alone; a third of it the split into fp16 parts), so with one query head and many streams the packed scans of
-// adkv_decode.cuh stay ahead (12 cycles with everything); the lines are in tensor_pays (adkv_host.h).  Against 64 bits the error of
-// a logit is 0.84 to 1.03 times that of one scan with fp32 sums, 0.97 in the mean over 16 sets (128 to 8000 tokens, 384 streams each).
+// adkv_decode.cuh stay ahead (12 cycles with everything); with one CTA on an SM the warps that move the sums, weigh and add, one after
+// the other, 2600 cycles a tile.  The lines are in tensor_pays (adkv_host.h).  Against 64 bits the error of a logit is 0.70 to 0.96
+// times that of one scan with fp32 sums, 0.89 in the mean over 14 sets (128 to 8000 tokens, 384 streams each).
 //
 // Only the appended token needs the encoder's exact state, and that comes from the tail.
 #include "adkv_host.h"
@@ -102,28 +103,56 @@ __device__ __noinline__ Window guarded_window(uint32_t w, float s, float beta, f
     r.s = s;
     return r;
 }
-// Code times scale of eight tokens (fields 0..7 of w); advances the scale.  safe: no channel of the warp can meet a bound in these
-// tokens; becomes the same for the next eight, so that the vote is under way while the values are split and stored.
+// Code times scale of eight tokens (fields 0..7 of w); advances the scale, without guards.  What every fourth product of the scale
+// loses in rounding goes into the next: two multiply-adds more in eight tokens than without, and logits end 6 to 12 % nearer to 64
+// bits than with every eighth, 256 streams x 8192 tokens 334 -> 337 us.
 template <int BITS>
-__device__ __forceinline__ void scale_window(uint32_t w, const FieldConsts<BITS> &fc, TensorChan &c, float smin, float smax, float (&x)[8], bool &safe)
+__device__ __forceinline__ void scale_window(uint32_t w, const FieldConsts<BITS> &fc, TensorChan &c, float (&x)[8])
+{
+    static_for<8>([&](auto jc) {
+        constexpr int j = decltype(jc)::value;
+        const float q = fc.template code<j % 4>(j < 4 ? w : w >> (4 * BITS));
+        x[j] = __fmul_rn(q, c.s);
+        const float f = fmaf(c.beta, fabsf(q), c.tc), s = c.s;
+        c.s = j % 4 == 0 ? fmaf(s, f, c.lost * f) : s * f;
+        if (j % 4 == 3) c.lost = fmaf(s, f, -c.s);
+    });
+}
+// The same with them, by a call.
+template <int BITS>
+__device__ __forceinline__ void scale_window_guarded(uint32_t w, TensorChan &c, float smin, float smax, float (&x)[8])
+{
+    const Window r = guarded_window<BITS>(w, c.s, c.beta, c.tc, smin * c.inv, smax * c.inv, kEps * c.inv);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = r.x[j];
+    c.s = r.s;
+    c.lost = 0.f;
+}
+// Sixteen tokens.  safe: no channel of the warp can meet a bound in the next eight.  The second eight run on that they cannot
+// either, and are done again where the scale between the two says otherwise: one vote for sixteen tokens instead of two, each of
+// which costs a warp with one other on its scheduler 22 cycles.
+template <int BITS>
+__device__ __forceinline__ void scale_windows(uint32_t wa, uint32_t wb, const FieldConsts<BITS> &fc, TensorChan &c, float smin, float smax,
+                                              float (&xa)[8], float (&xb)[8], bool &safe)
 {
     if (safe) {
-        static_for<8>([&](auto jc) {
-            constexpr int j = decltype(jc)::value;
-            const float q = fc.template code<j % 4>(j < 4 ? w : w >> (4 * BITS));
-            x[j] = __fmul_rn(q, c.s);
-            const float f = fmaf(c.beta, fabsf(q), c.tc), s = c.s;
-            c.s = j == 0 ? fmaf(s, f, c.lost * f) : s * f;
-            if (j == 7) c.lost = fmaf(s, f, -c.s);
-        });
+        scale_window<BITS>(wa, fc, c, xa);
+        const float between = c.s;
+        scale_window<BITS>(wb, fc, c, xb);
+        const bool held = between >= c.lo && between <= c.hi;
+        safe = __all_sync(kFull, held && c.s >= c.lo && c.s <= c.hi);
+        if (!safe) {
+            if (!__all_sync(kFull, held)) {
+                c.s = between;
+                scale_window_guarded<BITS>(wb, c, smin, smax, xb);
+            }
+            safe = c.safe();
+        }
     } else {
-        const Window r = guarded_window<BITS>(w, c.s, c.beta, c.tc, smin * c.inv, smax * c.inv, kEps * c.inv);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) x[j] = r.x[j];
-        c.s = r.s;
-        c.lost = 0.f;
+        scale_window_guarded<BITS>(wa, c, smin, smax, xa);
+        scale_window_guarded<BITS>(wb, c, smin, smax, xb);
+        safe = c.safe();
     }
-    safe = c.safe();
 }
 
 __device__ __forceinline__ float redux_max(float v)
@@ -148,7 +177,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
     extern __shared__ __align__(128) uint8_t smem_raw[];
     using Shared = TensorShared<BITS, G>;
     Shared &sh = *reinterpret_cast<Shared *>(smem_raw);
-    constexpr int kSums = G == 4 ? 4 : 6;    // see the products of K
+    constexpr int kSums = G == 4 ? 2 : 4;    // see the products of K
     constexpr int TPW = Codec<BITS>::TPW, KN = Shared::KN, VN = Shared::VN, KG = Shared::KG, VG = Shared::VG, NB = Shared::NB, ST = Shared::ST;
     constexpr int ROWS = kTcTok / TPW;       // word rows of a tile
     // columns of tensor memory: V values (rounded, then remainders) and sums of V, NB buffers each; sums of K
@@ -304,38 +333,39 @@ __global__ void __launch_bounds__(kTcThreads, 2)
 #pragma unroll 1
         for (int i = 0; i < n_tiles; ++i) {
             const int buf = i % NB, st = i % ST;
-            const int rows = (min(ROWS, n_rows - i * ROWS) + 16 / TPW - 1) / (16 / TPW) * (16 / TPW);   // products of V take 16 tokens at a time
+            const int rounds = (min(ROWS, n_rows - i * ROWS) + 16 / TPW - 1) / (16 / TPW);   // of 16 tokens, as the products of V take
             // the words have come, and the products that read this buffer before are done
             if (!(ok = mbar_wait_both(&loaded[st], i / ST & 1, i >= NB ? &freed[buf] : nullptr, (i / NB & 1) ^ 1, kStatKWait))) break;
             tc_fence_after();
             const uint32_t *row = &sh.words[which][st][0][c];
             uint8_t *k_dst = reinterpret_cast<uint8_t *>(&sh.a[buf][0][0][c][0]);
-            uint32_t v_dst = lanes + kVBuf * buf, w = *row;
-#pragma unroll 1
-            for (int r = 0; r < rows; ++r) {
-                row += kD;
-                const uint32_t w_next = *row;   // behind the last row of a tile: whatever lies there, not used
-#pragma unroll
-                for (int u = 0; u < TPW / 8; ++u) {
-                    float x[8];
-                    scale_window<BITS>(w, fc, ch, ka.smin, ka.smax, x, safe);
-                    uint4 hi, lo;
-                    hi.x = pack_half2(x[0], x[1]); lo.x = pack_remainder(hi.x, x[0], x[1]);
-                    hi.y = pack_half2(x[2], x[3]); lo.y = pack_remainder(hi.y, x[2], x[3]);
-                    hi.z = pack_half2(x[4], x[5]); lo.z = pack_remainder(hi.z, x[4], x[5]);
-                    hi.w = pack_half2(x[6], x[7]); lo.w = pack_remainder(hi.w, x[6], x[7]);
-                    if (is_k) {
-                        *reinterpret_cast<uint4 *>(k_dst) = hi;
-                        *reinterpret_cast<uint4 *>(k_dst + sizeof(sh.a[0][0])) = lo;
-                    } else {
-                        tmem_st4(v_dst, hi.x, hi.y, hi.z, hi.w);
-                        tmem_st4(v_dst + kVPart, lo.x, lo.y, lo.z, lo.w);
-                    }
-                    k_dst += kD * 16;
-                    v_dst += 4;
-                    if (TPW == 16) w >>= 16;
+            uint32_t v_dst = lanes + kVBuf * buf, wa = row[0], wb = BITS == 4 ? row[kD] : wa >> 16;
+            const auto store = [&](const float (&x)[8]) {
+                uint4 hi, lo;
+                hi.x = pack_half2(x[0], x[1]); lo.x = pack_remainder(hi.x, x[0], x[1]);
+                hi.y = pack_half2(x[2], x[3]); lo.y = pack_remainder(hi.y, x[2], x[3]);
+                hi.z = pack_half2(x[4], x[5]); lo.z = pack_remainder(hi.z, x[4], x[5]);
+                hi.w = pack_half2(x[6], x[7]); lo.w = pack_remainder(hi.w, x[6], x[7]);
+                if (is_k) {
+                    *reinterpret_cast<uint4 *>(k_dst) = hi;
+                    *reinterpret_cast<uint4 *>(k_dst + sizeof(sh.a[0][0])) = lo;
+                } else {
+                    tmem_st4(v_dst, hi.x, hi.y, hi.z, hi.w);
+                    tmem_st4(v_dst + kVPart, lo.x, lo.y, lo.z, lo.w);
                 }
-                w = w_next;
+                k_dst += kD * 16;
+                v_dst += 4;
+            };
+#pragma unroll 1
+            for (int n = 0; n < rounds; ++n) {
+                row += 16 / TPW * kD;
+                const uint32_t next_a = row[0], next_b = BITS == 4 ? row[kD] : next_a >> 16;   // behind a tile: whatever lies there, not used
+                float xa[8], xb[8];
+                scale_windows<BITS>(wa, wb, fc, ch, ka.smin, ka.smax, xa, xb, safe);
+                store(xa);
+                store(xb);
+                wa = next_a;
+                wb = next_b;
             }
             if (is_k) {
                 fence_async_shared();
@@ -386,15 +416,22 @@ __global__ void __launch_bounds__(kTcThreads, 2)
             const int buf = i % NB;
             if (!mbar_wait(&sh.kdone[buf], i / NB & 1, kStatLFullWait)) return false;
             tc_fence_after();
-            constexpr int C = G == 1 ? 4 : G == 2 ? 8 : 16;   // columns to read
+            constexpr int C = G == 1 ? 4 : G == 2 ? 8 : 16, AT = G == 4 ? 2 : 4;   // columns to read, loads in flight
             float sum[3 * G];
 #pragma unroll
-            for (int n = 0; n < kSums; ++n) {
-                uint32_t r[C];
-                tmem_ld(r, lanes + kDK + KN * n);
-                tmem_wait_ld(r);
+            for (int n = 0; n < kSums; n += AT) {
+                uint32_t r[AT][C];
 #pragma unroll
-                for (int k = 0; k < 3 * G; ++k) sum[k] = n ? sum[k] + __uint_as_float(r[k]) : __uint_as_float(r[k]);
+                for (int m = 0; m < AT; ++m) tmem_ld(r[m], lanes + kDK + KN * (n + m));
+#pragma unroll
+                for (int m = 0; m < AT; ++m) tmem_wait_ld(r[m]);
+#pragma unroll
+                for (int k = 0; k < 3 * G; ++k) {
+                    float part = __uint_as_float(r[0][k]);
+#pragma unroll
+                    for (int m = 1; m < AT; ++m) part += __uint_as_float(r[m][k]);
+                    sum[k] = n ? sum[k] + part : part;
+                }
             }
             tc_fence_before();
             arrive_warp(&sh.kread, lane);
@@ -415,8 +452,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
             const float mk0 = mask_row && in0 ? mask_row[t_begin + t0] * 1.4426950408889634f : 0.f;
             const float mk1 = mask_row && in1 ? mask_row[t_begin + t0 + 1] * 1.4426950408889634f : 0.f;
             if (!mbar_wait(&sh.lfull[buf], i / NB & 1, kStatLFullWait)) return false;
-            // the products that read this buffer of weights before are done
-            if (i >= NB && !mbar_wait(&sh.vdone[buf], (i / NB & 1) ^ 1, kStatVWait)) return false;
+            // the products that read this buffer of weights before are done: add_sums(i - 2) has waited for them
             const float ba = sh.back[g][0], bb = sh.back[g][1];
             const float2 a_hi = *reinterpret_cast<const float2 *>(&sh.lbuf[buf][0][g][0][2 * lane]);
             const float2 a_lo = *reinterpret_cast<const float2 *>(&sh.lbuf[buf][1][g][0][2 * lane]);
@@ -543,8 +579,9 @@ __global__ void __launch_bounds__(kTcThreads, 2)
                 if (!(ok = mbar_wait(&sh.kfull[buf], phase, kStatKWait))) break;
                 tc_fence_after();
                 if (elect_one()) {
-                    // Accumulation rounds towards zero.  One running sum over the eight steps put logits 3 to 6 % further from 64 bits than
-                    // a scan with fp32 sums (4 bits, 2000 and 4096 tokens); sums of one or two steps each, added up in fp32, do not.
+                    // Accumulation rounds towards zero.  One running sum over the eight steps puts logits 1 to 5 % further from 64 bits
+                    // than several that are added up in fp32; more sums are more to read: four heads, 4-bit, 256 streams x 4096
+                    // tokens, four sums 159 us, two 155 us, one 156 us; one and two heads the same with six, four and two.
                     const uint64_t a = mn_major_desc(&sh.a[buf][0][0][0][0], 128, kD * 16), bd = mn_major_desc(&sh.kb[0][0][0], 128, KG == 1 ? 0 : kD * 16);
 #pragma unroll
                     for (int n = 0; n < kD / 16; ++n) mma_smem(tmem + kDK + KN * (n % kSums), a + 16 * n, bd + 16 * n, k_desc, n >= kSums);
