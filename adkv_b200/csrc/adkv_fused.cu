@@ -112,8 +112,11 @@ ADKV_DEFINE_TU_STATUS(adkv_tu_status_fused)
 
 // Token segments of a stream side by side (adkv_segments.cu), next to tail states: up to one stream per SM and from 128
 // tokens on (max_tokens: the tokens of every sequence, or what the cache can hold of them where the lengths are on the
-// device).  Device time on a B200, the split head of adkv_narrow.cu / whole head / segments, where no scale meets a clamp and,
-// in brackets, where one channel of every head rests at a bound:
+// device).  The tensor-core kernel goes first, so what comes here is 2-bit caches with one query head and more than kSegmentsAhead
+// tokens, and scale bounds that kernel cannot take (tensor_can).  Device time on a B200, segments / tensor cores, 2-bit, one head, 128
+// to 148 streams: x 500 tokens 18.9 / 18.2 us, x 700 24.7 / 22.5 us, x 1000 30.0 / 30.7 us, x 12000 256 / 272 us.
+// Split head of adkv_narrow.cu / whole head / segments, where no scale meets a clamp and, in brackets, where one channel of every
+// head rests at a bound:
 //    4-bit                 128 streams x 256 tokens 16.4 / 16.7 / 12.4 us, x 2000 93 / 89 / 49 us (179 / 109 / 80 us)
 //    2-bit, four heads     128 streams x 256 tokens 22.0 / 24.4 / 16.0 us, x 2000 141 / 140 / 73 us (185 / 146 / 102 us)
 // Measured with tiles of 32 tokens everywhere, split head -> segments: 32 streams x 8000 tokens, 4-bit, 376 -> 176 us (728 -> 322 us);
@@ -124,7 +127,7 @@ ADKV_DEFINE_TU_STATUS(adkv_tu_status_fused)
 // to: 256 streams x 8000 tokens with four segments each, 2-bit, 442 -> 378 us / 478 -> 655 us, with eight KV heads 595 ->
 // 522 us / 646 -> 788 us.
 constexpr long long kSegmentsMaxStreams = kSMs;
-constexpr int kSegmentsMinTokens = 128;
+constexpr int kSegmentsMinTokens = 128, kSegmentsAhead = 700;
 
 static bool use_segments(const KArgs &ka, int B, int max_tokens, bool exact, unsigned flags)
 {
@@ -135,6 +138,7 @@ static bool use_segments(const KArgs &ka, int B, int max_tokens, bool exact, uns
 static bool use_tensor(const KArgs &ka, int B, int bits, int max_tokens, bool device_lengths, bool exact, unsigned flags)
 {
     const int G = ka.Hq / ka.Hkv;
+    if (bits == 2 && G == 1 && max_tokens > kSegmentsAhead && use_segments(ka, B, max_tokens, exact, flags)) return false;
     return ka.tail && !exact && !(flags & (ADKV_FLAG_SPLIT_CHANNELS | ADKV_FLAG_NO_SPLIT_CHANNELS)) && tensor_can(G, ka.smin, ka.smax) &&
            tensor_pays(bits, G, (long long)B * ka.Hkv, max_tokens, device_lengths);
 }

@@ -14,18 +14,19 @@ constexpr int kSMs = 148, kSchedulers = 4 * kSMs;   // B200: what the choice of 
 // 296 run at once, and up to 444 and 740 the last round is half full where the 64-thread CTAs of the other kernels pile up on
 // some SMs.  A value costs this kernel about the same whatever the number of query heads, the others a multiply-add and an
 // eighth of a sum over the lanes per head.  Device time on a B200, us, before -> this kernel (16 heads x 128 wide unless noted):
-//   one head     4-bit 128 x 300 14.5 -> 11.2, 128 x 3000 71.8 -> 65.4, 256 x 3000 132 -> 107, 400 x 300 27.5 -> 24.5, 400 x 200
-//                19.4 -> 19.8, 592 x 1500 102 -> 109; 2-bit 128 x 300 14.5 -> 11.9, 148 x 12000 256 -> 272, 440 x 150 16.6 -> 16.3
-//   two heads    4-bit 128 x 300 17.0 -> 11.7, 256 x 3000 158 -> 113, 740 x 256 37 -> 35, 740 x 1024 117 -> 101, 888 x 1024 118 -> 119
-//   four heads   4-bit 128 x 300 18.9 -> 13.0, 256 x 3000 195 -> 124, 740 x 150 33 -> 31, 1184 x 256 59 -> 58, 2400 x 512 201 -> 193,
-//                4096 x 512 300 -> 313; 2-bit 256 x 8192 551 -> 330
+//   one head     4-bit 128 x 300 14.3 -> 11.2, 128 x 3000 71.7 -> 68.6, 256 x 3000 132 -> 110, 400 x 300 26.6 -> 24.3, 400 x 200
+//                19.4 -> 19.8, 592 x 1500 102 -> 109; 2-bit 128 x 300 14.7 -> 12.3, 256 x 3000 139 -> 124, 440 x 1024 73 -> 70
+//   two heads    4-bit 128 x 300 16.9 -> 11.4, 256 x 3000 158 -> 111, 740 x 256 37 -> 34, 740 x 1024 117 -> 98, 888 x 1024 118 -> 119
+//   four heads   4-bit 128 x 300 19.1 -> 12.3, 256 x 3000 195 -> 118, 740 x 150 33 -> 30, 1184 x 256 59 -> 57, 1480 x 512 123 -> 114,
+//                4096 x 512 300 -> 313; 2-bit 256 x 3000 209 -> 132
+//   segments     4-bit, one head, between checkpoints 512 tokens apart: 8 streams x 8000 30 -> 19; 2-bit, 4096 apart, 8 x 9000 199 -> 96
 // Below 32 tokens set-up counts (148 x 16 tokens 5.0 -> 5.2, 296 x 32 tokens 6.7 -> 6.8).  Device-side lengths may be short whatever the cache
-// holds: 592 sequences of four heads, 50 to 100 tokens 22 -> 21, 100 to 1000 tokens 94 -> 60; of one head, 768 x 600 61 -> 76.
-// With one channel of every head at a bound 256 x 1000: one head 59 -> 51, four heads 76 -> 57.
+// holds: 384 sequences of four heads, 50 to 100 tokens 19 -> 18, 100 to 2000 tokens 146 -> 69; of one head, 768 x 600 61 -> 76.
+// With one channel of every head at a bound 256 x 1000: one head 59 -> 51, four heads 76 -> 55.
 static inline bool tensor_pays(int bits, int G, long long ctas, int tokens, bool device_lengths)
 {
     if (device_lengths && (tokens < 128 || (G == 1 && ctas > kSMs))) return false;
-    if (ctas <= kSMs) return tokens >= 32 && !(bits == 2 && G == 1 && tokens > 2000);
+    if (ctas <= kSMs) return tokens >= 32;
     if (ctas <= 2 * kSMs) return tokens >= 64;
     if (device_lengths) return tokens >= 512 && ctas <= (G == 2 ? 4 : 5) * kSMs;
     if (ctas <= 3 * kSMs) return tokens >= (G > 1 ? 100 : bits == 4 ? 256 : 128);
