@@ -106,6 +106,38 @@ def test_ranges(Hq, bits, kind):
     np.testing.assert_allclose(got, want, rtol=RTOL, atol=ATOL * np.abs(want).max())
 
 
+@pytest.mark.parametrize("rising", [False, True])
+@pytest.mark.parametrize("Hq,bits", [(32, 2), (32, 4), (128, 4)])
+def test_bound_met_at_every_token(Hq, bits, rising):
+    """One channel of every head meets a bound, a token later from head to head: each place of the 16 tokens between two votes."""
+    H, T, smin, smax = 32, 100, 0.05, 2.0
+    case = make_case(1950, 1, Hq, H, T, bits)
+    for n, c in (("kp", 5), ("vp", 70)):
+        zp, sc, al, be, tg = (t.clone() for t in case[n])
+        be[:, c], tg[:, c] = 2 ** -6, -8.0 if rising else 8.0      # 12 % a token and up, 12 % and less down
+        away = 1.125 ** (10 + torch.arange(H, dtype=torch.float32))
+        sc[:, c] = (smax / away if rising else smin * away).to(sc.dtype)
+        case[n] = (zp, sc, al, be, tg)
+    args, kw, ck = _filled(case, 1, H, T, smin, smax, bits, 64)
+    want = gemv.decode_attn(*args, T, 0.08, smin, smax, **kw, split_channels=False)
+    outs = [gemv.decode_attn(*args, T, 0.08, smin, smax, **kw), gemv.decode_attn(*args, T, 0.08, smin, smax, **kw, **ck)]
+    _status_ok()
+    for got in outs:
+        np.testing.assert_allclose(got.float().cpu().numpy(), want.float().cpu().numpy(), rtol=RTOL, atol=ATOL)
+
+
+@pytest.mark.parametrize("T", [699, 700, 701])
+def test_line_to_token_segments(T):
+    """2-bit, one query head: the longest streams of this kernel and the shortest that are cut into segments; between checkpoints never."""
+    case = make_case(1960, 1, 2, 2, T, 2)
+    args, kw, ck = _filled(case, 1, 2, T, SMIN, SMAX, 2, 1024)
+    want = gemv.decode_attn(*args, T, 0.08, SMIN, SMAX, **kw, split_channels=False)
+    outs = [gemv.decode_attn(*args, T, 0.08, SMIN, SMAX, **kw), gemv.decode_attn(*args, T, 0.08, SMIN, SMAX, **kw, **ck)]
+    _status_ok()
+    for got in outs:
+        np.testing.assert_allclose(got.float().cpu().numpy(), want.float().cpu().numpy(), rtol=RTOL, atol=ATOL)
+
+
 @pytest.mark.parametrize("B,Hkv,Hq,T,bits", [(37, 8, 8, 260, 2), (40, 8, 32, 130, 4), (56, 8, 16, 300, 4), (93, 8, 32, 300, 2)])
 def test_more_streams_than_a_round(B, Hkv, Hq, T, bits):
     """296, 320, 448 and 744 streams: two share an SM and its tensor memory, the others follow."""
