@@ -25,7 +25,7 @@
 // 1500 to 4096 tokens, 4 and 2 bits), because the segments start from less rounding.
 //
 // Steps 1 and 2 add a third to the work, two thirds where a clamp is met, so this pays only while a stream per warp pair
-// leaves schedulers idle: see use_segments in adkv_fused.cu.
+// leaves schedulers idle, and where the tensor-core kernel (adkv_tensor.cu) is no faster: see use_segments in adkv_fused.cu.
 #include "adkv_host.h"
 
 #include "adkv_softmax.cuh"
