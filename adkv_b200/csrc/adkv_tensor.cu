@@ -79,7 +79,7 @@ __device__ __forceinline__ uint32_t pack_remainder(uint32_t h, float a, float b)
     return pack_half2(d0, d1);
 }
 
-// What one thread keeps of its channel.  The scale is held in units of a power of two near the first one, so that the fp16 parts
+// What one thread keeps of its channel.  The scale is held in units of a power of two below the upper bound, so that the fp16 parts
 // of the dequantised values have their bits where they are needed; scaling by it rounds nothing.
 struct TensorChan {
     float s, beta, tc, lo, hi;   // scale, constants of its update, interval in which eight updates cannot meet a bound
@@ -153,6 +153,13 @@ __device__ __forceinline__ void scale_windows(uint32_t wa, uint32_t wb, const Fi
         scale_window_guarded<BITS>(wb, c, smin, smax, xb);
         safe = c.safe();
     }
+}
+
+// The code of the first token of a channel.
+template <int BITS>
+__device__ __noinline__ float first_code(const uint8_t *cache, size_t at)
+{
+    return code_f_rt<BITS>(reinterpret_cast<const uint32_t *>(cache)[at], 0);
 }
 
 __device__ __forceinline__ float redux_max(float v)
@@ -245,8 +252,15 @@ __global__ void __launch_bounds__(kTcThreads, 2)
             zp = __half2float(p.zp_init[po]);
             s = __half2float(p.scale_init[po]);
         }
-        // eight times the largest scale stays in the range of fp16
-        const int e = min(max(max(exponent_field(s), exponent_field(ka.smax) + 1 - 12), 127 - 40), 127 + 40);
+        // The unit goes by the upper bound: eight times that stays in the range of fp16, and a lower bound no further away than
+        // tensor_can allows leaves every value its 22 bits, wherever the scale moves.  Only scale_init may lie above the bound, and
+        // counts where its code is not zero (the values of this channel then start that large, too).  One branch for the warp and a
+        // call: a branch for each thread, or the word read in any case, costs long streams 1 % and a step of 300 tokens 0.25 us.
+        int e = max(exponent_field(s), exponent_field(ka.smax)) - 11;
+        if ((!PART || seg == 0) && __any_sync(kFull, e > exponent_field(ka.smax) - 11)) {
+            if (first_code<BITS>(is_k ? ka.cache : va.cache, size_t(bh) * ka.n_super_cap * kD + c) == 0.f) e = exponent_field(ka.smax) - 11;
+        }
+        e = min(max(e, 127 - 40), 127 + 40);
         const float inv = pow2_bits(254 - e);
         unit = pow2_bits(e);
         ch.s = s * inv;
@@ -314,9 +328,9 @@ __global__ void __launch_bounds__(kTcThreads, 2)
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
                     const uint32_t top = max(max(sh.top[0][2 * g + i], sh.top[1][2 * g + i]), max(sh.top[2][2 * g + i], sh.top[3][2 * g + i]));
-                    const int e = max(int(top >> 23), 11);
-                    up[i] = pow2_bits(264 - e);
-                    if (c == 0) sh.back[g][i] = pow2_bits(e - 10);
+                    const int e = max(int(top >> 23), 15);
+                    up[i] = pow2_bits(268 - e);
+                    if (c == 0) sh.back[g][i] = pow2_bits(e - 14);
                 }
                 const float qa = alpha * q[g] * unit * up[1];
                 col[3 * g] = __float2half_rn(q[g] * unit * up[0]);

@@ -235,7 +235,7 @@ def test_few_and_many_streams_agree(T, bits):
     _status_ok()
 
 
-def _replay64(cache, params, T, at, bits):
+def _replay64(cache, params, T, at, bits, smin=SMIN, smax=SMAX):
     """The recurrence in 64 bits over the stored codes: values of the tokens in ``at``, [len(at), streams, 128]."""
     B, H = cache.shape[:2]
     words = cache.view(B * H, -1, 128 * 4).contiguous().view(torch.int32)
@@ -248,12 +248,14 @@ def _replay64(cache, params, T, at, bits):
         if t in at:
             out.append(zp + rh)
         zp = zp + al * rh
-        s = (s * (1.0 - be * tg + be * q.abs())).clamp(SMIN, SMAX)
+        s = (s * (1.0 - be * tg + be * q.abs())).clamp(smin, smax)
     return torch.stack(out)
 
 
-def _logit_errors(B, T, bits, pinned, variants, seed=5):
+def _logit_errors(B, T, bits, pinned, variants, seed=5, G=1, smin=SMIN, smax=SMAX, init=None, gain=1.0):
     """Root mean square error of single logits against 64 bits, one figure per entry of ``variants`` (split_channels).
+    G query heads, all alike; ``init``: scale_init of every fourth channel; ``gain``: K and its scales are made smaller by
+    it and q larger.
 
     A mask leaves one cached token and the appended one, and cancels the cached token's exact logit against the appended
     token's; the scaling magnifies what remains.  The output is then v_self + a * (v_cached - v_self), where a / (1 - a) is
@@ -261,17 +263,21 @@ def _logit_errors(B, T, bits, pinned, variants, seed=5):
     """
     D, scaling = 128, 2000.0
     k, v = (synth.gen_kv(seed + i, B, 1, T + 1, D, device="cuda") for i in (0, 1))
-    q = synth.gen_q(seed + 2, B, 1, D, device="cuda")
+    q = (synth.gen_q(seed + 2, B, 1, D, device="cuda") * gain).expand(B, G, 1, D).contiguous()
+    k = k / gain
     kp, vp = (synth.gen_params(seed + 3 + i, 1, D, bits, device="cuda") for i in (0, 1))
+    kp[1].div_(gain)
+    if init is not None:
+        kp[1][:, ::4] = init
     if pinned:      # one channel of the head whose scale rests at scale_min
         kp[4][:, 17] = float(1 << (bits - 1))
         vp[4][:, 17] = float(1 << (bits - 1))
     kc = torch.zeros(orc.cache_shape(B, 1, orc.n_super_for(T + 1, bits), D), dtype=torch.uint8, device="cuda")
     vc = torch.zeros_like(kc)
     kt, vt = torch.zeros(B, 1, 2, D, device="cuda"), torch.zeros(B, 1, 2, D, device="cuda")
-    gemv.encode_kv_pair(kc, k[:, :, :T], kp, vc, v[:, :, :T], vp, SMIN, SMAX, bits=bits, k_tail=kt, v_tail=vt)
+    gemv.encode_kv_pair(kc, k[:, :, :T], kp, vc, v[:, :, :T], vp, smin, smax, bits=bits, k_tail=kt, v_tail=vt)
     at = sorted({T - 1, T - T // 8 - 1, T // 2 + 5})
-    kx, vx = _replay64(kc, kp, T, at, bits), _replay64(vc, vp, T, at, bits)
+    kx, vx = _replay64(kc, kp, T, at, bits, smin, smax), _replay64(vc, vp, T, at, bits, smin, smax)
 
     def appended(cache, tail):     # the appended token, from the tail it is quantised with
         word = cache.view(B, -1, D * 4).contiguous().view(torch.int32)[:, T // (32 // bits)]
@@ -282,7 +288,7 @@ def _logit_errors(B, T, bits, pinned, variants, seed=5):
     for split in variants:
         sq, n = 0.0, 0
         for i, t in enumerate(at):
-            args = (q, kc, vc, k[:, :, T:], v[:, :, T:], kp, vp, T, scaling, SMIN, SMAX)
+            args = (q, kc, vc, k[:, :, T:], v[:, :, T:], kp, vp, T, scaling, smin, smax)
             kw = dict(bits=bits, k_tail=kt, v_tail=vt, tail_keep=True, split_channels=split)
             gemv.decode_attn(*args, **kw)      # writes the appended codes
             ks, vs = appended(kc, kt), appended(vc, vt)
@@ -291,12 +297,12 @@ def _logit_errors(B, T, bits, pinned, variants, seed=5):
             mask[:, T] = 0.0
             shift = (scaling * (qd * (ks - kx[i])).sum(-1)).float()
             mask[:, t] = shift
-            out = gemv.decode_attn(*args, mask=mask, **kw)[:, 0].double()
-            d = vx[i] - vs
-            a = ((out - vs) * d).sum(-1) / (d * d).sum(-1)
+            out = gemv.decode_attn(*args, mask=mask, **kw).double()
+            d = (vx[i] - vs)[:, None]
+            a = ((out - vs[:, None]) * d).sum(-1) / (d * d).sum(-1)
             left = scaling * (qd * (kx[i] - ks)).sum(-1) + shift.double()     # what the rounding of the mask leaves
-            err = (torch.log(a / (1.0 - a)) - left) / scaling
-            sq, n = sq + float((err * err).sum()), n + B
+            err = (torch.log(a / (1.0 - a)) - left[:, None]) / scaling
+            sq, n = sq + float((err * err).sum()), n + err.numel()
         errors.append((sq / n) ** 0.5)
     _status_ok()
     return errors

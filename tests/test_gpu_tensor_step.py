@@ -7,6 +7,7 @@ import torch
 
 from adkv_b200 import gemv
 from oracle import adkv_oracle as orc
+from tests.test_gpu_segments import _logit_errors
 from tests.test_gpu_tail_state import ATOL, RTOL, _bits_equal, _oracle_tail, _prefill, _status_ok
 from tests.util import SMAX, SMIN, dev, make_case, np_params
 
@@ -69,10 +70,10 @@ def test_checkpoint_segments(T, interval, Hq, bits):
         assert _bits_equal(ck["k_ckpt"][:, :, n], kw["k_tail"].cpu().numpy()) and _bits_equal(ck["v_ckpt"][:, :, n], kw["v_tail"].cpu().numpy())
 
 
-@pytest.mark.parametrize("kind", ["large", "small", "zero_start", "fast_zero_point", "zero_query", "large_query"])
+@pytest.mark.parametrize("kind", ["large", "small", "zero_start", "large_first_value", "fast_zero_point", "zero_query", "large_query"])
 @pytest.mark.parametrize("Hq,bits", [(2, 2), (8, 4)])
 def test_ranges(Hq, bits, kind):
-    """Scales of thousands, of 1e-5, from zero; alpha above one; queries at either end: as the scan with fp32 sums gives it, in units of
+    """Scales of thousands, of 1e-5, from zero, one beyond scale_max in the first token; alpha above one; queries at either end: as the scan with fp32 sums gives it, in units of
     the result."""
     T, smin, smax, scaling = 150, SMIN, SMAX, 0.08
     case = make_case(1700, 2, Hq, 2, T, bits)
@@ -80,10 +81,10 @@ def test_ranges(Hq, bits, kind):
     for n in ("kp", "vp"):
         zp, sc, al, be, tg = (t.clone() for t in case[n])
         if kind == "large":
-            smax = 30000.0
+            smin, smax = 4.0, 30000.0
             sc[:, ::3] = 9000.0
         elif kind == "small":
-            smin, smax = 1e-7, 1.0
+            smin, smax = 1e-6, 2.0 ** -7
             sc[:] = 2e-5
         elif kind == "zero_start":
             sc[:, ::4] = 0.0
@@ -94,6 +95,8 @@ def test_ranges(Hq, bits, kind):
         case["k"], case["v"], scaling = (k.float().clamp(-100, 100) * 600).half(), (v.float().clamp(-100, 100) * 600).half(), 1e-5
     elif kind == "small":
         case["k"], case["v"], scaling = (k.float() * 2e-5).half(), (v.float() * 2e-5).half(), 2000.0
+    elif kind == "large_first_value":         # the code of the large scale is one
+        k[:, :, 0, ::7], v[:, :, 0, ::7], scaling = 60000.0, 60000.0, 1e-5
     elif kind == "zero_query":
         case["q"] = torch.zeros_like(q)
     elif kind == "large_query":
@@ -165,3 +168,20 @@ def test_no_upper_bound(Hq, T, bits, smax):
     got = gemv.decode_attn(*args, T, 0.08, SMIN, smax, **kw)
     _status_ok()
     np.testing.assert_allclose(got.float().cpu().numpy(), want.float().cpu().numpy(), rtol=RTOL, atol=ATOL)
+
+
+# scale_init far above the scales that follow; bounds too far apart for one unit of fp16 pairs (then the scans with fp32 values);
+# bounds as far apart as pairs may go, with scales at the lower one
+FAR_SCALES = {"large_init": dict(init=60000.0), "wide_bounds": dict(smin=1e-6, smax=32768.0, gain=1000.0),
+              "at_lower_bound": dict(smin=2.0 ** -7, smax=64.0, gain=50.0)}
+
+
+@pytest.mark.parametrize("bits,G", [(4, 1), (4, 2), (4, 4), (2, 1), (2, 2), (2, 4)])
+@pytest.mark.parametrize("scales", ["usual", *FAR_SCALES])
+def test_logit_error_is_that_of_a_whole_scan(scales, bits, G):
+    """No further from 64 bits than the scan with fp32 values."""
+    pairs = [_logit_errors(64, 600, bits, False, (None, False), seed=s, G=G, **FAR_SCALES.get(scales, {})) for s in (5, 25, 45)]
+    got, whole = (sum(e * e for e in errors) ** 0.5 for errors in zip(*pairs))
+    # 576 logits; eight sets of 2000 tokens: 0.85 to 0.98, and 1.02 with every scale at the lower bound (4-bit), where no rounding
+    # of a scale is carried on
+    assert got <= whole * (1.05 if scales == "at_lower_bound" else 1.0), (got, whole)
