@@ -38,7 +38,7 @@ static inline bool tensor_pays(int bits, int G, long long ctas, int tokens, bool
 // of keys of 1e-3 were 2 % off.  Values never use a scale below the quantiser's eps.
 static inline bool tensor_can(int G, float smin, float smax)
 {
-    return G <= 4 && smin == smin && smax > 0.f && smax <= 32768.f && smax <= 8192.f * fmaxf(smin, kEps);
+    return G <= 4 && smin == smin && smax >= kEps && smax <= 32768.f && smax <= 8192.f * fmaxf(smin, kEps);
 }
 
 static inline ParamPtrs to_ptrs(const adkv_params *p)

@@ -70,10 +70,10 @@ def test_checkpoint_segments(T, interval, Hq, bits):
         assert _bits_equal(ck["k_ckpt"][:, :, n], kw["k_tail"].cpu().numpy()) and _bits_equal(ck["v_ckpt"][:, :, n], kw["v_tail"].cpu().numpy())
 
 
-@pytest.mark.parametrize("kind", ["large", "small", "zero_start", "large_first_value", "fast_zero_point", "zero_query", "large_query"])
+@pytest.mark.parametrize("kind", ["large", "small", "tiny_bounds", "zero_start", "large_first_value", "fast_zero_point", "zero_query", "large_query"])
 @pytest.mark.parametrize("Hq,bits", [(2, 2), (8, 4)])
 def test_ranges(Hq, bits, kind):
-    """Scales of thousands, of 1e-5, from zero, one beyond scale_max in the first token; alpha above one; queries at either end: as the scan with fp32 sums gives it, in units of
+    """Scales of thousands, of 1e-5, of the quantiser's eps, from zero, one beyond scale_max in the first token; alpha above one; queries at either end: as the scan with fp32 sums gives it, in units of
     the result."""
     T, smin, smax, scaling = 150, SMIN, SMAX, 0.08
     case = make_case(1700, 2, Hq, 2, T, bits)
@@ -86,6 +86,11 @@ def test_ranges(Hq, bits, kind):
         elif kind == "small":
             smin, smax = 1e-6, 2.0 ** -7
             sc[:] = 2e-5
+        elif kind == "tiny_bounds":
+            smin, smax = 1e-10, 1e-9          # below the quantiser's eps, by which the values go then
+            zp[:], sc[:] = 1.0, 0.0
+        elif kind == "large_first_value":
+            sc[:, ::7] = 50000.0
         elif kind == "zero_start":
             sc[:, ::4] = 0.0
         elif kind == "fast_zero_point":
