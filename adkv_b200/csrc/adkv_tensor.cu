@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
     if (threadIdx.x == 0) {
         for (int i = 0; i < NB; ++i) {
             mbar_init(&sh.kfull[i], 4);
-            mbar_init(&sh.kdone[i], 1);
+            mbar_init(&sh.kdone[i], 2);
             mbar_init(&sh.vfull[i], 4);
             mbar_init(&sh.wfull[i], G);
             mbar_init(&sh.vdone[i], 2);
@@ -599,6 +599,7 @@ __global__ void __launch_bounds__(kTcThreads, 2)
                     const uint64_t a = mn_major_desc(&sh.a[buf][0][0][0][0], 128, kD * 16), bd = mn_major_desc(&sh.kb[0][0][0], 128, KG == 1 ? 0 : kD * 16);
 #pragma unroll
                     for (int n = 0; n < kD / 16; ++n) mma_smem(tmem + kDK + KN * (n % kSums), a + 16 * n, bd + 16 * n, k_desc, n >= kSums);
+                    mbar_arrive(&sh.kdone[buf]);   // and this thread has seen back and z0 written: the commit is for the products alone
                     mma_commit(&sh.kdone[buf]);
                 }
             } else {
