@@ -34,8 +34,8 @@ static inline bool tensor_pays(int bits, int G, long long ctas, int tokens, bool
     return G == 4 && (ctas <= 8 * kSMs ? tokens >= 256 : ctas <= 16 * kSMs && tokens >= 512);
 }
 // What that kernel can do: its values are pairs of fp16 numbers in units of 2^-11 of scale_max, which have 22 bits from a quarter of
-// a unit on.  Bounds further apart than 2^13 (exp(-4) and exp(4) are 2^11.5) go to the kernels with fp32 values: between 1e-6 and 32768, logits
-// of keys of 1e-3 were 2 % off.  Values never use a scale below the quantiser's eps.
+// a unit on.  Bounds further apart than 2^13 (exp(-4) and exp(4) are 2^11.5) go to the kernels with fp32 values: between 1e-6 and 32768 a
+// scale of 3e-4 would leave its values 11 bits.  Values never use a scale below the quantiser's eps.
 static inline bool tensor_can(int G, float smin, float smax)
 {
     return G <= 4 && smin == smin && smax >= kEps && smax <= 32768.f && smax <= 8192.f * fmaxf(smin, kEps);
