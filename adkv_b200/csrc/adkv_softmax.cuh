@@ -161,7 +161,7 @@ constexpr int kPartStride = 4 + kD;   // floats per (stream, segment, head): max
 struct CkptArgs {
     float *k_ckpt, *v_ckpt;   // [B*Hkv][n_ckpt_cap][2][kD]; entry k = state before token (k+1)*interval
     int interval, n_ckpt_cap;
-    bool mute_k;              // self-test (ADKV_FLAG_SELFTEST_MUTE_K): the K warps do nothing, so every V warp's wait runs out
+    bool mute_k;              // self-test (ADKV_FLAG_SELFTEST_MUTE_K): the K warps do nothing, so the waits behind them run out
 };
 
 // Device-side lengths: the sequence that comes r-th when they are ordered by length, longest first (equal ones by index).

@@ -258,7 +258,7 @@ int adkv_decode_attn_ckpt(const void *q, void *k_cache, void *v_cache, const voi
     const int n_seg = T / interval + 1;
     if (n_seg > 65535) return ADKV_E_SHAPE;
     const dim3 grid(B * Hkv, n_seg);
-    if (ka.tail && !exact && !ck.mute_k && tensor_can(Hq / Hkv, scale_min, scale_max) &&
+    if (ka.tail && !exact && tensor_can(Hq / Hkv, scale_min, scale_max) &&
         tensor_pays(bits, Hq / Hkv, (long long)B * Hkv * n_seg, min(T, interval), false)) {
         if (int rc = adkv_tensor_decode_attn(ka, va, static_cast<const float *>(mask), mask_stride_b, scaling, B, bits, nullptr, 0, ck, n_seg,
                                              static_cast<float *>(scratch), s))

@@ -207,7 +207,8 @@ __global__ void __launch_bounds__(kTcThreads, 2)
     const int bh = b * ka.Hkv + h, T = ka.T;
     const int seg = PART ? blockIdx.y : 0, n_seg = PART ? gridDim.y : 1;
     const int t_begin = PART ? seg * ck.interval : 0, t_end = PART ? min(T, t_begin + ck.interval) : T;
-    const bool append = seg == n_seg - 1;
+    const bool mute_k = PART && ck.mute_k;   // self-test: K is not scanned, and every wait behind that runs out
+    const bool append = seg == n_seg - 1 && !mute_k;
     const int ntok = t_end - t_begin, n_tiles = (ntok + kTcTok - 1) / kTcTok;
     const int n_rows = (ntok + TPW - 1) / TPW;
 
@@ -344,8 +345,9 @@ __global__ void __launch_bounds__(kTcThreads, 2)
         uint64_t *loaded = sh.loaded[which], *freed = is_k ? sh.kdone : sh.vdone, *full = is_k ? sh.kfull : sh.vfull;
         const uint32_t lanes = tmem + (uint32_t(32 * (warp & 3)) << 16);
         bool safe = ch.safe();
+        if (mute_k && is_k) ok = false;
 #pragma unroll 1
-        for (int i = 0; i < n_tiles; ++i) {
+        for (int i = mute_k && is_k ? n_tiles : 0; i < n_tiles; ++i) {
             const int buf = i % NB, st = i % ST;
             const int rounds = (min(ROWS, n_rows - i * ROWS) + 16 / TPW - 1) / (16 / TPW);   // of 16 tokens, as the products of V take
             // the words have come, and the products that read this buffer before are done

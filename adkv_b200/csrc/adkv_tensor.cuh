@@ -84,16 +84,28 @@ __device__ __forceinline__ void tmem_st4(uint32_t at, uint32_t a, uint32_t b, ui
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// mbar_wait_bounded by number of polls instead of by time: reading the timer takes longer than most of these waits.  try_wait
-// itself waits for a while, so a warp that waits takes few issue slots.
-constexpr int kWaitPolls = 8000000;   // at 100 ns or more each, about a second
+// mbar_wait_bounded with the SM's cycle counter for a clock, which makes less code at every wait: one that reads the timer, inline or
+// called, costs a step 1 to 4 %.  A poll waits by itself, up to 3.9 us here, so a warp that waits takes few issue slots.
+constexpr uint32_t kWaitCycles = 2000000000u;   // a second at 1.965 GHz; the counter starts again after 2.2 times that
+__device__ __forceinline__ uint32_t cycles()
+{
+    uint32_t t;
+    asm volatile("mov.u32 %0, %%clock;" : "=r"(t));
+    return t;
+}
 template <class Done>
 __device__ __forceinline__ bool wait_polled(const Done &done, int code)
 {
     bool ok = done();
-    for (int left = kWaitPolls; !ok && left > 0; --left) {
-        __nanosleep(64);
-        ok = done();
+    if (!ok) {
+        uint32_t spent = 0, last = cycles();
+        do {
+            const uint32_t now = cycles();
+            __nanosleep(64);
+            ok = done();
+            spent += now - last;
+            last = now;
+        } while (!ok && spent < kWaitCycles);
     }
     ok = __all_sync(kFull, ok);
     if (!ok && (threadIdx.x & 31) == 0) atomicExch(&g_status, code);

@@ -89,9 +89,10 @@ extern "C" {
 #define ADKV_FLAG_SPLIT_CHANNELS 8u
 #define ADKV_FLAG_NO_SPLIT_CHANNELS 16u
 /* Self-test of the failure path of adkv_decode_attn_ckpt (no counterpart in the reference): the K warps return at
- * once, so every V warp waits for logits that never come.  Each wait gives up after its 1 s limit, the kernels end
- * normally, adkv_device_status reports 3, nothing is appended, and every element of `out` is NaN -- a segment that
- * could not be finished marks its partial result instead of leaving whatever the scratch memory held. */
+ * once, so whatever waits for logits waits for ever.  Each wait gives up after its 1 s limit (the tensor cores' kernel counts it
+ * in cycles, 2e9), the kernels end normally, adkv_device_status reports a wait that ran out (3, or 1 to 4 of that kernel), nothing
+ * is appended, and every element of `out` is NaN -- a segment that could not be finished marks its partial result instead of
+ * leaving whatever the scratch memory held. */
 #define ADKV_FLAG_SELFTEST_MUTE_K 0x80000000u
 
 /* The five per-(kv head, channel) parameter tensors, fp16 [Hkv, D] each
@@ -282,7 +283,8 @@ int adkv_device_status(int *status, void *stream);
 /* Self-test of the bounded waits (no counterpart in the reference): launches one warp that waits on a barrier
  * nothing will ever complete.  The wait gives up after limit_ms (1..2000), the kernel ends normally, and
  * adkv_device_status then reports 7.  Every wait in the library's kernels uses the same routine with a 1 s
- * limit, so a lost copy or a missing partner ends as a status code, not as a hang. */
+ * limit, or one that counts 2e9 cycles (adkv_tensor.cuh), so a lost copy or a missing partner ends as a status code, not
+ * as a hang. */
 int adkv_selftest_wait_timeout(int limit_ms, void *stream);
 
 #ifdef __cplusplus

@@ -1,11 +1,14 @@
 """Decode steps on the tensor cores (next to tail states, up to four query heads per KV head) against the oracle and the
 one-warp-per-tensor scan.  Sizes are the edges of the 64-token tiles and of the 16 tokens that a product of V takes, scales
 at and outside the clamp bounds, values near the ends of fp16, more streams than a round of the chip holds.  Needs a B200."""
+import ctypes
+import time
+
 import numpy as np
 import pytest
 import torch
 
-from adkv_b200 import gemv
+from adkv_b200 import _lib, gemv
 from oracle import adkv_oracle as orc
 from tests.test_gpu_segments import _logit_errors
 from tests.test_gpu_tail_state import ATOL, RTOL, _bits_equal, _oracle_tail, _prefill, _status_ok
@@ -190,3 +193,40 @@ def test_logit_error_is_that_of_a_whole_scan(scales, bits, G):
     # 576 logits; eight sets of 2000 tokens: 0.85 to 0.98, and 1.02 with every scale at the lower bound (4-bit), where no rounding
     # of a scale is carried on
     assert got <= whole * (1.05 if scales == "at_lower_bound" else 1.0), (got, whole)
+
+
+@pytest.mark.parametrize("Hq,bits", [(2, 4), (8, 2)])
+def test_step_that_gives_up_marks_its_result(Hq, bits):
+    """With the K scan muted no sums of K ever come: every wait behind them runs out, the kernel ends by itself, nothing is appended
+    and the output is NaN; the next call is as before."""
+    T, interval, H = 496, 256, 2              # the appended token begins a word
+    case = make_case(1980, 1, Hq, H, T, bits)
+    args, kw, ck = _filled(case, 1, H, T, SMIN, SMAX, bits, interval)
+    scratch = torch.empty(gemv.decode_scratch_bytes(1, Hq, H, T, interval), dtype=torch.uint8, device="cuda")
+    good = gemv.decode_attn(*args, T, 0.08, SMIN, SMAX, **kw, **ck, scratch=scratch)
+    _status_ok()
+    q, kc, vc, kn, vn, kp, vp = args
+    kt, vt, kk, vk = kw["k_tail"], kw["v_tail"], ck["k_ckpt"], ck["v_ckpt"]
+    row = T // (32 // bits)
+    kc[:, :, row], vc[:, :, row] = 0, 0
+    before = [t.clone() for t in (kc, vc, kt, vt, kk, vk)]
+    out = torch.zeros_like(good)
+    pk, pv = (_lib.Params(*[t.data_ptr() for t in ps]) for ps in (kp, vp))
+    torch.cuda.synchronize()
+    t0 = time.perf_counter()
+    rc = _lib.load().adkv_decode_attn_ckpt(
+        q.data_ptr(), kc.data_ptr(), vc.data_ptr(), kn.data_ptr(), vn.data_ptr(), ctypes.addressof(pk), ctypes.addressof(pv),
+        kt.data_ptr(), vt.data_ptr(), kk.data_ptr(), vk.data_ptr(), interval, kk.shape[2], None, 0, out.data_ptr(), scratch.data_ptr(),
+        scratch.numel(), 1, Hq, H, T, 128, kc.shape[2], bits, 0.08, SMIN, SMAX, _lib.FLAG_SELFTEST_MUTE_K | _lib.FLAG_FAST_REPLAY,
+        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    torch.cuda.synchronize()
+    seconds = time.perf_counter() - t0
+    assert 1 <= gemv.device_status() <= 4
+    assert torch.isnan(out).all()
+    for t, old in zip((kc, vc, kt, vt, kk, vk), before):
+        assert torch.equal(t, old)
+    assert 0.9 < seconds < 4.0, seconds      # 2e9 cycles at 1.965 GHz or less
+    again = gemv.decode_attn(*args, T, 0.08, SMIN, SMAX, **kw, **ck, scratch=scratch)
+    _status_ok()
+    assert torch.equal(again, good)
