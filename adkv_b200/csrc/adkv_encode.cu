@@ -529,6 +529,10 @@ static int launch_encode(const EncBatch &b, int n, int B, int H, int T, int D, i
     if (split) {
         const auto first = bits == 4 ? encode_kernel<4, false, 2, kFirstPart> : encode_kernel<2, false, 2, kFirstPart>;
         const auto second = bits == 4 ? encode_kernel<4, false, 1, kSecondPart> : encode_kernel<2, false, 1, kSecondPart>;
+        // A refusal must not leave half of the prefill written: the second kernel is loaded (asking for its attributes does that) before
+        // the first runs, and where it may not run beside the first it follows as an ordinary launch.
+        cudaFuncAttributes unused;
+        if (cudaFuncGetAttributes(&unused, second) != cudaSuccess) return launch_status();
         first<<<split, kEncThreads, 0, s>>>(b, cs, 0, n_slices, H, T, n_super_cap, t_start, smin, smax);
         if (int rc = launch_status()) return rc;
         cudaLaunchAttribute attr{};
@@ -540,8 +544,11 @@ static int launch_encode(const EncBatch &b, int n, int B, int H, int T, int D, i
         cfg.stream = s;
         cfg.attrs = &attr;
         cfg.numAttrs = 1;
-        const cudaError_t e = cudaLaunchKernelEx(&cfg, second, b, cs, split, n_slices, H, T, n_super_cap, t_start, smin, smax);
-        return e == cudaSuccess ? launch_status() : int(e);
+        if (cudaLaunchKernelEx(&cfg, second, b, cs, split, n_slices, H, T, n_super_cap, t_start, smin, smax) != cudaSuccess) {
+            cudaGetLastError();
+            second<<<cfg.gridDim, cfg.blockDim, 0, s>>>(b, cs, split, n_slices, H, T, n_super_cap, t_start, smin, smax);
+        }
+        return launch_status();
     }
     kernel<<<dim3(n_slices, n), D == kD && few ? kD : kEncThreads, 0, s>>>(b, cs, 0, n_slices, H, T, n_super_cap, t_start, smin, smax);
     return launch_status();
