@@ -5,6 +5,7 @@ from __future__ import annotations
 import ctypes
 import functools
 import os
+import re
 import shutil
 import subprocess
 import tempfile
@@ -55,3 +56,31 @@ _pp = ctypes.addressof(_params)
 def prefill(B, H, T, bits=4, fail=()):
     ns = T // (32 // bits) + 1
     return run("adkv_encode_kv", PTR, PTR, _pp, PTR, PTR, PTR, _pp, PTR, B, H, T, 128, ns, bits, 0, 0.02, 50.0, None, fail=fail)
+
+
+FAST = _lib.FLAG_FAST_REPLAY
+
+
+def _step(name, *args):
+    """The decode kernel of one step, without ``decode_attn_`` and ``_kernel`` and its template arguments, and its CTAs."""
+    rc, got = run(name, *args)
+    assert rc == 0, rc
+    kernel = re.search(r"decode_attn_?(\w*?)_?kernelI", got[0][0]).group(1)
+    return kernel or "whole", got[0][1]
+
+
+def decode(bits, G, B, Hkv, T, bounds, tails=True, flags=FAST):
+    tail = PTR if tails else None
+    return _step("adkv_decode_attn", PTR, PTR, PTR, PTR, PTR, _pp, _pp, tail, tail, None, 0, PTR, B, G * Hkv, Hkv, T, 128, T + 1, bits,
+                 0.1, *bounds, flags, None)
+
+
+def decode_varlen(bits, G, B, Hkv, room, bounds, flags=FAST):
+    ns = -(-room // (32 // bits))
+    return _step("adkv_decode_attn_varlen", PTR, PTR, PTR, PTR, PTR, _pp, _pp, PTR, PTR, PTR, PTR, B, G * Hkv, Hkv, 128, ns, bits, 0.1,
+                 *bounds, flags, None)
+
+
+def decode_ckpt(bits, G, B, Hkv, T, interval, bounds, flags=FAST):
+    return _step("adkv_decode_attn_ckpt", PTR, PTR, PTR, PTR, PTR, _pp, _pp, PTR, PTR, PTR, PTR, interval, T, None, 0, PTR, PTR, 1 << 40, B,
+                 G * Hkv, Hkv, T, 128, T + 1, bits, 0.1, *bounds, flags, None)

@@ -1,9 +1,10 @@
-"""Decode steps next to tail states against the oracle and against 64 bits, over token segments (up to 148 streams of 128
-tokens and more, any device-side length) and with one warp pair per stream; prefill and append by number of streams.  Needs
-a B200.
+"""Decode steps next to tail states against the oracle and against 64 bits: what the library picks for few streams (the tensor
+cores, but for 2-bit codes of one query head from 700 tokens on), token segments (the same streams of 128 tokens and more,
+any device-side length, where the scale bounds are too far apart for the tensor cores), and one warp pair per stream; prefill and
+append by number of streams.  Needs a B200.
 
 Sizes are the edges of the split: no token, fewer tiles than segments, whole tiles, one token more or less; scales that
-never clamp, clamp at one bound, at both, and start outside the bounds.
+never clamp, clamp at one bound, at both, and start outside the bounds.  test_launches.py holds which kernel a call takes.
 """
 import numpy as np
 import pytest
@@ -12,7 +13,7 @@ import torch
 from adkv_b200 import gemv, synth
 from oracle import adkv_oracle as orc
 from tests.test_gpu_tail_state import ATOL, RTOL, _bits_equal, _oracle_tail, _prefill, _status_ok
-from tests.util import SMAX, SMIN, dev, make_case, np_params
+from tests.util import SMAX, SMIN, WIDE, dev, make_case, np_params
 
 pytestmark = pytest.mark.gpu
 
@@ -34,17 +35,22 @@ def _clamping(case, kind):
         case[n] = (zp, sc, al, be, tg)
 
 
-@pytest.mark.parametrize("split", [None, False], ids=["segments", "whole_head"])
-@pytest.mark.parametrize("clamp", ["none", "pinned_low", "both", "start_outside", "odd_factor"])
-@pytest.mark.parametrize("B,Hq,Hkv,T,bits", [
+BOUNDS = {"usual": (SMIN, SMAX), "wide": WIDE}
+SHAPES = [
     (1, 2, 2, 0, 4), (1, 2, 2, 1, 2), (2, 2, 2, 31, 4), (1, 4, 2, 32, 4), (1, 4, 1, 33, 2), (2, 2, 2, 255, 4), (1, 2, 1, 256, 2),
     (1, 2, 2, 257, 4), (1, 8, 2, 290, 2), (1, 2, 2, 777, 2), (2, 4, 2, 1031, 4),
     (1, 2, 2, 127, 4), (1, 4, 2, 128, 2), (1, 2, 2, 129, 4), (1, 8, 2, 225, 4),
-])
-def test_against_oracle(B, Hq, Hkv, T, bits, clamp, split):
+]
+
+
+@pytest.mark.parametrize("bounds,split", [("usual", None), ("wide", None), ("usual", False)], ids=["library", "segments", "whole_head"])
+@pytest.mark.parametrize("clamp", ["none", "pinned_low", "both", "start_outside", "odd_factor"])
+@pytest.mark.parametrize("B,Hq,Hkv,T,bits", SHAPES)
+def test_against_oracle(B, Hq, Hkv, T, bits, clamp, bounds, split):
+    smin, smax = BOUNDS[bounds]
     case = make_case(500 + T, B, Hq, Hkv, T, bits)
     _clamping(case, clamp)
-    dk, dv, tk, tv, ok_, ov_, sk, sv = _prefill(case, T + 1)
+    dk, dv, tk, tv, ok_, ov_, sk, sv = _prefill(case, T + 1, (smin, smax))
     kn, vn = case["k"][:, :, T], case["v"][:, :, T]
     mask = torch.zeros(B, 1, 1, T + 1)
     mask[0, 0, 0, :T // 3] = torch.finfo(torch.float16).min
@@ -53,21 +59,23 @@ def test_against_oracle(B, Hq, Hkv, T, bits, clamp, split):
         ok2, ov2 = ok_.copy(), ov_.copy()
         want = orc.decode_attn(case["q"][:, :, 0].numpy(), ok2, ov2, kn.numpy(), vn.numpy(), np_params(case["kp"]),
                                np_params(case["vp"]), T, 0.07, mask=None if m is None else m[:, 0].numpy(), bits=bits,
-                               scale_min=SMIN, scale_max=SMAX)
+                               scale_min=smin, scale_max=smax)
         got = gemv.decode_attn(dev(case["q"]), dk, dv, dev(kn[:, :, None]), dev(vn[:, :, None]), dev(case["kp"]), dev(case["vp"]),
-                               T, 0.07, SMIN, SMAX, mask=None if m is None else dev(m), bits=bits, k_tail=tk, v_tail=tv,
+                               T, 0.07, smin, smax, mask=None if m is None else dev(m), bits=bits, k_tail=tk, v_tail=tv,
                                tail_keep=name == "mask", split_channels=split)
         _status_ok()
         np.testing.assert_allclose(got.float().cpu().numpy(), want, rtol=RTOL, atol=ATOL)
         assert np.array_equal(dk.cpu().numpy(), ok2) and np.array_equal(dv.cpu().numpy(), ov2)
-    orc.append_token(ok_.copy(), kn.numpy(), sk, T, np_params(case["kp"]), bits, SMIN, SMAX)
-    orc.append_token(ov_.copy(), vn.numpy(), sv, T, np_params(case["vp"]), bits, SMIN, SMAX)
+    orc.append_token(ok_.copy(), kn.numpy(), sk, T, np_params(case["kp"]), bits, smin, smax)
+    orc.append_token(ov_.copy(), vn.numpy(), sv, T, np_params(case["vp"]), bits, smin, smax)
     assert _bits_equal(tk, _oracle_tail(sk)) and _bits_equal(tv, _oracle_tail(sv))
 
 
+@pytest.mark.parametrize("bounds", BOUNDS)
 @pytest.mark.parametrize("bits", [4, 2])
-def test_segments_varlen(bits):
+def test_segments_varlen(bits, bounds):
     """Ragged lengths, one of them zero: every sequence as the dense call on it alone gives it."""
+    smin, smax = BOUNDS[bounds]
     B, Hq, Hkv, D, lens = 3, 4, 2, 128, [0, 97, 640]
     case = make_case(77, B, Hq, Hkv, max(lens), bits)
     ns = orc.n_super_for(max(lens) + 1, bits)
@@ -78,22 +86,24 @@ def test_segments_varlen(bits):
     kp, vp = dev(case["kp"]), dev(case["vp"])
     for b, n in enumerate(lens):
         gemv.encode_kv_pair(dk[b:b + 1], dev(case["k"][b:b + 1, :, :n]), kp, dv[b:b + 1], dev(case["v"][b:b + 1, :, :n]), vp,
-                            SMIN, SMAX, bits=bits, k_tail=tk[b:b + 1], v_tail=tv[b:b + 1])
+                            smin, smax, bits=bits, k_tail=tk[b:b + 1], v_tail=tv[b:b + 1])
     kn, vn = dev(case["k"][:, :, -1:]), dev(case["v"][:, :, -1:])
     q = dev(case["q"])
     want = torch.cat([gemv.decode_attn(q[b:b + 1], dk[b:b + 1].clone(), dv[b:b + 1].clone(), kn[b:b + 1], vn[b:b + 1], kp, vp, n,
-                                       0.09, SMIN, SMAX, bits=bits, k_tail=tk[b:b + 1], v_tail=tv[b:b + 1], tail_keep=True,
+                                       0.09, smin, smax, bits=bits, k_tail=tk[b:b + 1], v_tail=tv[b:b + 1], tail_keep=True,
                                        split_channels=False) for b, n in enumerate(lens)])
-    got = gemv.decode_attn_varlen(q, dk, dv, kn, vn, kp, vp, torch.tensor(lens, dtype=torch.int32, device="cuda"), 0.09, SMIN,
-                                  SMAX, bits=bits, k_tail=tk, v_tail=tv)
+    got = gemv.decode_attn_varlen(q, dk, dv, kn, vn, kp, vp, torch.tensor(lens, dtype=torch.int32, device="cuda"), 0.09, smin,
+                                  smax, bits=bits, k_tail=tk, v_tail=tv)
     _status_ok()
     np.testing.assert_allclose(got.float().cpu().numpy(), want.float().cpu().numpy(), rtol=RTOL, atol=ATOL)
 
 
+@pytest.mark.parametrize("bounds", BOUNDS)
 @pytest.mark.parametrize("Hq,Hkv,bits", [(2, 2, 4), (8, 2, 2)])
-def test_segments_varlen_short(Hq, Hkv, bits):
+def test_segments_varlen_short(Hq, Hkv, bits, bounds):
     """Sequences from one token to a few tiles, and one past the capacity, in caches with room for 700: one tile is
     one segment.  The sequence that does not fit is reported and left alone."""
+    smin, smax = BOUNDS[bounds]
     lens, D = [1, 32, 33, 95, 96, 97, 128, 129, 224, 225, 700], 128
     B, cap = len(lens), 700
     case = make_case(78, B, Hq, Hkv, cap, bits)
@@ -104,29 +114,31 @@ def test_segments_varlen_short(Hq, Hkv, bits):
     kp, vp = dev(case["kp"]), dev(case["vp"])
     for b, n in enumerate(lens):
         gemv.encode_kv_pair(dk[b:b + 1], dev(case["k"][b:b + 1, :, :n]), kp, dv[b:b + 1], dev(case["v"][b:b + 1, :, :n]), vp,
-                            SMIN, SMAX, bits=bits, k_tail=tk[b:b + 1], v_tail=tv[b:b + 1])
+                            smin, smax, bits=bits, k_tail=tk[b:b + 1], v_tail=tv[b:b + 1])
     lens[-1] = dk.shape[2] * (32 // bits)
     kn, vn, q = dev(case["k"][:, :, -1:]), dev(case["v"][:, :, -1:]), dev(case["q"])
     before = [t.clone() for t in (dk, dv, tk, tv)]
     want = torch.cat([gemv.decode_attn(q[b:b + 1], dk[b:b + 1].clone(), dv[b:b + 1].clone(), kn[b:b + 1], vn[b:b + 1], kp, vp, n,
-                                       0.09, SMIN, SMAX, bits=bits, k_tail=tk[b:b + 1], v_tail=tv[b:b + 1], tail_keep=True,
+                                       0.09, smin, smax, bits=bits, k_tail=tk[b:b + 1], v_tail=tv[b:b + 1], tail_keep=True,
                                        split_channels=False) for b, n in enumerate(lens[:-1])])
-    got = gemv.decode_attn_varlen(q, dk, dv, kn, vn, kp, vp, torch.tensor(lens, dtype=torch.int32, device="cuda"), 0.09, SMIN,
-                                  SMAX, bits=bits, k_tail=tk, v_tail=tv)
+    got = gemv.decode_attn_varlen(q, dk, dv, kn, vn, kp, vp, torch.tensor(lens, dtype=torch.int32, device="cuda"), 0.09, smin,
+                                  smax, bits=bits, k_tail=tk, v_tail=tv)
     assert gemv.device_status() == 6 and gemv.device_status() == 0
     np.testing.assert_allclose(got[:-1].float().cpu().numpy(), want.float().cpu().numpy(), rtol=RTOL, atol=ATOL)
     for t, old in zip((dk, dv, tk, tv), before):
         assert torch.equal(t[-1], old[-1])
 
 
+@pytest.mark.parametrize("bounds", BOUNDS)
 @pytest.mark.parametrize("Hq,T,bits", [(2, 300, 4), (8, 531, 2)])
-def test_masked_segments(Hq, T, bits):
+def test_masked_segments(Hq, T, bits, bounds):
     """Additive masks that leave out whole segments, every cached token, and everything; the lowest fp32 and fp16 values
     as well as minus infinity."""
+    smin, smax = BOUNDS[bounds]
     case = make_case(610, 1, Hq, 2, T, bits)
-    dk, dv, tk, tv, *_ = _prefill(case, T + 1)
+    dk, dv, tk, tv, *_ = _prefill(case, T + 1, (smin, smax))
     args = (dev(case["q"]), dk, dv, dev(case["k"][:, :, T:]), dev(case["v"][:, :, T:]), dev(case["kp"]), dev(case["vp"]), T, 0.08,
-            SMIN, SMAX)
+            smin, smax)
     kw = dict(bits=bits, k_tail=tk, v_tail=tv, tail_keep=True)
     for low in (-float("inf"), torch.finfo(torch.float32).min, torch.finfo(torch.float16).min):
         for out in (slice(0, T // 2), slice(T // 4, T), slice(0, T), slice(0, T + 1)):
@@ -308,13 +320,16 @@ def _logit_errors(B, T, bits, pinned, variants, seed=5, G=1, smin=SMIN, smax=SMA
     return errors
 
 
+@pytest.mark.parametrize("bounds", BOUNDS)
 @pytest.mark.parametrize("B,T,bits,pinned", [(64, 4096, 2, False), (128, 8192, 2, False), (64, 2000, 4, False), (128, 4096, 4, False),
                                              (64, 4096, 4, True), (64, 8192, 2, True)])
-def test_logit_error_is_that_of_a_whole_scan(B, T, bits, pinned):
-    """Segments start from products of their predecessors' factors: no further from 64 bits than one scan over the stream.
-    Sums of 192 to 384 squared errors each; segments start from less rounding, which leaves 0.6 to 0.85 of the whole scan's."""
-    segments, whole = _logit_errors(B, T, bits, pinned, (None, False))
-    assert segments <= whole, (segments, whole)
+def test_logit_error_is_that_of_a_whole_scan(B, T, bits, pinned, bounds):
+    """Segments start from products of their predecessors' factors, the tensor cores sum pairs of fp16 numbers: no further from
+    64 bits than one scan over the stream.  Sums of 192 to 384 squared errors each; segments start from less rounding, which
+    leaves 0.6 to 0.85 of the whole scan's."""
+    smin, smax = BOUNDS[bounds]
+    got, whole = _logit_errors(B, T, bits, pinned, (None, False), smin=smin, smax=smax)
+    assert got <= whole, (got, whole)
 
 
 @pytest.mark.parametrize("T,bits", [(70, 4), (161, 2)])

@@ -31,7 +31,7 @@ def _oracle_tail(st) -> np.ndarray:
     return np.stack([st.zp, st.s], axis=2).astype(np.float32)
 
 
-def _prefill(case, capacity_tokens, **kw):
+def _prefill(case, capacity_tokens, bounds=(SMIN, SMAX), **kw):
     """Prefill on the GPU with tails; oracle caches and states for the same tokens."""
     B, Hkv, T, bits, D = case["B"], case["Hkv"], case["T"], case["bits"], case["D"]
     ns = orc.n_super_for(capacity_tokens, bits)
@@ -40,11 +40,11 @@ def _prefill(case, capacity_tokens, **kw):
     tk = torch.zeros(B, Hkv, 2, D, dtype=torch.float32, device="cuda")
     tv = torch.zeros_like(tk)
     gemv.encode_kv_pair(dk, dev(case["k"][:, :, :T]), dev(case["kp"]), dv, dev(case["v"][:, :, :T]), dev(case["vp"]),
-                        SMIN, SMAX, bits=bits, k_tail=tk, v_tail=tv, **kw)
+                        *bounds, bits=bits, k_tail=tk, v_tail=tv, **kw)
     ok_ = np.zeros(orc.cache_shape(B, Hkv, ns, D), np.uint8)
     ov_ = np.zeros_like(ok_)
-    _, sk = orc.encode_kv(ok_, case["k"][:, :, :T].numpy(), np_params(case["kp"]), bits, SMIN, SMAX)
-    _, sv = orc.encode_kv(ov_, case["v"][:, :, :T].numpy(), np_params(case["vp"]), bits, SMIN, SMAX)
+    _, sk = orc.encode_kv(ok_, case["k"][:, :, :T].numpy(), np_params(case["kp"]), bits, *bounds)
+    _, sv = orc.encode_kv(ov_, case["v"][:, :, :T].numpy(), np_params(case["vp"]), bits, *bounds)
     if T:
         assert np.array_equal(dk.cpu().numpy(), ok_) and np.array_equal(dv.cpu().numpy(), ov_)
     assert _bits_equal(tk, _oracle_tail(sk)) and _bits_equal(tv, _oracle_tail(sv))

@@ -151,7 +151,8 @@ def test_line_to_token_segments(T):
 
 @pytest.mark.parametrize("B,Hkv,Hq,T,bits", [(37, 8, 8, 260, 2), (40, 8, 32, 130, 4), (56, 8, 16, 300, 4), (93, 8, 32, 300, 2)])
 def test_more_streams_than_a_round(B, Hkv, Hq, T, bits):
-    """296, 320, 448 and 744 streams: two share an SM and its tensor memory, the others follow."""
+    """296, 320, 448 and 744 streams: two share an SM and its tensor memory, the others follow.  With device-side lengths these take
+    one warp per tensor."""
     case = make_case(1800 + T, 1, Hq, Hkv, T, bits)
     (q, kc, vc, kn, vn, kp, vp), kw, _ = _filled(case, 1, Hkv, T, SMIN, SMAX, bits)
     rep = lambda t: t.repeat(B, *([1] * (t.dim() - 1)))
@@ -164,6 +165,42 @@ def test_more_streams_than_a_round(B, Hkv, Hq, T, bits):
     for out in (got, again):
         np.testing.assert_allclose(out[:1].float().cpu().numpy(), want.float().cpu().numpy(), rtol=RTOL, atol=ATOL)
         assert torch.equal(out, rep(out[:1]))
+
+
+# device-side lengths: up to a round of CTAs, more than that, sequences that are ranked by length (up to 128) and that are not
+RAGGED = [(37, 4, 4, 2, 300), (60, 5, 2, 4, 600), (128, 4, 2, 2, 520), (129, 4, 4, 4, 560), (100, 7, 4, 2, 1100)]
+
+
+@pytest.mark.parametrize("B,Hkv,G,bits,room", RAGGED)
+def test_ragged_lengths(B, Hkv, G, bits, room):
+    """Empty sequences, equal lengths, full caches, and one sequence past the capacity, which is reported and left alone; the others
+    as the dense call on them alone gives it."""
+    D, g = 128, torch.Generator().manual_seed(B)
+    cap = gemv.n_super_for(room, bits) * (32 // bits)
+    lens = torch.randint(0, room, (B,), generator=g)
+    lens[::7] = lens[0]
+    lens[1], lens[B - 2], lens[B // 2] = 0, cap - 1, cap
+    kp, vp = (tuple(dev(p)) for p in (make_case(1, 1, Hkv, Hkv, 1, bits)[n] for n in ("kp", "vp")))
+    shape = (B, Hkv, gemv.n_super_for(room, bits), D // 4, 4, 4)
+    kc, vc = (torch.zeros(shape, dtype=torch.uint8, device="cuda") for _ in range(2))
+    k, v = (torch.randn(B, Hkv, cap - 1, D, generator=torch.Generator("cuda").manual_seed(i), device="cuda").half() for i in (B, B + 1))
+    gemv.encode_kv_pair(kc, k, kp, vc, v, vp, SMIN, SMAX, bits=bits)
+    kt, vt = (torch.rand(B, Hkv, 2, D, generator=g).cuda() + 0.1 for _ in range(2))
+    q = torch.randn(B, Hkv * G, 1, D, generator=g).half().cuda()
+    kn, vn = (torch.randn(B, Hkv, 1, D, generator=g).half().cuda() for _ in range(2))
+    refs = [x.clone() for x in (kc, vc, kt, vt)]
+    got = gemv.decode_attn_varlen(q, kc, vc, kn, vn, kp, vp, lens.int().cuda(), 0.05, SMIN, SMAX, bits=bits, k_tail=kt, v_tail=vt)
+    assert gemv.device_status() == 6 and gemv.device_status() == 0
+    rest = [b for b in range(B) if b != B // 2]
+    want = torch.empty_like(got)
+    for b in rest:
+        one = slice(b, b + 1)
+        want[one] = gemv.decode_attn(q[one], refs[0][one], refs[1][one], kn[one], vn[one], kp, vp, int(lens[b]), 0.05, SMIN, SMAX, bits=bits,
+                                     k_tail=refs[2][one], v_tail=refs[3][one], split_channels=False)
+    _status_ok()
+    np.testing.assert_allclose(got[rest].float().cpu().numpy(), want[rest].float().cpu().numpy(), rtol=RTOL, atol=ATOL)
+    for a, b in zip((kc, vc, kt, vt), refs):
+        assert torch.equal(a, b)
 
 
 @pytest.mark.parametrize("smax", [1e6, float("inf")])

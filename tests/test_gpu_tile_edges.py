@@ -8,7 +8,7 @@ from adkv_b200 import gemv
 from oracle import adkv_oracle as orc
 from tests import test_gpu_half_state
 from tests.test_gpu_tail_state import ATOL, RTOL, _prefill, _status_ok
-from tests.util import SMAX, SMIN, dev, make_case, np_params
+from tests.util import SMAX, SMIN, WIDE, dev, make_case, np_params
 
 pytestmark = pytest.mark.gpu
 
@@ -100,17 +100,20 @@ def test_tiles_by_size(bits, G, n, T):
     _status_ok()
 
 
-@pytest.mark.parametrize("bits,G,T", [(2, 1, 256), (2, 2, 257), (4, 2, 300), (2, 1, 512), (4, 2, 513), (2, 4, 384), (2, 4, 385), (4, 4, 513)])
+SEGMENTS = [(2, 1, 256), (2, 2, 257), (4, 2, 300), (2, 1, 512), (4, 2, 513), (2, 4, 384), (2, 4, 385), (4, 4, 513)]
+
+
+@pytest.mark.parametrize("bits,G,T", SEGMENTS)
 def test_segments_by_size(bits, G, T):
-    """Token segments at the lengths where their tiles change."""
+    """Token segments at the lengths where their tiles change, with scale bounds that the tensor cores do not take."""
     B, Hkv = 2, 2
     case = make_case(1300 + T, B, G * Hkv, Hkv, T, bits)
-    dk, dv, tk, tv, ok_, ov_, *_ = _prefill(case, T + 1)
+    dk, dv, tk, tv, ok_, ov_, *_ = _prefill(case, T + 1, WIDE)
     kn, vn = case["k"][:, :, T], case["v"][:, :, T]
     want = orc.decode_attn(case["q"][:, :, 0].numpy(), ok_, ov_, kn.numpy(), vn.numpy(), np_params(case["kp"]), np_params(case["vp"]), T,
-                           0.07, bits=bits, scale_min=SMIN, scale_max=SMAX)
+                           0.07, bits=bits, scale_min=WIDE[0], scale_max=WIDE[1])
     got = gemv.decode_attn(dev(case["q"]), dk, dv, dev(kn[:, :, None]), dev(vn[:, :, None]), dev(case["kp"]), dev(case["vp"]), T, 0.07,
-                           SMIN, SMAX, bits=bits, k_tail=tk, v_tail=tv)
+                           *WIDE, bits=bits, k_tail=tk, v_tail=tv)
     np.testing.assert_allclose(got.float().cpu().numpy(), want, rtol=RTOL, atol=ATOL)
     assert np.array_equal(dk.cpu().numpy(), ok_) and np.array_equal(dv.cpu().numpy(), ov_)
     _status_ok()

@@ -8,6 +8,8 @@ from adkv_b200 import synth
 from oracle import adkv_oracle as orc
 
 SMIN, SMAX = synth.SCALE_MIN, synth.SCALE_MAX
+# further apart than the tensor cores' kernel takes (2 ** 13): the other kernels serve these
+WIDE = (synth.SCALE_MAX / 2 ** 14, synth.SCALE_MAX)
 
 
 def np_params(params):
