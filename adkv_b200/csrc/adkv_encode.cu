@@ -500,13 +500,16 @@ static int ckpt_check(const void *k_ckpt, const void *v_ckpt, int interval, int 
 // An odd number of two-warp CTAs on an SM leaves two of its schedulers a warp more than the other two, and all wait for those.  Then
 // the CTAs beyond the even number come as four warps of one channel a thread, one for each scheduler: two launches side by side
 // (the second is a programmatic dependent that starts as soon as the first is in place).  Device time on a B200, K and V of 32 heads, 4-bit,
-// one launch -> two: 16 x 8192 tokens (6.9 CTAs an SM) 856 -> 790 us, 15 x 4000 426 -> 392 us, 11 x 4000 (4.8) 346 -> 323 us, 19 x 2000 (8.2)
-// 262 -> 243 us, 16 x 256 34.8 -> 33.2 us; 2-bit 16 x 8192 852 -> 818 us, 14 x 2000 (6.1) 216 -> 206 us.  With more than one left over
-// for an SM the two do not come out even.  Returns the size of the first, 0 for one launch.
-static int side_by_side(long long grid, int T)
+// one launch -> two: 16 x 8192 tokens (6.9 CTAs an SM) 856 -> 796 us, 15 x 4000 426 -> 392 us, 11 x 4000 (4.8) 346 -> 323 us, 19 x 2000 (8.2)
+// 262 -> 243 us, 1628 slices (11) x 1024 162 -> 148 us, 612 (4.1) x 256 25.7 -> 25.4 us; 2-bit 16 x 8192 852 -> 818 us, 14 x 2000 (6.1) 216 -> 206
+// us, 1628 x 1024 157 -> 152 us.  Short 2-bit prefills of few CTAs an SM do not gain: 612 x 256 24.9 -> 27.2 us, x 768 66.2 -> 68.3 us, x 2048 173.1 ->
+// 171.2 us; 908 (6.1) x 256 29.3 -> 30.1 us, x 384 42.7 -> 41.9 us; 1204 (8.1) x 256 34.5 -> 34.3 us.  With more than one left over for an SM
+// the two do not come out even; twelve CTAs an SM would gain as eleven do.  Returns the size of the first, 0 for one launch.
+static int side_by_side(long long grid, int T, int bits)
 {
     const long long even = grid / (2 * kSMs) * (2 * kSMs), rest = grid - even;
-    return even >= 4 * kSMs && even <= 10 * kSMs && rest > 0 && rest <= kSMs && T >= 256 ? int(even) : 0;
+    const int from = bits == 4 || even > 6 * kSMs ? 256 : even > 4 * kSMs ? 384 : 2048;
+    return even >= 4 * kSMs && even <= 10 * kSMs && rest > 0 && rest <= kSMs && T >= from ? int(even) : 0;
 }
 
 static int launch_encode(const EncBatch &b, int n, int B, int H, int T, int D, int n_super_cap, int bits,
@@ -525,7 +528,7 @@ static int launch_encode(const EncBatch &b, int n, int B, int H, int T, int D, i
     const auto kernel = D == kD ? (bits == 4 ? (few ? encode_kernel<4, false, 1> : encode_kernel<4, false, 2>)
                                              : (few ? encode_kernel<2, false, 1> : encode_kernel<2, false, 2>))
                                 : (bits == 4 ? encode_kernel<4, true, 2> : encode_kernel<2, true, 2>);
-    const int split = D == kD && !few ? side_by_side(grid, T) : 0;
+    const int split = D == kD && !few ? side_by_side(grid, T, bits) : 0;
     if (split) {
         const auto first = bits == 4 ? encode_kernel<4, false, 2, kFirstPart> : encode_kernel<2, false, 2, kFirstPart>;
         const auto second = bits == 4 ? encode_kernel<4, false, 1, kSecondPart> : encode_kernel<2, false, 1, kSecondPart>;

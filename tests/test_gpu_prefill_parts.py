@@ -29,9 +29,13 @@ def _prefill(case, n, H, T, bits, interval, start):
     return run, (kc, vc, kt, vt)
 
 
-# 600, 740, 890 and 1036 slices leave 8, 148, 2 and 148 over an even number on 148 SMs; 742 leaves 150 and stays one launch
-@pytest.mark.parametrize("B,H,T,bits,interval,start", [(60, 5, 256, 4, 0, 0), (74, 5, 259, 2, 0, 0), (89, 5, 300, 4, 128, 0),
-                                                       (74, 7, 305, 2, 96, 0), (74, 5, 600, 4, 0, 331), (53, 7, 260, 4, 0, 0)])
+# 600, 740, 890, 1036 and 1224 slices leave 8, 148, 2, 148 and 40 over an even number on 148 SMs; 742 leaves 150 and stays one launch, as do
+# 740 slices of 2-bit codes below 2048 tokens and 1036 below 384
+SHAPES = [(60, 5, 256, 4, 0, 0), (74, 5, 259, 2, 0, 0), (89, 5, 300, 4, 128, 0), (74, 7, 405, 2, 96, 0), (74, 7, 305, 2, 96, 0), (74, 5, 600, 4, 0, 331),
+          (53, 7, 260, 4, 0, 0), (102, 6, 259, 2, 0, 0), (37, 10, 2050, 2, 0, 0)]
+
+
+@pytest.mark.parametrize("B,H,T,bits,interval,start", SHAPES)
 def test_parts_of_a_prefill(B, H, T, bits, interval, start):
     case = make_case(2000 + T, 1, H, H, T, bits)
     many, one = (_prefill(case, n, H, T, bits, interval, start)[0]() for n in (B, 1))

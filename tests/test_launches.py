@@ -2,7 +2,7 @@
 import pytest
 
 from adkv_b200 import _lib
-from tests import launches, test_gpu_segments, test_gpu_tensor_step, test_gpu_tile_edges
+from tests import launches, test_gpu_prefill_parts, test_gpu_segments, test_gpu_tensor_step, test_gpu_tile_edges
 from tests.util import SMAX, SMIN, WIDE
 
 USUAL = (SMIN, SMAX)
@@ -13,6 +13,14 @@ def test_prefill_in_two_parts_covers_every_slice():
     assert rc == 0 and [g[1:] for g in got] == [(888, 64, False), (136, 128, True)]
     rc, got = launches.prefill(16, 32, 255)
     assert rc == 0 and [g[1:] for g in got] == [(1024, 64, False)]
+
+
+@pytest.mark.parametrize("slices,T,bits,split", [(592, 4000, 4, 0), (594, 256, 4, 592), (594, 255, 4, 0), (740, 256, 4, 592), (742, 4000, 4, 0),
+                                                 (740, 2047, 2, 0), (740, 2048, 2, 592), (890, 383, 2, 0), (890, 384, 2, 888), (1186, 255, 2, 0),
+                                                 (1186, 256, 2, 1184), (1628, 256, 4, 1480), (1778, 4000, 4, 0), (446, 4000, 4, 0)])
+def test_lines_of_the_second_part(slices, T, bits, split):
+    rc, got = launches.prefill(slices // 2, 1, T, bits)
+    assert rc == 0 and [g[1] for g in got] == ([split, slices - split] if split else [slices])
 
 
 @pytest.mark.parametrize("bits", [4, 2])
@@ -98,3 +106,5 @@ def test_gpu_tests_reach_the_kernels_they_name():
     assert launches.decode(4, 1, 1, 2, 700, (0.0, 4.0))[0] == "segments"
     for B, Hkv, G, bits, room in test_gpu_tensor_step.RAGGED:
         assert launches.decode_varlen(bits, G, B, Hkv, room, USUAL) == ("tensor", B * Hkv)
+    two = [len(launches.prefill(B, H, T - start, bits)[1]) == 2 for B, H, T, bits, interval, start in test_gpu_prefill_parts.SHAPES]
+    assert two == [True, False, True, True, False, True, False, True, True]
