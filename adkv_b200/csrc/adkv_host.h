@@ -17,12 +17,14 @@ constexpr int kSMs = 148, kSchedulers = 4 * kSMs;   // B200: what the choice of 
 //   one head     4-bit 128 x 300 14.3 -> 11.2, 128 x 3000 71.7 -> 68.6, 256 x 3000 132 -> 110, 400 x 300 26.6 -> 24.3, 400 x 200
 //                19.4 -> 19.8, 592 x 1500 102 -> 109; 2-bit 128 x 300 14.7 -> 12.3, 256 x 3000 139 -> 124, 440 x 1024 73 -> 70
 //   two heads    4-bit 128 x 300 16.9 -> 11.4, 256 x 3000 158 -> 111, 740 x 256 37 -> 34, 740 x 1024 117 -> 98, 888 x 1024 118 -> 119
-//   four heads   4-bit 128 x 300 19.1 -> 12.3, 256 x 3000 195 -> 118, 740 x 150 33 -> 30, 1184 x 256 59 -> 57, 1480 x 512 123 -> 114,
-//                4096 x 512 300 -> 313; 2-bit 256 x 3000 209 -> 132
+//   four heads   4-bit 128 x 300 19.1 -> 12.3, 256 x 3000 195 -> 118, 740 x 150 33 -> 30, 1184 x 256 59 -> 57, 1480 x 512 121 -> 112,
+//                2368 x 512 182 -> 174, 2368 x 3000 973 -> 860; 2-bit 256 x 3000 209 -> 132, 2368 x 512 192 -> 185, x 3000 1033 -> 942.  The
+//                kernel stays ahead beyond (4096 x 512 301 / 297, 2-bit 318 / 311), which the line does not use
 //   segments     4-bit, one head, between checkpoints 512 tokens apart: 8 streams x 8000 30 -> 19; 2-bit, 4096 apart, 8 x 9000 199 -> 96
 // Below 32 tokens set-up counts (148 x 16 tokens 5.0 -> 5.2, 296 x 32 tokens 6.7 -> 6.8).  Device-side lengths may be short whatever the cache
 // holds: 384 sequences of four heads, 50 to 100 tokens 19 -> 18, 100 to 2000 tokens 146 -> 69; of one head, 768 x 600 61 -> 76.
-// With one channel of every head at a bound 256 x 1000: one head 59 -> 51, four heads 76 -> 55.
+// With one channel of every head at a bound 256 x 1000: one head 59 -> 51, four heads 76 -> 55; but where the line for one head ends, 444 x
+// 1500 4-bit 110 -> 114, 2-bit 105 -> 113 (without 99 -> 86 and 98 -> 86), and for four, 4-bit 2368 x 512 208 -> 215.
 static inline bool tensor_pays(int bits, int G, long long ctas, int tokens, bool device_lengths)
 {
     if (device_lengths && (tokens < 128 || (G == 1 && ctas > kSMs))) return false;
