@@ -108,3 +108,8 @@ def test_gpu_tests_reach_the_kernels_they_name():
         assert launches.decode_varlen(bits, G, B, Hkv, room, USUAL) == ("tensor", B * Hkv)
     two = [len(launches.prefill(B, H, T - start, bits)[1]) == 2 for B, H, T, bits, interval, start in test_gpu_prefill_parts.SHAPES]
     assert two == [True, False, True, True, False, True, False, True, True]
+
+
+def test_smoke_run_reaches_the_default_kernels():
+    assert launches.decode(4, 2, 2, 2, 260, USUAL)[0] == "tensor"
+    assert len(launches.prefill(298, 2, 260)[1]) == 2
