@@ -21,8 +21,12 @@
 // in flight.  What bounds it: issue and register reads of the scans, 10 cycles a value and scheduler with four warps, 13 with two
 // (measured alone; a third of it the split into fp16 parts), so with one query head and many streams the packed scans of
 // adkv_decode.cuh stay ahead (12 cycles with everything); with one CTA on an SM the warps that move the sums, weigh and add, one after
-// the other, 2600 cycles a tile.  The lines are in tensor_pays (adkv_host.h).  Against 64 bits the error of a logit is 0.70 to 0.96
-// times that of one scan with fp32 sums, 0.89 in the mean over 14 sets (128 to 8000 tokens, 384 streams each).
+// the other, 2600 cycles a tile.  The lines are in tensor_pays (adkv_host.h).  Against 64 bits the error of a logit is 0.85 to 0.98
+// times that of one scan with fp32 sums (eight sets of 2000 tokens pooled, 192 logits each, for either code width and every number of
+// query heads; three sets of 16000: 0.88 to 0.97; single sets 0.7 to 1.25), with one channel of a head at a bound 0.85 to 1.00, with every
+// scale of a 4-bit cache at the lower bound 1.01 to 1.02.  A whole result, before it is rounded to fp16: 0.8 to 1.2, 0.90 where
+// the weights are flat.  Carrying what the scale loses in guarded windows, too, would leave 0.87 at the lower bound and cost
+// 5 to 10 % of such steps and up to 4 % of all.
 //
 // Only the appended token needs the encoder's exact state, and that comes from the tail.
 #include "adkv_host.h"

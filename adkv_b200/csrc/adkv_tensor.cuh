@@ -4,7 +4,7 @@
 
 namespace adkv {
 
-__device__ __forceinline__ void tmem_alloc(uint32_t *at, uint32_t columns)   // one whole warp; blocks until the columns are free
+__device__ __forceinline__ void tmem_alloc(uint32_t *at, uint32_t columns)   // one whole warp; blocks, without a limit of its own, until another kernel on the SM has given its columns back
 {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(at)), "r"(columns) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");

@@ -69,22 +69,27 @@ extern "C" {
 #define ADKV_FLAG_TAIL_KEEP 4u
 /* adkv_decode_attn, head dim 128, fp32 arithmetic: how a (batch, kv head) stream is laid over warps.  By default the
  * library decides from the number of streams and tokens of the call:
- *   - tensor cores: next to tail states, with the contracted replay, up to four query heads per KV head and scale_max up to
- *     32768, few streams (up to 296; more with two and four query heads and long streams) of 32 tokens or more have their sums
- *     over channels and tokens formed by the tensor cores;
- *   - token segments: under the same conditions, up to 148 streams (one per SM) of 128 tokens or more that the tensor cores
- *     do not take (2 bits, one query head, more than 700 tokens; larger scale_max) are cut along the token axis over eight K
- *     and eight V warps;
+ *   - tensor cores: next to tail states, with the contracted replay, up to four query heads per KV head, scale bounds no further
+ *     apart than 2^13 (scale_min counted from the quantiser's 1e-8 on) and scale_max from 1e-8 to 32768, few streams have their
+ *     sums over channels and tokens formed by the tensor cores: up to 148 of 32 tokens or more, up to 296 of 64, up to 444 of
+ *     256 (128 at 2 bits; 100 with two or four query heads), with two query heads up to 740 of 256, with four up to 740 of 128, 1184 of
+ *     256 and 2368 of 512;
+ *   - token segments: next to tail states, with the contracted replay and up to four query heads per KV head, up to 148 streams
+ *     (one per SM) of 128 tokens or more that the tensor cores do not take (2 bits, one query head, more than 700 tokens; other
+ *     scale bounds) are cut along the token axis over eight K and eight V warps;
  *   - split heads: otherwise, up to 148 streams (160 of fewer than 256 tokens) have the channels of a head split over two K
  *     and two V warps;
  *   - whole heads: everything else keeps one warp per tensor and stream, which needs the fewest instructions in all.
  * Next to tail states appended codes and tails do not depend on the layout, bit for bit.  Outputs of split and whole
  * heads agree up to the summation order of the logits; token segments start from products of the scale factors before
- * them and merge partial softmax sums, the tensor cores sum fp16 pairs of the values (22 bits) in fp32, and both stay as close to
- * exact arithmetic as a whole head does.
+ * them and merge partial softmax sums, the tensor cores sum pairs of fp16 numbers (22 bits) in fp32: values, queries times alpha,
+ * weights.  Both stay as close to exact arithmetic as a whole head does (error of a logit 0.85 to 1.0 times, with every scale of
+ * a 4-bit cache at scale_min 1.02); of a channel whose scale_init lies above scale_max and whose first code is not zero, the
+ * tensor cores keep the bits in units of scale_init.
  * SPLIT forces split heads, NO_SPLIT whole heads (tests, tuning; with both set, SPLIT wins); either one rules out tensor cores
  * and token segments, and nothing forces those.  adkv_decode_attn_varlen has no split heads: caches with room for 128 tokens or
- * more take tensor cores or token segments under the same conditions, the rest, and calls with either flag, whole heads.
+ * more take tensor cores (one query head: up to 148 streams; two and four: up to 296, and with room for 512 up to 592 and 740) or
+ * token segments under the same conditions, the rest, and calls with either flag, whole heads.
  * The segments of adkv_decode_attn_ckpt take the tensor cores by the same line. */
 #define ADKV_FLAG_SPLIT_CHANNELS 8u
 #define ADKV_FLAG_NO_SPLIT_CHANNELS 16u
