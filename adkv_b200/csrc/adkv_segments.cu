@@ -438,9 +438,8 @@ static int launch_segments(const KArgs &ka, const VArgs &va, const float *mask, 
     constexpr int bytes = int(sizeof(SegShared<BITS, G, TOK>));
     static_assert(bytes <= 227 * 1024, "shared memory of one CTA");
     // per device and process: cheap enough (a host-side call) to be made before every launch
-    const cudaError_t e = cudaFuncSetAttribute(decode_attn_segments_kernel<BITS, G, TOK>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return int(e);
+    if (cudaFuncSetAttribute(decode_attn_segments_kernel<BITS, G, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+        return launch_status();
     decode_attn_segments_kernel<BITS, G, TOK><<<B * ka.Hkv, 64 * NS, bytes, s>>>(ka, va, mask, mask_stride_b, scaling, seq_lens);
     return launch_status();
 }

@@ -213,8 +213,8 @@ static int launch_merge(const float *scratch, __half *out, int B, int Hq, int Hk
     cfg.stream = s;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, n_seg <= kMergeFew ? merge_few_kernel : merge_partials_kernel, scratch, out, Hq, Hkv, n_seg);
-    return e == cudaSuccess ? launch_status() : int(e);
+    (void)cudaLaunchKernelEx(&cfg, n_seg <= kMergeFew ? merge_few_kernel : merge_partials_kernel, scratch, out, Hq, Hkv, n_seg);
+    return launch_status();
 }
 
 extern "C" {
@@ -307,14 +307,12 @@ static std::mutex g_static_scratch_lock;
 static int static_scratch_of_current_device(float **addr)
 {
     int dev = -1;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return int(e);
+    if (cudaGetDevice(&dev) != cudaSuccess) return launch_status();
     if (dev < 0 || dev >= kMaxDevices) return ADKV_E_SHAPE;
     std::lock_guard<std::mutex> guard(g_static_scratch_lock);
     if (!g_static_scratch_known[dev]) {
         void *p = nullptr;
-        e = cudaGetSymbolAddress(&p, g_static_scratch);
-        if (e != cudaSuccess) return int(e);
+        if (cudaGetSymbolAddress(&p, g_static_scratch) != cudaSuccess) return launch_status();
         g_static_scratch_addr[dev] = static_cast<float *>(p);
         g_static_scratch_known[dev] = true;
     }

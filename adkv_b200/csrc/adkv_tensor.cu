@@ -656,8 +656,7 @@ static int launch_tensor(const KArgs &ka, const VArgs &va, const float *mask, lo
     constexpr int size = int(sizeof(TensorShared<BITS, G>)), bytes = size > 78 * 1024 ? size : 78 * 1024;
     static_assert(2 * (bytes + 1024) <= 228 * 1024, "shared memory of an SM");
     const auto kernel = decode_attn_tensor_kernel<BITS, G, PART>;
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e != cudaSuccess) return int(e);
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return launch_status();
     kernel<<<grid, kTcThreads, bytes, s>>>(ka, va, mask, mask_stride_b, scaling, seq_lens, n_rank, ck, scratch);
     return launch_status();
 }

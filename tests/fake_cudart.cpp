@@ -50,6 +50,7 @@ const char *fake_launch(int i, unsigned *grid, unsigned *block, int *beside)
     return launches[i].kernel.c_str();
 }
 void fake_reset() { launches.clear(); calls.clear(); fail_at.clear(); last = cudaSuccess; }
+int fake_last_error() { return last; }
 void fake_fail(const char *function, int nth) { fail_at[function] = nth; }
 
 // what the library uses
@@ -82,7 +83,7 @@ HIDDEN cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *
 HIDDEN cudaError_t cudaGetLastError() { const cudaError_t e = last; last = cudaSuccess; return e; }
 HIDDEN cudaError_t cudaFuncSetAttribute(const void *, cudaFuncAttribute, int) { return enter("cudaFuncSetAttribute"); }
 HIDDEN cudaError_t cudaFuncGetAttributes(cudaFuncAttributes *, const void *) { return enter("cudaFuncGetAttributes"); }
-HIDDEN cudaError_t cudaGetDevice(int *d) { *d = 0; return cudaSuccess; }
+HIDDEN cudaError_t cudaGetDevice(int *d) { *d = 0; return enter("cudaGetDevice"); }
 HIDDEN const char *cudaGetErrorString(cudaError_t) { return "fake"; }
 HIDDEN cudaError_t cudaGetSymbolAddress(void **p, const void *) { *p = reinterpret_cast<void *>(256); return cudaSuccess; }
 HIDDEN cudaError_t cudaMemcpyFromSymbol(void *p, const void *, size_t n, size_t, cudaMemcpyKind) { std::memset(p, 0, n); return cudaSuccess; }

@@ -61,18 +61,21 @@ def prefill(B, H, T, bits=4, fail=()):
 FAST = _lib.FLAG_FAST_REPLAY
 
 
-def _step(name, *args):
-    """The decode kernel of one step, without ``decode_attn_`` and ``_kernel`` and its template arguments, and its CTAs."""
-    rc, got = run(name, *args)
+def _step(name, *args, fail=()):
+    """The decode kernel of one step, without ``decode_attn_`` and ``_kernel`` and its template arguments, and its CTAs; the return code
+    and all launches where something is to fail."""
+    rc, got = run(name, *args, fail=fail)
+    if fail:
+        return rc, got
     assert rc == 0, rc
     kernel = re.search(r"decode_attn_?(\w*?)_?kernelI", got[0][0]).group(1)
     return kernel or "whole", got[0][1]
 
 
-def decode(bits, G, B, Hkv, T, bounds, tails=True, flags=FAST):
+def decode(bits, G, B, Hkv, T, bounds, tails=True, flags=FAST, fail=()):
     tail = PTR if tails else None
     return _step("adkv_decode_attn", PTR, PTR, PTR, PTR, PTR, _pp, _pp, tail, tail, None, 0, PTR, B, G * Hkv, Hkv, T, 128, T + 1, bits,
-                 0.1, *bounds, flags, None)
+                 0.1, *bounds, flags, None, fail=fail)
 
 
 def decode_varlen(bits, G, B, Hkv, room, bounds, flags=FAST):
@@ -81,6 +84,11 @@ def decode_varlen(bits, G, B, Hkv, room, bounds, flags=FAST):
                  *bounds, flags, None)
 
 
-def decode_ckpt(bits, G, B, Hkv, T, interval, bounds, flags=FAST):
+def decode_ckpt(bits, G, B, Hkv, T, interval, bounds, flags=FAST, fail=()):
     return _step("adkv_decode_attn_ckpt", PTR, PTR, PTR, PTR, PTR, _pp, _pp, PTR, PTR, PTR, PTR, interval, T, None, 0, PTR, PTR, 1 << 40, B,
-                 G * Hkv, Hkv, T, 128, T + 1, bits, 0.1, *bounds, flags, None)
+                 G * Hkv, Hkv, T, 128, T + 1, bits, 0.1, *bounds, flags, None, fail=fail)
+
+
+def decode_static(bits, G, B, Hkv, T, interval, bounds, flags=FAST, fail=()):
+    return _step("adkv_decode_attn_ckpt_static", PTR, PTR, PTR, PTR, PTR, _pp, _pp, PTR, PTR, PTR, PTR, interval, T, None, 0, PTR, B, G * Hkv, Hkv,
+                 T, 128, T + 1, bits, 0.1, *bounds, flags, None, fail=fail)

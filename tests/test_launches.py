@@ -113,3 +113,25 @@ def test_gpu_tests_reach_the_kernels_they_name():
 def test_smoke_run_reaches_the_default_kernels():
     assert launches.decode(4, 2, 2, 2, 260, USUAL)[0] == "tensor"
     assert len(launches.prefill(298, 2, 260)[1]) == 2
+
+
+@pytest.mark.parametrize("step", [lambda **kw: launches.decode(4, 1, 8, 8, 500, USUAL, **kw), lambda **kw: launches.decode(4, 1, 8, 8, 500, WIDE, **kw),
+                                  lambda **kw: launches.decode_ckpt(4, 1, 8, 8, 500, 256, USUAL, **kw)], ids=["tensor", "segments", "ckpt"])
+@pytest.mark.parametrize("function", ["cudaFuncSetAttribute", "cudaLaunchKernel"])
+def test_error_of_a_refused_step_is_its_own(step, function):
+    """The call reports it, launches nothing, and the next call does not find it."""
+    rc, got = step(fail=[(function, 1)])
+    assert rc == 701 and got == []
+    assert launches.library().fake_last_error() == 0
+
+
+def test_error_before_a_static_step_is_its_own():
+    rc, got = launches.decode_static(4, 1, 8, 8, 500, 256, USUAL, fail=[("cudaGetDevice", 1)])
+    assert rc == 701 and got == [] and launches.library().fake_last_error() == 0
+    assert launches.decode_static(4, 1, 8, 8, 500, 256, USUAL)[0] == "tensor"
+
+
+def test_error_of_a_refused_merge_is_its_own():
+    rc, got = launches.decode_ckpt(4, 1, 8, 8, 500, 256, USUAL, fail=[("cudaLaunchKernelExC", 1), ("cudaLaunchKernel", 2)])
+    assert rc == 701 and len(got) == 1
+    assert launches.library().fake_last_error() == 0
