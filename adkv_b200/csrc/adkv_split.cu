@@ -213,7 +213,12 @@ static int launch_merge(const float *scratch, __half *out, int B, int Hq, int Hk
     cfg.stream = s;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    (void)cudaLaunchKernelEx(&cfg, n_seg <= kMergeFew ? merge_few_kernel : merge_partials_kernel, scratch, out, Hq, Hkv, n_seg);
+    const auto kernel = n_seg <= kMergeFew ? merge_few_kernel : merge_partials_kernel;
+    if (cudaLaunchKernelEx(&cfg, kernel, scratch, out, Hq, Hkv, n_seg) != cudaSuccess) {
+        // the step has appended its token by now: where the merge may not wait beside it, it follows as an ordinary launch
+        cudaGetLastError();
+        kernel<<<cfg.gridDim, cfg.blockDim, 0, s>>>(scratch, out, Hq, Hkv, n_seg);
+    }
     return launch_status();
 }
 

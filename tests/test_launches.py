@@ -131,6 +131,13 @@ def test_error_before_a_static_step_is_its_own():
     assert launches.decode_static(4, 1, 8, 8, 500, 256, USUAL)[0] == "tensor"
 
 
+@pytest.mark.parametrize("T", [500, 4000])      # the merge of few segments, and the other
+def test_merge_refused_beside_the_segments_follows_them(T):
+    rc, got = launches.decode_ckpt(4, 1, 8, 8, T, 256, USUAL, fail=[("cudaLaunchKernelExC", 1)])
+    assert rc == 0 and "merge" in got[1][0] and not got[1][3]
+    assert launches.library().fake_last_error() == 0
+
+
 def test_error_of_a_refused_merge_is_its_own():
     rc, got = launches.decode_ckpt(4, 1, 8, 8, 500, 256, USUAL, fail=[("cudaLaunchKernelExC", 1), ("cudaLaunchKernel", 2)])
     assert rc == 701 and len(got) == 1
