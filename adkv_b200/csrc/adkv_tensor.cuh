@@ -98,7 +98,7 @@ __device__ __forceinline__ bool wait_polled(const Done &done, int code)
 {
     bool ok = done();
     if (!ok) {
-        uint32_t spent = 0, last = cycles();
+        uint32_t spent = 0, last = cycles();   // from one round to the next: two readings within a round may be moved together
         do {
             const uint32_t now = cycles();
             __nanosleep(64);
